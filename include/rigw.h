@@ -70,7 +70,10 @@ enum rigw_status {
 /* Arithmetic of the chi0 = M D M^T contraction (the eps factorization, Sigma and
  * the QP solve are FP64 in every mode). */
 enum rigw_precision {
-  RIGW_FP64 = 0,           /* FP64 DMMA tensor cores end to end (the drop-in)            */
+  RIGW_FP64 = 0,           /* FP64 end to end (the drop-in): chi0 on the FP64 DMMA cores, or,
+                              from 384 auxiliary functions on, from exact int8 digit products
+                              of 55-bit operands whose error is no larger than that of the
+                              FP64 sums                                                  */
   RIGW_BF16X3 = 1,         /* split BF16 hi/lo products on tcgen05, FP32 accumulation    */
   RIGW_OZAKI_INT8 = 16     /* + s (3 <= s <= 7): Ozaki-sliced INT8 products on tcgen05,
                               s signed 7-bit slices per row, exact INT32 accumulation,

@@ -43,6 +43,17 @@ Status run_batch(Context& c, rigw::PlanMode mode, int n, const rigw_problem* pro
     fresh.reset(new Plan());
     bs = fresh->build(&c, mode, shapes, factors);
   }
+  if (bs.code == RIGW_ERR_NOMEM) {   // without the digit buffers of the FP64 chi0
+    bool any = false;
+    for (Shape& sh : shapes) {
+      any = any || rigw::use_digits(sh);
+      sh.no_digits = 1;
+    }
+    if (any) {
+      fresh.reset(new Plan());
+      bs = fresh->build(&c, mode, shapes, factors);
+    }
+  }
   RIGW_TRY(bs);
   Plan* plan = fresh.get();
   RIGW_TRY(plan->stage_inputs(probs, c.stream));

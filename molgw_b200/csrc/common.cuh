@@ -18,6 +18,7 @@ constexpr int kSplitGroup = 8;                 // frequencies sharing one bf16 h
 constexpr size_t kSplitWholeBytes = size_t(1) << 30;   // below this, one buffer for all frequencies
 constexpr size_t kSplitProblemBytes = size_t(4) << 30; // split buffer of one problem at most (>= one frequency)
 constexpr size_t kSplitL2Bytes = size_t(48) << 20;     // split buffers that stay resident in the 126 MB L2
+constexpr int kFp64Digits = 7;                 // int8 digits of the FP64 chi0 (55 bits; digit_gemm.cu)
 constexpr int kSplitT = 256;                   // transitions per item of the split / slice kernels
 
 // Device-side error flags (bitmask written with atomicOr, read by the host after a stage).

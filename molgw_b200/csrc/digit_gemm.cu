@@ -1,0 +1,497 @@
+// FP64-accurate chi0 contraction from exact int8 digit products on the 5th-generation
+// tensor cores (RIGW_FP64 for all but the smallest problems).
+//
+//   eps(iw)[p][q] = delta_pq + sum_t A_pt B_qt,   A = M D_w,   B = M
+//
+// Row p of an operand is scaled by a power of two to its largest entry and rounded once
+// to an integer X of 8 NS - 1 bits; X is cut into NS balanced base-256 digits d_1 (most
+// significant) .. d_NS, each an int8:  x = 2^(e_p - (8 NS - 1)) sum_i d_i 256^(NS - i).
+//   (A B^T)_pq = 2^(e_p + f_q - 2 (8 NS - 1)) sum_{d=2}^{NS+1} 256^(2 NS - d) L_d(p,q),
+//   L_d = sum_{i+j=d} A_i B_j^T      (28 of the 49 digit products for NS = 7)
+// L_d is an exact INT32 sum (tcgen05.mma kind::i8) over chunks of kChunkTiles k-tiles: for
+// NS = 7, |L_d| <= 7 * 128^2 * 16384 < 2^31.  The levels are joined in 64-bit integers,
+// converted to FP64 once per chunk and summed in FP64.
+//
+// Error, NS = 7 (55-bit X): the products left out (i + j > 8) are digit products of zero
+// mean with weight 2^-70 of the two row scales; K of them add up to about
+// 2^-56 sqrt(K) max|A_p| max|B_q|.  An FP64 sum of K products rounds its running sum K
+// times, about 2^-55 K sigma^2 for entries of size sigma: for K >= 300 and a row maximum of
+// 5 sigma the digit sum is the closer one, at K = 4347 by a factor of 5.  Because a row
+// maximum never exceeds the row's norm, the error relative to sqrt(eps_pp eps_qq) stays at
+// the level of an FP64 sum whatever the spread of the entries (rms, normal entries: 1.3e-17
+// against 2.2e-16 at K = 4347; three decades of spread: 5.8e-17 against 1.8e-16, and at 512
+// transitions 7.5e-17 against 5.7e-17).
+//
+// 840 auxiliary functions, 4347 transitions, 32 frequencies: row maxima 0.04 ms, digits
+// 0.16 ms, products 1.23 ms (3.4 Pop/s int8), against 4.25 ms on DMMA (23 of 35 TF/s);
+// 2000 / 25000 / 32: 0.37 + 2.26 + 30.2 ms against 112 ms.
+// A row that holds an infinity or a NaN gives NaN, as the FP64 sums did.
+//
+// digit_rowmax_kernel: high words of max_t |A_pt| per frequency and row (integer maximum).
+// digit_slice_kernel:  the digits of one frequency group, in the order in which the tensor
+//   cores read them: [slab][row block of 128][k-tile of 64][digit][row group of 8][16-byte
+//   k chunk][row][16 bytes], i.e. contiguous 8 x 16-byte core matrices, so that one TMA box
+//   fetches all the digits of a tile.  Slab 0 is B (the same for every frequency).
+// digit_syrk_kernel:   one 256 x 128 tile of eps(iw) per pair of CTAs (cta_group::2).
+#include <cuda.h>
+#include <cudaTypedefs.h>
+
+#include "engine.cuh"
+#include "tc_common.cuh"
+
+namespace rigw {
+
+namespace {
+
+constexpr int kNaNExp = 1 << 20;                 // row exponent of a row with a non-finite entry
+constexpr int kDigThreads = 320;                 // warp 0 TMA, warp 1 MMA, warps 2..9 drain
+constexpr int kChunkTiles = 256;                 // k-tiles (of 64) per exact INT32 accumulation
+constexpr int kTileA = 128 * 64;                 // bytes of one digit of an A tile (128 rows)
+constexpr int kTileB = 64 * 64;                  // bytes of one digit of half a B tile (64 rows)
+
+template <int NS>
+struct DigCfg {
+  static constexpr int kLo = NS < 4 ? NS : 4;    // levels of the low pass: NS + 2 - kLo .. NS + 1
+  static constexpr int kHi = NS - kLo;           // levels of the high pass: 2 .. kHi + 1 (digits 1 .. kHi)
+  static constexpr int kSlot = NS * (kTileA + kTileB);
+  static constexpr int kSlots = (216 * 1024) / kSlot < 6 ? (216 * 1024) / kSlot : 6;
+  static constexpr int kPerHi = kHi > 0 ? NS / kHi : 1;   // k-tiles of the high pass per slot
+  static constexpr size_t kSmem = size_t(kSlots) * kSlot + 1024 + 256;
+};
+
+// Exponent of a row from the high word of its largest |x|: |x| <= 0.996 * 2^e, so that the
+// leading digit of rint(x 2^(8 NS - 1 - e)) is at most 127.
+RIGW_DEVICE_INLINE int row_exponent(unsigned hi) {
+  const int E = int(hi >> 20);
+  if (E >= 2047) return kNaNExp;
+  int e = (E == 0 ? 1 : E) - 1022;
+  if (E > 0 && (hi & 0xfffffu) + 1u + 0x100000u > 2088763u) ++e;   // mantissa above 0.996
+  return e < -960 ? -960 : e;
+}
+
+RIGW_DEVICE_INLINE double pow2(int e) { return __hiloint2double((e + 1023) << 20, 0); }   // -1022 <= e <= 1023
+
+}  // namespace
+
+__global__ void __launch_bounds__(256) digit_zero_kernel(const ProbDev* __restrict__ probs,
+                                                         const WorkItem* __restrict__ items) {
+  const WorkItem wi = items[blockIdx.x];
+  const ProbDev& p = probs[wi.prob];
+  const int n = (1 + p.nomega) * p.npad;
+  for (int k = threadIdx.x; k < 4096; k += 256)
+    if (wi.a + k < n) p.dmax[wi.a + k] = 0u;
+}
+
+// item: (prob, t0, row block): split_t transitions from t0, 128 rows, B and every frequency.
+// Thread (row, half) keeps 32 entries of its row in registers and walks the frequencies:
+// one FP64 product and one integer maximum per entry and frequency.
+__global__ void __launch_bounds__(256) digit_rowmax_kernel(const ProbDev* __restrict__ probs,
+                                                           const WorkItem* __restrict__ items) {
+  const WorkItem wi = items[blockIdx.x];
+  const ProbDev& p = probs[wi.prob];
+  constexpr int kWb = 16;
+  __shared__ double sd[kWb][64];
+  const int tid = threadIdx.x, row = tid & 127, half = tid >> 7;
+  const int r = wi.b * 128 + row;
+  const int tend = min(p.nia_pad, wi.a + p.split_t);
+  for (int t0 = wi.a; t0 < tend; t0 += 64) {
+    double v[32];
+    unsigned mb = 0;
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {
+      v[i] = p.mp[size_t(t0 + half * 32 + i) * p.npad + r];
+      mb = max(mb, unsigned(__double2hiint(v[i])) & 0x7fffffffu);
+    }
+    if (mb) atomicMax(p.dmax + r, mb);
+    for (int wb = 0; wb < p.nomega; wb += kWb) {
+      const int nwb = min(kWb, p.nomega - wb);
+      __syncthreads();
+      for (int i = tid; i < nwb * 64; i += 256) sd[i >> 6][i & 63] = p.dscale[size_t(wb + (i >> 6)) * p.nia_pad + t0 + (i & 63)];
+      __syncthreads();
+      for (int w = 0; w < nwb; ++w) {
+        unsigned m = 0;
+#pragma unroll
+        for (int i = 0; i < 32; ++i)
+          m = max(m, unsigned(__double2hiint(v[i] * sd[w][half * 32 + i])) & 0x7fffffffu);
+        if (m) atomicMax(p.dmax + size_t(1 + wb + w) * p.npad + r, m);
+      }
+    }
+  }
+}
+
+namespace {
+
+// 4 x 4 byte transpose: o[b] = byte b of w0, w1, w2, w3.
+RIGW_DEVICE_INLINE void bytes4(uint32_t w0, uint32_t w1, uint32_t w2, uint32_t w3, uint32_t (&o)[4]) {
+  const uint32_t a = __byte_perm(w0, w1, 0x5140), b = __byte_perm(w2, w3, 0x5140);
+  const uint32_t c = __byte_perm(w0, w1, 0x7362), d = __byte_perm(w2, w3, 0x7362);
+  o[0] = __byte_perm(a, b, 0x5410);
+  o[1] = __byte_perm(a, b, 0x7632);
+  o[2] = __byte_perm(c, d, 0x5410);
+  o[3] = __byte_perm(c, d, 0x7632);
+}
+
+// The NS digits of 16 consecutive transitions of one row: X = rint(v scale), a carry-in of
+// 128 in every byte but the leading one makes the digits balanced, and 16 bytes per digit
+// go to core-matrix row `dst` (digit planes kTileA bytes apart).
+template <int NS>
+RIGW_DEVICE_INLINE void write_digits(const double (&v)[16], double scale, int8_t* dst) {
+  constexpr uint64_t kBias = NS >= 8 ? 0x0080808080808080ull : (0x8080808080808080ull & ((1ull << (8 * (NS - 1))) - 1));
+  uint32_t out[NS][4];
+#pragma unroll
+  for (int g = 0; g < 4; ++g) {
+    uint32_t lo[4], hi[4], o[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const uint64_t y = (uint64_t(__double2ll_rn(v[4 * g + i] * scale)) + kBias) ^ kBias;
+      lo[i] = uint32_t(y);
+      hi[i] = uint32_t(y >> 32);
+    }
+    bytes4(lo[0], lo[1], lo[2], lo[3], o);
+#pragma unroll
+    for (int b = 0; b < 4 && b < NS; ++b) out[NS - 1 - b][g] = o[b];
+    if (NS > 4) {
+      bytes4(hi[0], hi[1], hi[2], hi[3], o);
+#pragma unroll
+      for (int b = 4; b < NS; ++b) out[NS - 1 - b][g] = o[b - 4];
+    }
+  }
+#pragma unroll
+  for (int s = 0; s < NS; ++s)
+    *reinterpret_cast<uint4*>(dst + size_t(s) * kTileA) = make_uint4(out[s][0], out[s][1], out[s][2], out[s][3]);
+}
+
+// Byte offset of (slab, row block, k-tile, digit 1, row, 16-byte chunk kc) in the digit array.
+RIGW_DEVICE_INLINE size_t digit_offset(int slab, int nrb, int rb, int nkt, int kt, int ns, int row, int kc) {
+  return (((size_t(slab) * nrb + rb) * nkt + kt) * ns) * kTileA + size_t(row >> 3) * 512 + kc * 128 + (row & 7) * 16;
+}
+
+}  // namespace
+
+// item: (prob, k-tile, row block, w0); w0 < 0: slab 0 (B), else the frequencies w0 .. w0 +
+// wgroup - 1 into slabs 1 ...  A warp writes 32 rows of one 16-byte chunk: four full lines
+// per digit.  Memory bound: NS bytes written per entry and frequency (840 auxiliary
+// functions, 32 frequencies: 0.87 GB).
+template <int NS>
+__global__ void __launch_bounds__(256) digit_slice_kernel(const ProbDev* __restrict__ probs,
+                                                          const WorkItem* __restrict__ items) {
+  const WorkItem wi = items[blockIdx.x];
+  const ProbDev& p = probs[wi.prob];
+  constexpr int kWb = 16;
+  __shared__ double sd[kWb][64];
+  const int tid = threadIdx.x, row = tid & 127, half = tid >> 7;
+  const int kt = wi.a, rb = wi.b, r = rb * 128 + row, t0 = kt * 64;
+  const int nrb = p.npad / 128, nkt = p.nia_pad / 64;
+  int8_t* dig = reinterpret_cast<int8_t*>(p.xs);
+  double v[2][16];
+#pragma unroll
+  for (int c = 0; c < 2; ++c)
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[c][i] = p.mp[size_t(t0 + (half * 2 + c) * 16 + i) * p.npad + r];
+  if (wi.c < 0) {
+    const int e = row_exponent(p.dmax[r]);
+    if (kt == 0 && half == 0) p.xexp[r] = e;
+    const double sc = pow2(8 * NS - 1 - (e == kNaNExp ? 0 : e));
+#pragma unroll
+    for (int c = 0; c < 2; ++c) write_digits<NS>(v[c], sc, dig + digit_offset(0, nrb, rb, nkt, kt, NS, row, half * 2 + c));
+    return;
+  }
+  const int w0 = wi.c, w1 = min(p.nomega, w0 + p.wgroup);
+  for (int wb = w0; wb < w1; wb += kWb) {
+    const int nwb = min(kWb, w1 - wb);
+    __syncthreads();
+    for (int i = tid; i < nwb * 64; i += 256) sd[i >> 6][i & 63] = p.dscale[size_t(wb + (i >> 6)) * p.nia_pad + t0 + (i & 63)];
+    __syncthreads();
+    for (int w = 0; w < nwb; ++w) {
+      const int e = row_exponent(p.dmax[size_t(1 + wb + w) * p.npad + r]);
+      if (kt == 0 && half == 0) p.xexp[size_t(1 + wb + w) * p.npad + r] = e;
+      const double sc = pow2(8 * NS - 1 - (e == kNaNExp ? 0 : e));
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        double x[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) x[i] = v[c][i] * sd[w][(half * 2 + c) * 16 + i];
+        write_digits<NS>(x, sc, dig + digit_offset(1 + wb - w0 + w, nrb, rb, nkt, kt, NS, row, half * 2 + c));
+      }
+    }
+  }
+}
+
+// One 256 x 128 tile per CTA pair: rank r holds A rows 128 r .. and B rows 64 r .. of the
+// tile and accumulates output rows 128 r ...  A slot of the ring holds every digit of one
+// k-tile (84 KB per CTA for NS = 7, two slots), so each digit tile that is loaded feeds all
+// the products it appears in; tcgen05 reads 96 bytes of shared memory per clock and CTA and
+// TMA writes 30, below the 128 that shared memory delivers (a 128 x 128 tile of one CTA
+// would read 128 and write 45).  TMEM holds four 128-column accumulators, so the levels go
+// in two passes over a chunk: NS + 1 down to NS - 2 (22 of the 28 products for NS = 7), and
+// the rest from the leading digits alone, several k-tiles per slot.
+template <int NS>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kDigThreads, 1)
+    digit_syrk_kernel(const DigitItem* __restrict__ items) {
+  using Cfg = DigCfg<NS>;
+  const DigitItem it = items[blockIdx.x >> 1];
+  const int jw = blockIdx.y;
+  if (jw >= it.nw) return;   // both CTAs of the pair, before any barrier or TMEM use
+  extern __shared__ uint8_t dig_smem_raw[];
+  uint8_t* smem =
+      reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dig_smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + Cfg::kSlots * Cfg::kSlot);   // used in rank 0
+  uint64_t* empty = full + Cfg::kSlots;     // slot read by the MMAs (both ranks)
+  uint64_t* accf = empty + Cfg::kSlots;     // pass accumulated (both ranks)
+  uint64_t* acce = accf + 1;                // pass drained by the 16 warps of the pair (rank 0)
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(acce + 1);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int rank = int(tc::cluster_rank());
+  if (tid == 0) {
+    for (int s = 0; s < Cfg::kSlots; ++s) {
+      tc::mbar_init(&full[s], 1);
+      tc::mbar_init(&empty[s], 1);
+    }
+    tc::mbar_init(accf, 1);
+    tc::mbar_init(acce, 16);
+    tc::fence_mbar_init();
+  }
+  if (warp == 0) tc::tmem_alloc_pair(tslot, 512);
+  __syncthreads();
+  tc::cluster_sync();        // the peer's barriers are initialised
+  tc::tc_fence_after();
+  const uint32_t tmem = *tslot;
+  const int nk = it.nkt;
+  const int nchunks = (nk + kChunkTiles - 1) / kChunkTiles;
+  constexpr int kPasses = Cfg::kHi > 0 ? 2 : 1;
+  // k-tiles of a slot in pass q (0: low levels, 1: high levels)
+  auto per_slot = [](int q) { return q == 0 ? 1 : Cfg::kPerHi; };
+  auto slot = [&](int s) { return smem + s * Cfg::kSlot; };
+
+  if (tid == 0) {
+    // ---- TMA producer of this CTA; rank 0's full barrier counts the bytes of both
+    const uint8_t* maps = static_cast<const uint8_t*>(it.maps);
+    for (int m = 0; m < (kPasses > 1 ? 4 : 2); ++m) tc::tmap_acquire(maps + 128 * m);
+    const int rowA = ((it.slab_a + jw) * it.nrb + it.rb_a + rank) * nk;
+    const int rowB = (it.slab_b * it.nrb + it.rb_b) * nk;
+    uint32_t issued = 0;
+    bool ok = true;
+    for (int c = 0; c < nchunks && ok; ++c)
+      for (int q = 0; q < kPasses && ok; ++q) {
+        const int k1 = min(nk, (c + 1) * kChunkTiles), ps = per_slot(q);
+        const int nd = q == 0 ? NS : Cfg::kHi;             // digits loaded
+        for (int k0 = c * kChunkTiles; k0 < k1; k0 += ps, ++issued) {
+          const int s = int(issued % Cfg::kSlots);
+          if (issued >= uint32_t(Cfg::kSlots) &&
+              !tc::mbar_wait(&empty[s], ((issued / Cfg::kSlots) - 1) & 1)) {
+            ok = false;
+            break;
+          }
+          const int nt = min(ps, k1 - k0);
+          if (rank == 0) tc::mbar_arrive_expect_tx(&full[s], uint32_t(2 * nt * nd * (kTileA + kTileB)));
+          const uint32_t bar = tc::mapa(&full[s], 0);
+          for (int t = 0; t < nt; ++t) {
+            uint8_t* d = slot(s) + t * nd * (kTileA + kTileB);
+            tc::tma_load_3d_pair(d, maps + 256 * q, bar, 0, 0, (rowA + k0 + t) * NS);
+            tc::tma_load_3d_pair(d + nd * kTileA, maps + 256 * q + 128, bar, 0, 32 * rank, (rowB + k0 + t) * NS);
+          }
+        }
+      }
+    if (!ok) atomicOr(it.err, kErrTimeout);
+    // copies still in flight on a timeout land before the CTA leaves (bounded wait)
+    if (rank == 0) {
+      for (uint32_t s = 0; s < uint32_t(Cfg::kSlots) && s < issued; ++s) {
+        const uint32_t last = issued - 1 - (issued - 1 - s) % Cfg::kSlots;
+        if (!tc::mbar_wait(&full[s], (last / Cfg::kSlots) & 1)) atomicOr(it.err, kErrTimeout);
+      }
+    } else if (!ok) {
+      const uint64_t t0 = tc::global_ns();
+      while (tc::global_ns() - t0 < 1000000ull) {
+      }
+    }
+  } else if (tid == 32 && rank == 0) {
+    // ---- MMA issuer of the pair
+    constexpr uint32_t idesc = tc::idesc_s8_s32(256, 128);
+    bool ok = true;
+    uint32_t step = 0;
+    int pass = 0;
+    for (int c = 0; c < nchunks && ok; ++c)
+#pragma unroll
+      for (int q = 0; q < kPasses; ++q) {
+        if (!ok) break;
+        if (pass > 0 && !tc::mbar_wait(acce, (pass - 1) & 1)) {
+          ok = false;
+          break;
+        }
+        ++pass;
+        tc::tc_fence_after();
+        const int k1 = min(nk, (c + 1) * kChunkTiles), ps = per_slot(q);
+        constexpr int kBytesLo = NS * (kTileA + kTileB);
+        uint32_t first = 0u;
+        for (int k0 = c * kChunkTiles; k0 < k1; k0 += ps, ++step) {
+          const int s = int(step % Cfg::kSlots);
+          if (!tc::mbar_wait(&full[s], (step / Cfg::kSlots) & 1)) {
+            ok = false;
+            break;
+          }
+          tc::tc_fence_after();
+          const int nt = min(ps, k1 - k0);
+          for (int t = 0; t < nt; ++t) {
+            const int nd = q == 0 ? NS : Cfg::kHi;
+            const uint8_t* base = slot(s) + (q == 0 ? 0 : t * nd * (kTileA + kTileB));
+            static_assert(kBytesLo == Cfg::kSlot, "one k-tile per slot in the low pass");
+            const uint64_t ad = tc::desc_kmajor_cores(base, 512);
+            const uint64_t bd = tc::desc_kmajor_cores(base + nd * kTileA, 512);
+            const int nl = q == 0 ? Cfg::kLo : Cfg::kHi;
+            const int d0 = q == 0 ? NS + 2 - Cfg::kLo : 2;
+#pragma unroll
+            for (int a = 0; a < nl; ++a) {
+              const int d = d0 + a;
+              const uint32_t dt = tmem + uint32_t(a * 128);
+              bool fresh = true;
+#pragma unroll
+              for (int i = 1; i <= NS; ++i) {
+                const int j = d - i;
+                if (j < 1 || j > NS) continue;
+#pragma unroll
+                for (int sub = 0; sub < 2; ++sub) {
+                  // 32 int8 along K = two core matrices = 256 bytes
+                  tc::mma_s8_pair(dt, ad + uint64_t(((i - 1) * kTileA + sub * 256) >> 4),
+                                  bd + uint64_t(((j - 1) * kTileB + sub * 256) >> 4), idesc,
+                                  (fresh && sub == 0) ? first : 1u);
+                }
+                fresh = false;
+              }
+            }
+            first = 1u;
+          }
+          tc::mma_commit_pair(&empty[s]);
+        }
+        if (ok) tc::mma_commit_pair(accf);
+      }
+    if (!ok) atomicOr(it.err, kErrTimeout);
+  } else if (warp >= 2) {
+    // ---- drain: join the levels of a pass in 64-bit integers, add to FP64 registers
+    const int quad = warp & 3;                 // TMEM lanes 32 quad .. (rows)
+    const int half = (warp - 2) >> 2;          // columns 64 half ..
+    const uint32_t done = tc::mapa(acce, 0);
+    double acc[64];
+#pragma unroll
+    for (int j = 0; j < 64; ++j) acc[j] = 0.0;
+    bool ok = true;
+    int pass = 0;
+    for (int c = 0; c < nchunks && ok; ++c)
+#pragma unroll
+      for (int q = 0; q < kPasses; ++q) {
+        if (!ok) break;
+        ok = __all_sync(0xffffffffu, tc::mbar_wait(accf, pass & 1));
+        if (!ok) break;
+        ++pass;
+        tc::tc_fence_after();
+        constexpr int kLoL = Cfg::kLo, kHiL = Cfg::kHi;
+        const double wq = q == 0 ? 1.0 : double(1ull << (8 * kLoL));
+#pragma unroll
+        for (int cb = 0; cb < 8; ++cb) {
+          const uint32_t base = tmem + uint32_t(half * 64 + cb * 8) + (uint32_t(quad * 32) << 16);
+          uint32_t r[4][8];
+          const int nl = q == 0 ? kLoL : kHiL;
+#pragma unroll
+          for (int a = 0; a < 4; ++a)
+            if (a < nl) tc::tmem_ld_32x8(base + uint32_t(a * 128), r[a]);
+          tc::tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            long long x = int(r[0][j]);
+#pragma unroll
+            for (int a = 1; a < 4; ++a)
+              if (a < nl) x = x * 256 + int(r[a][j]);
+            acc[cb * 8 + j] += double(x) * wq;
+          }
+        }
+        tc::tc_fence_before();
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive_cluster(done);
+      }
+    const int rb = it.rb_a + rank, cb = it.rb_b;
+    if (!ok) {
+      if (lane == 0) atomicOr(it.err, kErrTimeout);
+    } else if (rb < it.nrb && rb <= cb) {      // blocks below the diagonal are not stored
+      const int row = rb * 128 + quad * 32 + lane, col0 = cb * 128 + half * 64;
+      const int er = it.exps[size_t(it.slab_e + jw) * it.ld + row];
+      constexpr int kShift = 8 * (NS - 1) - 2 * (8 * NS - 1);
+      double* dst = it.C + jw * it.sC + size_t(row) * it.ld + col0;
+#pragma unroll
+      for (int j = 0; j < 64; j += 2) {
+        double v[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const int ec = it.exps[col0 + j + u];
+          v[u] = (er == kNaNExp || ec == kNaNExp) ? __longlong_as_double(0x7ff8000000000000ll)
+                                                   : ldexp(acc[j + u], er + ec + kShift);
+          if (col0 + j + u == row) v[u] += 1.0;
+        }
+        *reinterpret_cast<double2*>(dst + j) = make_double2(v[0], v[1]);
+      }
+    }
+  }
+  tc::tc_fence_before();
+  __syncthreads();
+  tc::cluster_sync();        // no CTA leaves while its peer may still reach its memory
+  if (warp == 0) {
+    __syncwarp();
+    tc::tmem_dealloc_pair(tmem, 512);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Host side
+namespace {
+PFN_cuTensorMapEncodeTiled_v12000 g_encode_dig = nullptr;
+
+template <int NS>
+cudaError_t prepare_ns() {
+  return cudaFuncSetAttribute(digit_syrk_kernel<NS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              int(DigCfg<NS>::kSmem));
+}
+}  // namespace
+
+// Four maps (512 bytes) of a digit array of `planes` digit planes (slabs x row blocks x
+// k-tiles x NS), each 64 core matrices of 128 bytes: all digits of an A tile and of half a
+// B tile, then the leading digits of the high pass.
+Status make_digit_tmaps(void* host_maps, const void* digits, long long planes, int ns) {
+  if (!g_encode_dig) {
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult qr;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qr) != cudaSuccess ||
+        qr != cudaDriverEntryPointSuccess || !fn) {
+      cudaGetLastError();
+      return Status::fail(RIGW_ERR_UNSUPPORTED, "cuTensorMapEncodeTiled unavailable");
+    }
+    g_encode_dig = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
+  }
+  CUtensorMap* maps = reinterpret_cast<CUtensorMap*>(host_maps);
+  const int nhi = ns > 4 ? ns - 4 : 1;
+  for (int m = 0; m < 4; ++m) {
+    cuuint64_t dims[3] = {128, 64, cuuint64_t(planes)};
+    cuuint64_t strides[2] = {128, 128 * 64};
+    cuuint32_t box[3] = {128, cuuint32_t(m & 1 ? 32 : 64), cuuint32_t(m < 2 ? ns : nhi)};
+    cuuint32_t estr[3] = {1, 1, 1};
+    CUresult e = g_encode_dig(&maps[m], CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(digits), dims, strides, box,
+                              estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (e != CUDA_SUCCESS) return Status::fail(RIGW_ERR_CUDA, "cuTensorMapEncodeTiled (digits) failed (%d)", int(e));
+  }
+  return Status::ok();
+}
+
+void launch_digit_zero(const ProbDev* probs, const WorkItem* items, int n, cudaStream_t s) {
+  if (n > 0) digit_zero_kernel<<<n, 256, 0, s>>>(probs, items);
+}
+void launch_digit_rowmax(const ProbDev* probs, const WorkItem* items, int n, cudaStream_t s) {
+  if (n > 0) digit_rowmax_kernel<<<n, 256, 0, s>>>(probs, items);
+}
+void launch_digit_slice(const ProbDev* probs, const WorkItem* items, int n, cudaStream_t s) {
+  if (n > 0) digit_slice_kernel<kFp64Digits><<<n, 256, 0, s>>>(probs, items);
+}
+void launch_digit_syrk(const DigitItem* items, int n, int ny, cudaStream_t s) {
+  if (n > 0 && ny > 0)
+    digit_syrk_kernel<kFp64Digits><<<dim3(2 * n, ny), kDigThreads, DigCfg<kFp64Digits>::kSmem, s>>>(items);
+}
+cudaError_t prepare_digit_kernels() { return prepare_ns<kFp64Digits>(); }
+
+}  // namespace rigw

@@ -19,8 +19,8 @@ inline int round_up(int v, int a) { return (v + a - 1) / a * a; }
 // ---------------------------------------------------------------------------
 bool Shape::operator<(const Shape& o) const {
   return std::tie(naux, nocc, nvirt, nomega, nstate_p, nsig, nc, nsigma_half, technique, precision, qp_only, nocc2,
-                  nvirt2) < std::tie(o.naux, o.nocc, o.nvirt, o.nomega, o.nstate_p, o.nsig, o.nc, o.nsigma_half,
-                                     o.technique, o.precision, o.qp_only, o.nocc2, o.nvirt2);
+                  nvirt2, no_digits) < std::tie(o.naux, o.nocc, o.nvirt, o.nomega, o.nstate_p, o.nsig, o.nc, o.nsigma_half,
+                                     o.technique, o.precision, o.qp_only, o.nocc2, o.nvirt2, o.no_digits);
 }
 
 Status make_shape(const rigw_problem& p, Shape* sh) {
@@ -49,6 +49,7 @@ Status make_shape(const rigw_problem& p, Shape* sh) {
   sh->nsigma_half = p.nomega_sigma / 2;
   sh->technique = p.technique;
   sh->precision = p.precision;
+  sh->no_digits = 0;
   sh->qp_only = (p.flags & RIGW_PROBLEM_QP_ONLY) ? 1 : 0;
   return Status::ok();
 }
@@ -148,6 +149,7 @@ Status Context::init(int dev, size_t budget_bytes, int want_priority, bool block
   RIGW_CUDA_TRY(prepare_syrk_f64_tma());
   RIGW_CUDA_TRY(prepare_tc_kernels());
   RIGW_CUDA_TRY(prepare_ozaki_kernels());
+  RIGW_CUDA_TRY(prepare_digit_kernels());
   RIGW_CUDA_TRY(cudaFuncSetAttribute(chol_diag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      int(chol_diag_smem_bytes())));
   return Status::ok();
@@ -243,6 +245,17 @@ Dims dims_of(const Shape& sh, PlanMode mode) {
 
 }  // namespace
 
+// The digit products need whole 256 x 128 tiles per pair of CTAs and three passes over the
+// operands before the product.  chi0 stage, DMMA against digits (12 / 32 frequencies, ms):
+// naux 200 0.051 / 0.064 against 0.066 / 0.096, 300 0.104 / 0.137 against 0.078 / 0.162,
+// 384 0.117 / 0.299 against 0.094 / 0.188, 512 0.262 / 0.664 against 0.127 / 0.317,
+// 840 (32) 4.25 against 1.41, 2000 (32) 112 against 33.  Below 512 transitions the passes
+// and the drains, which do not shrink with the sum, take over.
+bool use_digits(const Shape& sh) {
+  return !sh.no_digits && sh.precision == RIGW_FP64 && sh.naux >= 384 &&
+         (long long)sh.nocc * sh.nvirt + (long long)sh.nocc2 * sh.nvirt2 >= 512;
+}
+
 // Bytes of one frequency's split operands (bf16 hi/lo, or the Ozaki slices).
 size_t split_bytes_per_frequency(const Shape& sh) {
   if (sh.precision == RIGW_FP64) return 0;
@@ -315,27 +328,29 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
   // Split precision: when the hi/lo buffers of every frequency of the batch are
   // small, one group holds all frequencies (one split and one tensor-core launch
   // with a full grid); otherwise groups of kSplitGroup frequencies share a buffer.
+  // bytes of the split operands of one frequency: bf16 hi/lo, slices, or FP64 digits
+  auto split_per_w = [&](const Shape& sh) -> size_t {
+    const Dims d = dims_of(sh, mode);
+    const int per = sh.precision == RIGW_FP64 ? (use_digits(sh) ? kFp64Digits : 0)
+                                              : (is_ozaki(sh.precision) ? ozaki_slices(sh.precision) : 4);
+    return size_t(d.npad) * d.nia_pad * per;
+  };
   size_t split_all = 0;
   for (const Shape& sh : shapes)
-    if (factor && sh.precision != RIGW_FP64) {
-      const Dims d = dims_of(sh, mode);
-      split_all += size_t(sh.nomega) * d.npad * d.nia_pad * (is_ozaki(sh.precision) ? ozaki_slices(sh.precision) : 4);
-    }
+    if (factor) split_all += size_t(sh.nomega) * split_per_w(sh);
   const bool split_whole = split_all <= kSplitWholeBytes;
   auto split_group = [&](const Shape& sh) {
     if (tune_.split_group > 0) return std::max(1, std::min(sh.nomega, tune_.split_group));
     if (split_whole) return std::max(1, sh.nomega);
     // at most kSplitGroup frequencies, and at most kSplitProblemBytes per problem
-    const Dims d = dims_of(sh, mode);
-    const size_t per_w = size_t(d.npad) * d.nia_pad * (is_ozaki(sh.precision) ? ozaki_slices(sh.precision) : 4);
-    const int cap = int(std::max<size_t>(1, kSplitProblemBytes / std::max<size_t>(per_w, 1)));
+    const int cap = int(std::max<size_t>(1, kSplitProblemBytes / std::max<size_t>(split_per_w(sh), 1)));
     return std::max(1, std::min({sh.nomega, kSplitGroup, cap}));
   };
 
   // ---- memory layout
   Layout L;
   struct Off {
-    size_t mp, xs, tmap, rmax, xexp, tnorm, dscale, eps, winv, logdet, rhs, colsq, mnorm, vchiv, ew, tr, en, sc, sr, qp;
+    size_t mp, xs, tmap, rmax, dmax, xexp, tnorm, dscale, eps, winv, logdet, rhs, colsq, mnorm, vchiv, ew, tr, en, sc, sr, qp;
   };
   std::vector<Off> off(np);
   for (int i = 0; i < np; ++i) {
@@ -358,7 +373,12 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
       pp.off_in_omega = L.take(size_t(sh.nomega) * D);
       pp.off_in_weight = L.take(size_t(sh.nomega) * D);
       off[i].mp = L.take(size_t(d.nia_pad) * d.npad * D);
-      if (sh.precision == RIGW_FP64) {
+      if (use_digits(sh)) {
+        off[i].xs = L.take(size_t(1 + split_group(sh)) * split_per_w(sh));
+        off[i].tmap = L.take(512);
+        off[i].dmax = L.take(size_t(1 + sh.nomega) * d.npad * sizeof(unsigned));
+        off[i].xexp = L.take(size_t(1 + sh.nomega) * d.npad * sizeof(int));
+      } else if (sh.precision == RIGW_FP64) {
         off[i].tmap = L.take(256);   // tensor maps of mp and dscale (TMA-staged FP64 chi0)
       } else if (sh.precision == RIGW_BF16X3) {
         off[i].xs = L.take(size_t(split_group(sh)) * 2 * d.npad * d.nia_pad * 2);
@@ -415,7 +435,7 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
       lists += size_t(kMaxChains + 1) * t * sizeof(GemmItem) +
                size_t(sh.nomega) * (d.npanel + 8) * sizeof(WorkItem) +
                size_t(d.nia_pad / 8 + d.npad * d.ldb / 1024 + 64) * 16;
-      if (sh.precision != RIGW_FP64) {   // split items: (group, split_t transitions, 64 aux), + row maxima
+      if (sh.precision != RIGW_FP64 || use_digits(sh)) {   // split items: (group, split_t transitions, 64 aux), + row maxima
         const int g = split_group(sh);
         lists += size_t((sh.nomega + g - 1) / g + 1) * (d.nia_pad / split_item_t(d) + 1) * (d.npad / 64) *
                      sizeof(WorkItem) +
@@ -479,7 +499,15 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
       }
       p.tnorm = dp(off[i].tnorm);
       p.dscale = dp(off[i].dscale);
-      if (sh.precision == RIGW_FP64) {
+      if (use_digits(sh)) {
+        p.xs = base + off[i].xs;
+        p.dmax = reinterpret_cast<unsigned*>(base + off[i].dmax);
+        p.xexp = reinterpret_cast<int*>(base + off[i].xexp);
+        alignas(64) unsigned char maps[512];
+        RIGW_TRY(make_digit_tmaps(maps, p.xs,
+                                  (long long)(1 + p.wgroup) * d.npanel * (d.nia_pad / 64) * kFp64Digits, kFp64Digits));
+        RIGW_CUDA_TRY(cudaMemcpyAsync(base + off[i].tmap, maps, sizeof(maps), cudaMemcpyHostToDevice, ctx->stream));
+      } else if (sh.precision == RIGW_FP64) {
         alignas(64) unsigned char maps[256];
         RIGW_TRY(make_f64_tmaps(maps, p.mp, d.npad, d.nia_pad, p.dscale, sh.nomega));
         RIGW_CUDA_TRY(cudaMemcpyAsync(base + off[i].tmap, maps, sizeof(maps), cudaMemcpyHostToDevice, ctx->stream));
@@ -616,7 +644,43 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
               (fused ? tl_ozaki4_ : tl_ozaki_)[w0 / p.wgroup].push_back(t);
             }
       }
-      if (sh.precision == RIGW_FP64) {
+      if (use_digits(sh)) {
+        // row maxima of M and of M D_w for every frequency, the digits of M, then per
+        // frequency group the digits of M D_w and the products
+        const int nkt = p.nia_pad / 64;
+        for (size_t e = 0; e < size_t(1 + sh.nomega) * npad; e += 4096) wl_dzero_.push_back({i, int(e), 0, 0});
+        for (int t0 = 0; t0 < p.nia_pad; t0 += p.split_t)
+          for (int rb = 0; rb < p.npanel; ++rb) wl_dmax_.push_back({i, t0, rb, 0});
+        for (int rb = 0; rb < p.npanel; ++rb)
+          for (int kt = 0; kt < nkt; ++kt) wl_dbase_.push_back({i, kt, rb, -1});
+        for (int w0 = 0, g = 0; w0 < sh.nomega; w0 += p.wgroup, ++g) {
+          if (int(wl_dslice_.size()) <= g) {
+            wl_dslice_.resize(g + 1);
+            dl_syrk_.resize(g + 1);
+          }
+          for (int rb = 0; rb < p.npanel; ++rb)
+            for (int kt = 0; kt < nkt; ++kt) wl_dslice_[g].push_back({i, kt, rb, w0});
+          for (int ra = 0; ra < p.npanel; ra += 2)
+            for (int cb = ra; cb < p.npanel; ++cb) {
+              DigitItem t{};
+              t.maps = base + off[i].tmap;
+              t.C = p.eps + size_t(w0) * npad * npad;
+              t.err = err_dev_;
+              t.exps = p.xexp;
+              t.rb_a = ra;
+              t.rb_b = cb;
+              t.nrb = p.npanel;
+              t.nkt = nkt;
+              t.slab_a = 1;
+              t.slab_b = 0;
+              t.slab_e = 1 + w0;
+              t.ld = npad;
+              t.nw = std::min(p.wgroup, sh.nomega - w0);
+              t.sC = (long long)npad * npad;
+              dl_syrk_[g].push_back(t);
+            }
+        }
+      } else if (sh.precision == RIGW_FP64) {
         // one item per tile covering every frequency (blockIdx.y); the tiles of a
         // row block start at its diagonal, so only the lower half of the
         // diagonal BMC x BMC block lies below it, and end at naux
@@ -794,6 +858,9 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
   for (auto& l : tl_ozaki_) std::stable_sort(l.begin(), l.end(), by_cost);
   for (auto& l : tl_ozaki4_) std::stable_sort(l.begin(), l.end(), by_cost);
 
+  for (auto& l : dl_syrk_)
+    std::stable_sort(l.begin(), l.end(), [](const DigitItem& a, const DigitItem& b) { return a.nkt > b.nkt; });
+
   // ---- upload the lists and the launch sequence
   size_t lbytes = 0;
   auto reserve = [&](size_t n) {
@@ -820,6 +887,8 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
       for (size_t j = 0; j < n; ++j) ny = std::max(ny, static_cast<const GemmItem*>(src)[j].nw);
     if (kind == 13 || kind == 20 || kind == 21)
       for (size_t j = 0; j < n; ++j) ny = std::max(ny, static_cast<const TcItem*>(src)[j].nw);
+    if (kind == 26)
+      for (size_t j = 0; j < n; ++j) ny = std::max(ny, static_cast<const DigitItem*>(src)[j].nw);
     if (kind == 22)
       for (size_t j = 0; j < n; ++j) ny = std::max(ny, static_cast<const F64SyrkItem*>(src)[j].nw);
     pend.push_back({kind, src, elem * n, int(n), arg, stream, wait_ev, rec_ev, ny});
@@ -833,6 +902,13 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
   for (size_t g = 0; g < wl_split_.size(); ++g) {
     add(12, wl_split_[g].data(), sizeof(WorkItem), wl_split_[g].size(), 0);
     add(13, tl_syrk_[g].data(), sizeof(TcItem), tl_syrk_[g].size(), 0);
+  }
+  add(23, wl_dzero_.data(), sizeof(WorkItem), wl_dzero_.size(), 0);
+  add(24, wl_dmax_.data(), sizeof(WorkItem), wl_dmax_.size(), 0);
+  add(25, wl_dbase_.data(), sizeof(WorkItem), wl_dbase_.size(), 0);
+  for (size_t g = 0; g < wl_dslice_.size(); ++g) {
+    add(25, wl_dslice_[g].data(), sizeof(WorkItem), wl_dslice_[g].size(), 0);
+    add(26, dl_syrk_[g].data(), sizeof(DigitItem), dl_syrk_[g].size(), 0);
   }
   add(17, wl_ozzero_.data(), sizeof(WorkItem), wl_ozzero_.size(), 0);
   add(18, wl_rowmax_.data(), sizeof(WorkItem), wl_rowmax_.size(), 0);
@@ -922,7 +998,8 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
 static int stage_of(int kind) {
   switch (kind) {
     case 0: case 2: case 3: return 0;
-    case 1: case 12: case 13: case 15: case 16: case 17: case 18: case 19: case 20: case 21: case 22: return 1;
+    case 1: case 12: case 13: case 15: case 16: case 17: case 18: case 19: case 20: case 21: case 22:
+    case 23: case 24: case 25: case 26: return 1;
     case -1: case 4: case 5: case 6: case 14: return 2;
     default: return 3;
   }
@@ -955,6 +1032,10 @@ void Plan::record(cudaStream_t s0, int stage) {
       case 12: launch_split_bf16x3(probs_dev_, wl, L.count, s); break;
       case 13: launch_syrk_bf16x3(reinterpret_cast<const TcItem*>(lb + L.off), L.count, L.ny, s); break;
       case 22: launch_syrk_f64_tma(reinterpret_cast<const F64SyrkItem*>(lb + L.off), L.count, L.ny, s); break;
+      case 23: launch_digit_zero(probs_dev_, wl, L.count, s); break;
+      case 24: launch_digit_rowmax(probs_dev_, wl, L.count, s); break;
+      case 25: launch_digit_slice(probs_dev_, wl, L.count, s); break;
+      case 26: launch_digit_syrk(reinterpret_cast<const DigitItem*>(lb + L.off), L.count, L.ny, s); break;
       case 17: launch_ozaki_zero(probs_dev_, wl, L.count, s); break;
       case 18: launch_ozaki_rowmax(probs_dev_, wl, L.count, s); break;
       case 19: launch_ozaki_slice(probs_dev_, wl, L.count, s); break;

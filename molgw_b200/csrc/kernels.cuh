@@ -115,6 +115,26 @@ struct F64SyrkItem {
 void launch_syrk_f64_tma(const F64SyrkItem* items, int n, int ny, cudaStream_t s);
 cudaError_t prepare_syrk_f64_tma();
 
+// FP64 chi0 from exact int8 digit products (digit_gemm.cu): one 256 x 128 upper tile of
+// eps(iw) = 1 + (M D_w) M^T per pair of CTAs, frequency = blockIdx.y.
+struct DigitItem {
+  const void* maps;     // four CUtensorMaps of the problem's digit array (make_digit_tmaps)
+  double* C;            // &eps[w0][0][0]
+  int* err;
+  const int* exps;      // row exponents: [0][ld] of M, [1 + w][ld] of M D_w
+  int rb_a, rb_b;       // 128-row blocks: output rows from 128 rb_a (two blocks), columns from 128 rb_b
+  int nrb, nkt;         // row blocks and k-tiles (64 transitions) of a slab
+  int slab_a, slab_b;   // slab of M D_w for j = 0 (+ j), slab of M
+  int slab_e;           // exponent row of M D_w for j = 0 (+ j)
+  int ld, nw;           // npad; frequencies covered
+  long long sC;         // doubles between the eps blocks of two frequencies
+};
+void launch_digit_zero(const ProbDev* probs, const WorkItem* items, int n, cudaStream_t s);
+void launch_digit_rowmax(const ProbDev* probs, const WorkItem* items, int n, cudaStream_t s);
+void launch_digit_slice(const ProbDev* probs, const WorkItem* items, int n, cudaStream_t s);
+void launch_digit_syrk(const DigitItem* items, int n, int ny, cudaStream_t s);
+cudaError_t prepare_digit_kernels();
+
 // Host-side launchers of the DMMA tile engine (gemm_f64.cu).
 // grid (n items) x (ny frequencies): CTAs with blockIdx.y >= item.nw return at once
 void launch_dgemm_128x128(const GemmItem* items, int n, int ny, cudaStream_t s);

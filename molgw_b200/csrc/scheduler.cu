@@ -142,12 +142,16 @@ Status solve_batch(Context& c, int n, const rigw_problem* probs, rigw_result* re
   std::vector<Unit> units;
   std::vector<std::vector<double>> om(n), wt(n);
   for (int i = 0; i < n; ++i) {
-    const Shape& sh = shapes[i];
-    int wc = sh.nomega;
-    for (; wc >= 1; --wc) {
-      Shape s2 = sh;
-      s2.nomega = wc;
-      if (Plan::measure({s2}, kPlanPartial) <= avail) break;
+    Shape& sh = shapes[i];
+    int wc = 0;
+    for (;;) {
+      for (wc = sh.nomega; wc >= 1; --wc) {
+        Shape s2 = sh;
+        s2.nomega = wc;
+        if (Plan::measure({s2}, kPlanPartial) <= avail) break;
+      }
+      if (wc >= 1 || !use_digits(sh)) break;
+      sh.no_digits = 1;   // one frequency with its digit buffers does not fit: DMMA needs none
     }
     if (wc < 1)
       return Status::fail(RIGW_ERR_NOMEM, "problem %d (naux=%d, nocc=%d, nvirt=%d) does not fit in %zu bytes even "

@@ -93,6 +93,60 @@ RIGW_DEVICE_INLINE void mma_s8(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, 
       "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc));
 }
+// --- CTA pairs (clusters of two, cta_group::2): the CTA of even rank issues the MMAs
+// for both; A rows 128 r .. and B rows r N/2 .. lie in the shared memory of rank r,
+// accumulator rows 128 r .. in its TMEM.
+RIGW_DEVICE_INLINE uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+RIGW_DEVICE_INLINE void cluster_sync() {
+  asm volatile(
+      "barrier.cluster.arrive.release;\n\t"
+      "barrier.cluster.wait.acquire;\n" ::: "memory");
+}
+// Address of the same shared variable in CTA `rank` of the cluster.
+RIGW_DEVICE_INLINE uint32_t mapa(const void* p, uint32_t rank) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+  return a;
+}
+RIGW_DEVICE_INLINE void mbar_arrive_cluster(uint32_t bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(bar) : "memory");
+}
+// 3-D TMA tile load into this CTA's shared memory, completing on an mbarrier of the pair.
+RIGW_DEVICE_INLINE void tma_load_3d_pair(void* dst, const void* tmap, uint32_t bar, int c0, int c1, int c2) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes "
+      "[%0], [%1, {%3, %4, %5}], [%2];\n" ::"r"(smem_u32(dst)),
+      "l"(tmap), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
+      : "memory");
+}
+RIGW_DEVICE_INLINE void tmem_alloc_pair(uint32_t* slot, uint32_t ncols) {
+  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(slot)),
+               "r"(ncols));
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;\n" ::);
+}
+RIGW_DEVICE_INLINE void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
+  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;\n" ::"r"(taddr), "r"(ncols));
+}
+RIGW_DEVICE_INLINE void mma_s8_pair(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc));
+}
+// Arrive on the mbarrier at this offset in both CTAs when all MMAs issued so far are done.
+RIGW_DEVICE_INLINE void mma_commit_pair(uint64_t* bar) {
+  asm volatile(
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n" ::"r"(
+          smem_u32(bar)),
+      "h"(uint16_t(3))
+      : "memory");
+}
+
 // Arrive on an mbarrier when all previously issued MMAs of this thread are done.
 RIGW_DEVICE_INLINE void mma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
@@ -112,6 +166,27 @@ RIGW_DEVICE_INLINE void tmem_ld_32x32(uint32_t taddr, uint32_t (&r)[32]) {
         "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
       : "r"(taddr));
   asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+}
+
+// 32 lanes x 8 columns of 32-bit words, without the wait (tmem_ld_wait).
+RIGW_DEVICE_INLINE void tmem_ld_32x8(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr));
+}
+RIGW_DEVICE_INLINE void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory"); }
+
+// Shared-memory matrix descriptor of a K-major tile stored as 8-row x 16-byte core
+// matrices of 128 contiguous bytes (no swizzle): neighbours along K are 128 bytes
+// apart, neighbouring 8-row groups sbo bytes.
+RIGW_DEVICE_INLINE uint64_t desc_kmajor_cores(const void* smem, uint32_t sbo) {
+  const uint64_t addr = smem_u32(smem);
+  uint64_t d = 0;
+  d |= (addr >> 4) & 0x3FFFull;            // start address
+  d |= uint64_t(128 >> 4) << 16;           // leading byte offset: next core matrix along K
+  d |= uint64_t(sbo >> 4) << 32;           // stride byte offset: next 8 rows
+  d |= uint64_t(1) << 46;                  // descriptor version (sm_100)
+  return d;
 }
 
 // Shared-memory matrix descriptor of a K-major tile whose rows are 128 bytes,

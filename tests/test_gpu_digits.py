@@ -1,0 +1,103 @@
+"""FP64 chi0 from int8 digit products (molgw_b200/csrc/digit_gemm.cu) at the edges of its
+tiles and chunks, against NumPy in FP64.
+
+Tolerance: an FP64 sum of K products of entries with row norms |A_p|, |B_q| is off by at most
+about K u |A_p| |B_q|, u = 2^-53; chi = eps^-1 - 1 is a contraction of that error (eps >= 1), so
+|d chi| <= 2 K u max diag(eps) with both sides' errors, and ten times that is allowed.  The row
+exponents and the layout of the digits would show as errors of 1e-2 and more."""
+import numpy as np
+import pytest
+
+from molgw_b200.rigw import Engine, RigwError
+from molgw_b200.synth import GWInstance, make_instance
+
+pytestmark = pytest.mark.gpu
+
+
+def molecule(nocc, nvirt, naux, nomega, seed=0, decades=0.0):
+    rng = np.random.default_rng(seed)
+    energy = np.concatenate([np.sort(rng.uniform(-1.1, -0.3, nocc)), np.sort(rng.uniform(0.02, 1.5, nvirt))])
+    m = rng.standard_normal((nocc, nvirt, naux)) * (0.35 / np.sqrt(nocc * nvirt + naux))
+    m *= 10.0 ** (-decades * rng.random(naux))[None, None, :]
+    ms = rng.standard_normal((2, nocc + nvirt, naux)) * 0.01
+    occ = np.concatenate([np.full(nocc, 2.0), np.zeros(nvirt)])
+    return GWInstance(nocc=nocc, nvirt=nvirt, naux=naux, nomega=nomega, energy=energy, occupation=occ, m_ia=m,
+                      m_sigma=ms, nsemin=nocc, nsemax=nocc + 1)
+
+
+def reference(inst, omega):
+    no, nv = inst.nocc, inst.nvirt
+    de = (inst.energy[no:][None, :] - inst.energy[:no][:, None]).ravel()
+    docc = (inst.occupation[:no][:, None] - inst.occupation[no:][None, :]).ravel()
+    m = inst.m_ia.reshape(no * nv, -1)
+    out, top = [], 0.0
+    for w in omega:
+        eps = np.eye(inst.naux) + m.T @ (m * (2.0 * docc * de / (w * w + de * de))[:, None])
+        top = max(top, np.abs(np.diag(eps)).max())
+        out.append(np.linalg.inv(eps) - np.eye(inst.naux))
+    return np.array(out), top
+
+
+def check(engine, inst):
+    from molgw_b200.rigw import imag_grid
+    erpa, egw, w = engine.polarizability_grid_scalapack(inst)
+    chi = w.chi()
+    w.release()
+    ref, top = reference(inst, imag_grid(inst.nomega)[0])
+    tol = 10 * 2 * inst.nocc * inst.nvirt * 2.0 ** -53 * top
+    assert np.abs(chi - ref).max() <= tol, (np.abs(chi - ref).max(), tol)
+    return erpa
+
+
+@pytest.mark.parametrize("nocc,nvirt,naux,nomega", [
+    (8, 64, 384, 3),       # whole tiles, K a multiple of the k-tile, smallest of the range
+    (9, 57, 385, 2),       # one row beyond a 128-row block, one transition beyond a k-tile
+    (7, 90, 511, 17),      # one row short of four blocks; more frequencies than one factor block
+    (11, 61, 513, 2),      # an odd number of row blocks: the last pair has one
+    (30, 547, 390, 2),     # 16410 transitions: two INT32 chunks, the second of one k-tile
+])
+def test_tile_and_chunk_edges(engine, nocc, nvirt, naux, nomega):
+    check(engine, molecule(nocc, nvirt, naux, nomega, seed=naux))
+
+
+def test_rows_of_very_different_size(engine):
+    check(engine, molecule(10, 70, 400, 3, seed=5, decades=150.0))
+
+
+def test_negative_factors(engine):
+    """A few inverted transitions (D < 0) that leave eps positive definite."""
+    inst = molecule(10, 70, 400, 3, seed=6)
+    inst.occupation[9], inst.occupation[10] = 0.5, 1.5
+    check(engine, inst)
+
+
+def test_frequency_groups_and_mixed_batch(engine):
+    """A batch in which some problems take the digit products and some the DMMA kernel gives
+    what each gives alone."""
+    insts = [make_instance(4, 30, 70, 8, seed=41), make_instance(9, 80, 400, 16, seed=42),
+             make_instance(12, 100, 520, 12, seed=43)]
+    alone = [engine.g0w0(i) for i in insts]
+    for a, b in zip(alone, engine.g0w0_batch(insts)):
+        assert abs(a.erpa - b.erpa) <= 1e-12 * abs(a.erpa)
+        assert np.abs(a.sigma_calc - b.sigma_calc).max() <= 1e-12 * np.abs(a.sigma_calc).max()
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_non_finite_input_is_reported(engine, bad):
+    inst = molecule(9, 64, 384, 2, seed=8)
+    inst.m_ia[3, 5, 17] = bad
+    with pytest.raises(RigwError):
+        engine.g0w0(inst)
+    check(engine, molecule(9, 64, 384, 2, seed=8))      # the context stays usable
+
+
+def test_without_room_for_the_digits(engine):
+    """A budget that holds one frequency without the digit buffers (about 115 MB) but not with
+    them (205 MB): the problem still runs, on DMMA."""
+    inst = molecule(30, 547, 390, 2, seed=9)
+    ref = engine.g0w0(inst)
+    small = Engine(0, hbm_budget_bytes=160 << 20)
+    out = small.g0w0(inst)
+    small.close()
+    assert abs(out.erpa - ref.erpa) <= 1e-10
+    assert np.abs(out.sigma_calc - ref.sigma_calc).max() <= 1e-11 * np.abs(ref.sigma_calc).max()
