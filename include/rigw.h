@@ -76,8 +76,9 @@ enum rigw_precision {
                               FP64 sums                                                  */
   RIGW_BF16X3 = 1,         /* split BF16 hi/lo products on tcgen05, FP32 accumulation    */
   RIGW_OZAKI_INT8 = 16     /* + s (3 <= s <= 7): Ozaki-sliced INT8 products on tcgen05,
-                              s signed 7-bit slices per row, exact INT32 accumulation,
-                              FP64 recombination; use RIGW_OZAKI(s)                      */
+                              s signed slices per row (8 bits each for chi0, 7 for AO->MO),
+                              exact INT32 accumulation, FP64 recombination; use
+                              RIGW_OZAKI(s)                                              */
 };
 #define RIGW_OZAKI(s) (RIGW_OZAKI_INT8 + (s))
 #define RIGW_OZAKI_MIN_SLICES 3

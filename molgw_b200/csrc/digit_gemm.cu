@@ -1,5 +1,5 @@
-// FP64-accurate chi0 contraction from exact int8 digit products on the 5th-generation
-// tensor cores (RIGW_FP64 for all but the smallest problems).
+// chi0 from exact int8 digit products on the 5th-generation tensor cores: NS = 7 digits
+// reach FP64 accuracy (RIGW_FP64 for all but the smallest problems), NS = s is RIGW_OZAKI(s).
 //
 //   eps(iw)[p][q] = delta_pq + sum_t A_pt B_qt,   A = M D_w,   B = M
 //
@@ -7,7 +7,7 @@
 // to an integer X of 8 NS - 1 bits; X is cut into NS balanced base-256 digits d_1 (most
 // significant) .. d_NS, each an int8:  x = 2^(e_p - (8 NS - 1)) sum_i d_i 256^(NS - i).
 //   (A B^T)_pq = 2^(e_p + f_q - 2 (8 NS - 1)) sum_{d=2}^{NS+1} 256^(2 NS - d) L_d(p,q),
-//   L_d = sum_{i+j=d} A_i B_j^T      (28 of the 49 digit products for NS = 7)
+//   L_d = sum_{i+j=d} A_i B_j^T      (NS (NS + 1) / 2 digit products: 28 of 49 for NS = 7)
 // L_d is an exact INT32 sum (tcgen05.mma kind::i8) over chunks of kChunkTiles k-tiles: for
 // NS = 7, |L_d| <= 7 * 128^2 * 16384 < 2^31.  The levels are joined in 64-bit integers,
 // converted to FP64 once per chunk and summed in FP64.
@@ -54,7 +54,7 @@ struct DigCfg {
   static constexpr int kLo = NS < 4 ? NS : 4;    // levels of the low pass: NS + 2 - kLo .. NS + 1
   static constexpr int kHi = NS - kLo;           // levels of the high pass: 2 .. kHi + 1 (digits 1 .. kHi)
   static constexpr int kSlot = NS * (kTileA + kTileB);
-  static constexpr int kSlots = (216 * 1024) / kSlot < 6 ? (216 * 1024) / kSlot : 6;
+  static constexpr int kSlots = (216 * 1024) / kSlot;
   static constexpr int kPerHi = kHi > 0 ? NS / kHi : 1;   // k-tiles of the high pass per slot
   static constexpr size_t kSmem = size_t(kSlots) * kSlot + 1024 + 256;
 };
@@ -67,6 +67,12 @@ RIGW_DEVICE_INLINE int row_exponent(unsigned hi) {
   int e = (E == 0 ? 1 : E) - 1022;
   if (E > 0 && (hi & 0xfffffu) + 1u + 0x100000u > 2088763u) ++e;   // mantissa above 0.996
   return e < -960 ? -960 : e;
+}
+
+// D_w(t); only the FP64 mode takes negative factors.
+RIGW_DEVICE_INLINE double factor(const ProbDev& p, int w, int t) {
+  const double d = p.dscale[size_t(w) * p.nia_pad + t];
+  return p.signed_d ? d : split_factor(d);
 }
 
 RIGW_DEVICE_INLINE double pow2(int e) { return __hiloint2double((e + 1023) << 20, 0); }   // -1022 <= e <= 1023
@@ -106,7 +112,7 @@ __global__ void __launch_bounds__(256) digit_rowmax_kernel(const ProbDev* __rest
     for (int wb = 0; wb < p.nomega; wb += kWb) {
       const int nwb = min(kWb, p.nomega - wb);
       __syncthreads();
-      for (int i = tid; i < nwb * 64; i += 256) sd[i >> 6][i & 63] = p.dscale[size_t(wb + (i >> 6)) * p.nia_pad + t0 + (i & 63)];
+      for (int i = tid; i < nwb * 64; i += 256) sd[i >> 6][i & 63] = factor(p, wb + (i >> 6), t0 + (i & 63));
       __syncthreads();
       for (int w = 0; w < nwb; ++w) {
         unsigned m = 0;
@@ -200,7 +206,7 @@ __global__ void __launch_bounds__(256) digit_slice_kernel(const ProbDev* __restr
   for (int wb = w0; wb < w1; wb += kWb) {
     const int nwb = min(kWb, w1 - wb);
     __syncthreads();
-    for (int i = tid; i < nwb * 64; i += 256) sd[i >> 6][i & 63] = p.dscale[size_t(wb + (i >> 6)) * p.nia_pad + t0 + (i & 63)];
+    for (int i = tid; i < nwb * 64; i += 256) sd[i >> 6][i & 63] = factor(p, wb + (i >> 6), t0 + (i & 63));
     __syncthreads();
     for (int w = 0; w < nwb; ++w) {
       const int e = row_exponent(p.dmax[size_t(1 + wb + w) * p.npad + r]);
@@ -219,8 +225,9 @@ __global__ void __launch_bounds__(256) digit_slice_kernel(const ProbDev* __restr
 
 // One 256 x 128 tile per CTA pair: rank r holds A rows 128 r .. and B rows 64 r .. of the
 // tile and accumulates output rows 128 r ...  A slot of the ring holds every digit of one
-// k-tile (84 KB per CTA for NS = 7, two slots), so each digit tile that is loaded feeds all
-// the products it appears in; tcgen05 reads 96 bytes of shared memory per clock and CTA and
+// k-tile of 64 transitions (84 KB per CTA for NS = 7, two slots; five slots of 32 transitions
+// measured 2% slower), so each digit tile that is loaded feeds all the products it appears
+// in; tcgen05 reads 96 bytes of shared memory per clock and CTA and
 // TMA writes 30, below the 128 that shared memory delivers (a 128 x 128 tile of one CTA
 // would read 128 and write 45).  TMEM holds four 128-column accumulators, so the levels go
 // in two passes over a chunk: NS + 1 down to NS - 2 (22 of the 28 products for NS = 7), and
@@ -448,12 +455,16 @@ cudaError_t prepare_ns() {
   return cudaFuncSetAttribute(digit_syrk_kernel<NS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               int(DigCfg<NS>::kSmem));
 }
+template <int NS>
+void syrk_ns(const DigitItem* items, int n, int ny, cudaStream_t s) {
+  digit_syrk_kernel<NS><<<dim3(2 * n, ny), kDigThreads, DigCfg<NS>::kSmem, s>>>(items);
+}
 }  // namespace
 
-// Four maps (512 bytes) of a digit array of `planes` digit planes (slabs x row blocks x
-// k-tiles x NS), each 64 core matrices of 128 bytes: all digits of an A tile and of half a
-// B tile, then the leading digits of the high pass.
-Status make_digit_tmaps(void* host_maps, const void* digits, long long planes, int ns) {
+// Four maps (512 bytes) of `planes` operand planes (slabs x row blocks x k-tiles x ns) of
+// `cores` core matrices of 128 bytes (64: int8 digits, 128: bf16): all planes of an A tile and
+// of half a B tile, then the leading digits of the high pass.
+Status make_digit_tmaps(void* host_maps, const void* digits, long long planes, int ns, int cores) {
   if (!g_encode_dig) {
     void* fn = nullptr;
     cudaDriverEntryPointQueryResult qr;
@@ -467,9 +478,9 @@ Status make_digit_tmaps(void* host_maps, const void* digits, long long planes, i
   CUtensorMap* maps = reinterpret_cast<CUtensorMap*>(host_maps);
   const int nhi = ns > 4 ? ns - 4 : 1;
   for (int m = 0; m < 4; ++m) {
-    cuuint64_t dims[3] = {128, 64, cuuint64_t(planes)};
-    cuuint64_t strides[2] = {128, 128 * 64};
-    cuuint32_t box[3] = {128, cuuint32_t(m & 1 ? 32 : 64), cuuint32_t(m < 2 ? ns : nhi)};
+    cuuint64_t dims[3] = {128, cuuint64_t(cores), cuuint64_t(planes)};
+    cuuint64_t strides[2] = {128, cuuint64_t(128 * cores)};
+    cuuint32_t box[3] = {128, cuuint32_t(m & 1 ? cores / 2 : cores), cuuint32_t(m < 2 ? ns : nhi)};
     cuuint32_t estr[3] = {1, 1, 1};
     CUresult e = g_encode_dig(&maps[m], CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(digits), dims, strides, box,
                               estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
@@ -485,13 +496,30 @@ void launch_digit_zero(const ProbDev* probs, const WorkItem* items, int n, cudaS
 void launch_digit_rowmax(const ProbDev* probs, const WorkItem* items, int n, cudaStream_t s) {
   if (n > 0) digit_rowmax_kernel<<<n, 256, 0, s>>>(probs, items);
 }
-void launch_digit_slice(const ProbDev* probs, const WorkItem* items, int n, cudaStream_t s) {
-  if (n > 0) digit_slice_kernel<kFp64Digits><<<n, 256, 0, s>>>(probs, items);
+void launch_digit_slice(int planes, const ProbDev* probs, const WorkItem* items, int n, cudaStream_t s) {
+  if (n <= 0) return;
+  switch (planes) {
+    case 3: digit_slice_kernel<3><<<n, 256, 0, s>>>(probs, items); break;
+    case 4: digit_slice_kernel<4><<<n, 256, 0, s>>>(probs, items); break;
+    case 5: digit_slice_kernel<5><<<n, 256, 0, s>>>(probs, items); break;
+    case 6: digit_slice_kernel<6><<<n, 256, 0, s>>>(probs, items); break;
+    default: digit_slice_kernel<7><<<n, 256, 0, s>>>(probs, items); break;
+  }
 }
-void launch_digit_syrk(const DigitItem* items, int n, int ny, cudaStream_t s) {
-  if (n > 0 && ny > 0)
-    digit_syrk_kernel<kFp64Digits><<<dim3(2 * n, ny), kDigThreads, DigCfg<kFp64Digits>::kSmem, s>>>(items);
+void launch_digit_syrk(int planes, const DigitItem* items, int n, int ny, cudaStream_t s) {
+  if (n <= 0 || ny <= 0) return;
+  switch (planes) {
+    case 3: syrk_ns<3>(items, n, ny, s); break;
+    case 4: syrk_ns<4>(items, n, ny, s); break;
+    case 5: syrk_ns<5>(items, n, ny, s); break;
+    case 6: syrk_ns<6>(items, n, ny, s); break;
+    default: syrk_ns<7>(items, n, ny, s); break;
+  }
 }
-cudaError_t prepare_digit_kernels() { return prepare_ns<kFp64Digits>(); }
+cudaError_t prepare_digit_kernels() {
+  for (cudaError_t e : {prepare_ns<3>(), prepare_ns<4>(), prepare_ns<5>(), prepare_ns<6>(), prepare_ns<7>()})
+    if (e != cudaSuccess) return e;
+  return cudaSuccess;
+}
 
 }  // namespace rigw

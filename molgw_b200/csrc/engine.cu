@@ -231,8 +231,7 @@ Dims dims_of(const Shape& sh, PlanMode mode) {
   d.npad = round_up(sh.naux, kPanel);
   d.npanel = d.npad / kPanel;
   d.nia = sh.nocc * sh.nvirt + sh.nocc2 * sh.nvirt2;
-  // the int8 tensor-core K tile is 128 transitions (128 bytes), the bf16 one 64
-  d.nia_pad = round_up(std::max(d.nia, 1), is_ozaki(sh.precision) ? 128 : 64);
+  d.nia_pad = round_up(std::max(d.nia, 1), 64);   // one k-tile of the tensor-core operands
   d.want_identity =
       (mode == kPlanPolar || ((mode == kPlanFused || mode == kPlanPartial) && !sh.qp_only)) ? 1 : 0;
   d.moff = d.want_identity ? d.npad : 0;
@@ -256,18 +255,23 @@ bool use_digits(const Shape& sh) {
          (long long)sh.nocc * sh.nvirt + (long long)sh.nocc2 * sh.nvirt2 >= 512;
 }
 
-// Bytes of one frequency's split operands (bf16 hi/lo, or the Ozaki slices).
+int operand_planes(const Shape& sh) {
+  if (sh.precision == RIGW_BF16X3) return 2;
+  if (is_ozaki(sh.precision)) return ozaki_slices(sh.precision);
+  return use_digits(sh) ? kFp64Digits : 0;
+}
+
+// Bytes of one frequency's split operands (bf16 hi/lo, or the digits).
 size_t split_bytes_per_frequency(const Shape& sh) {
-  if (sh.precision == RIGW_FP64) return 0;
+  const int planes = operand_planes(sh);
   const int npad = round_up(sh.naux, kPanel);
-  const int nia = sh.nocc * sh.nvirt + sh.nocc2 * sh.nvirt2;
-  const int nia_pad = round_up(std::max(nia, 1), is_ozaki(sh.precision) ? 128 : 64);
-  return size_t(npad) * nia_pad * (is_ozaki(sh.precision) ? ozaki_slices(sh.precision) : 4);
+  const int nia_pad = round_up(std::max(sh.nocc * sh.nvirt + sh.nocc2 * sh.nvirt2, 1), 64);
+  return size_t(npad) * nia_pad * planes * (planes == 2 ? 2 : 1);
 }
 
 namespace {
 
-// Transitions per item of the split / slice / row-max kernels: wide items for
+// Transitions per item of the row-maximum kernel: wide items for
 // large problems (fewer items to build), 64 otherwise (enough CTAs to fill the GPU).
 int split_item_t(const Dims& d) { return (size_t(d.nia_pad / 64) * (d.npad / 64) >= 8192) ? kSplitT : 64; }
 
@@ -328,29 +332,22 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
   // Split precision: when the hi/lo buffers of every frequency of the batch are
   // small, one group holds all frequencies (one split and one tensor-core launch
   // with a full grid); otherwise groups of kSplitGroup frequencies share a buffer.
-  // bytes of the split operands of one frequency: bf16 hi/lo, slices, or FP64 digits
-  auto split_per_w = [&](const Shape& sh) -> size_t {
-    const Dims d = dims_of(sh, mode);
-    const int per = sh.precision == RIGW_FP64 ? (use_digits(sh) ? kFp64Digits : 0)
-                                              : (is_ozaki(sh.precision) ? ozaki_slices(sh.precision) : 4);
-    return size_t(d.npad) * d.nia_pad * per;
-  };
   size_t split_all = 0;
   for (const Shape& sh : shapes)
-    if (factor) split_all += size_t(sh.nomega) * split_per_w(sh);
+    if (factor) split_all += size_t(sh.nomega) * split_bytes_per_frequency(sh);
   const bool split_whole = split_all <= kSplitWholeBytes;
   auto split_group = [&](const Shape& sh) {
     if (tune_.split_group > 0) return std::max(1, std::min(sh.nomega, tune_.split_group));
     if (split_whole) return std::max(1, sh.nomega);
     // at most kSplitGroup frequencies, and at most kSplitProblemBytes per problem
-    const int cap = int(std::max<size_t>(1, kSplitProblemBytes / std::max<size_t>(split_per_w(sh), 1)));
+    const int cap = int(std::max<size_t>(1, kSplitProblemBytes / std::max<size_t>(split_bytes_per_frequency(sh), 1)));
     return std::max(1, std::min({sh.nomega, kSplitGroup, cap}));
   };
 
   // ---- memory layout
   Layout L;
   struct Off {
-    size_t mp, xs, tmap, rmax, dmax, xexp, tnorm, dscale, eps, winv, logdet, rhs, colsq, mnorm, vchiv, ew, tr, en, sc, sr, qp;
+    size_t mp, xs, tmap, dmax, xexp, tnorm, dscale, eps, winv, logdet, rhs, colsq, mnorm, vchiv, ew, tr, en, sc, sr, qp;
   };
   std::vector<Off> off(np);
   for (int i = 0; i < np; ++i) {
@@ -373,21 +370,15 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
       pp.off_in_omega = L.take(size_t(sh.nomega) * D);
       pp.off_in_weight = L.take(size_t(sh.nomega) * D);
       off[i].mp = L.take(size_t(d.nia_pad) * d.npad * D);
-      if (use_digits(sh)) {
-        off[i].xs = L.take(size_t(1 + split_group(sh)) * split_per_w(sh));
+      if (const int planes = operand_planes(sh)) {
+        off[i].xs = L.take(size_t((planes > 2) + split_group(sh)) * split_bytes_per_frequency(sh));
         off[i].tmap = L.take(512);
-        off[i].dmax = L.take(size_t(1 + sh.nomega) * d.npad * sizeof(unsigned));
-        off[i].xexp = L.take(size_t(1 + sh.nomega) * d.npad * sizeof(int));
-      } else if (sh.precision == RIGW_FP64) {
+        if (planes > 2) {
+          off[i].dmax = L.take(size_t(1 + sh.nomega) * d.npad * sizeof(unsigned));
+          off[i].xexp = L.take(size_t(1 + sh.nomega) * d.npad * sizeof(int));
+        }
+      } else {
         off[i].tmap = L.take(256);   // tensor maps of mp and dscale (TMA-staged FP64 chi0)
-      } else if (sh.precision == RIGW_BF16X3) {
-        off[i].xs = L.take(size_t(split_group(sh)) * 2 * d.npad * d.nia_pad * 2);
-        off[i].tmap = L.take(128);
-      } else if (is_ozaki(sh.precision)) {
-        off[i].xs = L.take(size_t(split_group(sh)) * ozaki_slices(sh.precision) * d.npad * d.nia_pad);
-        off[i].tmap = L.take(128);
-        off[i].rmax = L.take(size_t(sh.nomega) * d.npad * sizeof(unsigned long long));
-        off[i].xexp = L.take(size_t(sh.nomega) * d.npad * sizeof(int));
       }
       off[i].tnorm = L.take(size_t(d.nia_pad) * D);
       off[i].dscale = L.take(size_t(sh.nomega) * d.nia_pad * D);
@@ -435,11 +426,12 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
       lists += size_t(kMaxChains + 1) * t * sizeof(GemmItem) +
                size_t(sh.nomega) * (d.npanel + 8) * sizeof(WorkItem) +
                size_t(d.nia_pad / 8 + d.npad * d.ldb / 1024 + 64) * 16;
-      if (sh.precision != RIGW_FP64 || use_digits(sh)) {   // split items: (group, split_t transitions, 64 aux), + row maxima
+      if (operand_planes(sh)) {   // planes per (group, k-tile, row block), row maxima, products
         const int g = split_group(sh);
-        lists += size_t((sh.nomega + g - 1) / g + 1) * (d.nia_pad / split_item_t(d) + 1) * (d.npad / 64) *
-                     sizeof(WorkItem) +
-                 size_t(sh.nomega) * d.npad / 4096 * sizeof(WorkItem) + 64;
+        const size_t groups = size_t(sh.nomega + g - 1) / g;
+        lists += (groups + 2) * (d.nia_pad / 64) * d.npanel * sizeof(WorkItem) +
+                 (size_t(1 + sh.nomega) * d.npad / 4096 + 1) * sizeof(WorkItem) +
+                 groups * (d.npanel / 2 + 1) * d.npanel * sizeof(DigitItem);
       }
     }
     *measure_only = L.cur + lists + (size_t(1) << 20);
@@ -479,35 +471,22 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
     p.want_identity = d.want_identity;
     if (factor) {
       p.mp = dp(off[i].mp);
-      p.kpad = d.nia_pad;
       p.wgroup = split_group(sh);
+      p.signed_d = sh.precision == RIGW_FP64;
       p.split_t = split_item_t(d);
-      if (sh.precision == RIGW_BF16X3) {
-        p.xs = base + off[i].xs;
-        alignas(64) unsigned char map[128];
-        RIGW_TRY(make_split_tmap(map, p.xs, d.nia_pad, (long long)p.wgroup * 2 * d.npad));
-        RIGW_CUDA_TRY(cudaMemcpyAsync(base + off[i].tmap, map, sizeof(map), cudaMemcpyHostToDevice, ctx->stream));
-      } else if (is_ozaki(sh.precision)) {
-        p.slices = ozaki_slices(sh.precision);
-        p.xs = base + off[i].xs;
-        p.rmax = reinterpret_cast<unsigned long long*>(base + off[i].rmax);
-        p.xexp = reinterpret_cast<int*>(base + off[i].xexp);
-        alignas(64) unsigned char map[128];
-        RIGW_TRY(make_ozaki_tmap(map, p.xs, d.nia_pad, (long long)p.wgroup * p.slices * d.npad,
-                                 p.slices <= kOzaFusedMaxSlices ? 64 : 128));
-        RIGW_CUDA_TRY(cudaMemcpyAsync(base + off[i].tmap, map, sizeof(map), cudaMemcpyHostToDevice, ctx->stream));
-      }
       p.tnorm = dp(off[i].tnorm);
       p.dscale = dp(off[i].dscale);
-      if (use_digits(sh)) {
+      if (const int planes = operand_planes(sh)) {
         p.xs = base + off[i].xs;
-        p.dmax = reinterpret_cast<unsigned*>(base + off[i].dmax);
-        p.xexp = reinterpret_cast<int*>(base + off[i].xexp);
+        if (planes > 2) {
+          p.dmax = reinterpret_cast<unsigned*>(base + off[i].dmax);
+          p.xexp = reinterpret_cast<int*>(base + off[i].xexp);
+        }
         alignas(64) unsigned char maps[512];
-        RIGW_TRY(make_digit_tmaps(maps, p.xs,
-                                  (long long)(1 + p.wgroup) * d.npanel * (d.nia_pad / 64) * kFp64Digits, kFp64Digits));
+        RIGW_TRY(make_digit_tmaps(maps, p.xs, (long long)((planes > 2) + p.wgroup) * d.npanel * (d.nia_pad / 64) * planes, planes,
+                                  planes == 2 ? 128 : 64));
         RIGW_CUDA_TRY(cudaMemcpyAsync(base + off[i].tmap, maps, sizeof(maps), cudaMemcpyHostToDevice, ctx->stream));
-      } else if (sh.precision == RIGW_FP64) {
+      } else {
         alignas(64) unsigned char maps[256];
         RIGW_TRY(make_f64_tmaps(maps, p.mp, d.npad, d.nia_pad, p.dscale, sh.nomega));
         RIGW_CUDA_TRY(cudaMemcpyAsync(base + off[i].tmap, maps, sizeof(maps), cudaMemcpyHostToDevice, ctx->stream));
@@ -574,92 +553,27 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
     const int npad = p.npad, ldb = p.ldb;
     if (factor) {
       for (int t0 = 0; t0 < p.nia_pad; t0 += 8) wl_pack_.push_back({i, t0, 0, 0});
-      if (sh.precision == RIGW_BF16X3) {
-        // frequencies in groups of p.wgroup sharing one hi/lo buffer: split(g), then chi0(g)
-        for (int w0 = 0, g = 0; w0 < sh.nomega; w0 += p.wgroup, ++g) {
-          if (int(wl_split_.size()) <= g) {
-            wl_split_.resize(g + 1);
-            tl_syrk_.resize(g + 1);
-          }
-          for (int t0 = 0; t0 < p.nia_pad; t0 += p.split_t)
-            for (int p0 = 0; p0 < npad; p0 += 64) wl_split_[g].push_back({i, t0, p0, w0});
-        }
-        // one item per (group, tile) covering the group's frequencies
-        for (int w0 = 0; w0 < sh.nomega; w0 += p.wgroup)
-          for (int ti = 0; ti < npad; ti += BMN)
-            for (int tj = ti; tj < npad; tj += BMN) {
-              TcItem t{};
-              t.tmap = base + off[i].tmap;
-              t.C = p.eps + size_t(w0) * npad * npad + size_t(ti) * npad + tj;
-              t.err = err_dev_;
-              t.row_a = ti;
-              t.row_b = tj;
-              t.lo_off = npad;
-              t.ktiles = p.kpad / 64;
-              t.ldc = npad;
-              t.diag = ti - tj;
-              t.nw = std::min(p.wgroup, sh.nomega - w0);
-              t.sC = (long long)npad * npad;
-              t.srow = 2 * npad;
-              tl_syrk_[w0 / p.wgroup].push_back(t);
-            }
-      }
-      // FP64 chi0: upper 128-wide column strips in 64-row items (two CTAs per SM),
-      // over the naux x naux block only; the identity pads are written afterwards
-      if (is_ozaki(sh.precision)) {
-        // row maxima of S over every frequency, then per frequency group: slices, chi0
-        for (size_t e = 0; e < size_t(sh.nomega) * npad; e += 4096) wl_ozzero_.push_back({i, int(e), 0, 0});
-        for (int t0 = 0; t0 < p.nia_pad; t0 += p.split_t)
-          for (int p0 = 0; p0 < npad; p0 += 64) wl_rowmax_.push_back({i, t0, p0, 0});
-        for (int w0 = 0, g = 0; w0 < sh.nomega; w0 += p.wgroup, ++g) {
-          if (int(wl_slice_.size()) <= g) {
-            wl_slice_.resize(g + 1);
-            tl_ozaki_.resize(g + 1);
-            tl_ozaki4_.resize(g + 1);
-          }
-          for (int t0 = 0; t0 < p.nia_pad; t0 += p.split_t)
-            for (int p0 = 0; p0 < npad; p0 += 64) wl_slice_[g].push_back({i, t0, p0, w0});
-        }
-        for (int w0 = 0; w0 < sh.nomega; w0 += p.wgroup)
-          for (int ti = 0; ti < npad; ti += BMN)
-            for (int tj = ti; tj < npad; tj += BMN) {
-              TcItem t{};
-              t.tmap = base + off[i].tmap;
-              t.C = p.eps + size_t(w0) * npad * npad + size_t(ti) * npad + tj;
-              t.err = err_dev_;
-              t.row_a = ti;
-              t.row_b = tj;
-              t.lo_off = npad;
-              const bool fused = p.slices <= kOzaFusedMaxSlices;
-              t.ktiles = p.kpad / (fused ? 64 : 128);
-              t.ldc = npad;
-              t.diag = ti - tj;
-              t.ea = p.xexp + size_t(w0) * npad + ti;
-              t.eb = p.xexp + size_t(w0) * npad + tj;
-              t.slices = p.slices;
-              t.nw = std::min(p.wgroup, sh.nomega - w0);
-              t.sC = (long long)npad * npad;
-              t.srow = p.slices * npad;
-              t.se = npad;
-              (fused ? tl_ozaki4_ : tl_ozaki_)[w0 / p.wgroup].push_back(t);
-            }
-      }
-      if (use_digits(sh)) {
-        // row maxima of M and of M D_w for every frequency, the digits of M, then per
-        // frequency group the digits of M D_w and the products
+      if (const int planes = operand_planes(sh)) {
+        // per frequency group the planes of M sqrt(D_w) (bf16) or M D_w (digits; before the first
+        // group those of M, and the row maxima of all of them), then the products
         const int nkt = p.nia_pad / 64;
-        for (size_t e = 0; e < size_t(1 + sh.nomega) * npad; e += 4096) wl_dzero_.push_back({i, int(e), 0, 0});
-        for (int t0 = 0; t0 < p.nia_pad; t0 += p.split_t)
-          for (int rb = 0; rb < p.npanel; ++rb) wl_dmax_.push_back({i, t0, rb, 0});
-        for (int rb = 0; rb < p.npanel; ++rb)
-          for (int kt = 0; kt < nkt; ++kt) wl_dbase_.push_back({i, kt, rb, -1});
+        if (planes > 2) {
+          for (size_t e = 0; e < size_t(1 + sh.nomega) * npad; e += 4096) wl_dzero_.push_back({i, int(e), 0, 0});
+          for (int t0 = 0; t0 < p.nia_pad; t0 += p.split_t)
+            for (int rb = 0; rb < p.npanel; ++rb) wl_dmax_.push_back({i, t0, rb, 0});
+        }
+        auto& slices = wl_slice_[planes];
+        auto& products = dl_syrk_[planes];
         for (int w0 = 0, g = 0; w0 < sh.nomega; w0 += p.wgroup, ++g) {
-          if (int(wl_dslice_.size()) <= g) {
-            wl_dslice_.resize(g + 1);
-            dl_syrk_.resize(g + 1);
+          if (int(slices.size()) <= g) {
+            slices.resize(g + 1);
+            products.resize(g + 1);
           }
           for (int rb = 0; rb < p.npanel; ++rb)
-            for (int kt = 0; kt < nkt; ++kt) wl_dslice_[g].push_back({i, kt, rb, w0});
+            for (int kt = 0; kt < nkt; ++kt) {
+              slices[g].push_back({i, kt, rb, w0});
+              if (g == 0 && planes > 2) slices[g].push_back({i, kt, rb, -1});
+            }
           for (int ra = 0; ra < p.npanel; ra += 2)
             for (int cb = ra; cb < p.npanel; ++cb) {
               DigitItem t{};
@@ -671,16 +585,16 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
               t.rb_b = cb;
               t.nrb = p.npanel;
               t.nkt = nkt;
-              t.slab_a = 1;
+              t.slab_a = planes > 2;
               t.slab_b = 0;
               t.slab_e = 1 + w0;
               t.ld = npad;
               t.nw = std::min(p.wgroup, sh.nomega - w0);
               t.sC = (long long)npad * npad;
-              dl_syrk_[g].push_back(t);
+              products[g].push_back(t);
             }
         }
-      } else if (sh.precision == RIGW_FP64) {
+      } else {
         // one item per tile covering every frequency (blockIdx.y); the tiles of a
         // row block start at its diagonal, so only the lower half of the
         // diagonal BMC x BMC block lies below it, and end at naux
@@ -851,15 +765,9 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
   std::stable_sort(gl_syrk_.begin(), gl_syrk_.end(), [](const GemmItem& a, const GemmItem& b) {
     return double(a.k) * a.m * a.n * std::max(a.nw, 1) > double(b.k) * b.m * b.n * std::max(b.nw, 1);
   });
-  auto by_cost = [](const TcItem& a, const TcItem& b) {
-    return double(a.ktiles) * std::max(a.nw, 1) > double(b.ktiles) * std::max(b.nw, 1);
-  };
-  for (auto& l : tl_syrk_) std::stable_sort(l.begin(), l.end(), by_cost);
-  for (auto& l : tl_ozaki_) std::stable_sort(l.begin(), l.end(), by_cost);
-  for (auto& l : tl_ozaki4_) std::stable_sort(l.begin(), l.end(), by_cost);
-
-  for (auto& l : dl_syrk_)
-    std::stable_sort(l.begin(), l.end(), [](const DigitItem& a, const DigitItem& b) { return a.nkt > b.nkt; });
+  for (auto& planes : dl_syrk_)
+    for (auto& l : planes)
+      std::stable_sort(l.begin(), l.end(), [](const DigitItem& a, const DigitItem& b) { return a.nkt > b.nkt; });
 
   // ---- upload the lists and the launch sequence
   size_t lbytes = 0;
@@ -885,8 +793,6 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
     int ny = 1;
     if (kind == 1 || kind == 5 || kind == 6 || kind == 14)
       for (size_t j = 0; j < n; ++j) ny = std::max(ny, static_cast<const GemmItem*>(src)[j].nw);
-    if (kind == 13 || kind == 20 || kind == 21)
-      for (size_t j = 0; j < n; ++j) ny = std::max(ny, static_cast<const TcItem*>(src)[j].nw);
     if (kind == 26)
       for (size_t j = 0; j < n; ++j) ny = std::max(ny, static_cast<const DigitItem*>(src)[j].nw);
     if (kind == 22)
@@ -899,23 +805,13 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
   add(3, wl_mnorm_.data(), sizeof(WorkItem), wl_mnorm_.size(), 0);
   add(1, gl_syrk_.data(), sizeof(GemmItem), gl_syrk_.size(), 0);
   add(22, fl_syrk_.data(), sizeof(F64SyrkItem), fl_syrk_.size(), 0);
-  for (size_t g = 0; g < wl_split_.size(); ++g) {
-    add(12, wl_split_[g].data(), sizeof(WorkItem), wl_split_[g].size(), 0);
-    add(13, tl_syrk_[g].data(), sizeof(TcItem), tl_syrk_[g].size(), 0);
-  }
   add(23, wl_dzero_.data(), sizeof(WorkItem), wl_dzero_.size(), 0);
   add(24, wl_dmax_.data(), sizeof(WorkItem), wl_dmax_.size(), 0);
-  add(25, wl_dbase_.data(), sizeof(WorkItem), wl_dbase_.size(), 0);
-  for (size_t g = 0; g < wl_dslice_.size(); ++g) {
-    add(25, wl_dslice_[g].data(), sizeof(WorkItem), wl_dslice_[g].size(), 0);
-    add(26, dl_syrk_[g].data(), sizeof(DigitItem), dl_syrk_[g].size(), 0);
-  }
-  add(17, wl_ozzero_.data(), sizeof(WorkItem), wl_ozzero_.size(), 0);
-  add(18, wl_rowmax_.data(), sizeof(WorkItem), wl_rowmax_.size(), 0);
-  for (size_t g = 0; g < wl_slice_.size(); ++g) {
-    add(19, wl_slice_[g].data(), sizeof(WorkItem), wl_slice_[g].size(), 0);
-    add(20, tl_ozaki_[g].data(), sizeof(TcItem), tl_ozaki_[g].size(), 0);
-    add(21, tl_ozaki4_[g].data(), sizeof(TcItem), tl_ozaki4_[g].size(), 0);
+  for (int np2 = 2; np2 < 8; ++np2) {
+    for (size_t g = 0; g < wl_slice_[np2].size(); ++g) {
+      add(25, wl_slice_[np2][g].data(), sizeof(WorkItem), wl_slice_[np2][g].size(), np2);
+      add(26, dl_syrk_[np2][g].data(), sizeof(DigitItem), dl_syrk_[np2][g].size(), np2);
+    }
   }
   add(16, wl_pad_.data(), sizeof(WorkItem), wl_pad_.size(), 0);
   add(15, wl_trace_.data(), sizeof(WorkItem), wl_trace_.size(), 0);
@@ -998,8 +894,7 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
 static int stage_of(int kind) {
   switch (kind) {
     case 0: case 2: case 3: return 0;
-    case 1: case 12: case 13: case 15: case 16: case 17: case 18: case 19: case 20: case 21: case 22:
-    case 23: case 24: case 25: case 26: return 1;
+    case 1: case 15: case 16: case 22: case 23: case 24: case 25: case 26: return 1;
     case -1: case 4: case 5: case 6: case 14: return 2;
     default: return 3;
   }
@@ -1029,18 +924,19 @@ void Plan::record(cudaStream_t s0, int stage) {
         break;
       case 15: trace_kernel<<<L.count, 256, 0, s>>>(probs_dev_, wl); break;
       case 16: pad_eps_kernel<<<L.count, 256, 0, s>>>(probs_dev_, wl); break;
-      case 12: launch_split_bf16x3(probs_dev_, wl, L.count, s); break;
-      case 13: launch_syrk_bf16x3(reinterpret_cast<const TcItem*>(lb + L.off), L.count, L.ny, s); break;
       case 22: launch_syrk_f64_tma(reinterpret_cast<const F64SyrkItem*>(lb + L.off), L.count, L.ny, s); break;
       case 23: launch_digit_zero(probs_dev_, wl, L.count, s); break;
+      case 25:
+        if (L.arg == 2) launch_split_bf16(probs_dev_, wl, L.count, s);
+        else launch_digit_slice(L.arg, probs_dev_, wl, L.count, s);
+        break;
+      case 26: {
+        const DigitItem* dl = reinterpret_cast<const DigitItem*>(lb + L.off);
+        if (L.arg == 2) launch_split_syrk(dl, L.count, L.ny, s);
+        else launch_digit_syrk(L.arg, dl, L.count, L.ny, s);
+        break;
+      }
       case 24: launch_digit_rowmax(probs_dev_, wl, L.count, s); break;
-      case 25: launch_digit_slice(probs_dev_, wl, L.count, s); break;
-      case 26: launch_digit_syrk(reinterpret_cast<const DigitItem*>(lb + L.off), L.count, L.ny, s); break;
-      case 17: launch_ozaki_zero(probs_dev_, wl, L.count, s); break;
-      case 18: launch_ozaki_rowmax(probs_dev_, wl, L.count, s); break;
-      case 19: launch_ozaki_slice(probs_dev_, wl, L.count, s); break;
-      case 20: launch_syrk_ozaki(reinterpret_cast<const TcItem*>(lb + L.off), L.count, L.ny, s); break;
-      case 21: launch_syrk_ozaki_fused(reinterpret_cast<const TcItem*>(lb + L.off), L.count, L.ny, s); break;
       case 2: init_rhs_kernel<<<L.count, 256, 0, s>>>(probs_dev_, wl); break;
       case 3: mnorm_kernel<<<L.count, 256, 0, s>>>(probs_dev_, wl); break;
       case 4: chol_diag_kernel<<<L.count, kDiagThreads, chol_diag_smem_bytes(), s>>>(probs_dev_, wl, L.arg); break;

@@ -108,7 +108,9 @@ struct Tuning {
 int precision_class(const std::vector<Shape>& shapes);
 // Whether the FP64 chi0 of a problem goes through the int8 digit products.
 bool use_digits(const Shape& sh);
-// Bytes of one frequency's split operands of a problem (0 for FP64).
+// Planes of the chi0 operands: 2 (bf16 hi/lo), 3 .. 7 (int8 digits), 0 (FP64 on DMMA).
+int operand_planes(const Shape& sh);
+// Bytes of one frequency's split operands of a problem (0 for FP64 on DMMA).
 size_t split_bytes_per_frequency(const Shape& sh);
 
 enum PlanMode : int {
@@ -172,14 +174,10 @@ class Plan {
   std::vector<std::vector<WorkItem>> wl_diag_;
   std::vector<GemmItem> gl_syrk_;
   std::vector<F64SyrkItem> fl_syrk_;              // FP64 chi0, TMA-staged (64-row items)
-  std::vector<std::vector<WorkItem>> wl_split_;   // per frequency group
-  std::vector<std::vector<TcItem>> tl_syrk_;
-  std::vector<WorkItem> wl_ozzero_, wl_rowmax_;    // Ozaki: row maxima over every frequency
-  std::vector<std::vector<WorkItem>> wl_slice_;   // Ozaki: per frequency group
-  std::vector<WorkItem> wl_dzero_, wl_dmax_, wl_dbase_;   // FP64 digits: row maxima, digits of M
-  std::vector<std::vector<WorkItem>> wl_dslice_;          // FP64 digits: per frequency group
-  std::vector<std::vector<DigitItem>> dl_syrk_;
-  std::vector<std::vector<TcItem>> tl_ozaki_, tl_ozaki4_;   // s >= 5 / s <= 4 (fused slice pairs)
+  std::vector<WorkItem> wl_dzero_, wl_dmax_;               // digits: row maxima
+  // chi0 on tcgen05, by the number of operand planes (2: bf16, 3 .. 7: digits)
+  std::vector<std::vector<WorkItem>> wl_slice_[8];         // per frequency group: planes of M D_w (first: and of M)
+  std::vector<std::vector<DigitItem>> dl_syrk_[8];         // and the products
   std::vector<std::vector<GemmItem>> gl_k2_, gl_k2n_, gl_k3_, gl_k3d_, gl_k3a_;
   std::vector<WorkItem> wl_trace_, wl_pad_;
   struct Launch {
@@ -302,9 +300,9 @@ Status make_split_tmap(void* host_map, const void* xs, int kpad, long long rows)
 // The two tensor maps of the TMA-staged FP64 chi0 (256 bytes at host_maps):
 // mp [nia_pad][npad] in 16 x 16 boxes with 128-byte swizzle, dscale [nomega][nia_pad] in 16 x 1 boxes.
 Status make_f64_tmaps(void* host_maps, const double* mp, int npad, int nia_pad, const double* dscale, int nomega);
-// The four tensor maps (512 bytes) of a digit array of `planes` digit planes (digit_gemm.cu).
-Status make_digit_tmaps(void* host_maps, const void* digits, long long planes, int ns);
-// box_bytes 128: 128-byte swizzle (syrk_ozaki_kernel); 64: 64-byte swizzle (syrk_ozaki_fused_kernel)
-Status make_ozaki_tmap(void* host_map, const void* xq, int kpad, long long rows, int box_bytes = 128);
+// The four tensor maps (512 bytes) of `planes` operand planes, ns per tile, of `cores` core
+// matrices (digit_gemm.cu).
+Status make_digit_tmaps(void* host_maps, const void* digits, long long planes, int ns, int cores);
+Status make_ozaki_tmap(void* host_map, const void* xq, int kpad, long long rows);
 
 }  // namespace rigw

@@ -35,32 +35,22 @@ struct AomoUnpackItem {
 };
 __global__ void aomo_unpack_kernel(const AomoUnpackItem* items);
 
-// Split-precision chi0 (syrk_bf16x3.cu): one 128x128 upper tile of eps(iw).
+// One 128 x 128 tile of a general tensor-core product A B^T of the AO->MO transform
+// (syrk_bf16x3.cu, syrk_ozaki.cu).
 struct TcItem {
-  const void* tmap;   // CUtensorMap of the problem's hi/lo tensor (rows: [wgroup][2][npad], cols: kpad)
-  double* C;          // &eps[w][i0][j0]
+  const void* tmap;     // CUtensorMap of A: rows of 128 bytes along K
+  const void* tmap_b;   // of B
+  double* C;
   int* err;
-  int row_a, row_b;   // tensor rows of the hi blocks of the A (i0) and B (j0) operands
-  int lo_off;         // rows from a hi block to its lo block (npad)
-  int ktiles;         // kpad / 64
-  int ldc;            // npad
-  int diag;           // i0 - j0: identity where (col - row) == diag
-  // Ozaki INT8 (syrk_ozaki.cu): row_a/row_b address slice 1, lo_off is the row
-  // distance between slices, ktiles = kpad / 128
-  const int* ea;      // row exponents of the A rows (e_p, p = i0 ..)
-  const int* eb;      // row exponents of the B rows (e_q, q = j0 ..)
+  int row_a, row_b;     // tensor rows of the hi planes (Ozaki: first slices)
+  int lo_off, lo_off_b; // rows from a plane to the next
+  int ktiles;           // k-tiles of 64 bf16 or 128 int8
+  int ldc;
+  const int* ea;        // Ozaki: row exponents of A and B
+  const int* eb;
   int slices;
-  // The item covers nw frequencies (nw <= 0: one): CTA (item, j) (blockIdx.y = j < nw) uses
-  // C + j*sC, tensor rows row_a/row_b + j*srow, exponents ea/eb + j*se.
-  long long sC, se;
-  int srow, nw;
-  // General products: B from its own tensor map (nullptr: the A map) whose lo
-  // rows (Ozaki: next slice) are lo_off_b below the hi rows (first slice); only
-  // the first mrows x ncols of the tile are stored, without identity (0: all 128).
-  const void* tmap_b;
-  int lo_off_b, mrows, ncols;
+  int mrows, ncols;     // rows and columns stored
 };
-void launch_split_bf16x3(const ProbDev* probs, const WorkItem* items, int n, cudaStream_t s);
 // Split of a general FP64 operand into K-major bf16 hi/lo for the tensor-core
 // kernel: element (r, k) of batch z is src[z*zs_src + r*rs + k*ks]; dst holds
 // [2][Rpad][Kpad] per batch (hi rows, then lo rows), zero padded.
@@ -86,14 +76,8 @@ struct SliceOp {
   int* exps;
 };
 void launch_slice_kmajor(const SliceOp& op, cudaStream_t s);
-void launch_syrk_bf16x3(const TcItem* items, int n, int ny, cudaStream_t s);
-void launch_ozaki_zero(const ProbDev* probs, const WorkItem* items, int n, cudaStream_t s);
-void launch_ozaki_rowmax(const ProbDev* probs, const WorkItem* items, int n, cudaStream_t s);
-void launch_ozaki_slice(const ProbDev* probs, const WorkItem* items, int n, cudaStream_t s);
-void launch_syrk_ozaki(const TcItem* items, int n, int ny, cudaStream_t s);
-// s <= 4: every slice pair of a k-tile from one stage (64-byte swizzled tensor map)
-void launch_syrk_ozaki_fused(const TcItem* items, int n, int ny, cudaStream_t s);
-constexpr int kOzaFusedMaxSlices = 4;
+void launch_syrk_bf16x3(const TcItem* items, int n, cudaStream_t s);
+void launch_syrk_ozaki(const TcItem* items, int n, cudaStream_t s);
 cudaError_t prepare_ozaki_kernels();
 cudaError_t prepare_tc_kernels();
 
@@ -115,13 +99,15 @@ struct F64SyrkItem {
 void launch_syrk_f64_tma(const F64SyrkItem* items, int n, int ny, cudaStream_t s);
 cudaError_t prepare_syrk_f64_tma();
 
-// FP64 chi0 from exact int8 digit products (digit_gemm.cu): one 256 x 128 upper tile of
-// eps(iw) = 1 + (M D_w) M^T per pair of CTAs, frequency = blockIdx.y.
+// chi0 on the tcgen05 cores: one 256 x 128 upper tile of eps(iw) = 1 + M D_w M^T per pair of
+// CTAs, frequency = blockIdx.y.  The operands are planes of M and M D_w, 3 to 7 int8 digits
+// (digit_gemm.cu; FP64: 7, RIGW_OZAKI(s): s), or the two bf16 parts of M sqrt(D_w) on both
+// sides (syrk_bf16x3.cu; slab_b and exps unused).
 struct DigitItem {
-  const void* maps;     // four CUtensorMaps of the problem's digit array (make_digit_tmaps)
+  const void* maps;     // CUtensorMaps of the problem's planes (make_digit_tmaps)
   double* C;            // &eps[w0][0][0]
   int* err;
-  const int* exps;      // row exponents: [0][ld] of M, [1 + w][ld] of M D_w
+  const int* exps;      // digits, row exponents: [0][ld] of M, [1 + w][ld] of M D_w
   int rb_a, rb_b;       // 128-row blocks: output rows from 128 rb_a (two blocks), columns from 128 rb_b
   int nrb, nkt;         // row blocks and k-tiles (64 transitions) of a slab
   int slab_a, slab_b;   // slab of M D_w for j = 0 (+ j), slab of M
@@ -131,8 +117,11 @@ struct DigitItem {
 };
 void launch_digit_zero(const ProbDev* probs, const WorkItem* items, int n, cudaStream_t s);
 void launch_digit_rowmax(const ProbDev* probs, const WorkItem* items, int n, cudaStream_t s);
-void launch_digit_slice(const ProbDev* probs, const WorkItem* items, int n, cudaStream_t s);
-void launch_digit_syrk(const DigitItem* items, int n, int ny, cudaStream_t s);
+// planes: digits per operand, 3 .. 7
+void launch_digit_slice(int planes, const ProbDev* probs, const WorkItem* items, int n, cudaStream_t s);
+void launch_digit_syrk(int planes, const DigitItem* items, int n, int ny, cudaStream_t s);
+void launch_split_bf16(const ProbDev* probs, const WorkItem* items, int n, cudaStream_t s);
+void launch_split_syrk(const DigitItem* items, int n, int ny, cudaStream_t s);
 cudaError_t prepare_digit_kernels();
 
 // Host-side launchers of the DMMA tile engine (gemm_f64.cu).

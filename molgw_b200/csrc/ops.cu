@@ -109,9 +109,9 @@ Status run_tc_items(Context& c, const std::vector<TcItem>& items, bool ozaki = f
   RIGW_CUDA_TRY(cudaMemcpyAsync(buf.data(), items.data(), items.size() * sizeof(TcItem), cudaMemcpyHostToDevice,
                                 c.stream));
   if (ozaki)
-    launch_syrk_ozaki(reinterpret_cast<const TcItem*>(buf.data()), int(items.size()), 1, c.stream);
+    launch_syrk_ozaki(reinterpret_cast<const TcItem*>(buf.data()), int(items.size()), c.stream);
   else
-    launch_syrk_bf16x3(reinterpret_cast<const TcItem*>(buf.data()), int(items.size()), 1, c.stream);
+    launch_syrk_bf16x3(reinterpret_cast<const TcItem*>(buf.data()), int(items.size()), c.stream);
   RIGW_CUDA_TRY(cudaGetLastError());
   return c.sync(c.stream);
 }
@@ -257,7 +257,6 @@ Status eri_3center_mo(Context& c, int nbf, int nstate, int npair, int naux, cons
           t.mrows = std::min(128, ncp - i0);
           t.ncols = std::min(128, wide - j0);
           t.err = errp;
-          t.nw = 1;
           if (ns > 0) {
             t.slices = ns;
             t.ea = exps_of(e_a1, 1, Rp1) + i0;
@@ -289,8 +288,7 @@ Status eri_3center_mo(Context& c, int nbf, int nstate, int npair, int naux, cons
             t.mrows = std::min(128, mcp - i0);
             t.ncols = std::min(128, pcp - j0);
             t.err = errp;
-            t.nw = 1;
-            if (ns > 0) {
+              if (ns > 0) {
               t.slices = ns;
               t.ea = exps_of(e_a2, 1, Rp2) + i0;
               t.eb = exps_of(e_b2, nc, Rpp) + size_t(n) * Rpp + j0;

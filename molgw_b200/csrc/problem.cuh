@@ -52,16 +52,13 @@ struct ProbDev {
   const double* zcalc;       // [nc] complex (re, im) evaluation points
   // ---- workspace (device)
   double* mp;
-  void* xs;                  // split precision: [wgroup][2][npad][kpad] bf16 hi/lo of M sqrt(D_w);
-                             // Ozaki: [wgroup][slices][npad][kpad] int8 slices of M sqrt(D_w) 2^-e
-                             // FP64 digits: [1 + wgroup] slabs of int8 digits of M, then of M D_w
-  int kpad;                  // transitions padded to the tensor-core K tile (== nia_pad)
-  int wgroup;                // frequencies per split group (one buffer, reused group by group)
-  int slices;                // Ozaki slices (0: not Ozaki)
-  int split_t;               // transitions per item of the split / slice / row-max kernels
-  unsigned long long* rmax;  // Ozaki: [nomega][npad] max_t |S_pt| as double bits (atomicMax)
-  unsigned* dmax;            // FP64 digits: [1 + nomega][npad] high words of max_t |M_pt|, max_t |(M D_w)_pt|
-  int* xexp;                 // Ozaki: [nomega][npad] row exponents e_p; FP64 digits: [1 + nomega][npad]
+  void* xs;                  // chi0 operand planes (layout in digit_gemm.cu): int8 digits, [1 + wgroup]
+                             // slabs of M, then of M D_w; bf16 hi/lo, [wgroup] slabs of M sqrt(D_w)
+  int wgroup;                // frequencies per group (one set of slabs, reused group by group)
+  int signed_d;              // D_w(t) < 0 is taken (FP64); the split precisions refuse it
+  int split_t;               // transitions per item of the row-maximum kernel
+  unsigned* dmax;            // digits: [1 + nomega][npad] high words of max_t |M_pt|, max_t |(M D_w)_pt|
+  int* xexp;                 // digits: [1 + nomega][npad] row exponents
   double* tnorm;
   double* dscale;
   double* eps;

@@ -1,17 +1,15 @@
-// Split-precision chi0 contraction on the 5th-generation tensor cores.
+// Split-precision products on the 5th-generation tensor cores.
 //
-//   eps(iw) = 1 + S S^T,   S = M diag(sqrt(D_w)),   S = S_hi + S_lo  (bf16 hi/lo split)
+//   eps(iw) = 1 + S S^T,   S = M diag(sqrt(D_w)) = S_hi + S_lo  (bf16 hi/lo split)
 //   S S^T  ~=  S_hi S_hi^T + S_hi S_lo^T + S_lo S_hi^T     (fp32 accumulation in TMEM)
 //
-// split_bf16x3_kernel: per 64x64 tile of the packed FP64 tensor, scales by
-//   sqrt(D_w(t)) for every frequency and writes the hi/lo bf16 pair in the
-//   K-major (transition-contiguous) layout the tensor cores read.
-// syrk_bf16x3_kernel: one 128x128 upper tile of eps(iw) per CTA.  One thread
-//   issues TMA loads (4 tiles of 128 rows x 64 bf16 per stage, 128-byte
-//   swizzle) into a 3-stage ring, one thread issues tcgen05.mma (M=128, N=128,
-//   K=16; 12 per stage) into two ping-pong TMEM accumulators, eight warps drain
-//   them chunk by chunk into FP64, add the identity and store.  All mbarrier
-//   waits are bounded.
+// split_bf16_kernel: scales the packed FP64 tensor by sqrt(D_w(t)) for every frequency of a
+//   group and writes the hi/lo pair in the order in which the tensor cores read it
+//   (8 x 16-byte core matrices, as digit_gemm.cu).
+// split_syrk_kernel: one 256 x 128 upper tile of eps(iw) per pair of CTAs (cta_group::2).
+// split_kmajor_kernel, syrk_bf16x3_kernel: the general products of the AO->MO transform,
+//   one 128 x 128 tile per CTA from K-major operands (128-byte swizzle).
+// All mbarrier waits are bounded.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cudaTypedefs.h>
@@ -26,50 +24,59 @@ constexpr int kTcTileBytes = 128 * 64 * 2;
 constexpr int kTcStageBytes = 4 * kTcTileBytes;
 constexpr size_t kTcSmemBytes = size_t(kTcStages) * kTcStageBytes + 1024 + 256;
 
-// item: (prob, t0, p0, w0): split_t transitions from t0 x 64 rows from p0, the
-// frequencies w0 .. w0+wgroup-1; 256 threads.
-__global__ void __launch_bounds__(256) split_bf16x3_kernel(const ProbDev* __restrict__ probs,
-                                                           const WorkItem* __restrict__ items) {
+// A bf16 value, as the bits of the float it is, in FP64.  Integer arithmetic: a conversion
+// instruction runs at a quarter of the FP64 rate, and three per entry bounded the kernel.  Exact
+// for normal values; below 2^-126 it is off by less than 2^-125, and a NaN or an infinity has
+// already gone into the high part.
+RIGW_DEVICE_INLINE double widen(uint32_t u) {
+  return __hiloint2double(int((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + 0x38000000u)), 0);
+}
+
+// item: (prob, k-tile, row block, w0): frequencies w0 .. w0 + wgroup - 1 into slabs 0 ...
+// Thread (row, half) keeps 32 entries of its row for all frequencies; a warp writes 32 rows
+// of one 16-byte chunk, four full lines.
+__global__ void __launch_bounds__(256) split_bf16_kernel(const ProbDev* __restrict__ probs,
+                                                         const WorkItem* __restrict__ items) {
   const WorkItem wi = items[blockIdx.x];
   const ProbDev& p = probs[wi.prob];
-  const int p0 = wi.b;
-  constexpr int kWb = 16;            // frequencies per block of scale factors
-  __shared__ double tile[64][65];   // [P][t]
-  __shared__ double sc[kWb][64];    // sqrt(D_w(t0 + t)) for kWb frequencies
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  __nv_bfloat16* xs = reinterpret_cast<__nv_bfloat16*>(p.xs);
-  const int w0 = wi.c, w1 = min(p.nomega, w0 + p.wgroup);   // this item's frequency group
-  const int tend = min(p.nia_pad, wi.a + p.split_t);
-  for (int t0 = wi.a; t0 < tend; t0 += 64) {               // 64-transition sub-tiles of the item
-    __syncthreads();
-    for (int idx = tid; idx < 64 * 64; idx += 256) {
-      const int tt = idx >> 6, pp = idx & 63;
-      tile[pp][tt] = p.mp[size_t(t0 + tt) * p.npad + p0 + pp];
-    }
-    // the scale factors of a block of frequencies, then its conversions without barriers
-    for (int wb = w0; wb < w1; wb += kWb) {
-      const int nwb = min(kWb, w1 - wb);
-      __syncthreads();
-      for (int idx = tid; idx < nwb * 64; idx += 256)
-        sc[idx >> 6][idx & 63] = sqrt(p.dscale[size_t(wb + (idx >> 6)) * p.nia_pad + t0 + (idx & 63)]);
-      __syncthreads();
-      for (int w = wb; w < wb + nwb; ++w) {
-        const int wl = w - w0;
-        const double s0 = sc[w - wb][2 * lane], s1 = sc[w - wb][2 * lane + 1];
+  constexpr int kWb = 16;
+  constexpr int kPlane = 128 * 128;     // bytes of hi or lo of 128 rows x 64 transitions
+  __shared__ double sd[kWb][64];
+  const int tid = threadIdx.x, row = tid & 127, half = tid >> 7;
+  const int kt = wi.a, rb = wi.b, r = rb * 128 + row, t0 = kt * 64 + half * 32;
+  const int nrb = p.npad / 128, nkt = p.nia_pad / 64;
+  double v[32];
 #pragma unroll
-        for (int pr = 0; pr < 8; ++pr) {
-          const int pp = warp * 8 + pr;
-          const double v0 = tile[pp][2 * lane] * s0, v1 = tile[pp][2 * lane + 1] * s1;
-          const __nv_bfloat16 h0 = __double2bfloat16(v0), h1 = __double2bfloat16(v1);
-          const __nv_bfloat16 l0 = __double2bfloat16(v0 - double(__bfloat162float(h0)));
-          const __nv_bfloat16 l1 = __double2bfloat16(v1 - double(__bfloat162float(h1)));
-          const size_t hi_row = (size_t(2 * wl) * p.npad + p0 + pp) * p.kpad + t0;
-          const size_t lo_row = (size_t(2 * wl + 1) * p.npad + p0 + pp) * p.kpad + t0;
-          reinterpret_cast<__nv_bfloat162*>(xs + hi_row)[lane] = __halves2bfloat162(h0, h1);
-          reinterpret_cast<__nv_bfloat162*>(xs + lo_row)[lane] = __halves2bfloat162(l0, l1);
-        }
+  for (int i = 0; i < 32; ++i) v[i] = p.mp[size_t(t0 + i) * p.npad + r];
+  uint8_t* out = static_cast<uint8_t*>(p.xs) + size_t(row >> 3) * 1024 + (row & 7) * 16 + half * 512;
+  auto write = [&](const double* d, int slab) {   // d: factors of the 32 transitions
+    uint8_t* dst = out + (((size_t(slab) * nrb + rb) * nkt + kt) * 2) * kPlane;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      uint32_t hi[4], lo[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int k = c * 8 + 2 * i;
+        const double x0 = v[k] * d[k], x1 = v[k + 1] * d[k + 1];
+        const __nv_bfloat162 h = __floats2bfloat162_rn(float(x0), float(x1));
+        hi[i] = *reinterpret_cast<const uint32_t*>(&h);
+        // the low part from the FP64 remainder, rounded once
+        const __nv_bfloat162 l = __floats2bfloat162_rn(float(x0 - widen(hi[i] << 16)),
+                                                       float(x1 - widen(hi[i] & 0xffff0000u)));
+        lo[i] = *reinterpret_cast<const uint32_t*>(&l);
       }
+      *reinterpret_cast<uint4*>(dst + c * 128) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+      *reinterpret_cast<uint4*>(dst + kPlane + c * 128) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
     }
+  };
+  const int w0 = wi.c, w1 = min(p.nomega, w0 + p.wgroup);
+  for (int wb = w0; wb < w1; wb += kWb) {
+    const int nwb = min(kWb, w1 - wb);
+    __syncthreads();
+    for (int i = tid; i < nwb * 64; i += 256)
+      sd[i >> 6][i & 63] = sqrt(p.dscale[size_t(wb + (i >> 6)) * p.nia_pad + kt * 64 + (i & 63)]);
+    __syncthreads();
+    for (int w = 0; w < nwb; ++w) write(&sd[w][half * 32], wb - w0 + w);
   }
 }
 
@@ -99,25 +106,181 @@ __global__ void __launch_bounds__(256) split_kmajor_kernel(const SplitOp op) {
   }
 }
 
-// K is consumed in chunks of kTcChunk k-tiles (512 transitions).  Each chunk
-// accumulates in fp32 in one of two TMEM accumulators (128 columns each); eight
-// epilogue warps drain a finished chunk into FP64 registers while the MMA warp
-// fills the other accumulator.  The fp32 accumulation length is therefore
-// bounded by the chunk, whatever the number of transitions.
+// K is consumed in chunks of 512 transitions that accumulate in fp32 in one of two TMEM
+// accumulators (128 columns each); eight drain warps per CTA add a finished chunk to FP64
+// registers while the MMA warp fills the other, so the fp32 accumulation length is bounded
+// whatever the number of transitions.
+//
+// Tile 256 x 128 per CTA pair: what bounds the products is shared memory, 128 bytes per
+// clock.  A 128 x 128 tile of one CTA reads 128 bytes per clock of MMA time and TMA writes
+// 85 more (64 KB per 768 clocks), so it could not pass 60%; the pair reads 96 (each CTA its
+// A rows and half of B; the hi part of A is held in the collector for two products, which
+// saves a sixth of that) and writes 62.  What remains is the traffic between L2 and shared
+// memory, 31 bytes per clock and SM (50% of the tensor pipe); half-size slots, twice as many of
+// them and wider TMA rows change nothing.  chi0 stage, one CTA per tile before: 840 auxiliary
+// functions, 32 frequencies 0.539 -> 0.530 ms, 4000 / 48 317 -> 290 ms, 16 ragged molecules
+// 98.4 -> 94.6 ms.
+constexpr int kSpPlaneA = 128 * 128;                       // hi or lo of 128 A rows, 64 transitions
+constexpr int kSpPlaneB = 64 * 128;                        // of half a B tile
+constexpr int kSpSlot = 2 * (kSpPlaneA + kSpPlaneB);       // 48 KB
+constexpr int kSpSlots = 4;
+constexpr int kSpChunk = 8;                                // k-tiles per fp32 accumulation
+constexpr int kSpThreads = 320;                            // warp 0 TMA, warp 1 MMA, warps 2..9 drain
+constexpr size_t kSpSmem = size_t(kSpSlots) * kSpSlot + 1024 + 256;
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kSpThreads, 1)
+    split_syrk_kernel(const DigitItem* __restrict__ items) {
+  const DigitItem it = items[blockIdx.x >> 1];
+  const int jw = blockIdx.y;
+  if (jw >= it.nw) return;   // both CTAs of the pair, before any barrier or TMEM use
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + kSpSlots * kSpSlot);   // used in rank 0
+  uint64_t* empty = full + kSpSlots;        // slot read by the MMAs (both ranks)
+  uint64_t* accf = empty + kSpSlots;        // [2] chunk accumulated (both ranks)
+  uint64_t* acce = accf + 2;                // [2] chunk drained by the 16 warps of the pair (rank 0)
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(acce + 2);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int rank = int(tc::cluster_rank());
+  if (tid == 0) {
+    for (int s = 0; s < kSpSlots; ++s) {
+      tc::mbar_init(&full[s], 1);
+      tc::mbar_init(&empty[s], 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      tc::mbar_init(&accf[b], 1);
+      tc::mbar_init(&acce[b], 16);
+    }
+    tc::fence_mbar_init();
+  }
+  if (warp == 0) tc::tmem_alloc_pair(tslot, 256);
+  __syncthreads();
+  tc::cluster_sync();        // the peer's barriers are initialised
+  tc::tc_fence_after();
+  const uint32_t tmem = *tslot;
+  const int nk = it.nkt;
+  const int nchunks = (nk + kSpChunk - 1) / kSpChunk;
+
+  if (tid == 0) {
+    // ---- TMA producer of this CTA; rank 0's full barrier counts the bytes of both
+    const uint8_t* maps = static_cast<const uint8_t*>(it.maps);
+    tc::tmap_acquire(maps);
+    tc::tmap_acquire(maps + 128);
+    const int rowA = ((it.slab_a + jw) * it.nrb + it.rb_a + rank) * nk;
+    const int rowB = ((it.slab_a + jw) * it.nrb + it.rb_b) * nk;
+    int issued = 0;
+    bool ok = true;
+    for (int kt = 0; kt < nk; ++kt, ++issued) {
+      const int s = kt % kSpSlots;
+      if (kt >= kSpSlots && !tc::mbar_wait(&empty[s], ((kt / kSpSlots) - 1) & 1)) {
+        ok = false;
+        break;
+      }
+      if (rank == 0) tc::mbar_arrive_expect_tx(&full[s], 2 * kSpSlot);
+      const uint32_t bar = tc::mapa(&full[s], 0);
+      uint8_t* d = smem + s * kSpSlot;
+      tc::tma_load_3d_pair(d, maps, bar, 0, 0, (rowA + kt) * 2);
+      tc::tma_load_3d_pair(d + 2 * kSpPlaneA, maps + 128, bar, 0, 64 * rank, (rowB + kt) * 2);
+    }
+    if (!ok) atomicOr(it.err, kErrTimeout);
+    // copies still in flight on a timeout land before the CTA leaves (bounded wait)
+    if (rank == 0) {
+      for (int s = 0; s < kSpSlots && s < issued; ++s)
+        if (!tc::mbar_wait(&full[s], (((issued - 1 - s) / kSpSlots)) & 1)) atomicOr(it.err, kErrTimeout);
+    } else if (!ok) {
+      const uint64_t t0 = tc::global_ns();
+      while (tc::global_ns() - t0 < 1000000ull) {
+      }
+    }
+  } else if (tid == 32 && rank == 0) {
+    // ---- MMA issuer of the pair
+    constexpr uint32_t idesc = tc::idesc_bf16_f32(256, 128);
+    bool ok = true;
+    for (int kt = 0; kt < nk && ok; ++kt) {
+      const int c = kt / kSpChunk, b = c & 1;
+      const bool first = (kt % kSpChunk) == 0;
+      if (first && c >= 2 && !tc::mbar_wait(&acce[b], ((c >> 1) - 1) & 1)) {
+        ok = false;
+        break;
+      }
+      const int s = kt % kSpSlots;
+      if (!tc::mbar_wait(&full[s], (kt / kSpSlots) & 1)) {
+        ok = false;
+        break;
+      }
+      tc::tc_fence_after();
+      const uint32_t d = tmem + uint32_t(b * 128);
+      const uint8_t* base = smem + s * kSpSlot;
+      const uint64_t ah = tc::desc_kmajor_cores(base, 1024), al = tc::desc_kmajor_cores(base + kSpPlaneA, 1024);
+      const uint64_t bh = tc::desc_kmajor_cores(base + 2 * kSpPlaneA, 1024);
+      const uint64_t bl = tc::desc_kmajor_cores(base + 2 * kSpPlaneA + kSpPlaneB, 1024);
+#pragma unroll
+      for (int sub = 0; sub < 4; ++sub) {
+        const uint64_t o = uint64_t(sub * 16);   // 16 bf16 along K = two core matrices = 256 bytes
+        tc::mma_bf16_pair<1>(d, ah + o, bh + o, idesc, (first && sub == 0) ? 0u : 1u);
+        tc::mma_bf16_pair<2>(d, ah + o, bl + o, idesc, 1u);
+        tc::mma_bf16_pair<0>(d, al + o, bh + o, idesc, 1u);
+      }
+      tc::mma_commit_pair(&empty[s]);
+      if ((kt % kSpChunk) == kSpChunk - 1 || kt == nk - 1) tc::mma_commit_pair(&accf[b]);
+    }
+    if (!ok) atomicOr(it.err, kErrTimeout);
+  } else if (warp >= 2) {
+    // ---- drain each chunk into FP64 registers, then store the tile
+    const int quad = warp & 3;                 // TMEM lanes 32 quad .. (rows)
+    const int half = (warp - 2) >> 2;          // columns 64 half ..
+    double acc[64];
+#pragma unroll
+    for (int j = 0; j < 64; ++j) acc[j] = 0.0;
+    bool ok = true;
+    for (int c = 0; c < nchunks; ++c) {
+      const int b = c & 1;
+      ok = __all_sync(0xffffffffu, tc::mbar_wait(&accf[b], (c >> 1) & 1));
+      if (!ok) break;
+      tc::tc_fence_after();
+      const uint32_t base = tmem + uint32_t(b * 128 + half * 64) + (uint32_t(quad * 32) << 16);
+#pragma unroll
+      for (int cb = 0; cb < 8; ++cb) {
+        uint32_t r[8];
+        tc::tmem_ld_32x8(base + cb * 8, r);
+        tc::tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[cb * 8 + j] += double(__uint_as_float(r[j]));
+      }
+      tc::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive_cluster(tc::mapa(&acce[b], 0));
+    }
+    const int rb = it.rb_a + rank, cb = it.rb_b;
+    if (!ok) {
+      if (lane == 0) atomicOr(it.err, kErrTimeout);
+    } else if (rb < it.nrb && rb <= cb) {      // blocks below the diagonal are not stored
+      const int row = rb * 128 + quad * 32 + lane, col0 = cb * 128 + half * 64;
+      double* dst = it.C + jw * it.sC + size_t(row) * it.ld + col0;
+#pragma unroll
+      for (int j = 0; j < 64; j += 2) {
+        double v0 = acc[j], v1 = acc[j + 1];
+        if (col0 + j == row) v0 += 1.0;
+        if (col0 + j + 1 == row) v1 += 1.0;
+        *reinterpret_cast<double2*>(dst + j) = make_double2(v0, v1);
+      }
+    }
+  }
+  tc::tc_fence_before();
+  __syncthreads();
+  tc::cluster_sync();        // no CTA leaves while its peer may still reach its memory
+  if (warp == 0) {
+    __syncwarp();
+    tc::tmem_dealloc_pair(tmem, 256);
+  }
+}
+
+// The general product of the AO->MO transform: the same chunks, one 128 x 128 tile per CTA.
 constexpr int kTcChunk = 8;
 constexpr int kTcThreads = 320;    // warp 0 TMA, warp 1 MMA, warps 2..9 epilogue
 
 __global__ void __launch_bounds__(kTcThreads, 1) syrk_bf16x3_kernel(const TcItem* __restrict__ items) {
-  TcItem it = items[blockIdx.x];
-  const int jw = blockIdx.y;
-  if (jw >= (it.nw > 0 ? it.nw : 1)) return;   // the whole CTA, before any barrier or TMEM use
-  it.C += jw * it.sC;
-  it.row_a += jw * it.srow;
-  it.row_b += jw * it.srow;
-  if (it.ea) {
-    it.ea += jw * it.se;
-    it.eb += jw * it.se;
-  }
+  const TcItem it = items[blockIdx.x];
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + kTcStages * kTcStageBytes);
@@ -148,10 +311,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) syrk_bf16x3_kernel(const TcItem
 
   if (tid == 0) {
     // ---- TMA producer
-    const void* tmb = it.tmap_b ? it.tmap_b : it.tmap;
-    const int lob = it.tmap_b ? it.lo_off_b : it.lo_off;
     tc::tmap_acquire(it.tmap);
-    if (it.tmap_b) tc::tmap_acquire(it.tmap_b);
+    tc::tmap_acquire(it.tmap_b);
     int issued[kTcStages] = {0, 0, 0};
     bool ok = true;
     for (int kt = 0; kt < nk && ok; ++kt) {
@@ -164,8 +325,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) syrk_bf16x3_kernel(const TcItem
       const int k0 = kt * 64;
       tc::tma_load_2d(tile(s, 0), it.tmap, &full[s], k0, it.row_a);
       tc::tma_load_2d(tile(s, 1), it.tmap, &full[s], k0, it.row_a + it.lo_off);
-      tc::tma_load_2d(tile(s, 2), tmb, &full[s], k0, it.row_b);
-      tc::tma_load_2d(tile(s, 3), tmb, &full[s], k0, it.row_b + lob);
+      tc::tma_load_2d(tile(s, 2), it.tmap_b, &full[s], k0, it.row_b);
+      tc::tma_load_2d(tile(s, 3), it.tmap_b, &full[s], k0, it.row_b + it.lo_off_b);
       ++issued[s];
     }
     if (!ok) atomicOr(it.err, kErrTimeout);
@@ -228,18 +389,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) syrk_bf16x3_kernel(const TcItem
       __syncwarp();
       if (lane == 0) tc::mbar_arrive(&acce[b]);
     }
-    if (ok && it.mrows == 0) {
-      double* dst = it.C + size_t(row) * it.ldc + half * 64;
-#pragma unroll
-      for (int j = 0; j < 64; j += 2) {
-        const int col = half * 64 + j;
-        double v0 = acc[j], v1 = acc[j + 1];
-        if (col - row == it.diag) v0 += 1.0;
-        if (col + 1 - row == it.diag) v1 += 1.0;
-        *reinterpret_cast<double2*>(dst + j) = make_double2(v0, v1);
-      }
-    } else if (ok) {
-      // edge tile of a general product: rows < mrows, columns < ncols, no identity
+    if (ok) {   // rows < mrows, columns < ncols
       if (row < it.mrows) {
         double* dst = it.C + size_t(row) * it.ldc;
 #pragma unroll
@@ -274,19 +424,17 @@ bool bf16x3_available() {
   return true;
 }
 
-// Row-major [rows][kpad] tensor read in boxes of 128 rows x box_bytes (128: 128-byte
-// swizzle; 64: 64-byte swizzle).
+// Row-major [rows][kpad] tensor read in boxes of 128 rows x 128 bytes (128-byte swizzle).
 static Status make_kmajor_tmap(void* host_map, CUtensorMapDataType type, int esize, const void* base, int kpad,
-                               long long rows, int box_bytes = 128) {
+                               long long rows) {
   if (!bf16x3_available()) return Status::fail(RIGW_ERR_UNSUPPORTED, "cuTensorMapEncodeTiled unavailable");
   CUtensorMap* m = reinterpret_cast<CUtensorMap*>(host_map);
   cuuint64_t dims[2] = {cuuint64_t(kpad), cuuint64_t(rows)};
   cuuint64_t strides[1] = {cuuint64_t(kpad) * esize};
-  cuuint32_t box[2] = {cuuint32_t(box_bytes / esize), 128};
+  cuuint32_t box[2] = {cuuint32_t(128 / esize), 128};
   cuuint32_t estr[2] = {1, 1};
   CUresult r = g_encode(m, type, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                        box_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B,
-                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                        CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return Status::fail(RIGW_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", int(r));
   return Status::ok();
@@ -296,12 +444,16 @@ Status make_split_tmap(void* host_map, const void* xs, int kpad, long long rows)
   return make_kmajor_tmap(host_map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, xs, kpad, rows);
 }
 
-Status make_ozaki_tmap(void* host_map, const void* xq, int kpad, long long rows, int box_bytes) {
-  return make_kmajor_tmap(host_map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, xq, kpad, rows, box_bytes);
+Status make_ozaki_tmap(void* host_map, const void* xq, int kpad, long long rows) {
+  return make_kmajor_tmap(host_map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, xq, kpad, rows);
 }
 
-void launch_split_bf16x3(const ProbDev* probs, const WorkItem* items, int n, cudaStream_t s) {
-  if (n > 0) split_bf16x3_kernel<<<n, 256, 0, s>>>(probs, items);
+void launch_split_bf16(const ProbDev* probs, const WorkItem* items, int n, cudaStream_t s) {
+  if (n > 0) split_bf16_kernel<<<n, 256, 0, s>>>(probs, items);
+}
+
+void launch_split_syrk(const DigitItem* items, int n, int ny, cudaStream_t s) {
+  if (n > 0 && ny > 0) split_syrk_kernel<<<dim3(2 * n, ny), kSpThreads, kSpSmem, s>>>(items);
 }
 
 void launch_split_kmajor(const SplitOp& op, cudaStream_t s) {
@@ -309,11 +461,13 @@ void launch_split_kmajor(const SplitOp& op, cudaStream_t s) {
     split_kmajor_kernel<<<dim3(op.Kpad / 64, op.Rpad / 64, op.nz), 256, 0, s>>>(op);
 }
 
-void launch_syrk_bf16x3(const TcItem* items, int n, int ny, cudaStream_t s) {
-  if (n > 0 && ny > 0) syrk_bf16x3_kernel<<<dim3(n, ny), kTcThreads, kTcSmemBytes, s>>>(items);
+void launch_syrk_bf16x3(const TcItem* items, int n, cudaStream_t s) {
+  if (n > 0) syrk_bf16x3_kernel<<<n, kTcThreads, kTcSmemBytes, s>>>(items);
 }
 
 cudaError_t prepare_tc_kernels() {
+  cudaError_t e = cudaFuncSetAttribute(split_syrk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSpSmem));
+  if (e != cudaSuccess) return e;
   return cudaFuncSetAttribute(syrk_bf16x3_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTcSmemBytes));
 }
 

@@ -138,6 +138,27 @@ RIGW_DEVICE_INLINE void mma_s8_pair(uint32_t d_tmem, uint64_t adesc, uint64_t bd
       "tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc));
 }
+// kind::f16 for the pair.  `keep`: 1 holds A in the collector buffer for the next MMA, 2 takes
+// it from there for the last time, 0 neither (an operand that consecutive MMAs share is read
+// from shared memory once).
+template <int keep>
+RIGW_DEVICE_INLINE void mma_bf16_pair(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
+  if constexpr (keep == 1)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16.collector::a::fill [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc));
+  else if constexpr (keep == 2)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16.collector::a::lastuse [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc));
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc));
+}
 // Arrive on the mbarrier at this offset in both CTAs when all MMAs issued so far are done.
 RIGW_DEVICE_INLINE void mma_commit_pair(uint64_t* bar) {
   asm volatile(
@@ -199,19 +220,6 @@ RIGW_DEVICE_INLINE uint64_t desc_kmajor_sw128(const void* smem) {
   d |= uint64_t(1024 >> 4) << 32;          // stride byte offset: 8 rows x 128 B
   d |= uint64_t(1) << 46;                  // descriptor version (sm_100)
   d |= uint64_t(2) << 61;                  // SWIZZLE_128B
-  return d;
-}
-
-// The same for rows of 64 bytes written with 64-byte swizzling (8-row atoms of
-// 512 bytes).
-RIGW_DEVICE_INLINE uint64_t desc_kmajor_sw64(const void* smem) {
-  const uint64_t addr = smem_u32(smem);
-  uint64_t d = 0;
-  d |= (addr >> 4) & 0x3FFFull;            // start address
-  d |= uint64_t(1) << 16;                  // leading byte offset (unused for swizzled K-major)
-  d |= uint64_t(512 >> 4) << 32;           // stride byte offset: 8 rows x 64 B
-  d |= uint64_t(1) << 46;                  // descriptor version (sm_100)
-  d |= uint64_t(4) << 61;                  // SWIZZLE_64B
   return d;
 }
 
