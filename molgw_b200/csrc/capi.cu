@@ -43,10 +43,10 @@ Status run_batch(Context& c, rigw::PlanMode mode, int n, const rigw_problem* pro
     fresh.reset(new Plan());
     bs = fresh->build(&c, mode, shapes, factors);
   }
-  if (bs.code == RIGW_ERR_NOMEM) {   // without the digit buffers of the FP64 chi0
+  if (bs.code == RIGW_ERR_NOMEM) {   // without the digit buffers of the FP64 products
     bool any = false;
     for (Shape& sh : shapes) {
-      any = any || rigw::use_digits(sh);
+      any = any || rigw::use_digits(sh) || rigw::use_factor_digits(sh);
       sh.no_digits = 1;
     }
     if (any) {

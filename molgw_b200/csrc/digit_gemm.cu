@@ -36,6 +36,8 @@
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
+#include <type_traits>
+
 #include "engine.cuh"
 #include "tc_common.cuh"
 
@@ -76,6 +78,11 @@ RIGW_DEVICE_INLINE double factor(const ProbDev& p, int w, int t) {
 }
 
 RIGW_DEVICE_INLINE double pow2(int e) { return __hiloint2double((e + 1023) << 20, 0); }   // -1022 <= e <= 1023
+
+// 2^e; NaN above 1023 (kNaNExp, also with a shift added), 2^-1022 at the least.
+RIGW_DEVICE_INLINE double pow2_of(int e) {
+  return e > 1023 ? __longlong_as_double(0x7ff8000000000000ll) : pow2(max(e, -1022));
+}
 
 }  // namespace
 
@@ -232,13 +239,10 @@ __global__ void __launch_bounds__(256) digit_slice_kernel(const ProbDev* __restr
 // would read 128 and write 45).  TMEM holds four 128-column accumulators, so the levels go
 // in two passes over a chunk: NS + 1 down to NS - 2 (22 of the 28 products for NS = 7), and
 // the rest from the leading digits alone, several k-tiles per slot.
-template <int NS>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kDigThreads, 1)
-    digit_syrk_kernel(const DigitItem* __restrict__ items) {
+template <int NS, class Item>
+__device__ __forceinline__ void digit_product(const Item& it, const int jw) {
   using Cfg = DigCfg<NS>;
-  const DigitItem it = items[blockIdx.x >> 1];
-  const int jw = blockIdx.y;
-  if (jw >= it.nw) return;   // both CTAs of the pair, before any barrier or TMEM use
+  constexpr bool kUpdate = std::is_same<Item, UpdateItem>::value;
   extern __shared__ uint8_t dig_smem_raw[];
   uint8_t* smem =
       reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dig_smem_raw) + 1023) & ~uintptr_t(1023));
@@ -263,8 +267,20 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kDigThreads, 1)
   tc::cluster_sync();        // the peer's barriers are initialised
   tc::tc_fence_after();
   const uint32_t tmem = *tslot;
-  const int nk = it.nkt;
-  const int nchunks = (nk + kChunkTiles - 1) / kChunkTiles;
+  int nk, chunk, slab_a, slab_b;      // k-tiles summed, k-tiles per chunk, operand slabs
+  int c0 = 0;                         // first chunk
+  if constexpr (kUpdate) {
+    nk = it.nk;
+    chunk = it.chunk;
+    c0 = it.first;
+    slab_a = slab_b = it.slab + jw * it.step;
+  } else {
+    nk = it.nkt;
+    chunk = kChunkTiles;
+    slab_a = it.slab_a + jw;
+    slab_b = it.slab_b;
+  }
+  const int nchunks = (nk + chunk - 1) / chunk;
   constexpr int kPasses = Cfg::kHi > 0 ? 2 : 1;
   // k-tiles of a slot in pass q (0: low levels, 1: high levels)
   auto per_slot = [](int q) { return q == 0 ? 1 : Cfg::kPerHi; };
@@ -274,15 +290,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kDigThreads, 1)
     // ---- TMA producer of this CTA; rank 0's full barrier counts the bytes of both
     const uint8_t* maps = static_cast<const uint8_t*>(it.maps);
     for (int m = 0; m < (kPasses > 1 ? 4 : 2); ++m) tc::tmap_acquire(maps + 128 * m);
-    const int rowA = ((it.slab_a + jw) * it.nrb + it.rb_a + rank) * nk;
-    const int rowB = (it.slab_b * it.nrb + it.rb_b) * nk;
+    const int rowA = (slab_a * it.nrb + it.rb_a + rank) * it.nkt;
+    const int rowB = (slab_b * it.nrb + it.rb_b) * it.nkt;
     uint32_t issued = 0;
     bool ok = true;
-    for (int c = 0; c < nchunks && ok; ++c)
+    for (int c = c0; c < nchunks && ok; ++c)
       for (int q = 0; q < kPasses && ok; ++q) {
-        const int k1 = min(nk, (c + 1) * kChunkTiles), ps = per_slot(q);
+        const int k1 = min(nk, (c + 1) * chunk), ps = per_slot(q);
         const int nd = q == 0 ? NS : Cfg::kHi;             // digits loaded
-        for (int k0 = c * kChunkTiles; k0 < k1; k0 += ps, ++issued) {
+        for (int k0 = c * chunk; k0 < k1; k0 += ps, ++issued) {
           const int s = int(issued % Cfg::kSlots);
           if (issued >= uint32_t(Cfg::kSlots) &&
               !tc::mbar_wait(&empty[s], ((issued / Cfg::kSlots) - 1) & 1)) {
@@ -317,7 +333,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kDigThreads, 1)
     bool ok = true;
     uint32_t step = 0;
     int pass = 0;
-    for (int c = 0; c < nchunks && ok; ++c)
+    for (int c = c0; c < nchunks && ok; ++c)
 #pragma unroll
       for (int q = 0; q < kPasses; ++q) {
         if (!ok) break;
@@ -327,10 +343,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kDigThreads, 1)
         }
         ++pass;
         tc::tc_fence_after();
-        const int k1 = min(nk, (c + 1) * kChunkTiles), ps = per_slot(q);
+        const int k1 = min(nk, (c + 1) * chunk), ps = per_slot(q);
         constexpr int kBytesLo = NS * (kTileA + kTileB);
         uint32_t first = 0u;
-        for (int k0 = c * kChunkTiles; k0 < k1; k0 += ps, ++step) {
+        for (int k0 = c * chunk; k0 < k1; k0 += ps, ++step) {
           const int s = int(step % Cfg::kSlots);
           if (!tc::mbar_wait(&full[s], (step / Cfg::kSlots) & 1)) {
             ok = false;
@@ -377,12 +393,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kDigThreads, 1)
     const int quad = warp & 3;                 // TMEM lanes 32 quad .. (rows)
     const int half = (warp - 2) >> 2;          // columns 64 half ..
     const uint32_t done = tc::mapa(acce, 0);
+    // weight of the lowest level of unit-scaled operands
+    constexpr int kShift = 8 * (NS - 1) - 2 * (8 * NS - 1);
     double acc[64];
 #pragma unroll
     for (int j = 0; j < 64; ++j) acc[j] = 0.0;
     bool ok = true;
     int pass = 0;
-    for (int c = 0; c < nchunks && ok; ++c)
+    for (int c = c0; c < nchunks && ok; ++c)
 #pragma unroll
       for (int q = 0; q < kPasses; ++q) {
         if (!ok) break;
@@ -392,6 +410,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kDigThreads, 1)
         tc::tc_fence_after();
         constexpr int kLoL = Cfg::kLo, kHiL = Cfg::kHi;
         const double wq = q == 0 ? 1.0 : double(1ull << (8 * kLoL));
+        // update: every chunk has row and column exponents of its own
+        double wr = wq;
+        const int* ecol = nullptr;
+        if constexpr (kUpdate) {
+          const int* e = it.exps + (size_t(slab_a) * it.ngroups + c) * it.nrb * 128;
+          wr *= pow2_of(e[min(it.rb_a + rank, it.nrb - 1) * 128 + quad * 32 + lane]);
+          ecol = e + it.rb_b * 128 + half * 64;
+        }
 #pragma unroll
         for (int cb = 0; cb < 8; ++cb) {
           const uint32_t base = tmem + uint32_t(half * 64 + cb * 8) + (uint32_t(quad * 32) << 16);
@@ -407,32 +433,46 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kDigThreads, 1)
 #pragma unroll
             for (int a = 1; a < 4; ++a)
               if (a < nl) x = x * 256 + int(r[a][j]);
-            acc[cb * 8 + j] += double(x) * wq;
+            if constexpr (kUpdate) acc[cb * 8 + j] += double(x) * (wr * pow2_of(ecol[cb * 8 + j] + kShift));
+            else acc[cb * 8 + j] += double(x) * wq;
           }
         }
         tc::tc_fence_before();
         __syncwarp();
         if (lane == 0) tc::mbar_arrive_cluster(done);
       }
-    const int rb = it.rb_a + rank, cb = it.rb_b;
     if (!ok) {
       if (lane == 0) atomicOr(it.err, kErrTimeout);
-    } else if (rb < it.nrb && rb <= cb) {      // blocks below the diagonal are not stored
-      const int row = rb * 128 + quad * 32 + lane, col0 = cb * 128 + half * 64;
-      const int er = it.exps[size_t(it.slab_e + jw) * it.ld + row];
-      constexpr int kShift = 8 * (NS - 1) - 2 * (8 * NS - 1);
-      double* dst = it.C + jw * it.sC + size_t(row) * it.ld + col0;
+    } else if constexpr (kUpdate) {
+      if (rank < it.rows_a && !(it.diag && it.rb_b < it.rb_a + rank)) {
+        double* dst = it.C + jw * it.sC + size_t(rank * 128 + quad * 32 + lane) * it.ld + half * 64;
 #pragma unroll
-      for (int j = 0; j < 64; j += 2) {
-        double v[2];
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          const int ec = it.exps[col0 + j + u];
-          v[u] = (er == kNaNExp || ec == kNaNExp) ? __longlong_as_double(0x7ff8000000000000ll)
-                                                   : ldexp(acc[j + u], er + ec + kShift);
-          if (col0 + j + u == row) v[u] += 1.0;
+        for (int j = 0; j < 64; j += 2) {
+          if (half * 64 + j >= it.ncol) break;     // an even number of columns
+          double2 v = *reinterpret_cast<const double2*>(dst + j);
+          v.x -= acc[j];
+          v.y -= acc[j + 1];
+          *reinterpret_cast<double2*>(dst + j) = v;
         }
-        *reinterpret_cast<double2*>(dst + j) = make_double2(v[0], v[1]);
+      }
+    } else {
+      const int rb = it.rb_a + rank, cb = it.rb_b;
+      if (rb < it.nrb && rb <= cb) {               // blocks below the diagonal are not stored
+        const int row = rb * 128 + quad * 32 + lane, col0 = cb * 128 + half * 64;
+        const int er = it.exps[size_t(it.slab_e + jw) * it.ld + row];
+        double* dst = it.C + jw * it.sC + size_t(row) * it.ld + col0;
+#pragma unroll
+        for (int j = 0; j < 64; j += 2) {
+          double v[2];
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            const int ec = it.exps[col0 + j + u];
+            v[u] = (er == kNaNExp || ec == kNaNExp) ? __longlong_as_double(0x7ff8000000000000ll)
+                                                     : ldexp(acc[j + u], er + ec + kShift);
+            if (col0 + j + u == row) v[u] += 1.0;
+          }
+          *reinterpret_cast<double2*>(dst + j) = make_double2(v[0], v[1]);
+        }
       }
     }
   }
@@ -443,6 +483,63 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kDigThreads, 1)
     __syncwarp();
     tc::tmem_dealloc_pair(tmem, 512);
   }
+}
+
+template <int NS>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kDigThreads, 1)
+    digit_syrk_kernel(const DigitItem* __restrict__ items) {
+  const DigitItem it = items[blockIdx.x >> 1];
+  if (int(blockIdx.y) >= it.nw) return;   // both CTAs of the pair, before any barrier or TMEM use
+  digit_product<NS>(it, blockIdx.y);
+}
+
+// C -= A^T B for the rows of one panel group, A and B columns of the finished rows above it
+// (the factorization of eps and its fused solves).  The columns' digits are scaled group of
+// rows by group of rows, so a chunk of the sum is one group and is joined with its own weights:
+// U's entries far above the diagonal are small, and one scale for a whole column would have to
+// cover its largest entry.  DMMA did these updates at 20 TF/s (64 x 128 tiles, K = 256 at a
+// time, every trailing tile read and written once per group); here each tile is written once
+// in all, with K of all rows above, at 100 TF/s (2000 auxiliary functions, K = 512).
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kDigThreads, 1)
+    digit_update_kernel(const UpdateItem* __restrict__ items) {
+  const UpdateItem it = items[blockIdx.x >> 1];
+  if (int(blockIdx.y) >= it.nw) return;
+  digit_product<kFp64Digits>(it, blockIdx.y);
+}
+
+// One block of 128 columns of a group of finished rows: column maxima, then the digits, both
+// passes over the same rows (the second one from L2).  Thread (column, half).
+__global__ void __launch_bounds__(256) factor_slice_kernel(const FactorSliceItem* __restrict__ items) {
+  const FactorSliceItem it = items[blockIdx.x];
+  const int jw = blockIdx.y;
+  if (jw >= it.nw) return;
+  __shared__ unsigned part[2][128];
+  const int tid = threadIdx.x, col = tid & 127, half = tid >> 7;
+  const double* src = it.src + jw * it.s_src + col;
+  const bool live = col < it.ncol;
+  unsigned m = 0;
+  if (live) {
+#pragma unroll 8
+    for (int r = half; r < it.rows; r += 2)
+      m = max(m, unsigned(__double2hiint(src[size_t(r) * it.ld])) & 0x7fffffffu);
+  }
+  part[half][col] = m;
+  __syncthreads();
+  const int e = row_exponent(max(part[0][col], part[1][col]));
+  const int slab = it.slab + jw * it.step;
+  if (half == 0) it.exps[((size_t(slab) * it.ngroups + it.group) * it.nrb + it.rb) * 128 + col] = e;
+  const double sc = pow2(8 * kFp64Digits - 1 - (e == kNaNExp ? 0 : e));
+  int8_t* dig = static_cast<int8_t*>(it.digits);
+  for (int kt = 0; kt < it.rows / 64; ++kt)
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const int kc = half * 2 + c;
+      double v[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) v[i] = live ? src[size_t(kt * 64 + kc * 16 + i) * it.ld] : 0.0;
+      write_digits<kFp64Digits>(v, sc,
+                                dig + digit_offset(slab, it.nrb, it.rb, it.nkt, it.kt + kt, kFp64Digits, col, kc));
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -506,6 +603,13 @@ void launch_digit_slice(int planes, const ProbDev* probs, const WorkItem* items,
     default: digit_slice_kernel<7><<<n, 256, 0, s>>>(probs, items); break;
   }
 }
+void launch_factor_slice(const FactorSliceItem* items, int n, int ny, cudaStream_t s) {
+  if (n > 0 && ny > 0) factor_slice_kernel<<<dim3(n, ny), 256, 0, s>>>(items);
+}
+void launch_digit_update(const UpdateItem* items, int n, int ny, cudaStream_t s) {
+  if (n > 0 && ny > 0)
+    digit_update_kernel<<<dim3(2 * n, ny), kDigThreads, DigCfg<kFp64Digits>::kSmem, s>>>(items);
+}
 void launch_digit_syrk(int planes, const DigitItem* items, int n, int ny, cudaStream_t s) {
   if (n <= 0 || ny <= 0) return;
   switch (planes) {
@@ -519,7 +623,8 @@ void launch_digit_syrk(int planes, const DigitItem* items, int n, int ny, cudaSt
 cudaError_t prepare_digit_kernels() {
   for (cudaError_t e : {prepare_ns<3>(), prepare_ns<4>(), prepare_ns<5>(), prepare_ns<6>(), prepare_ns<7>()})
     if (e != cudaSuccess) return e;
-  return cudaSuccess;
+  return cudaFuncSetAttribute(digit_update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              int(DigCfg<kFp64Digits>::kSmem));
 }
 
 }  // namespace rigw

@@ -255,6 +255,11 @@ bool use_digits(const Shape& sh) {
          (long long)sh.nocc * sh.nvirt + (long long)sh.nocc2 * sh.nvirt2 >= 512;
 }
 
+// From seven panels on a group of four leaves something to update.  Factorization stage, DMMA
+// against digits (32 frequencies, ms): naux 500 0.46 / 0.48, 840 1.91 / 1.88, 1152 3.51 / 3.14,
+// 1483 7.15 / 5.36, 2000 18.4 / 12.9, 4000 (48 frequencies, QP only) 139 / 67.
+bool use_factor_digits(const Shape& sh) { return !sh.no_digits && sh.naux > 768; }
+
 int operand_planes(const Shape& sh) {
   if (sh.precision == RIGW_BF16X3) return 2;
   if (is_ozaki(sh.precision)) return ozaki_slices(sh.precision);
@@ -346,8 +351,13 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
 
   // ---- memory layout
   Layout L;
+  // digit blocks of the factor [U | right-hand sides], and the bytes of its digits
+  auto factor_blocks = [&](const Dims& d) { return d.npanel + (d.ldb + kPanel - 1) / kPanel; };
+  auto factor_bytes = [&](const Shape& sh, const Dims& d) {
+    return size_t(sh.nomega) * factor_blocks(d) * kPanel * d.npad * kFp64Digits;
+  };
   struct Off {
-    size_t mp, xs, tmap, dmax, xexp, tnorm, dscale, eps, winv, logdet, rhs, colsq, mnorm, vchiv, ew, tr, en, sc, sr, qp;
+    size_t fmap, fexp, mp, xs, tmap, dmax, xexp, tnorm, dscale, eps, winv, logdet, rhs, colsq, mnorm, vchiv, ew, tr, en, sc, sr, qp;
   };
   std::vector<Off> off(np);
   for (int i = 0; i < np; ++i) {
@@ -370,8 +380,17 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
       pp.off_in_omega = L.take(size_t(sh.nomega) * D);
       pp.off_in_weight = L.take(size_t(sh.nomega) * D);
       off[i].mp = L.take(size_t(d.nia_pad) * d.npad * D);
-      if (const int planes = operand_planes(sh)) {
-        off[i].xs = L.take(size_t((planes > 2) + split_group(sh)) * split_bytes_per_frequency(sh));
+      // the chi0 operands and, after them, the digits of the factor
+      const int planes = operand_planes(sh);
+      const bool fd = use_factor_digits(sh);
+      off[i].xs = L.take(std::max(planes ? size_t((planes > 2) + split_group(sh)) * split_bytes_per_frequency(sh) : 0,
+                                  fd ? factor_bytes(sh, d) : 0));
+      if (fd) {
+        off[i].fmap = L.take(512);
+        off[i].fexp = L.take(size_t(sh.nomega) * ((d.npanel + kDigitGroup - 1) / kDigitGroup) * factor_blocks(d) *
+                             kPanel * sizeof(int));
+      }
+      if (planes) {
         off[i].tmap = L.take(512);
         if (planes > 2) {
           off[i].dmax = L.take(size_t(1 + sh.nomega) * d.npad * sizeof(unsigned));
@@ -423,6 +442,9 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
       const Dims d = dims_of(sh, mode);
       const size_t t = size_t(d.npanel + 2) * (d.npanel + 2 + (d.ldb + 127) / 128) * 4;
       // GEMM items cover all frequencies of a chain; the WorkItem lists stay per frequency
+      if (factor && use_factor_digits(sh))
+        lists += size_t(kMaxChains) * (d.npanel / kDigitGroup + 1) * factor_blocks(d) *
+                 (sizeof(FactorSliceItem) + (kDigitGroup / 2) * sizeof(UpdateItem));
       lists += size_t(kMaxChains + 1) * t * sizeof(GemmItem) +
                size_t(sh.nomega) * (d.npanel + 8) * sizeof(WorkItem) +
                size_t(d.nia_pad / 8 + d.npad * d.ldb / 1024 + 64) * 16;
@@ -491,6 +513,12 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
         RIGW_TRY(make_f64_tmaps(maps, p.mp, d.npad, d.nia_pad, p.dscale, sh.nomega));
         RIGW_CUDA_TRY(cudaMemcpyAsync(base + off[i].tmap, maps, sizeof(maps), cudaMemcpyHostToDevice, ctx->stream));
       }
+      if (use_factor_digits(sh)) {
+        alignas(64) unsigned char maps[512];
+        RIGW_TRY(make_digit_tmaps(maps, base + off[i].xs,
+                                  (long long)sh.nomega * factor_blocks(d) * (d.npad / 64) * kFp64Digits, kFp64Digits, 64));
+        RIGW_CUDA_TRY(cudaMemcpyAsync(base + off[i].fmap, maps, sizeof(maps), cudaMemcpyHostToDevice, ctx->stream));
+      }
       p.eps = dp(off[i].eps);
       p.winv = dp(off[i].winv);
       p.logdet = dp(off[i].logdet);
@@ -545,7 +573,8 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
   gl_k2n_.assign(nlists, {});
   gl_k3_.assign(nlists, {});
   gl_k3d_.assign(nlists, {});
-  gl_k3a_.assign(nlists, {});
+  fl_slice_.assign(nlists, {});
+  ul_update_.assign(nlists, {});
   int pair = 0;
   for (int i = 0; i < np; ++i) {
     const Shape& sh = shapes[i];
@@ -703,11 +732,79 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
         // the whole group, so each trailing tile is read and written once per group.
         // Items of the next diagonal block go to their own list (in both forms) so that
         // its factorization can start while the rest of the update runs (lookahead).
-        const int jg = k % group_;
-        const bool first_of_pair = jg != group_ - 1;           // not the group's last panel
+        // Problems on digit products take groups of kDigitGroup panels, and after the last
+        // panel of a group only the rows of the next group are updated, with every row
+        // above them (left-looking), on the int8 tensor cores.
+        const bool fd = factor && use_factor_digits(sh);
+        const int gsize = fd ? kDigitGroup : group_;
+        const int jg = k % gsize;
+        const bool inside = jg != gsize - 1;                    // not the group's last panel
         const int kp = k - jg;                                  // first panel of the U rows used
         const int kdim = (jg + 1) * kPanel;
-        const int iend = first_of_pair ? std::min(npad, r0 + kPanel) : npad;
+        const int iend = inside ? std::min(npad, r0 + kPanel) : npad;
+        if (fd && !inside && r0 < npad) {
+          int* fexp = reinterpret_cast<int*>(base + off[i].fexp);
+          const int nrb = p.npanel + (ldb + kPanel - 1) / kPanel, nkt = npad / 64;
+          const int ngroups = (p.npanel + kDigitGroup - 1) / kDigitGroup;
+          auto slice = [&](const double* X, int ldx, long long stride, int c0, int n, int rb) {
+            FactorSliceItem f{};
+            f.src = X + size_t(kp) * kPanel * ldx + c0;
+            f.digits = base + off[i].xs;
+            f.exps = fexp;
+            f.ld = ldx;
+            f.ncol = n;
+            f.rows = kdim;
+            f.nrb = nrb;
+            f.nkt = nkt;
+            f.rb = rb;
+            f.kt = kp * (kPanel / 64);
+            f.ngroups = ngroups;
+            f.group = k / kDigitGroup;
+            f.slab = w0;
+            f.step = nchains_;
+            f.nw = nw;
+            f.s_src = stride;
+            fl_slice_[li].push_back(f);
+          };
+          auto update = [&](double* X, int ldx, long long stride, int ra, int c0, int n, int rb, int first, int diag) {
+            UpdateItem u{};
+            u.maps = base + off[i].fmap;
+            u.C = X + size_t(ra) * kPanel * ldx + c0;
+            u.err = err_dev_;
+            u.exps = fexp;
+            u.rb_a = ra;
+            u.rb_b = rb;
+            u.nrb = nrb;
+            u.nkt = nkt;
+            u.nk = r0 / 64;
+            u.chunk = kDigitGroup * kPanel / 64;
+            u.first = first;
+            u.ngroups = ngroups;
+            u.slab = w0;
+            u.step = nchains_;
+            u.rows_a = std::min(2, p.npanel - ra);
+            u.ncol = n;
+            u.diag = diag;
+            u.ld = ldx;
+            u.nw = nw;
+            u.sC = stride;
+            ul_update_[li].push_back(u);
+          };
+          for (int cb = k + 1; cb < p.npanel; ++cb) slice(E, npad, sE, cb * kPanel, kPanel, cb);
+          if (p.want_identity)
+            for (int cb = 0; cb <= k; ++cb) slice(R, ldb, sR, cb * kPanel, kPanel, p.npanel + cb);
+          for (int c0 = p.moff; c0 < ldb; c0 += kPanel)
+            slice(R, ldb, sR, c0, std::min(kPanel, ldb - c0), p.npanel + c0 / kPanel);
+          for (int ra = k + 1; ra < std::min(p.npanel, k + 1 + kDigitGroup); ra += 2) {
+            for (int cb = ra; cb < p.npanel; ++cb) update(E, npad, sE, ra, cb * kPanel, kPanel, cb, 0, 1);
+            if (p.want_identity)
+              for (int cb = 0; cb <= k; ++cb)
+                update(R, ldb, sR, ra, cb * kPanel, kPanel, p.npanel + cb, cb / kDigitGroup, 0);
+            for (int c0 = p.moff; c0 < ldb; c0 += kPanel)
+              update(R, ldb, sR, ra, c0, std::min(kPanel, ldb - c0), p.npanel + c0 / kPanel, 0, 0);
+          }
+          continue;
+        }
         auto k3 = [&](const double* Bsrc, int ldbs, double* Cdst, int ldc, int i0, int c0, int m, int n,
                       std::vector<GemmItem>& dst) {
           GemmItem g{};
@@ -729,7 +826,7 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
           g.sC = (Cdst == E) ? sE : sR;
           dst.push_back(g);
         };
-        std::vector<GemmItem>& rest = first_of_pair ? gl_k3a_[li] : gl_k3_[li];
+        std::vector<GemmItem>& rest = gl_k3_[li];
         for (int i0 = r0; i0 < iend; i0 += BM) {
           const int m = std::min(BM, iend - i0);
           if (factor)
@@ -793,6 +890,10 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
     int ny = 1;
     if (kind == 1 || kind == 5 || kind == 6 || kind == 14)
       for (size_t j = 0; j < n; ++j) ny = std::max(ny, static_cast<const GemmItem*>(src)[j].nw);
+    if (kind == 27)
+      for (size_t j = 0; j < n; ++j) ny = std::max(ny, static_cast<const FactorSliceItem*>(src)[j].nw);
+    if (kind == 28)
+      for (size_t j = 0; j < n; ++j) ny = std::max(ny, static_cast<const UpdateItem*>(src)[j].nw);
     if (kind == 26)
       for (size_t j = 0; j < n; ++j) ny = std::max(ny, static_cast<const DigitItem*>(src)[j].nw);
     if (kind == 22)
@@ -835,8 +936,8 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
       if (k == 0 && add(4, wl_diag_[L(0)].data(), sizeof(WorkItem), wl_diag_[L(0)].size(), 0, sm, pending))
         pending = -1;
       const bool next = k + 1 < max_panels && !wl_diag_[L(k + 1)].empty();
-      std::vector<GemmItem>& rest3 = k % group_ != group_ - 1 ? gl_k3a_[L(k)] : gl_k3_[L(k)];
-      if (next && !gl_k2n_[L(k)].empty() && !gl_k3d_[L(k)].empty()) {
+      std::vector<GemmItem>& rest3 = gl_k3_[L(k)];
+      if (next && ul_update_[L(k)].empty() && !gl_k2n_[L(k)].empty() && !gl_k3d_[L(k)].empty()) {
         const int ea = nev++, eb = nev++;
         add(5, gl_k2n_[L(k)].data(), sizeof(GemmItem), gl_k2n_[L(k)].size(), k, sm, pending, ea);
         pending = -1;
@@ -847,11 +948,15 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
         pending = eb;
         continue;
       }
-      // no next panel (or nothing to update ahead of it): everything on the main stream
+      // no next panel, nothing to update ahead of it, or a panel group on digit products ends
+      // here (its digits need the whole panel solve): everything on the main stream
       if (add(5, gl_k2n_[L(k)].data(), sizeof(GemmItem), gl_k2n_[L(k)].size(), k, sm, pending)) pending = -1;
       if (add(5, gl_k2_[L(k)].data(), sizeof(GemmItem), gl_k2_[L(k)].size(), k, sm, pending)) pending = -1;
       if (add(14, gl_k3d_[L(k)].data(), sizeof(GemmItem), gl_k3d_[L(k)].size(), k, sm, pending)) pending = -1;
       if (add(6, rest3.data(), sizeof(GemmItem), rest3.size(), k, sm, pending)) pending = -1;
+      if (add(27, fl_slice_[L(k)].data(), sizeof(FactorSliceItem), fl_slice_[L(k)].size(), k, sm, pending))
+        pending = -1;
+      if (add(28, ul_update_[L(k)].data(), sizeof(UpdateItem), ul_update_[L(k)].size(), k, sm, pending)) pending = -1;
       if (next && add(4, wl_diag_[L(k + 1)].data(), sizeof(WorkItem), wl_diag_[L(k + 1)].size(), k + 1, sm,
                       pending))
         pending = -1;
@@ -895,7 +1000,7 @@ static int stage_of(int kind) {
   switch (kind) {
     case 0: case 2: case 3: return 0;
     case 1: case 15: case 16: case 22: case 23: case 24: case 25: case 26: return 1;
-    case -1: case 4: case 5: case 6: case 14: return 2;
+    case -1: case 4: case 5: case 6: case 14: case 27: case 28: return 2;
     default: return 3;
   }
 }
@@ -936,6 +1041,10 @@ void Plan::record(cudaStream_t s0, int stage) {
         else launch_digit_syrk(L.arg, dl, L.count, L.ny, s);
         break;
       }
+      case 27:
+        launch_factor_slice(reinterpret_cast<const FactorSliceItem*>(lb + L.off), L.count, L.ny, s);
+        break;
+      case 28: launch_digit_update(reinterpret_cast<const UpdateItem*>(lb + L.off), L.count, L.ny, s); break;
       case 24: launch_digit_rowmax(probs_dev_, wl, L.count, s); break;
       case 2: init_rhs_kernel<<<L.count, 256, 0, s>>>(probs_dev_, wl); break;
       case 3: mnorm_kernel<<<L.count, 256, 0, s>>>(probs_dev_, wl); break;

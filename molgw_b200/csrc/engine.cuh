@@ -90,7 +90,7 @@ struct Shape {
   int naux, nocc, nvirt, nomega, nstate_p, nsig, nc, nsigma_half, technique, precision;
   int qp_only;
   int nocc2 = 0, nvirt2 = 0;   // second spin channel of the W window
-  int no_digits = 0;           // FP64 chi0 by DMMA alone: set where the digit buffers do not fit
+  int no_digits = 0;           // FP64 products by DMMA alone: set where the digit buffers do not fit
   bool operator<(const Shape& o) const;
 };
 
@@ -108,6 +108,10 @@ struct Tuning {
 int precision_class(const std::vector<Shape>& shapes);
 // Whether the FP64 chi0 of a problem goes through the int8 digit products.
 bool use_digits(const Shape& sh);
+// Whether the updates between panel groups of the factorization go through digit products, and
+// the panels of such a group.
+bool use_factor_digits(const Shape& sh);
+constexpr int kDigitGroup = 4;
 // Planes of the chi0 operands: 2 (bf16 hi/lo), 3 .. 7 (int8 digits), 0 (FP64 on DMMA).
 int operand_planes(const Shape& sh);
 // Bytes of one frequency's split operands of a problem (0 for FP64 on DMMA).
@@ -178,7 +182,9 @@ class Plan {
   // chi0 on tcgen05, by the number of operand planes (2: bf16, 3 .. 7: digits)
   std::vector<std::vector<WorkItem>> wl_slice_[8];         // per frequency group: planes of M D_w (first: and of M)
   std::vector<std::vector<DigitItem>> dl_syrk_[8];         // and the products
-  std::vector<std::vector<GemmItem>> gl_k2_, gl_k2n_, gl_k3_, gl_k3d_, gl_k3a_;
+  std::vector<std::vector<GemmItem>> gl_k2_, gl_k2n_, gl_k3_, gl_k3d_;
+  std::vector<std::vector<FactorSliceItem>> fl_slice_;   // digits of a finished panel group
+  std::vector<std::vector<UpdateItem>> ul_update_;       // and the update of the next group's rows
   std::vector<WorkItem> wl_trace_, wl_pad_;
   struct Launch {
     int kind;        // see Plan::record

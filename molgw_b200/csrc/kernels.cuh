@@ -115,6 +115,37 @@ struct DigitItem {
   int ld, nw;           // npad; frequencies covered
   long long sC;         // doubles between the eps blocks of two frequencies
 };
+// Update of finished rows on the digit products (digit_gemm.cu): C -= A^T B with A and B columns
+// of [U | U^-T | U^-T M_sigma], digits of all rows above the tile, frequency = blockIdx.y.
+struct UpdateItem {
+  const void* maps;     // tensor maps of the problem's factor digits
+  double* C;            // first row and column of the tile's region for j = 0
+  int* err;
+  const int* exps;      // [slab][group][128 nrb] column exponents
+  int rb_a, rb_b;       // digit blocks of the output rows (two, of rows_a) and of the columns
+  int nrb, nkt;         // digit blocks and k-tiles of a slab
+  int nk, chunk;        // k-tiles summed; k-tiles per exponent group
+  int first;            // first group that contributes (columns of U^-T are zero above their own)
+  int ngroups;          // groups of a slab
+  int slab, step;       // slab (frequency) for j = 0, and its increment
+  int rows_a, ncol;     // row blocks present (1 or 2); columns stored
+  int diag;             // 1: blocks below the diagonal (rb_b < row block) are not stored
+  int ld, nw;
+  long long sC;         // doubles between the regions of two j
+};
+// Digits of a group of finished rows: 128 columns of U, U^-T or U^-T M_sigma.
+struct FactorSliceItem {
+  const double* src;    // [rows][ld] for j = 0
+  void* digits;
+  int* exps;
+  int ld, ncol, rows;
+  int nrb, nkt, rb, kt; // digit blocks and k-tiles of a slab; block of the columns, first k-tile
+  int ngroups, group;
+  int slab, step, nw;
+  long long s_src;
+};
+void launch_factor_slice(const FactorSliceItem* items, int n, int ny, cudaStream_t s);
+void launch_digit_update(const UpdateItem* items, int n, int ny, cudaStream_t s);
 void launch_digit_zero(const ProbDev* probs, const WorkItem* items, int n, cudaStream_t s);
 void launch_digit_rowmax(const ProbDev* probs, const WorkItem* items, int n, cudaStream_t s);
 // planes: digits per operand, 3 .. 7

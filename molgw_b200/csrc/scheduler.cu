@@ -150,7 +150,7 @@ Status solve_batch(Context& c, int n, const rigw_problem* probs, rigw_result* re
         s2.nomega = wc;
         if (Plan::measure({s2}, kPlanPartial) <= avail) break;
       }
-      if (wc >= 1 || !use_digits(sh)) break;
+      if (wc >= 1 || !(use_digits(sh) || use_factor_digits(sh))) break;
       sh.no_digits = 1;   // one frequency with its digit buffers does not fit: DMMA needs none
     }
     if (wc < 1)

@@ -82,6 +82,43 @@ def test_frequency_groups_and_mixed_batch(engine):
         assert np.abs(a.sigma_calc - b.sigma_calc).max() <= 1e-12 * np.abs(a.sigma_calc).max()
 
 
+def sigma_reference(inst, omega, weight, z):
+    no, nv = inst.nocc, inst.nvirt
+    de = (inst.energy[no:][None, :] - inst.energy[:no][:, None]).ravel()
+    docc = (inst.occupation[:no][:, None] - inst.occupation[no:][None, :]).ravel()
+    m = inst.m_ia.reshape(no * nv, -1)
+    out = np.zeros((2, z.size), complex)
+    for w, wt in zip(omega, weight):
+        eps = np.eye(inst.naux) + m.T @ (m * (2.0 * docc * de / (w * w + de * de))[:, None])
+        for s in range(2):
+            v = np.einsum("pi,pi->p", inst.m_sigma[s], np.linalg.solve(eps, inst.m_sigma[s].T).T) - \
+                np.sum(inst.m_sigma[s] ** 2, axis=1)
+            x = z[:, None] - inst.energy[None, :]
+            out[s] -= wt / (2 * np.pi) * ((1.0 / (x + 1j * w) + 1.0 / (x - 1j * w)) @ v)
+    return out
+
+
+@pytest.mark.parametrize("nocc,nvirt,naux,nomega", [
+    (9, 60, 769, 3),       # seven panels: the group after the first has three
+    (8, 70, 1030, 5),      # nine panels: the last group has one, its pair of row blocks too
+    (10, 65, 1100, 2),     # M columns that end inside a 128-column block
+])
+@pytest.mark.parametrize("qp_only", [False, True])
+def test_factorization_updates_by_digits(engine, nocc, nvirt, naux, nomega, qp_only):
+    """The updates between panel groups on digit products: chi from the identity part and
+    Sigma_c from the M columns.  |U^-T M|^2 - |M|^2 is a difference of sums of naux terms, each
+    rounded: 1e-13 of the largest Sigma covers naux u sqrt(naux) for these sizes."""
+    from molgw_b200.rigw import imag_grid
+    inst = molecule(nocc, nvirt, naux, nomega, seed=naux)
+    if not qp_only:
+        check(engine, inst)
+    om, wt = imag_grid(nomega)
+    out = engine.g0w0(inst, qp_only=qp_only)
+    ef = 0.5 * (inst.energy[nocc - 1] + inst.energy[nocc])
+    ref = sigma_reference(inst, om, wt, ef + 1j * inst.step_sigma_calc * np.arange(inst.nomega_sigma_calc))
+    assert np.abs(out.sigma_calc - ref).max() <= 1e-13 * np.abs(ref).max()
+
+
 @pytest.mark.parametrize("bad", [np.nan, np.inf])
 def test_non_finite_input_is_reported(engine, bad):
     inst = molecule(9, 64, 384, 2, seed=8)
