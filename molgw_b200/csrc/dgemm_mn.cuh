@@ -19,6 +19,7 @@ enum GemmFlags : int {
   kUpperA = 4,        // A[k][m] = 0 for k > m, with m counted from the item's first row (the
                       // triangular inverse of the panel solves): the warps of rows
                       // m < wm0 + 64 skip the MMAs of k >= wm0 + 64, which add exact zeros
+  kTransposed = 8,    // element (m, n) is stored at C[n * ldc + m] (plain products only)
 };
 
 struct GemmItem {
@@ -192,6 +193,21 @@ dgemm_mn_kernel(const GemmItem* __restrict__ items) {
   // columns wn0 + 8j + 2r + e (j < 4, e < 2).
   const bool ident = (it.flags & (kAddIdentity | kSubIdentity)) != 0;
   const double idv = (it.flags & kSubIdentity) ? -1.0 : 1.0;
+  if (it.flags & kTransposed) {   // rows 8q .. 8q + 7 of a column are contiguous: 64 bytes
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int col = wn0 + 8 * j + 2 * r + e;
+        if (col >= it.n) continue;
+        double* dst = it.C + size_t(col) * it.ldc + wm0 + 8 * q;
+#pragma unroll
+        for (int i = 0; i < 8; i += 2)
+          if (wm0 + 8 * q + i < it.m)
+            *reinterpret_cast<double2*>(dst + i) = make_double2(it.alpha * acc[i][j][e], it.alpha * acc[i + 1][j][e]);
+      }
+    return;
+  }
   double csq[4][2];
 #pragma unroll
   for (int j = 0; j < 4; ++j) csq[j][0] = csq[j][1] = 0.0;

@@ -17,8 +17,21 @@ void launch_dgemm_64x128(const GemmItem* items, int n, int ny, cudaStream_t s) {
   launch_dgemm<64, 128>(items, n, ny, s);
 }
 
+void launch_dgemm_256x32(const GemmItem* items, int n, int ny, cudaStream_t s) {
+  launch_dgemm<256, 32>(items, n, ny, s);
+}
+void launch_dgemm_128x64(const GemmItem* items, int n, int ny, cudaStream_t s) {
+  launch_dgemm<128, 64>(items, n, ny, s);
+}
+
 cudaError_t prepare_dgemm_kernels() {
-  cudaError_t e = cudaFuncSetAttribute(dgemm_mn_kernel<128, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  cudaError_t e = cudaFuncSetAttribute(dgemm_mn_kernel<256, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       int(DgemmCfg<256, 32>::kSmemBytes));
+  if (e != cudaSuccess) return e;
+  e = cudaFuncSetAttribute(dgemm_mn_kernel<128, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           int(DgemmCfg<128, 64>::kSmemBytes));
+  if (e != cudaSuccess) return e;
+  e = cudaFuncSetAttribute(dgemm_mn_kernel<128, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        int(DgemmCfg<128, 128>::kSmemBytes));
   if (e != cudaSuccess) return e;
   return cudaFuncSetAttribute(dgemm_mn_kernel<64, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize,

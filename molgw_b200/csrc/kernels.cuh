@@ -33,7 +33,9 @@ struct AomoUnpackItem {
   double* bfull;          // [nbf][nbf][naux_pad]
   int naux, naux_pad, npair, nbf, p0;
 };
-__global__ void aomo_unpack_kernel(const AomoUnpackItem* items);
+__global__ void aomo_unpack_kernel(AomoUnpackItem it);
+// out[r][p0 + P] = src[(n, m)][P]: rows r = n mc + m of naux entries from a chunk [n][mcp][pcp].
+__global__ void aomo_store_kernel(const double* src, double* out, int mc, int mcp, int pcp, int cnt, long long naux);
 
 // One 128 x 128 tile of a general tensor-core product A B^T of the AO->MO transform
 // (syrk_bf16x3.cu, syrk_ozaki.cu).
@@ -159,6 +161,8 @@ cudaError_t prepare_digit_kernels();
 // grid (n items) x (ny frequencies): CTAs with blockIdx.y >= item.nw return at once
 void launch_dgemm_128x128(const GemmItem* items, int n, int ny, cudaStream_t s);
 void launch_dgemm_64x128(const GemmItem* items, int n, int ny, cudaStream_t s);
+void launch_dgemm_256x32(const GemmItem* items, int n, int ny, cudaStream_t s);   // narrow products
+void launch_dgemm_128x64(const GemmItem* items, int n, int ny, cudaStream_t s);
 cudaError_t prepare_dgemm_kernels();
 
 }  // namespace rigw

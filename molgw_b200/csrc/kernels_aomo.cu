@@ -11,9 +11,8 @@
 
 namespace rigw {
 
-// item: tile of 32 pairs x 32 auxiliary functions; block (32, 8).
-__global__ void __launch_bounds__(256) aomo_unpack_kernel(const AomoUnpackItem* __restrict__ items) {
-  const AomoUnpackItem it = items[0];
+// Tile of 32 pairs x 32 auxiliary functions; block (32, 8).
+__global__ void __launch_bounds__(256) aomo_unpack_kernel(const AomoUnpackItem it) {
   const int pair0 = blockIdx.x * 32;
   const int paux0 = blockIdx.y * 32;          // relative to the chunk start p0
   __shared__ double tile[32][33];
@@ -40,6 +39,14 @@ __global__ void __launch_bounds__(256) aomo_unpack_kernel(const AomoUnpackItem* 
       it.bfull[(size_t(nu) * it.nbf + mu) * it.naux_pad + P] = v;
     }
   }
+}
+
+__global__ void __launch_bounds__(256) aomo_store_kernel(const double* __restrict__ src, double* __restrict__ out,
+                                                         int mc, int mcp, int pcp, int cnt, long long naux) {
+  const int r = blockIdx.x, n = r / mc, m = r % mc;
+  const double* s = src + (size_t(n) * mcp + m) * pcp;
+  double* d = out + size_t(r) * naux;
+  for (int q = threadIdx.x; q < cnt; q += 256) d[q] = s[q];
 }
 
 }  // namespace rigw

@@ -9,6 +9,7 @@ namespace rigw {
 
 namespace {
 inline int round_up(int v, int a) { return (v + a - 1) / a * a; }
+constexpr int kMaxGridY = 65535;
 
 Status run_gemm_items(Context& c, const std::vector<GemmItem>& items, bool wide) {
   if (items.empty()) return Status::ok();
@@ -135,31 +136,45 @@ Status eri_3center_mo(Context& c, int nbf, int nstate, int npair, int naux, cons
   if (mstate_min < 1 || mstate_max > nstate || mstate_min > mstate_max || nstate_min < 1 ||
       nstate_max > nstate || nstate_min > nstate_max)
     return Status::fail(RIGW_ERR_ARG, "eri_3center_mo: state ranges outside [1, %d]", nstate);
-  for (int q = 0; q < 2 * npair; ++q)
-    if (index_basis[q] < 1 || index_basis[q] > nbf)
-      return Status::fail(RIGW_ERR_ARG, "eri_3center_mo: index_basis entry %d out of [1, %d]", q, nbf);
+  // every pair present: the unpacked block is written completely and needs no clearing
+  size_t missing = size_t(nbf) * (nbf + 1) / 2;
+  std::vector<char> seen(size_t(npair) >= missing ? size_t(nbf) * nbf : 0, 0);
+  for (int q = 0; q < npair; ++q) {
+    const int a = index_basis[2 * q], b = index_basis[2 * q + 1];
+    if (a < 1 || a > nbf || b < 1 || b > nbf)
+      return Status::fail(RIGW_ERR_ARG, "eri_3center_mo: index_basis entry %d out of [1, %d]",
+                          2 * q + (a < 1 || a > nbf ? 0 : 1), nbf);
+    if (!seen.empty()) {
+      char& f = seen[size_t(std::max(a, b) - 1) * nbf + std::min(a, b) - 1];
+      missing -= f == 0;
+      f = 1;
+    }
+  }
   const int mc = mstate_max - mstate_min + 1, nc = nstate_max - nstate_min + 1;
   const int mcp = round_up(mc, 2), ncp = round_up(nc, 2);
-  // C^T restricted to the two ranges: ctm[mu][m], ctn[nu][n] (m, n contiguous, even widths)
-  std::vector<double> ctm(size_t(nbf) * mcp, 0.0), ctn(size_t(nbf) * ncp, 0.0);
-  for (int mu = 0; mu < nbf; ++mu) {
-    for (int m = 0; m < mc; ++m) ctm[size_t(mu) * mcp + m] = c_matrix[size_t(mstate_min - 1 + m) * nbf + mu];
-    for (int n = 0; n < nc; ++n) ctn[size_t(mu) * ncp + n] = c_matrix[size_t(nstate_min - 1 + n) * nbf + mu];
-  }
   // auxiliary chunk so that the unpacked (nu, mu, P) block stays below ~2 GB
   const size_t per_aux = size_t(nbf) * nbf * sizeof(double);
   int pc = int(std::max<size_t>(8, (size_t(2) << 30) / per_aux / 8 * 8));
   pc = std::min(pc, round_up(naux, 8));
   const int pcp = round_up(pc, 8);
-  DeviceBuffer b_ctm, b_ctn, b_idx, b_eri, b_full, b_t, b_out, b_item;
-  RIGW_TRY(b_ctm.allocate(&c, ctm.size() * 8, "aomo ctm"));
-  RIGW_TRY(b_ctn.allocate(&c, ctn.size() * 8, "aomo ctn"));
-  RIGW_TRY(b_idx.allocate(&c, size_t(2) * npair * sizeof(int), "aomo index"));
-  if (!on_dev) RIGW_TRY(b_eri.allocate(&c, size_t(pc) * npair * 8, "aomo eri3 chunk"));
-  RIGW_TRY(b_full.allocate(&c, size_t(nbf) * nbf * pcp * 8, "aomo unpacked"));
-  RIGW_TRY(b_t.allocate(&c, size_t(ncp) * nbf * pcp * 8, "aomo half"));
-  RIGW_TRY(b_out.allocate(&c, size_t(ncp) * mcp * pcp * 8, "aomo out chunk"));
-  RIGW_TRY(b_item.allocate(&c, sizeof(AomoUnpackItem), "aomo item"));
+  // One arena: every buffer of the call is allocated at once (each allocation waits for the
+  // stream), and the items of both FP64 products go up with one copy per chunk.
+  const int max_items = (ncp + 127) / 128 * ((nbf * pcp + 127) / 128) + ((mcp + 127) / 128) * ((pcp + 127) / 128) *
+                        ((nc + kMaxGridY - 1) / kMaxGridY) + 4;
+  size_t arena = 0;
+  auto take = [&](size_t bytes) {
+    const size_t o = arena;
+    arena += (std::max<size_t>(bytes, 1) + 255) / 256 * 256;
+    return o;
+  };
+  const size_t o_ctm = take(size_t(nbf) * mcp * 8), o_ctn = take(size_t(nbf) * ncp * 8), o_idx = take(size_t(2) * npair * sizeof(int));
+  const size_t o_eri = take(on_dev ? 0 : size_t(pc) * npair * 8);
+  const size_t o_full = take(size_t(nbf) * nbf * pcp * 8), o_t = take(size_t(ncp) * nbf * pcp * 8);
+  const size_t o_out = take(size_t(ncp) * mcp * pcp * 8);
+  const size_t o_item = take(split ? 0 : size_t(max_items) * sizeof(GemmItem));
+  DeviceBuffer b_all;
+  RIGW_TRY(b_all.allocate(&c, arena, "aomo buffers"));
+  char* const ab = b_all.data();
   cudaStream_t s = c.stream;
   // stage times (CUDA events on the stream): AO tensor upload + unpack, the two
   // products with their operand splits, result download
@@ -179,14 +194,25 @@ Status eri_3center_mo(Context& c, int nbf, int nstate, int npair, int naux, cons
     return double(ms);
   };
   RIGW_CUDA_TRY(cudaEventRecord(ev.e[4], s));
-  RIGW_CUDA_TRY(cudaMemcpyAsync(b_ctm.data(), ctm.data(), ctm.size() * 8, cudaMemcpyHostToDevice, s));
-  RIGW_CUDA_TRY(cudaMemcpyAsync(b_ctn.data(), ctn.data(), ctn.size() * 8, cudaMemcpyHostToDevice, s));
-  RIGW_CUDA_TRY(cudaMemcpyAsync(b_idx.data(), index_basis, size_t(2) * npair * sizeof(int), cudaMemcpyHostToDevice, s));
-  double* dctm = reinterpret_cast<double*>(b_ctm.data());
-  double* dctn = reinterpret_cast<double*>(b_ctn.data());
-  double* dfull = reinterpret_cast<double*>(b_full.data());
-  double* dt = reinterpret_cast<double*>(b_t.data());
-  double* dout = reinterpret_cast<double*>(b_out.data());
+  RIGW_CUDA_TRY(cudaMemcpyAsync(ab + o_idx, index_basis, size_t(2) * npair * sizeof(int), cudaMemcpyHostToDevice, s));
+  double* dctm = reinterpret_cast<double*>(ab + o_ctm);
+  double* dctn = reinterpret_cast<double*>(ab + o_ctn);
+  double* dfull = reinterpret_cast<double*>(ab + o_full);
+  double* dt = reinterpret_cast<double*>(ab + o_t);
+  double* dout = reinterpret_cast<double*>(ab + o_out);
+  std::vector<double> ctm, ctn;
+  auto upload_c = [&]() -> Status {
+    // C^T restricted to the two ranges: ctm[mu][m], ctn[nu][n] (m, n contiguous, even widths)
+    ctm.assign(size_t(nbf) * mcp, 0.0);
+    ctn.assign(size_t(nbf) * ncp, 0.0);
+    for (int mu = 0; mu < nbf; ++mu) {
+      for (int m = 0; m < mc; ++m) ctm[size_t(mu) * mcp + m] = c_matrix[size_t(mstate_min - 1 + m) * nbf + mu];
+      for (int n = 0; n < nc; ++n) ctn[size_t(mu) * ncp + n] = c_matrix[size_t(nstate_min - 1 + n) * nbf + mu];
+    }
+    RIGW_CUDA_TRY(cudaMemcpyAsync(ab + o_ctm, ctm.data(), ctm.size() * 8, cudaMemcpyHostToDevice, s));
+    RIGW_CUDA_TRY(cudaMemcpyAsync(ab + o_ctn, ctn.data(), ctn.size() * 8, cudaMemcpyHostToDevice, s));
+    return Status::ok();
+  };
   // split precision: C^T blocks split once; the unpacked tensor and the half
   // transform are split per auxiliary chunk (BF16x3 products, FP64 results)
   const int Kp = round_up(nbf, ns > 0 ? 128 : 64);   // 64 bf16 or 128 int8 per k-tile
@@ -197,6 +223,7 @@ Status eri_3center_mo(Context& c, int nbf, int nstate, int npair, int naux, cons
   char* maps = nullptr;
   int* errp = nullptr;
   if (split) {
+    RIGW_TRY(upload_c());
     RIGW_TRY(s_maps.allocate(&c, 4 * 128, "split tensor maps"));
     RIGW_TRY(s_err.allocate(&c, sizeof(int), "split error flag"));
     maps = s_maps.data();
@@ -222,18 +249,20 @@ Status eri_3center_mo(Context& c, int nbf, int nstate, int npair, int naux, cons
     RIGW_CUDA_TRY(cudaEventRecord(ev.e[0], s));
     const double* chunk = eri3 + size_t(p0) * npair;
     if (!on_dev) {
-      RIGW_CUDA_TRY(cudaMemcpyAsync(b_eri.data(), chunk, size_t(cnt) * npair * 8, cudaMemcpyHostToDevice, s));
-      chunk = reinterpret_cast<const double*>(b_eri.data());
+      RIGW_CUDA_TRY(cudaMemcpyAsync(ab + o_eri, chunk, size_t(cnt) * npair * 8, cudaMemcpyHostToDevice, s));
+      chunk = reinterpret_cast<const double*>(ab + o_eri);
     }
-    RIGW_CUDA_TRY(cudaMemsetAsync(dfull, 0, size_t(nbf) * nbf * pcp * 8, s));
-    AomoUnpackItem it{chunk, reinterpret_cast<const int*>(b_idx.data()), dfull, cnt, pcp, npair, nbf, 0};
-    RIGW_CUDA_TRY(cudaMemcpyAsync(b_item.data(), &it, sizeof(it), cudaMemcpyHostToDevice, s));
+    // columns P >= cnt of the last chunk stay as they are: no product mixes columns, and they
+    // are not copied out (the split paths scale rows of this block by column P, too)
+    if (missing) RIGW_CUDA_TRY(cudaMemsetAsync(dfull, 0, size_t(nbf) * nbf * pcp * 8, s));
+    const AomoUnpackItem it{chunk, reinterpret_cast<const int*>(ab + o_idx), dfull, cnt, pcp, npair, nbf, 0};
     dim3 grid((npair + 31) / 32, (cnt + 31) / 32);
-    aomo_unpack_kernel<<<grid, 256, 0, s>>>(reinterpret_cast<const AomoUnpackItem*>(b_item.data()));
+    aomo_unpack_kernel<<<grid, 256, 0, s>>>(it);
     RIGW_CUDA_TRY(cudaGetLastError());
     RIGW_CUDA_TRY(cudaEventRecord(ev.e[1], s));
     launches += 1 + (split ? (ns > 0 ? 6 : 4) : 2);
     const int wide = nbf * pcp;
+    bool stored = false;      // the products wrote the caller's array
     if (split) {
       // step 1: T[n][j] = sum_nu ctn^T[n][nu] B^T[j][nu],  j = (mu, P)
       const SplitOp b1{dfull, 1, wide, 0, wide, nbf, Rpw, Kp, 1, nullptr, 0};
@@ -301,9 +330,33 @@ Status eri_3center_mo(Context& c, int nbf, int nstate, int npair, int naux, cons
       RIGW_TRY(c.sync(s));
       if (herr) return Status::fail(RIGW_ERR_TIMEOUT, "eri_3center_mo: a bounded device wait expired");
     } else {
-    // step 1: T[n][(mu,P)] = sum_nu ctn[nu][n] B[nu][(mu,P)]
-    std::vector<GemmItem> g1;
-    for (int i0 = 0; i0 < ncp; i0 += 128)
+    // step 1: T[n][(mu,P)] = sum_nu ctn[nu][n] B[nu][(mu,P)].  Few n (the occupied states): the
+    // (mu,P) side takes the rows of the tile and the result is stored transposed, since a
+    // 128-row tile over n would multiply mostly padding (21 states: 0.44 ms of 0.54; 0.1 ms so).
+    // The items cover runs of equal tiles (grid y), so the list is a few entries long; C^T and
+    // the list are made on the host while the tensor is unpacked.
+    if (p0 == 0) RIGW_TRY(upload_c());
+    std::vector<GemmItem> items;
+    const int bm = ncp <= 32 ? 256 : 128, bn = ncp <= 32 ? 32 : (ncp <= 64 ? 64 : 128);
+    for (int i0 = 0; bn < 128 && i0 < wide;) {
+      GemmItem g{};
+      g.nw = std::max(1, std::min((wide - i0) / bm, kMaxGridY));   // whole tiles, then the rest
+      g.A = dfull + i0;
+      g.lda = wide;
+      g.B = dctn;
+      g.ldb = ncp;
+      g.C = dt + i0;
+      g.ldc = wide;
+      g.m = std::min(bm, wide - i0);
+      g.n = ncp;
+      g.k = nbf;
+      g.flags = kTransposed;
+      g.alpha = 1.0;
+      g.sA = g.sC = bm;
+      items.push_back(g);
+      i0 += g.nw * bm;
+    }
+    for (int i0 = 0; bn == 128 && i0 < ncp; i0 += 128)
       for (int j0 = 0; j0 < wide; j0 += 128) {
         GemmItem g{};
         g.A = dctn + i0;
@@ -316,35 +369,53 @@ Status eri_3center_mo(Context& c, int nbf, int nstate, int npair, int naux, cons
         g.n = std::min(128, wide - j0);
         g.k = nbf;
         g.alpha = 1.0;
-        g1.push_back(g);
+        items.push_back(g);
       }
-    RIGW_TRY(run_gemm_items(c, g1, true));
-    // step 2: O[n][m][P] = sum_mu ctm[mu][m] T[n][mu][P]
-    std::vector<GemmItem> g2;
-    for (int n = 0; n < nc; ++n)
+    const int c1 = int(items.size());
+    // step 2: O[n][m][P] = sum_mu ctm[mu][m] T[n][mu][P], into the caller's device array where
+    // its rows can be written in 16-byte pairs
+    const bool direct = on_dev && cnt == naux && naux % 2 == 0 &&
+                        reinterpret_cast<uintptr_t>(out) % 16 == 0;
+    stored = direct;
+    for (int n = 0; n < nc; n += kMaxGridY)
       for (int i0 = 0; i0 < mcp; i0 += 128)
-        for (int j0 = 0; j0 < pcp; j0 += 128) {
+        for (int j0 = 0; j0 < (direct ? cnt : pcp); j0 += 128) {
           GemmItem g{};
+          g.nw = std::min(nc - n, kMaxGridY);
+          g.sB = wide;
+          g.sC = direct ? (long long)mc * naux : (long long)mcp * pcp;
           g.A = dctm + i0;
           g.lda = mcp;
           g.B = dt + size_t(n) * wide + j0;
           g.ldb = pcp;
-          g.C = dout + (size_t(n) * mcp + i0) * pcp + j0;
-          g.ldc = pcp;
-          g.m = std::min(128, mcp - i0);
-          g.n = std::min(128, pcp - j0);
+          g.C = direct ? out + (size_t(n) * mc + i0) * naux + j0 : dout + (size_t(n) * mcp + i0) * pcp + j0;
+          g.ldc = direct ? naux : pcp;
+          g.m = std::min(128, (direct ? mc : mcp) - i0);   // rows: an odd count is fine
+          g.n = std::min(128, (direct ? cnt : pcp) - j0);
           g.k = nbf;
           g.alpha = 1.0;
-          g2.push_back(g);
+          items.push_back(g);
         }
-    RIGW_TRY(run_gemm_items(c, g2, true));
+    const GemmItem* d_items = reinterpret_cast<const GemmItem*>(ab + o_item);
+    RIGW_CUDA_TRY(cudaMemcpyAsync(ab + o_item, items.data(), items.size() * sizeof(GemmItem), cudaMemcpyHostToDevice, s));
+    const int ny1 = std::max(1, items[0].nw), ny2 = std::min(nc, kMaxGridY);
+    if (bn == 32) launch_dgemm_256x32(d_items, c1, ny1, s);
+    else if (bn == 64) launch_dgemm_128x64(d_items, c1, ny1, s);
+    else launch_dgemm_128x128(d_items, c1, 1, s);
+    launch_dgemm_128x128(d_items + c1, int(items.size()) - c1, ny2, s);
+    RIGW_CUDA_TRY(cudaGetLastError());
     }
     // out[n][m][p0 : p0+cnt]
     RIGW_CUDA_TRY(cudaEventRecord(ev.e[2], s));
-    for (int n = 0; n < nc; ++n)
-      RIGW_CUDA_TRY(cudaMemcpy2DAsync(out + (size_t(n) * mc) * naux + p0, size_t(naux) * 8,
-                                      dout + size_t(n) * mcp * pcp, size_t(pcp) * 8, size_t(cnt) * 8, mc,
-                                      on_dev ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, s));
+    if (on_dev) {
+      if (!stored) aomo_store_kernel<<<nc * mc, 256, 0, s>>>(dout, out + p0, mc, mcp, pcp, cnt, naux);
+      RIGW_CUDA_TRY(cudaGetLastError());
+    } else {
+      for (int n = 0; n < nc; ++n)
+        RIGW_CUDA_TRY(cudaMemcpy2DAsync(out + (size_t(n) * mc) * naux + p0, size_t(naux) * 8,
+                                        dout + size_t(n) * mcp * pcp, size_t(pcp) * 8, size_t(cnt) * 8, mc,
+                                        cudaMemcpyDeviceToHost, s));
+    }
     RIGW_CUDA_TRY(cudaEventRecord(ev.e[3], s));
     RIGW_CUDA_TRY(cudaStreamSynchronize(s));
     stage[0] += elapsed(0, 1);

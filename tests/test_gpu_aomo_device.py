@@ -36,6 +36,37 @@ def test_device_mode_equals_host_mode(engine, precision):
         assert np.array_equal(host, dev.cpu().numpy())
 
 
+@pytest.mark.parametrize("nbf,naux,ranges", [
+    (41, 96, (10, 41, 1, 9)),       # narrow tile of 32 states, an even number of auxiliary functions
+    (150, 131, (34, 149, 1, 33)),   # 64 states, odd number of auxiliary functions: rows copied out
+    (150, 130, (70, 150, 2, 66)),   # 65 states: the 128-row tile
+    (37, 64, (5, 5, 1, 32)),        # one state on the wide side, all 32 columns used
+])
+@pytest.mark.parametrize("screened", [False, True])
+def test_first_product_tiles(engine, nbf, naux, ranges, screened):
+    """The first product's tile follows the number of states n, and the unpacked block is
+    cleared only where pairs are missing.  Two FP64 sums of nbf terms of size 1 x 1/sqrt(nbf):
+    an error of 4 nbf u max|B| covers both orders of summation."""
+    import torch
+    rng = np.random.default_rng(nbf + naux)
+    pairs = _pairs(nbf)
+    if screened:
+        pairs = pairs[rng.random(len(pairs)) > 0.1]
+    eri3 = rng.standard_normal((naux, len(pairs)))
+    c = np.linalg.qr(rng.standard_normal((nbf, nbf)))[0].T.copy()
+    full = np.zeros((naux, nbf, nbf))
+    full[:, pairs[:, 0] - 1, pairs[:, 1] - 1] = eri3
+    full = full + full.transpose(0, 2, 1)
+    m0, m1, n0, n1 = ranges
+    ref = np.einsum("na,Pab,mb->nmP", c[n0 - 1:n1], full, c[m0 - 1:m1], optimize=True)
+    dirty = torch.full((1 << 24,), float("nan"), dtype=torch.float64, device="cuda")
+    del dirty                                     # whatever the arena holds must not reach the result
+    dev = engine.calculate_eri_3center_mo(torch.from_numpy(eri3).cuda(), pairs, c, m0, m1, n0, n1).cpu().numpy()
+    host = engine.calculate_eri_3center_mo(eri3, pairs, c, m0, m1, n0, n1)
+    assert np.array_equal(dev, host)
+    assert np.abs(dev - ref).max() <= 4 * nbf * 2.0 ** -53 * np.abs(full).max() * np.sqrt(nbf)
+
+
 def test_ao_tensor_to_qp_energies_he(engine):
     """The He AO tensor B(mu nu, P) (pair-packed, diagonal x0.5 as the reference
     stores it, src/m_eri_calculate.f90:1841) and the HF orbitals through both
