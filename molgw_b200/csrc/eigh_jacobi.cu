@@ -9,6 +9,12 @@
 // orthogonal Q.  (Solving S to convergence instead changes neither the number
 // of outer sweeps nor the result: on the test matrices both take 11 outer
 // sweeps at n = 512, the single inner sweep with a quarter of the inner work.)
+// The entries inside A_II and A_JJ are rotated in the first round of a sweep
+// only, where every block is in one pair (63 inner rounds); the other rounds
+// rotate the 32 x 32 entries of A_IJ alone (32 inner rounds), so a sweep visits
+// every entry once instead of the inner ones nb - 1 times.  That takes one outer
+// sweep more (12 at n = 512) and half the inner work: 22 matrices of 512,
+// subproblems 21.2 -> 11 ms, the whole batch 32.3 -> 23 ms.
 // The whole matrix is then updated with the round's rotation J (the pairs' Q
 // embedded at their rows and columns): every row and column belongs to exactly
 // one pair, so tile (p, q) of J^T A J is Q_p^T A[P, Q] Q_q and depends only on
@@ -77,6 +83,18 @@ __global__ void __launch_bounds__(1024) eigh_init_kernel(const double* __restric
   }
 }
 
+// Pair k of inner round r: all pairs of the 64 indices over 63 rounds, or, kCross,
+// those of one index from each block over 32.
+template <bool kCross>
+RIGW_DEVICE_INLINE void inner_pair(int r, int k, int& a, int& b) {
+  if (kCross) {
+    a = k;
+    b = kB + ((k + r) & (kB - 1));
+  } else {
+    rr_pair(r, k, kS, a, b);
+  }
+}
+
 // One cyclic Jacobi sweep on the 64 x 64 symmetric S (stride kLd) in shared
 // memory, accumulating the rotations into Q (starts as the identity).  Per round:
 // warp 0 forms the round's 32 rotations (lane k: pair k); then, after one barrier,
@@ -107,6 +125,7 @@ RIGW_DEVICE_INLINE void rotate_block(double* S, int ak, int bk, int al, int bl, 
   }
 }
 
+template <bool kCross>
 __device__ void inner_jacobi_sweep(double* S, double* Q, double* cs, double* sn, const int* blk, double tau) {
   const int tid = threadIdx.x;
   constexpr int kNblk = (kS / 2) * (kS / 2 + 1) / 2;   // upper 2 x 2 block pairs (528)
@@ -122,10 +141,10 @@ __device__ void inner_jacobi_sweep(double* S, double* Q, double* cs, double* sn,
     bl[m] = kl >> 8;
   }
   const int kq = tid & 31, g = tid >> 5;   // Q: pair kq, rows 8 g .. 8 g + 7
-  for (int r = 0; r < kS - 1; ++r) {
+  for (int r = 0; r < (kCross ? kB : kS - 1); ++r) {
     if (tid < 32) {
       int a, b;
-      rr_pair(r, tid, kS, a, b);
+      inner_pair<kCross>(r, tid, a, b);
       const double apq = S[a * kLd + b];
       double c = 1.0, s = 0.0;
       if (fabs(apq) > tau) {
@@ -145,8 +164,8 @@ __device__ void inner_jacobi_sweep(double* S, double* Q, double* cs, double* sn,
 #pragma unroll
       for (int m = 0; m < 2; ++m) {
         act[m] = sn[bk[m]] != 0.0 || sn[bl[m]] != 0.0;
-        rr_pair(r, bk[m], kS, ia[m][0], ia[m][1]);
-        rr_pair(r, bl[m], kS, ia[m][2], ia[m][3]);
+        inner_pair<kCross>(r, bk[m], ia[m][0], ia[m][1]);
+        inner_pair<kCross>(r, bl[m], ia[m][2], ia[m][3]);
         if (!act[m]) continue;
         x[m][0] = S[ia[m][0] * kLd + ia[m][2]];
         x[m][1] = S[ia[m][0] * kLd + ia[m][3]];
@@ -161,8 +180,8 @@ __device__ void inner_jacobi_sweep(double* S, double* Q, double* cs, double* sn,
     }
     if (bk[2] >= 0 && (sn[bk[2]] != 0.0 || sn[bl[2]] != 0.0)) {
       int ak, bkk, al, bll;
-      rr_pair(r, bk[2], kS, ak, bkk);
-      rr_pair(r, bl[2], kS, al, bll);
+      inner_pair<kCross>(r, bk[2], ak, bkk);
+      inner_pair<kCross>(r, bl[2], al, bll);
       const double x00 = S[ak * kLd + al], x01 = S[ak * kLd + bll], x10 = S[bkk * kLd + al], x11 = S[bkk * kLd + bll];
       rotate_block(S, ak, bkk, al, bll, bk[2] != bl[2], cs[bk[2]], sn[bk[2]], cs[bl[2]], sn[bl[2]], x00, x01, x10,
                    x11);
@@ -172,7 +191,7 @@ __device__ void inner_jacobi_sweep(double* S, double* Q, double* cs, double* sn,
     if (sq != 0.0) {
       const double cq = cs[kq];
       int qa_i, qb_i;
-      rr_pair(r, kq, kS, qa_i, qb_i);
+      inner_pair<kCross>(r, kq, qa_i, qb_i);
       double qa[8], qb[8];
 #pragma unroll
       for (int jj = 0; jj < 8; ++jj) {
@@ -190,8 +209,9 @@ __device__ void inner_jacobi_sweep(double* S, double* Q, double* cs, double* sn,
 }
 
 // One CTA per (pair k of round r, matrix w = blockIdx.y): one sweep on the
-// subproblem, its Q to Qbuf.  flags[w][k] says whether the pair rotated;
+// subproblem (kCross: on the pairs of A_IJ, and only their entries decide), its Q to Qbuf.  flags[w][k] says whether the pair rotated;
 // rot[w] whether any pair of matrix w did.
+template <bool kCross>
 __global__ void __launch_bounds__(kThreads, 3) eigh_pair_kernel(const double* __restrict__ Aall,
                                                              double* __restrict__ Qbuf, int* __restrict__ flags,
                                                              int* __restrict__ rot, const double* __restrict__ tau,
@@ -214,7 +234,7 @@ __global__ void __launch_bounds__(kThreads, 3) eigh_pair_kernel(const double* __
     const double x = A[size_t(sub_index(i, I, J)) * n + sub_index(j, I, J)];
     S[i * kLd + j] = x;
     Q[i * kLd + j] = (i == j) ? 1.0 : 0.0;
-    if (i != j && fabs(x) > tw) big = 1;
+    if ((kCross ? (i < kB && j >= kB) : i != j) && fabs(x) > tw) big = 1;
   }
   if (!__syncthreads_or(big)) {
     if (tid == 0) flags[w * npairs + k] = 0;
@@ -228,7 +248,7 @@ __global__ void __launch_bounds__(kThreads, 3) eigh_pair_kernel(const double* __
     for (int l = e; l < kS / 2; ++l) blk[row0 + l - e] = e | (l << 8);
   }
   __syncthreads();
-  inner_jacobi_sweep(S, Q, cs, sn, blk, 0.25 * tw);
+  inner_jacobi_sweep<kCross>(S, Q, cs, sn, blk, 0.25 * tw);
   if (tid == 0) {
     flags[w * npairs + k] = 1;
     atomicOr(rot + w, 1);
@@ -366,7 +386,8 @@ Status eigh_jacobi_batched(Context& c, double* A, double* V, int n, int nw, cuda
   if (n <= 0 || n % kS != 0 || nw <= 0)
     return Status::fail(RIGW_ERR_ARG, "eigh_jacobi_batched: n must be a positive multiple of %d", kS);
   // per device (cheap): the current device is the context's
-  RIGW_CUDA_TRY(cudaFuncSetAttribute(eigh_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kPairSmem)));
+  for (auto* k : {&eigh_pair_kernel<false>, &eigh_pair_kernel<true>})
+    RIGW_CUDA_TRY(cudaFuncSetAttribute(*k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kPairSmem)));
   RIGW_CUDA_TRY(cudaFuncSetAttribute(eigh_apply_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kApplySmem)));
   const int nb = n / kB, npairs = nb / 2, chunks = n / kS, ntri = npairs * (npairs + 1) / 2;
   const long long sA = (long long)n * n;
@@ -387,7 +408,8 @@ Status eigh_jacobi_batched(Context& c, double* A, double* V, int n, int nw, cuda
   for (; sweep < kOuterMaxSweeps && !converged; ++sweep) {
     RIGW_CUDA_TRY(cudaMemsetAsync(rot, 0, size_t(nw) * sizeof(int), s));
     for (int r = 0; r < nb - 1; ++r) {
-      eigh_pair_kernel<<<dim3(npairs, nw), kThreads, kPairSmem, s>>>(A, qbuf, flags, rot, tau, n, sA, r);
+      if (r == 0) eigh_pair_kernel<false><<<dim3(npairs, nw), kThreads, kPairSmem, s>>>(A, qbuf, flags, rot, tau, n, sA, r);
+      else eigh_pair_kernel<true><<<dim3(npairs, nw), kThreads, kPairSmem, s>>>(A, qbuf, flags, rot, tau, n, sA, r);
       eigh_apply_kernel<<<dim3(ntri + npairs * chunks, nw), kThreads, kApplySmem, s>>>(A, V, qbuf, flags, n, sA, r);
       nl += 2;
     }
