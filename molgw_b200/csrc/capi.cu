@@ -25,8 +25,9 @@ int finish(rigw_ctx* ctx, const Status& s) {
 }
 
 Status run_batch(Context& c, rigw::PlanMode mode, int n, const rigw_problem* probs, rigw_result* res,
-                 std::unique_ptr<Plan>* owned_plan, const std::vector<const rigw::ProbDev*>& factors,
-                 const double* const* sigma_in) {
+                 std::unique_ptr<Plan>* owned_plan, const Plan* parent, const double* const* sigma_in) {
+  std::vector<const rigw::ProbDev*> factors;   // of the W a Sigma plan reads
+  if (parent) factors.push_back(&const_cast<Plan*>(parent)->problems()[0].dev);
   std::vector<Shape> shapes(n);
   for (int i = 0; i < n; ++i) RIGW_TRY(rigw::make_shape(probs[i], &shapes[i]));
   if (mode != rigw::kPlanPolar)
@@ -36,26 +37,39 @@ Status run_batch(Context& c, rigw::PlanMode mode, int n, const rigw_problem* pro
   for (int i = 0; i < n; ++i)
     if (probs[i].precision != RIGW_FP64 && !rigw::bf16x3_available())
       return Status::fail(RIGW_ERR_UNSUPPORTED, "precision %d not available", probs[i].precision);
-  std::unique_ptr<Plan> fresh(new Plan());
-  Status bs = fresh->build(&c, mode, shapes, factors);
-  if (bs.code == RIGW_ERR_NOMEM && !c.plan_cache.empty()) {   // cached plans hold memory: drop them, retry once
-    c.plan_cache.clear();
+  // a plan of an earlier call of this kind, or a new one
+  std::unique_ptr<Plan> fresh = c.take_idle(mode, shapes, parent);
+  Status bs;
+  if (!fresh) {
     fresh.reset(new Plan());
     bs = fresh->build(&c, mode, shapes, factors);
-  }
-  if (bs.code == RIGW_ERR_NOMEM) {   // without the digit buffers of the FP64 products
-    bool any = false;
-    for (Shape& sh : shapes) {
-      any = any || rigw::use_digits(sh) || rigw::use_factor_digits(sh);
-      sh.no_digits = 1;
-    }
-    if (any) {
+    if (bs.code == RIGW_ERR_NOMEM && !c.plan_cache.empty()) {   // cached plans hold memory: drop them, retry once
+      c.plan_cache.clear();
       fresh.reset(new Plan());
       bs = fresh->build(&c, mode, shapes, factors);
+    }
+    if (bs.code == RIGW_ERR_NOMEM) {   // without the digit buffers of the FP64 products
+      bool any = false;
+      for (Shape& sh : shapes) {
+        any = any || rigw::use_digits(sh) || rigw::use_factor_digits(sh);
+        sh.no_digits = 1;
+      }
+      if (any) {
+        fresh.reset(new Plan());
+        bs = fresh->build(&c, mode, shapes, factors);
+      }
     }
   }
   RIGW_TRY(bs);
   Plan* plan = fresh.get();
+  // a W plan that fails here goes, and the idle Sigma plans on its factors with it
+  struct Guard {
+    Context& c;
+    std::unique_ptr<Plan>& p;
+    ~Guard() {
+      if (p) c.drop_children(p.get());
+    }
+  } guard{c, fresh};
   RIGW_TRY(plan->stage_inputs(probs, c.stream));
   if (sigma_in)
     for (int i = 0; i < n; ++i) RIGW_TRY(plan->stage_sigma_calc(i, sigma_in[i], c.stream));
@@ -73,6 +87,7 @@ Status run_batch(Context& c, rigw::PlanMode mode, int n, const rigw_problem* pro
   RIGW_TRY(err);
   if (res) RIGW_TRY(plan->fetch_results(probs, res, c.stream));
   if (owned_plan) *owned_plan = std::move(fresh);
+  else c.put_idle(std::move(fresh), parent);
   return Status::ok();
 }
 
@@ -156,7 +171,7 @@ int rigw_polarizability_imag(rigw_ctx* ctx, const rigw_problem* prob, double* er
   rigw_wpol* w = new (std::nothrow) rigw_wpol();
   if (!w) return finish(ctx, Status::fail(RIGW_ERR_NOMEM, "host allocation"));
   rigw_result r{};
-  Status s = run_batch(ctx->impl, rigw::kPlanPolar, 1, prob, &r, &w->impl.plan, {}, nullptr);
+  Status s = run_batch(ctx->impl, rigw::kPlanPolar, 1, prob, &r, &w->impl.plan, nullptr, nullptr);
   if (!s.good()) {
     delete w;
     return finish(ctx, s);
@@ -184,19 +199,15 @@ int rigw_gw_selfenergy_imag(rigw_ctx* ctx, const rigw_wpol* wpol, const rigw_pro
     return finish(ctx, Status::fail(RIGW_ERR_ARG, "problem does not match the resident polarizability"));
   std::lock_guard<std::mutex> lock(ctx->impl.mu);
   cudaSetDevice(ctx->impl.device);
-  std::vector<const rigw::ProbDev*> f{&wpol->impl.plan->problems()[0].dev};
-  std::unique_ptr<Plan> tmp;
-  return finish(ctx, run_batch(ctx->impl, rigw::kPlanSigma, 1, prob, result, &tmp, f, nullptr));
+  return finish(ctx, run_batch(ctx->impl, rigw::kPlanSigma, 1, prob, result, nullptr, wpol->impl.plan.get(), nullptr));
 }
 
-int rigw_wpol_release(rigw_ctx* ctx, rigw_wpol* wpol) {
+int rigw_wpol_release(rigw_ctx* /*ctx*/, rigw_wpol* wpol) {
   if (!wpol) return RIGW_ERR_ARG;
-  if (ctx) {
-    std::lock_guard<std::mutex> lock(ctx->impl.mu);
-    cudaSetDevice(ctx->impl.device);
-    delete wpol;
-    return RIGW_OK;
-  }
+  Context* own = wpol->impl.ctx;   // the context that made it (alive: it owns the plan's memory)
+  std::lock_guard<std::mutex> lock(own->mu);
+  cudaSetDevice(own->device);
+  own->put_idle(std::move(wpol->impl.plan), nullptr);
   delete wpol;
   return RIGW_OK;
 }
@@ -206,9 +217,8 @@ int rigw_qp_solve(rigw_ctx* ctx, const rigw_problem* prob, const double* sigma_c
   if (!prob || !sigma_calc || !result) return finish(ctx, Status::fail(RIGW_ERR_ARG, "null argument"));
   std::lock_guard<std::mutex> lock(ctx->impl.mu);
   cudaSetDevice(ctx->impl.device);
-  std::unique_ptr<Plan> tmp;
   const double* sc[1] = {sigma_calc};
-  return finish(ctx, run_batch(ctx->impl, rigw::kPlanQP, 1, prob, result, &tmp, {}, sc));
+  return finish(ctx, run_batch(ctx->impl, rigw::kPlanQP, 1, prob, result, nullptr, nullptr, sc));
 }
 
 int rigw_sox_selfenergy_imag(rigw_ctx* ctx, const rigw_sox_problem* prob, double* sigma_sox) {

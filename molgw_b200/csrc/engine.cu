@@ -69,7 +69,10 @@ Status DeviceBuffer::allocate(Context* ctx, size_t bytes, const char* name) {
     ctx->spare_bytes = 0;
     return Status::ok();   // already counted in in_use
   }
-  if (ctx->budget && ctx->in_use + bytes > ctx->budget) ctx->free_spare();
+  if (ctx->budget && ctx->in_use + bytes > ctx->budget) {
+    ctx->idle.clear();
+    ctx->free_spare();
+  }
   if (ctx->budget && ctx->in_use + bytes > ctx->budget)
     return Status::fail(RIGW_ERR_NOMEM, "%s: %zu bytes exceed the HBM budget (%zu in use of %zu)", name, bytes,
                         ctx->in_use, ctx->budget);
@@ -77,8 +80,9 @@ Status DeviceBuffer::allocate(Context* ctx, size_t bytes, const char* name) {
   // stays mapped in the pool and is handed to the next plan without remapping.
   const auto t0 = std::chrono::steady_clock::now();
   cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(&ptr_), bytes, ctx->stream);
-  if (e != cudaSuccess && ctx->spare_ptr) {   // the spare block may be what is missing
+  if (e != cudaSuccess && (ctx->spare_ptr || !ctx->idle.empty())) {   // what is kept may be what is missing
     cudaGetLastError();
+    ctx->idle.clear();
     ctx->free_spare();
     e = cudaMallocAsync(reinterpret_cast<void**>(&ptr_), bytes, ctx->stream);
   }
@@ -119,6 +123,44 @@ Status Context::reserve(size_t bytes) {
   RIGW_TRY(b.allocate(this, bytes, "reserved arena"));
   b.release();   // a block of at least kSpareMin bytes becomes the spare block
   return Status::ok();
+}
+
+std::unique_ptr<Plan> Context::take_idle(int mode, const std::vector<Shape>& shapes, const Plan* parent) {
+  for (size_t k = idle.size(); k-- > 0;) {
+    IdlePlan& e = idle[k];
+    if (e.mode != mode || e.parent != parent || e.shapes < shapes || shapes < e.shapes) continue;
+    std::unique_ptr<Plan> p = std::move(e.plan);
+    idle.erase(idle.begin() + k);
+    return p;
+  }
+  return nullptr;
+}
+
+void Context::drop_children(const Plan* parent) {
+  for (size_t k = idle.size(); k-- > 0;)
+    if (idle[k].parent == parent) idle.erase(idle.begin() + k);
+}
+
+size_t Context::idle_bytes() const {
+  size_t n = 0;
+  for (const IdlePlan& e : idle) n += e.plan->bytes();
+  return n;
+}
+
+void Context::put_idle(std::unique_ptr<Plan> plan, const Plan* parent) {
+  const Plan* raw = plan.get();
+  if (raw->bytes() > kIdleBytes) {
+    drop_children(raw);
+    return;
+  }
+  const int mode = raw->mode();
+  const std::vector<Shape> shapes = raw->shapes();
+  idle.push_back({mode, shapes, parent, std::move(plan)});
+  while (idle.size() > kIdlePlans || idle_bytes() > kIdleBytes) {
+    std::unique_ptr<Plan> old = std::move(idle.front().plan);
+    idle.erase(idle.begin());
+    drop_children(old.get());
+  }
 }
 
 void Context::free_spare() {
@@ -198,6 +240,7 @@ Status Context::sync(cudaStream_t s) {
 
 Context::~Context() {
   plan_cache.clear();
+  idle.clear();
   free_spare();
   if (stream) {
     cudaStreamSynchronize(stream);

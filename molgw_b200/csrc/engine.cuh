@@ -154,7 +154,7 @@ class Plan {
   Status check_errors(cudaStream_t s);
   float last_ms() const { return last_ms_; }
   std::vector<PlanProblem>& problems() { return probs_; }
-  size_t bytes() const { return arena_.size(); }
+  size_t bytes() const { return arena_.size() + lists_.size(); }
   PlanMode mode() const { return mode_; }
   const std::vector<Shape>& shapes() const { return shapes_; }
   ~Plan();
@@ -229,6 +229,24 @@ class Context {
   std::mutex mu;
   // plans by (mode, shapes); a repeated batch replays its CUDA graphs
   std::map<std::pair<int, std::vector<Shape>>, std::unique_ptr<Plan>> plan_cache;
+  // Plans of the stand-alone calls that are not in use (a released W, the Sigma and QP plans of
+  // finished calls): a repeated sequence of such calls finds its lists uploaded and its graphs
+  // captured.  A Sigma plan belongs to the W (parent) whose factors its items point to and goes
+  // with it.  At most kIdlePlans and kIdleBytes; all are given back when an allocation would
+  // fail, before an autotuning run and with the context.
+  struct IdlePlan {
+    int mode;
+    std::vector<Shape> shapes;
+    const Plan* parent;
+    std::unique_ptr<Plan> plan;
+  };
+  static constexpr size_t kIdlePlans = 6;
+  static constexpr size_t kIdleBytes = size_t(1) << 30;
+  std::vector<IdlePlan> idle;   // oldest first
+  std::unique_ptr<Plan> take_idle(int mode, const std::vector<Shape>& shapes, const Plan* parent);
+  void put_idle(std::unique_ptr<Plan> plan, const Plan* parent);
+  void drop_children(const Plan* parent);   // idle Sigma plans of a W that goes
+  size_t idle_bytes() const;
   bool use_graphs = true;
   rigw_stats last_stats{};
   double host_build_ms = 0.0, host_capture_ms = 0.0;   // host time in plan builds / graph captures

@@ -120,6 +120,7 @@ Status solve_batch(Context& c, int n, const rigw_problem* probs, rigw_result* re
   // plans cached for other shapes count as free memory for this decision
   size_t cached = 0;
   for (auto& kv : c.plan_cache) cached += kv.second->bytes();
+  cached += c.idle_bytes();
   const size_t usable = avail + cached;
 
   // ---- fits: one fused plan
@@ -135,6 +136,7 @@ Status solve_batch(Context& c, int n, const rigw_problem* probs, rigw_result* re
 
   // ---- frequency chunks and waves
   c.plan_cache.clear();
+  c.idle.clear();
   avail = available_bytes(c);
   struct Unit {
     int prob, w0, nw;
@@ -246,6 +248,7 @@ Status autotune(Context& c, int n, const rigw_problem* probs, rigw_tune_report* 
   RIGW_TRY(validate_batch(n, probs, &shapes));
   std::memset(rep, 0, sizeof(*rep));
   c.plan_cache.clear();
+  c.idle.clear();
   const size_t avail = available_bytes(c);
   const int cls = precision_class(shapes);
   bool any_fp64 = false;
@@ -324,6 +327,7 @@ Status autotune(Context& c, int n, const rigw_problem* probs, rigw_tune_report* 
   RIGW_TRY(try_field(&Tuning::panel_group, {2, 8, 16}, 2));
   c.tuned[{int(kPlanFused), cls}] = best;
   c.plan_cache.clear();
+  c.idle.clear();
   rep->chi0_rows = best.chi0_rows;
   rep->update_rows = best.update_rows;
   rep->split_group = best.split_group;

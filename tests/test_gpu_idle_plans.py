@@ -1,0 +1,79 @@
+"""Plans of the stand-alone calls that the context keeps between calls: a repeated sequence gives
+the same bits, a W in use is never handed out twice, a failed W takes its Sigma plans with it,
+and kept plans make room when an allocation needs it."""
+from dataclasses import replace
+
+import numpy as np
+import pytest
+
+from molgw_b200.rigw import Engine, RigwError
+from molgw_b200.synth import make_instance
+
+pytestmark = pytest.mark.gpu
+
+
+def sequence(eng, inst):
+    erpa, egw, w = eng.polarizability_grid_scalapack(inst)
+    s = eng.gw_selfenergy_imag_scalapack(w, inst)
+    q = eng.qp_solve(inst, s)
+    w.release()
+    return erpa, egw, s, q.energy_qp_g
+
+
+def same(a, b):
+    return a[0] == b[0] and a[1] == b[1] and np.array_equal(a[2], b[2]) and np.array_equal(a[3], b[3])
+
+
+def test_repeated_sequences_and_other_inputs():
+    a, b = make_instance(5, 40, 90, 8, seed=1), make_instance(5, 40, 90, 8, seed=2)   # same shapes
+    c = make_instance(6, 44, 140, 8, seed=3)
+    first = []
+    for inst in (a, b, c):
+        eng = Engine(0)
+        first.append(sequence(eng, inst))
+        eng.close()
+    eng = Engine(0)
+    for _ in range(3):                    # the third round replays captured graphs
+        for inst, ref in zip((a, b, c), first):
+            assert same(sequence(eng, inst), ref)
+    eng.close()
+
+
+def test_two_resident_w_of_one_shape():
+    a, b = make_instance(5, 40, 90, 8, seed=1), make_instance(5, 40, 90, 8, seed=2)
+    eng = Engine(0)
+    ra, rb = sequence(eng, a), sequence(eng, b)
+    _, _, wa = eng.polarizability_grid_scalapack(a)
+    _, _, wb = eng.polarizability_grid_scalapack(b)
+    for _ in range(2):
+        assert np.array_equal(eng.gw_selfenergy_imag_scalapack(wa, a), ra[2])
+        assert np.array_equal(eng.gw_selfenergy_imag_scalapack(wb, b), rb[2])
+    wa.release()
+    assert np.array_equal(eng.gw_selfenergy_imag_scalapack(wb, b), rb[2])
+    wb.release()
+    eng.close()
+
+
+def test_failed_w_is_not_kept():
+    good = make_instance(5, 40, 90, 8, seed=1)
+    bad = replace(good, occupation=2.0 - good.occupation, m_ia=good.m_ia * 3.0)   # chi0 > 1: not positive definite
+    eng = Engine(0)
+    ref = sequence(eng, good)
+    for _ in range(2):
+        with pytest.raises(RigwError):
+            eng.polarizability_grid_scalapack(bad)
+        assert same(sequence(eng, good), ref)
+    eng.close()
+
+
+def test_kept_plans_give_way_to_an_allocation():
+    small, large = make_instance(5, 40, 90, 8, seed=1), make_instance(8, 60, 260, 16, seed=4)
+    probe = Engine(0)
+    ref = sequence(probe, large)
+    peak = probe.last_stats()["device_bytes_peak"]
+    probe.close()
+    eng = Engine(0, hbm_budget_bytes=int(peak * 1.02))
+    sequence(eng, small)
+    sequence(eng, replace(small, nomega=6))
+    assert same(sequence(eng, large), ref)
+    eng.close()
