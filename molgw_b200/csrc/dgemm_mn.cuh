@@ -18,7 +18,7 @@ enum GemmFlags : int {
   kSubIdentity = 2,   // C -= 1 where (col - row) == diag
   kUpperA = 4,        // A[k][m] = 0 for k > m, with m counted from the item's first row (the
                       // triangular inverse of the panel solves): the warps of rows
-                      // m < wm0 + 64 skip the MMAs of k >= wm0 + 64, which add exact zeros
+                      // m < wm0 + WM skip the MMAs of k >= wm0 + WM, which add exact zeros
   kTransposed = 8,    // element (m, n) is stored at C[n * ldc + m] (plain products only)
 };
 
@@ -40,9 +40,10 @@ struct GemmItem {
   int nw;
 };
 
-template <int BM, int BN, int ST = 3>
+// WM: rows of a warp's tile (its columns are 32).
+template <int BM, int BN, int ST = 3, int WM = 64>
 struct DgemmCfg {
-  static constexpr int kWarpsM = BM / 64;
+  static constexpr int kWarpsM = BM / WM;
   static constexpr int kWarpsN = BN / 32;
   static constexpr int kThreads = kWarpsM * kWarpsN * 32;
   static constexpr int kBK = 16;
@@ -53,10 +54,11 @@ struct DgemmCfg {
   static constexpr size_t kSmemBytes = size_t(kStages) * kStageDoubles * sizeof(double);
 };
 
-template <int BM, int BN, int STAGES = 3>
-__global__ void __launch_bounds__(DgemmCfg<BM, BN, STAGES>::kThreads, 1)
+template <int BM, int BN, int STAGES = 3, int WM = 64>
+__global__ void __launch_bounds__(DgemmCfg<BM, BN, STAGES, WM>::kThreads, 1)
 dgemm_mn_kernel(const GemmItem* __restrict__ items) {
-  using Cfg = DgemmCfg<BM, BN, STAGES>;
+  using Cfg = DgemmCfg<BM, BN, STAGES, WM>;
+  constexpr int FM = WM / 8;   // 8-row fragments of a warp; lane (q, r) owns rows FM q ..
   constexpr int BK = Cfg::kBK;
   constexpr int ST = Cfg::kStages;
   constexpr int NT = Cfg::kThreads;
@@ -78,11 +80,11 @@ dgemm_mn_kernel(const GemmItem* __restrict__ items) {
   const int warp = tid >> 5;
   const int wm = warp % Cfg::kWarpsM;
   const int wn = warp / Cfg::kWarpsM;
-  const int wm0 = wm * 64;
+  const int wm0 = wm * WM;
   const int wn0 = wn * 32;
   const int ktiles = (it.k + BK - 1) / BK;
   const bool has_scale = it.kscale != nullptr;
-  const int klim = (it.flags & kUpperA) ? min(it.k, wm0 + 64) : it.k;   // warp-uniform
+  const int klim = (it.flags & kUpperA) ? min(it.k, wm0 + WM) : it.k;   // warp-uniform
 
   auto stage_a = [&](int s) { return smem + s * Cfg::kStageDoubles; };
   auto stage_b = [&](int s) { return smem + s * Cfg::kStageDoubles + BK * Cfg::kLdaS; };
@@ -116,9 +118,9 @@ dgemm_mn_kernel(const GemmItem* __restrict__ items) {
     }
   };
 
-  double acc[8][4][2];
+  double acc[FM][4][2];
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+  for (int i = 0; i < FM; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
 
@@ -152,16 +154,16 @@ dgemm_mn_kernel(const GemmItem* __restrict__ items) {
     }
     const int s = kt % ST;
     if (kt * BK >= klim) continue;   // this warp's rows see only zeros of A from here on
-    const double* as = stage_a(s) + wm0 + 8 * q;
+    const double* as = stage_a(s) + wm0 + FM * q;
     const double* bs = stage_b(s) + wn0 + q;
     const double* ks = stage_k(s);
 #pragma unroll
     for (int k4 = 0; k4 < BK / 4; ++k4) {
       const int kk = k4 * 4 + r;
-      double a[8], b[4];
+      double a[FM], b[4];
       const double2* ap = reinterpret_cast<const double2*>(as + kk * Cfg::kLdaS);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
+      for (int i = 0; i < FM / 2; ++i) {
         const double2 v = ap[i];
         a[2 * i] = v.x;
         a[2 * i + 1] = v.y;
@@ -169,13 +171,13 @@ dgemm_mn_kernel(const GemmItem* __restrict__ items) {
       if (has_scale) {
         const double sc = ks[kk];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) a[i] *= sc;
+        for (int i = 0; i < FM; ++i) a[i] *= sc;
       }
 #pragma unroll
       for (int j = 0; j < 4; ++j) b[j] = bs[kk * Cfg::kLdbS + 8 * j];
       if (nfrag == 4) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
+        for (int i = 0; i < FM; ++i)
 #pragma unroll
           for (int j = 0; j < 4; ++j) dmma_8x8x4(acc[i][j][0], acc[i][j][1], a[i], b[j]);
       } else {
@@ -183,27 +185,27 @@ dgemm_mn_kernel(const GemmItem* __restrict__ items) {
         for (int j = 0; j < 4; ++j)
           if (j < nfrag)
 #pragma unroll
-            for (int i = 0; i < 8; ++i) dmma_8x8x4(acc[i][j][0], acc[i][j][1], a[i], b[j]);
+            for (int i = 0; i < FM; ++i) dmma_8x8x4(acc[i][j][0], acc[i][j][1], a[i], b[j]);
       }
     }
   }
   cp_async_wait<0>();
 
-  // Epilogue.  Lane (q, r) of warp (wm, wn) owns rows wm0 + 8q + i (i < 8) and
+  // Epilogue.  Lane (q, r) of warp (wm, wn) owns rows wm0 + FM q + i (i < FM) and
   // columns wn0 + 8j + 2r + e (j < 4, e < 2).
   const bool ident = (it.flags & (kAddIdentity | kSubIdentity)) != 0;
   const double idv = (it.flags & kSubIdentity) ? -1.0 : 1.0;
-  if (it.flags & kTransposed) {   // rows 8q .. 8q + 7 of a column are contiguous: 64 bytes
+  if (it.flags & kTransposed) {   // the lane's FM rows of a column are contiguous
 #pragma unroll
     for (int j = 0; j < 4; ++j)
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
         const int col = wn0 + 8 * j + 2 * r + e;
         if (col >= it.n) continue;
-        double* dst = it.C + size_t(col) * it.ldc + wm0 + 8 * q;
+        double* dst = it.C + size_t(col) * it.ldc + wm0 + FM * q;
 #pragma unroll
-        for (int i = 0; i < 8; i += 2)
-          if (wm0 + 8 * q + i < it.m)
+        for (int i = 0; i < FM; i += 2)
+          if (wm0 + FM * q + i < it.m)
             *reinterpret_cast<double2*>(dst + i) = make_double2(it.alpha * acc[i][j][e], it.alpha * acc[i + 1][j][e]);
       }
     return;
@@ -212,8 +214,8 @@ dgemm_mn_kernel(const GemmItem* __restrict__ items) {
 #pragma unroll
   for (int j = 0; j < 4; ++j) csq[j][0] = csq[j][1] = 0.0;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int row = wm0 + 8 * q + i;
+  for (int i = 0; i < FM; ++i) {
+    const int row = wm0 + FM * q + i;
     if (row >= it.m) continue;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {

@@ -870,13 +870,13 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
           dst.push_back(g);
         };
         std::vector<GemmItem>& rest = gl_k3_[li];
+        if (factor && r0 < iend) k3(E, npad, E, npad, r0, r0, kPanel, kPanel, gl_k3d_[li]);
         for (int i0 = r0; i0 < iend; i0 += BM) {
           const int m = std::min(BM, iend - i0);
           if (factor)
-            for (int j0 = i0 / BMN * BMN; j0 < npad; j0 += BMN) {
-              const bool next_diag = i0 < r0 + kPanel && j0 == r0;
-              k3(E, npad, E, npad, i0, j0, m, std::min(BMN, npad - j0), next_diag ? gl_k3d_[li] : rest);
-            }
+            for (int j0 = i0 / BMN * BMN; j0 < npad; j0 += BMN)
+              if (i0 >= r0 + kPanel || j0 != r0)
+                k3(E, npad, E, npad, i0, j0, m, std::min(BMN, npad - j0), rest);
           // I block: columns below r0 only (the U rows of panel kp have zeros beyond it there)
           if (p.want_identity)
             for (int c0 = 0; c0 < r0; c0 += BMN) k3(R, ldb, R, ldb, i0, c0, m, std::min(BMN, r0 - c0), rest);
@@ -908,6 +908,27 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
   for (auto& planes : dl_syrk_)
     for (auto& l : planes)
       std::stable_sort(l.begin(), l.end(), [](const DigitItem& a, const DigitItem& b) { return a.nkt > b.nkt; });
+
+  // Products of the factorization that would leave SMs idle are cut into 32-column tiles.
+  // Returns whether the list was cut (the launch argument).
+  auto narrow = [&](std::vector<GemmItem>& l) {
+    size_t ctas = 0;
+    for (const GemmItem& g : l) ctas += std::max(g.nw, 1);
+    if (l.empty() || ctas > kNarrowCtas) return 0;
+    std::vector<GemmItem> cut;
+    for (const GemmItem& g : l)
+      for (int c = 0; c < g.n; c += 32) {
+        GemmItem t = g;
+        t.B += c;
+        t.C += c;
+        if (t.Cin) t.Cin += c;
+        if (t.colsq) t.colsq += c;
+        t.n = std::min(32, g.n - c);
+        cut.push_back(t);
+      }
+    l.swap(cut);
+    return 1;
+  };
 
   // ---- upload the lists and the launch sequence
   size_t lbytes = 0;
@@ -982,21 +1003,23 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
       std::vector<GemmItem>& rest3 = gl_k3_[L(k)];
       if (next && ul_update_[L(k)].empty() && !gl_k2n_[L(k)].empty() && !gl_k3d_[L(k)].empty()) {
         const int ea = nev++, eb = nev++;
-        add(5, gl_k2n_[L(k)].data(), sizeof(GemmItem), gl_k2n_[L(k)].size(), k, sm, pending, ea);
+        const int nn = narrow(gl_k2n_[L(k)]), nd = narrow(gl_k3d_[L(k)]), n2 = narrow(gl_k2_[L(k)]), n3 = narrow(rest3);
+        add(5, gl_k2n_[L(k)].data(), sizeof(GemmItem), gl_k2n_[L(k)].size(), nn, sm, pending, ea);
         pending = -1;
-        add(14, gl_k3d_[L(k)].data(), sizeof(GemmItem), gl_k3d_[L(k)].size(), k, sl, ea);
+        add(14, gl_k3d_[L(k)].data(), sizeof(GemmItem), gl_k3d_[L(k)].size(), nd, sl, ea);
         add(4, wl_diag_[L(k + 1)].data(), sizeof(WorkItem), wl_diag_[L(k + 1)].size(), k + 1, sl, -1, eb);
-        add(5, gl_k2_[L(k)].data(), sizeof(GemmItem), gl_k2_[L(k)].size(), k, sm);
-        add(6, rest3.data(), sizeof(GemmItem), rest3.size(), k, sm);
+        add(5, gl_k2_[L(k)].data(), sizeof(GemmItem), gl_k2_[L(k)].size(), n2, sm);
+        add(6, rest3.data(), sizeof(GemmItem), rest3.size(), n3, sm);
         pending = eb;
         continue;
       }
       // no next panel, nothing to update ahead of it, or a panel group on digit products ends
       // here (its digits need the whole panel solve): everything on the main stream
-      if (add(5, gl_k2n_[L(k)].data(), sizeof(GemmItem), gl_k2n_[L(k)].size(), k, sm, pending)) pending = -1;
-      if (add(5, gl_k2_[L(k)].data(), sizeof(GemmItem), gl_k2_[L(k)].size(), k, sm, pending)) pending = -1;
-      if (add(14, gl_k3d_[L(k)].data(), sizeof(GemmItem), gl_k3d_[L(k)].size(), k, sm, pending)) pending = -1;
-      if (add(6, rest3.data(), sizeof(GemmItem), rest3.size(), k, sm, pending)) pending = -1;
+      const int nn = narrow(gl_k2n_[L(k)]), nd = narrow(gl_k3d_[L(k)]), n2 = narrow(gl_k2_[L(k)]), n3 = narrow(rest3);
+      if (add(5, gl_k2n_[L(k)].data(), sizeof(GemmItem), gl_k2n_[L(k)].size(), nn, sm, pending)) pending = -1;
+      if (add(5, gl_k2_[L(k)].data(), sizeof(GemmItem), gl_k2_[L(k)].size(), n2, sm, pending)) pending = -1;
+      if (add(14, gl_k3d_[L(k)].data(), sizeof(GemmItem), gl_k3d_[L(k)].size(), nd, sm, pending)) pending = -1;
+      if (add(6, rest3.data(), sizeof(GemmItem), rest3.size(), n3, sm, pending)) pending = -1;
       if (add(27, fl_slice_[L(k)].data(), sizeof(FactorSliceItem), fl_slice_[L(k)].size(), k, sm, pending))
         pending = -1;
       if (add(28, ul_update_[L(k)].data(), sizeof(UpdateItem), ul_update_[L(k)].size(), k, sm, pending)) pending = -1;
@@ -1066,8 +1089,14 @@ void Plan::record(cudaStream_t s0, int stage) {
         if (tune_.chi0_rows == 128) launch_dgemm_128x128(gl, L.count, L.ny, s);
         else launch_dgemm_64x128(gl, L.count, L.ny, s);
         break;
-      case 6: case 14:
-        if (tune_.update_rows == 128) launch_dgemm_128x128(gl, L.count, L.ny, s);
+      case 14:   // the next diagonal block: one 128 x 128 item per frequency set
+        if (L.arg) launch_dgemm_128x32(gl, L.count, L.ny, s);
+        else launch_dgemm_128x128(gl, L.count, L.ny, s);
+        break;
+      case 6:
+        if (L.arg && tune_.update_rows == 128) launch_dgemm_128x32(gl, L.count, L.ny, s);
+        else if (L.arg) launch_dgemm_64x32(gl, L.count, L.ny, s);
+        else if (tune_.update_rows == 128) launch_dgemm_128x128(gl, L.count, L.ny, s);
         else launch_dgemm_64x128(gl, L.count, L.ny, s);
         break;
       case 15: trace_kernel<<<L.count, 256, 0, s>>>(probs_dev_, wl); break;
@@ -1092,7 +1121,10 @@ void Plan::record(cudaStream_t s0, int stage) {
       case 2: init_rhs_kernel<<<L.count, 256, 0, s>>>(probs_dev_, wl); break;
       case 3: mnorm_kernel<<<L.count, 256, 0, s>>>(probs_dev_, wl); break;
       case 4: chol_diag_kernel<<<L.count, kDiagThreads, chol_diag_smem_bytes(), s>>>(probs_dev_, wl, L.arg); break;
-      case 5: launch_dgemm_128x128(gl, L.count, L.ny, s); break;
+      case 5:
+        if (L.arg) launch_dgemm_128x32(gl, L.count, L.ny, s);
+        else launch_dgemm_128x128(gl, L.count, L.ny, s);
+        break;
       case 7: energy_kernel<<<L.count, 256, 0, s>>>(probs_dev_, wl); break;
       case 8: energy_sum_kernel<<<(L.count + 127) / 128, 128, 0, s>>>(probs_dev_, L.count); break;
       case 9: vchiv_kernel<<<L.count, 256, 0, s>>>(probs_dev_, wl); break;

@@ -163,6 +163,8 @@ void launch_dgemm_128x128(const GemmItem* items, int n, int ny, cudaStream_t s);
 void launch_dgemm_64x128(const GemmItem* items, int n, int ny, cudaStream_t s);
 void launch_dgemm_256x32(const GemmItem* items, int n, int ny, cudaStream_t s);   // narrow products
 void launch_dgemm_128x64(const GemmItem* items, int n, int ny, cudaStream_t s);
+void launch_dgemm_128x32(const GemmItem* items, int n, int ny, cudaStream_t s);   // 32-row warps
+void launch_dgemm_64x32(const GemmItem* items, int n, int ny, cudaStream_t s);
 cudaError_t prepare_dgemm_kernels();
 
 }  // namespace rigw
