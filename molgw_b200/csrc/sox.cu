@@ -74,7 +74,7 @@ struct SoxArgs {
   double* partial;     // [pc][gridDim.x][nw][2]
 };
 
-// One block per (unit stripe, Sigma state of the chunk).  Every thread keeps
+// One block per (unit stripe, Sigma state of the chunk, kSoxW points).  Every thread keeps
 // sum_e w_e (x / d) and sum_e w_e / d for kSoxW points (x = Re z - delta,
 // d = |z - delta|^2), so that sum_e w_e / (z - delta) = ar - i Im(z) as.  The
 // per-block sums go to `partial` in a fixed order (deterministic results).
@@ -85,7 +85,8 @@ __global__ void __launch_bounds__(kSoxThreads, 2) sox_contract_kernel(SoxArgs a)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const double* C = a.C + (long long)blockIdx.y * a.sp;
   const double* ev = a.e + a.no;
-  for (int w0 = 0; w0 < a.nw; w0 += kSoxW) {
+  {
+    const int w0 = blockIdx.z * kSoxW;
     const int nwc = min(kSoxW, a.nw - w0);
     double zr[kSoxW], zi2[kSoxW], ar[kSoxW], as[kSoxW];
 #pragma unroll
@@ -172,20 +173,25 @@ __global__ void __launch_bounds__(kSoxThreads, 2) sox_contract_kernel(SoxArgs a)
   }
 }
 
-// out[pl][w] = sum over blocks of partial[pl][blk][w], in block order.
+// out[pl][w] = sum over blocks of partial[pl][blk][w]: one warp per (pl, w), lanes over blocks,
+// a fixed tree (one thread walking the blocks took 80 us, each step a trip to L2; 4 us so).
 __global__ void sox_reduce_kernel(const double* __restrict__ partial, int nblk, int nw, int pc,
                                   double* __restrict__ out) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= pc * nw) return;
+  const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (t >= pc * nw) return;   // whole warps
   const int pl = t / nw, w = t % nw;
   double r = 0.0, im = 0.0;
-  for (int b = 0; b < nblk; ++b) {
+  for (int b = lane; b < nblk; b += 32) {
     const double* q = partial + (((long long)pl * nblk + b) * nw + w) * 2;
     r += q[0];
     im += q[1];
   }
-  out[2 * (long long)t] = r;
-  out[2 * (long long)t + 1] = im;
+  r = warp_sum(r);
+  im = warp_sum(im);
+  if (lane == 0) {
+    out[2 * (long long)t] = r;
+    out[2 * (long long)t + 1] = im;
+  }
 }
 
 }  // namespace
@@ -272,7 +278,8 @@ Status sox_selfenergy_imag(Context& c, const rigw_sox_problem& pr, double* sigma
   a.vt = (nv + kSoxTile - 1) / kSoxTile;
   a.tpairs = a.vt * (a.vt + 1) / 2;
   a.units = a.units1 + no * a.tpairs;
-  const int nblk = std::max(1, std::min(a.units, sms * 4 / pc));
+  // the points go over grid z, so two blocks per SM and point group balance the unit stripes
+  const int nblk = std::max(1, std::min(a.units, sms * 2 / pc));
   RIGW_TRY(b_part.allocate(&c, size_t(pc) * nblk * nw * 16, "sox partial sums"));
   a.partial = reinterpret_cast<double*>(b_part.data());
   double* out = sigma_sox;
@@ -316,10 +323,10 @@ Status sox_selfenergy_imag(Context& c, const rigw_sox_problem& pr, double* sigma
     RIGW_CUDA_TRY(cudaGetLastError());
     RIGW_CUDA_TRY(cudaEventRecord(e[3], s));
     a.C = cbuf;
-    sox_contract_kernel<<<dim3(nblk, pcn), kSoxThreads, 0, s>>>(a);
+    sox_contract_kernel<<<dim3(nblk, pcn, (nw + kSoxW - 1) / kSoxW), kSoxThreads, 0, s>>>(a);
     RIGW_CUDA_TRY(cudaGetLastError());
     const int nred = pcn * nw;
-    sox_reduce_kernel<<<(nred + 127) / 128, 128, 0, s>>>(a.partial, nblk, nw, pcn, out + size_t(p0) * nw * 2);
+    sox_reduce_kernel<<<(nred + 3) / 4, 128, 0, s>>>(a.partial, nblk, nw, pcn, out + size_t(p0) * nw * 2);
     RIGW_CUDA_TRY(cudaGetLastError());
     launches += 3;
     RIGW_CUDA_TRY(cudaEventRecord(e[1], s));
