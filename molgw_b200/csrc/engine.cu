@@ -604,9 +604,12 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
   // as two chains on their own streams, each with its own one-panel lookahead,
   // so that one chain's launch tails and diagonal blocks overlap the other's GEMMs.
   // frequency chains: independent factorization sequences on their own streams,
-  // at least kChainPairs (problem, frequency) pairs each
+  // at least kChainPairs (problem, frequency) pairs each.  One problem of up to 12 panels
+  // leaves room for four (840 / 32 frequencies: 1.81 -> 1.68 ms, 1483: 5.29 -> 5.15 ms; 16
+  // panels 12.0 -> 12.5 ms, 16 molecules 68 -> 74 ms)
   nchains_ = tune_.chains > 0 ? std::max(1, std::min({tune_.chains, kMaxChains, npairs}))
-                              : std::max(1, std::min(kAutoChains, npairs / kChainPairs));
+                              : std::max(1, std::min(np == 1 && max_panels <= 12 ? 2 * kAutoChains : kAutoChains,
+                                                     npairs / kChainPairs));
   // panels per trailing update: longer updates pay off when many problems keep
   // the GPU busy; one or few problems keep pairs, whose factorization chain is shorter
   group_ = tune_.panel_group > 0 ? std::max(1, std::min(tune_.panel_group, 32)) : (np >= 4 ? 16 : 2);
@@ -1126,7 +1129,7 @@ void Plan::record(cudaStream_t s0, int stage) {
         else launch_dgemm_128x128(gl, L.count, L.ny, s);
         break;
       case 7: energy_kernel<<<L.count, 256, 0, s>>>(probs_dev_, wl); break;
-      case 8: energy_sum_kernel<<<(L.count + 127) / 128, 128, 0, s>>>(probs_dev_, L.count); break;
+      case 8: energy_sum_kernel<<<(L.count + 3) / 4, 128, 0, s>>>(probs_dev_, L.count); break;
       case 9: vchiv_kernel<<<L.count, 256, 0, s>>>(probs_dev_, wl); break;
       case 10: sigma_kernel<<<L.count, 256, 0, s>>>(probs_dev_, wl); break;
       case 11: pade_qp_kernel<<<L.count, 256, 0, s>>>(probs_dev_, wl); break;
