@@ -210,6 +210,9 @@ class ClockSampler:
                 "window": "samples taken inside the timed region"}
 
 
+FP64_DIGIT_PRODUCTS = 28   # int8 digit products of one FP64 product (seven digits, levels i + j <= 8)
+
+
 def measured_fp64_peak(torch) -> float:
     """cuBLAS DGEMM throughput (TFLOP/s) on this GPU: 8192^3 float64, best of 5."""
     n = 8192
@@ -655,7 +658,8 @@ def run_sweep_block(fp64_peak: float, bf16_peak: float) -> dict:
     torch.cuda.synchronize()
     f_chi0 = float(nw) * na * (na + 1) * (no * nv)
     out, ref = {}, None
-    for name, prec, products, peak in (("fp64", RIGW_FP64, 1, fp64_peak), ("bf16x3", RIGW_BF16X3, 3, bf16_peak),
+    for name, prec, products, peak in (("fp64", RIGW_FP64, FP64_DIGIT_PRODUCTS, 2.0 * bf16_peak),
+                                       ("bf16x3", RIGW_BF16X3, 3, bf16_peak),
                                        ("ozaki4", RIGW_OZAKI(4), 10, 2.0 * bf16_peak)):
         eng = Engine(0)
         eng.g0w0(inst, prec, dev, qp_only=True)
@@ -697,7 +701,8 @@ def run_sweep_line(args):
     clocks = ClockSampler(0)
     clocks.start()
     out, ref = {}, None
-    plan = [("fp64", RIGW_FP64, 1, fp64_peak, "measured cuBLAS DGEMM"),
+    plan = [("fp64", RIGW_FP64, FP64_DIGIT_PRODUCTS, 2.0 * bf16_peak,
+             "2 x MEASURED_PEAKS.json bf16_tflops (28 int8 digit products)"),
             ("bf16x3", RIGW_BF16X3, 3, bf16_peak, "MEASURED_PEAKS.json bf16_tflops")]
     plan += [(f"ozaki{k}", RIGW_OZAKI(k), k * (k + 1) // 2, 2.0 * bf16_peak,
               "2 x MEASURED_PEAKS.json bf16_tflops (dense int8 rate = 2 x bf16 on B200)") for k in range(3, 8)]
@@ -1189,14 +1194,21 @@ def main():
         fp64_peak = measured_fp64_peak(torch)
         peaks = json.loads((ROOT / "MEASURED_PEAKS.json").read_text()) if (ROOT / "MEASURED_PEAKS.json").exists() else {}
         chi0_avg = float(np.mean(chi0_ms))
-        achieved = chi0_flops(inst) / (chi0_avg * 1e-3) / 1e12
-        traffic = profile_traffic("chi0_syrk_fp64_naux840.txt")
-        roofline = {"kernel": "chi0 contraction M D M^T (dgemm_mn_kernel<64,128>, FP64 DMMA)",
-                    "bound": "tensor", "achieved": achieved, "peak": fp64_peak, "unit": "TFLOP/s",
-                    "frac": achieved / fp64_peak, "traffic": traffic,
-                    "peak_source": "measured cuBLAS DGEMM 8192^3 on this GPU (torch.matmul float64, best of 6); "
-                                   "MEASURED_PEAKS.json has no FP64 figure",
+        # FP64 chi0: 28 exact int8 digit products per FP64 product; split precisions: theirs
+        products = {"fp64": FP64_DIGIT_PRODUCTS, "bf16x3": 3}.get(args.precision, FP64_DIGIT_PRODUCTS)
+        int8_peak = (1.0 if args.precision == "bf16x3" else 2.0) * float(peaks.get("bf16_tflops", 1590.0))
+        achieved = products * chi0_flops(inst) / (chi0_avg * 1e-3) / 1e12
+        traffic = profile_traffic("digit_syrk_naux840.txt")
+        roofline = {"kernel": "chi0 stage (row maxima, digits, digit_syrk_kernel<7>: 28 exact int8 digit products "
+                              "of 55-bit operands on tcgen05, FP64 result)" if products == FP64_DIGIT_PRODUCTS else
+                              "chi0 stage (split_bf16_kernel, split_syrk_kernel: 3 bf16 products on tcgen05)",
+                    "bound": "tensor", "achieved": achieved, "peak": int8_peak, "unit": "TFLOP/s",
+                    "frac": achieved / int8_peak, "traffic": traffic,
+                    "peak_source": "MEASURED_PEAKS.json bf16_tflops (burst)" + (
+                        "" if products == 3 else " x 2 (dense int8 rate = 2 x bf16)"),
                     "algorithmic_flops_per_launch": chi0_flops(inst),
+                    "fp64_tflops_algorithmic": chi0_flops(inst) / (chi0_avg * 1e-3) / 1e12,
+                    "fp64_peak_measured_dgemm": fp64_peak,
                     "chi0_ms_per_launch": chi0_avg}
         line = {
             "metric": METRIC, "value": value, "unit": "solves/s", "n_gpus": world, "steps": args.steps,
@@ -1227,7 +1239,7 @@ def main():
             # the tcgen05 kernel does 3 bf16 products of the chi0 contraction
             bf = peaks.get("bf16_tflops")
             ach = 3.0 * chi0_flops(inst) / (alt["chi0_ms"] * 1e-3) / 1e12
-            alt["roofline_chi0"] = {"kernel": "split_bf16x3_kernel + syrk_bf16x3_kernel (tcgen05, 3 bf16 products)",
+            alt["roofline_chi0"] = {"kernel": "split_bf16_kernel + split_syrk_kernel (tcgen05, 3 bf16 products)",
                                     "bound": "tensor", "achieved": ach, "peak": bf, "unit": "TFLOP/s",
                                     "frac": ach / bf if bf else None,
                                     "peak_source": "MEASURED_PEAKS.json bf16_tflops (burst, of measured)"}

@@ -298,10 +298,15 @@ bool use_digits(const Shape& sh) {
          (long long)sh.nocc * sh.nvirt + (long long)sh.nocc2 * sh.nvirt2 >= 512;
 }
 
-// From seven panels on a group of four leaves something to update.  Factorization stage, DMMA
-// against digits (32 frequencies, ms): naux 500 0.46 / 0.48, 840 1.91 / 1.88, 1152 3.51 / 3.14,
-// 1483 7.15 / 5.36, 2000 18.4 / 12.9, 4000 (48 frequencies, QP only) 139 / 67.
+// Factorization stage, DMMA against digits in groups of four panels (32 frequencies, ms): naux
+// 500 0.46 / 0.48, 840 1.91 / 1.88, 1152 3.51 / 3.14, 1483 7.15 / 5.36, 2000 18.4 / 12.9, 4000
+// (48 frequencies, QP only) 139 / 67.
 bool use_factor_digits(const Shape& sh) { return !sh.no_digits && sh.naux > 768; }
+
+// Two panels leave the least to DMMA; from 24 panels on the sums are long enough that the four
+// of a group, drained once per group, win (stage, groups of 2 / 4 / 8, ms: 8 molecules up to
+// 1152 7.0 / 7.7 / 7.8, 1483 5.07 / 5.28 / 5.78, 2000 12.0 / 12.5 / 15.1, 4000 71.6 / 69.7 / 72.3).
+int factor_group(const Shape& sh) { return sh.naux > 23 * kPanel ? 4 : 2; }
 
 int operand_planes(const Shape& sh) {
   if (sh.precision == RIGW_BF16X3) return 2;
@@ -430,7 +435,7 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
                                   fd ? factor_bytes(sh, d) : 0));
       if (fd) {
         off[i].fmap = L.take(512);
-        off[i].fexp = L.take(size_t(sh.nomega) * ((d.npanel + kDigitGroup - 1) / kDigitGroup) * factor_blocks(d) *
+        off[i].fexp = L.take(size_t(sh.nomega) * ((d.npanel + factor_group(sh) - 1) / factor_group(sh)) * factor_blocks(d) *
                              kPanel * sizeof(int));
       }
       if (planes) {
@@ -486,8 +491,8 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
       const size_t t = size_t(d.npanel + 2) * (d.npanel + 2 + (d.ldb + 127) / 128) * 4;
       // GEMM items cover all frequencies of a chain; the WorkItem lists stay per frequency
       if (factor && use_factor_digits(sh))
-        lists += size_t(kMaxChains) * (d.npanel / kDigitGroup + 1) * factor_blocks(d) *
-                 (sizeof(FactorSliceItem) + (kDigitGroup / 2) * sizeof(UpdateItem));
+        lists += size_t(kMaxChains) * (d.npanel / factor_group(sh) + 1) * factor_blocks(d) *
+                 (sizeof(FactorSliceItem) + (factor_group(sh) / 2) * sizeof(UpdateItem));
       lists += size_t(kMaxChains + 1) * t * sizeof(GemmItem) +
                size_t(sh.nomega) * (d.npanel + 8) * sizeof(WorkItem) +
                size_t(d.nia_pad / 8 + d.npad * d.ldb / 1024 + 64) * 16;
@@ -778,11 +783,11 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
         // the whole group, so each trailing tile is read and written once per group.
         // Items of the next diagonal block go to their own list (in both forms) so that
         // its factorization can start while the rest of the update runs (lookahead).
-        // Problems on digit products take groups of kDigitGroup panels, and after the last
+        // Problems on digit products take groups of factor_group panels, and after the last
         // panel of a group only the rows of the next group are updated, with every row
         // above them (left-looking), on the int8 tensor cores.
         const bool fd = factor && use_factor_digits(sh);
-        const int gsize = fd ? kDigitGroup : group_;
+        const int fg = factor_group(sh), gsize = fd ? fg : group_;
         const int jg = k % gsize;
         const bool inside = jg != gsize - 1;                    // not the group's last panel
         const int kp = k - jg;                                  // first panel of the U rows used
@@ -791,7 +796,7 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
         if (fd && !inside && r0 < npad) {
           int* fexp = reinterpret_cast<int*>(base + off[i].fexp);
           const int nrb = p.npanel + (ldb + kPanel - 1) / kPanel, nkt = npad / 64;
-          const int ngroups = (p.npanel + kDigitGroup - 1) / kDigitGroup;
+          const int ngroups = (p.npanel + fg - 1) / fg;
           auto slice = [&](const double* X, int ldx, long long stride, int c0, int n, int rb) {
             FactorSliceItem f{};
             f.src = X + size_t(kp) * kPanel * ldx + c0;
@@ -805,7 +810,7 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
             f.rb = rb;
             f.kt = kp * (kPanel / 64);
             f.ngroups = ngroups;
-            f.group = k / kDigitGroup;
+            f.group = k / fg;
             f.slab = w0;
             f.step = nchains_;
             f.nw = nw;
@@ -823,7 +828,7 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
             u.nrb = nrb;
             u.nkt = nkt;
             u.nk = r0 / 64;
-            u.chunk = kDigitGroup * kPanel / 64;
+            u.chunk = fg * kPanel / 64;
             u.first = first;
             u.ngroups = ngroups;
             u.slab = w0;
@@ -841,11 +846,11 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
             for (int cb = 0; cb <= k; ++cb) slice(R, ldb, sR, cb * kPanel, kPanel, p.npanel + cb);
           for (int c0 = p.moff; c0 < ldb; c0 += kPanel)
             slice(R, ldb, sR, c0, std::min(kPanel, ldb - c0), p.npanel + c0 / kPanel);
-          for (int ra = k + 1; ra < std::min(p.npanel, k + 1 + kDigitGroup); ra += 2) {
+          for (int ra = k + 1; ra < std::min(p.npanel, k + 1 + fg); ra += 2) {
             for (int cb = ra; cb < p.npanel; ++cb) update(E, npad, sE, ra, cb * kPanel, kPanel, cb, 0, 1);
             if (p.want_identity)
               for (int cb = 0; cb <= k; ++cb)
-                update(R, ldb, sR, ra, cb * kPanel, kPanel, p.npanel + cb, cb / kDigitGroup, 0);
+                update(R, ldb, sR, ra, cb * kPanel, kPanel, p.npanel + cb, cb / fg, 0);
             for (int c0 = p.moff; c0 < ldb; c0 += kPanel)
               update(R, ldb, sR, ra, c0, std::min(kPanel, ldb - c0), p.npanel + c0 / kPanel, 0, 0);
           }

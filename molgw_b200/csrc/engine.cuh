@@ -109,9 +109,9 @@ int precision_class(const std::vector<Shape>& shapes);
 // Whether the FP64 chi0 of a problem goes through the int8 digit products.
 bool use_digits(const Shape& sh);
 // Whether the updates between panel groups of the factorization go through digit products, and
-// the panels of such a group.
+// the panels of such a group (even: rows are updated in pairs of panels).
 bool use_factor_digits(const Shape& sh);
-constexpr int kDigitGroup = 4;
+int factor_group(const Shape& sh);
 // Planes of the chi0 operands: 2 (bf16 hi/lo), 3 .. 7 (int8 digits), 0 (FP64 on DMMA).
 int operand_planes(const Shape& sh);
 // Bytes of one frequency's split operands of a problem (0 for FP64 on DMMA).

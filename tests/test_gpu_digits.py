@@ -99,9 +99,10 @@ def sigma_reference(inst, omega, weight, z):
 
 
 @pytest.mark.parametrize("nocc,nvirt,naux,nomega", [
-    (9, 60, 769, 3),       # seven panels: the group after the first has three
-    (8, 70, 1030, 5),      # nine panels: the last group has one, its pair of row blocks too
+    (9, 60, 769, 3),       # seven panels in groups of two: the last group has one
+    (8, 70, 1030, 5),      # nine panels, one column block of the right-hand sides ends early
     (10, 65, 1100, 2),     # M columns that end inside a 128-column block
+    (6, 86, 3200, 1),      # 25 panels in groups of four: the last group has one
 ])
 @pytest.mark.parametrize("qp_only", [False, True])
 def test_factorization_updates_by_digits(engine, nocc, nvirt, naux, nomega, qp_only):
