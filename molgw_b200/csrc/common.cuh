@@ -58,12 +58,6 @@ RIGW_DEVICE_INLINE void dmma_8x8x4(double& c0, double& c1, double a, double b) {
                : "d"(a), "d"(b));
 }
 
-// D_w(t) of the sliced precisions, which take positive factors only: a negative one (inverted
-// occupations) becomes NaN, and eps is then reported as not positive definite.
-RIGW_DEVICE_INLINE double split_factor(double d) {
-  return d < 0.0 ? __longlong_as_double(0x7ff8000000000000ll) : d;
-}
-
 RIGW_DEVICE_INLINE double warp_sum(double v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

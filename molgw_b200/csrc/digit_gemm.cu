@@ -1,37 +1,43 @@
 // chi0 from exact int8 digit products on the 5th-generation tensor cores: NS = 7 digits
 // reach FP64 accuracy (RIGW_FP64 for all but the smallest problems), NS = s is RIGW_OZAKI(s).
 //
-//   eps(iw)[p][q] = delta_pq + sum_t A_pt B_qt,   A = M D_w,   B = M
+//   eps(iw)[p][q] = delta_pq + sum_t S_pt S_qt,   S = M sqrt(D_w)
 //
-// Row p of an operand is scaled by a power of two to its largest entry and rounded once
+// Row p of S is scaled by a power of two to its largest entry and rounded once
 // to an integer X of 8 NS - 1 bits; X is cut into NS balanced base-256 digits d_1 (most
 // significant) .. d_NS, each an int8:  x = 2^(e_p - (8 NS - 1)) sum_i d_i 256^(NS - i).
-//   (A B^T)_pq = 2^(e_p + f_q - 2 (8 NS - 1)) sum_{d=2}^{NS+1} 256^(2 NS - d) L_d(p,q),
-//   L_d = sum_{i+j=d} A_i B_j^T      (NS (NS + 1) / 2 digit products: 28 of 49 for NS = 7)
+//   (S S^T)_pq = 2^(e_p + e_q - 2 (8 NS - 1)) sum_{d=2}^{NS+1} 256^(2 NS - d) L_d(p,q),
+//   L_d = sum_{i+j=d} S_i S_j^T      (NS (NS + 1) / 2 digit products: 28 of 49 for NS = 7)
 // L_d is an exact INT32 sum (tcgen05.mma kind::i8) over chunks of kChunkTiles k-tiles: for
 // NS = 7, |L_d| <= 7 * 128^2 * 16384 < 2^31.  The levels are joined in 64-bit integers,
 // converted to FP64 once per chunk and summed in FP64.
 //
 // Error, NS = 7 (55-bit X): the products left out (i + j > 8) are digit products of zero
 // mean with weight 2^-70 of the two row scales; K of them add up to about
-// 2^-56 sqrt(K) max|A_p| max|B_q|.  An FP64 sum of K products rounds its running sum K
-// times, about 2^-55 K sigma^2 for entries of size sigma: for K >= 300 and a row maximum of
-// 5 sigma the digit sum is the closer one, at K = 4347 by a factor of 5.  Because a row
-// maximum never exceeds the row's norm, the error relative to sqrt(eps_pp eps_qq) stays at
-// the level of an FP64 sum whatever the spread of the entries (rms, normal entries: 1.3e-17
-// against 2.2e-16 at K = 4347; three decades of spread: 5.8e-17 against 1.8e-16, and at 512
-// transitions 7.5e-17 against 5.7e-17).
+// 2^-56 sqrt(K) max|S_p| max|S_q|, at most 2^-56 sqrt(K) sqrt(eps_pp eps_qq), because a row
+// maximum never exceeds the row's norm.  An FP64 sum of K products rounds its running sum K
+// times.  (M D_w and M in place of S on both sides would not be bounded so: max|M_q| can
+// exceed sqrt(eps_qq) by sqrt(max D / min D), 9 times the error of the FP64 sum for gaps over
+// three decades and amplitudes that grow as their square roots, 512 transitions.)
 //
 // 840 auxiliary functions, 4347 transitions, 32 frequencies: row maxima 0.04 ms, digits
 // 0.16 ms, products 1.23 ms (3.4 Pop/s int8), against 4.25 ms on DMMA (23 of 35 TF/s);
 // 2000 / 25000 / 32: 0.37 + 2.26 + 30.2 ms against 112 ms.
-// A row that holds an infinity or a NaN gives NaN, as the FP64 sums did.
+// The operands are the same on both sides, so on the diagonal the products that are left out
+// hold squares, whose mean is not zero.  For even NS the largest of them, digit NS/2 + 1 against
+// itself, has the weight of the first level left out and would lower eps_pp by 1e-9 for NS = 4:
+// digit_slice_kernel sums it per row, and it is added to the diagonal.  For odd NS the first
+// squares are 2^-8 below that level.
+// A row that holds an infinity or a NaN gives NaN, as the FP64 sums did.  A negative D_w
+// (inverted occupations) has no root: RIGW_FP64 then takes the DMMA kernel, which is launched
+// behind these and returns at once unless digit_rowmax_kernel met one; in the sliced
+// precisions the root is NaN and eps is reported as not positive definite.
 //
-// digit_rowmax_kernel: high words of max_t |A_pt| per frequency and row (integer maximum).
+// digit_rowmax_kernel: high words of max_t |S_pt| per frequency and row (integer maximum).
 // digit_slice_kernel:  the digits of one frequency group, in the order in which the tensor
 //   cores read them: [slab][row block of 128][k-tile of 64][digit][row group of 8][16-byte
 //   k chunk][row][16 bytes], i.e. contiguous 8 x 16-byte core matrices, so that one TMA box
-//   fetches all the digits of a tile.  Slab 0 is B (the same for every frequency).
+//   fetches all the digits of a tile.  One slab per frequency of the group.
 // digit_syrk_kernel:   one 256 x 128 tile of eps(iw) per pair of CTAs (cta_group::2).
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -71,12 +77,6 @@ RIGW_DEVICE_INLINE int row_exponent(unsigned hi) {
   return e < -960 ? -960 : e;
 }
 
-// D_w(t); only the FP64 mode takes negative factors.
-RIGW_DEVICE_INLINE double factor(const ProbDev& p, int w, int t) {
-  const double d = p.dscale[size_t(w) * p.nia_pad + t];
-  return p.signed_d ? d : split_factor(d);
-}
-
 RIGW_DEVICE_INLINE double pow2(int e) { return __hiloint2double((e + 1023) << 20, 0); }   // -1022 <= e <= 1023
 
 // 2^e; NaN above 1023 (kNaNExp, also with a shift added), 2^-1022 at the least.
@@ -90,12 +90,16 @@ __global__ void __launch_bounds__(256) digit_zero_kernel(const ProbDev* __restri
                                                          const WorkItem* __restrict__ items) {
   const WorkItem wi = items[blockIdx.x];
   const ProbDev& p = probs[wi.prob];
-  const int n = (1 + p.nomega) * p.npad;
+  const int n = p.nomega * p.npad;
+  if (p.negative && wi.a == 0 && threadIdx.x == 0) *p.negative = 0;
   for (int k = threadIdx.x; k < 4096; k += 256)
-    if (wi.a + k < n) p.dmax[wi.a + k] = 0u;
+    if (wi.a + k < n) {
+      p.dmax[wi.a + k] = 0u;
+      if (p.squares) p.squares[wi.a + k] = 0;
+    }
 }
 
-// item: (prob, t0, row block): split_t transitions from t0, 128 rows, B and every frequency.
+// item: (prob, t0, row block): split_t transitions from t0, 128 rows, every frequency.
 // Thread (row, half) keeps 32 entries of its row in registers and walks the frequencies:
 // one FP64 product and one integer maximum per entry and frequency.
 __global__ void __launch_bounds__(256) digit_rowmax_kernel(const ProbDev* __restrict__ probs,
@@ -109,24 +113,23 @@ __global__ void __launch_bounds__(256) digit_rowmax_kernel(const ProbDev* __rest
   const int tend = min(p.nia_pad, wi.a + p.split_t);
   for (int t0 = wi.a; t0 < tend; t0 += 64) {
     double v[32];
-    unsigned mb = 0;
 #pragma unroll
-    for (int i = 0; i < 32; ++i) {
-      v[i] = p.mp[size_t(t0 + half * 32 + i) * p.npad + r];
-      mb = max(mb, unsigned(__double2hiint(v[i])) & 0x7fffffffu);
-    }
-    if (mb) atomicMax(p.dmax + r, mb);
+    for (int i = 0; i < 32; ++i) v[i] = p.mp[size_t(t0 + half * 32 + i) * p.npad + r];
     for (int wb = 0; wb < p.nomega; wb += kWb) {
       const int nwb = min(kWb, p.nomega - wb);
       __syncthreads();
-      for (int i = tid; i < nwb * 64; i += 256) sd[i >> 6][i & 63] = factor(p, wb + (i >> 6), t0 + (i & 63));
+      for (int i = tid; i < nwb * 64; i += 256) {
+        const double d = p.dscale[size_t(wb + (i >> 6)) * p.nia_pad + t0 + (i & 63)];
+        if (d < 0.0 && p.negative) *p.negative = 1;   // any thread: the same value
+        sd[i >> 6][i & 63] = sqrt(d);
+      }
       __syncthreads();
       for (int w = 0; w < nwb; ++w) {
         unsigned m = 0;
 #pragma unroll
         for (int i = 0; i < 32; ++i)
           m = max(m, unsigned(__double2hiint(v[i] * sd[w][half * 32 + i])) & 0x7fffffffu);
-        if (m) atomicMax(p.dmax + size_t(1 + wb + w) * p.npad + r, m);
+        if (m) atomicMax(p.dmax + size_t(wb + w) * p.npad + r, m);
       }
     }
   }
@@ -146,9 +149,10 @@ RIGW_DEVICE_INLINE void bytes4(uint32_t w0, uint32_t w1, uint32_t w2, uint32_t w
 
 // The NS digits of 16 consecutive transitions of one row: X = rint(v scale), a carry-in of
 // 128 in every byte but the leading one makes the digits balanced, and 16 bytes per digit
-// go to core-matrix row `dst` (digit planes kTileA bytes apart).
+// go to core-matrix row `dst` (digit planes kTileA bytes apart).  Returns the sum of the squares
+// of digit NS/2 + 1.
 template <int NS>
-RIGW_DEVICE_INLINE void write_digits(const double (&v)[16], double scale, int8_t* dst) {
+RIGW_DEVICE_INLINE int write_digits(const double (&v)[16], double scale, int8_t* dst) {
   constexpr uint64_t kBias = NS >= 8 ? 0x0080808080808080ull : (0x8080808080808080ull & ((1ull << (8 * (NS - 1))) - 1));
   uint32_t out[NS][4];
 #pragma unroll
@@ -172,6 +176,10 @@ RIGW_DEVICE_INLINE void write_digits(const double (&v)[16], double scale, int8_t
 #pragma unroll
   for (int s = 0; s < NS; ++s)
     *reinterpret_cast<uint4*>(dst + size_t(s) * kTileA) = make_uint4(out[s][0], out[s][1], out[s][2], out[s][3]);
+  int sq = 0;
+#pragma unroll
+  for (int g = 0; g < 4; ++g) sq = __dp4a(int(out[NS / 2][g]), int(out[NS / 2][g]), sq);
+  return sq;
 }
 
 // Byte offset of (slab, row block, k-tile, digit 1, row, 16-byte chunk kc) in the digit array.
@@ -181,8 +189,8 @@ RIGW_DEVICE_INLINE size_t digit_offset(int slab, int nrb, int rb, int nkt, int k
 
 }  // namespace
 
-// item: (prob, k-tile, row block, w0); w0 < 0: slab 0 (B), else the frequencies w0 .. w0 +
-// wgroup - 1 into slabs 1 ...  A warp writes 32 rows of one 16-byte chunk: four full lines
+// item: (prob, k-tile, row block, w0): the frequencies w0 .. w0 + wgroup - 1 into slabs 0 ...
+// A warp writes 32 rows of one 16-byte chunk: four full lines
 // per digit.  Memory bound: NS bytes written per entry and frequency (840 auxiliary
 // functions, 32 frequencies: 0.87 GB).
 template <int NS>
@@ -190,6 +198,7 @@ __global__ void __launch_bounds__(256) digit_slice_kernel(const ProbDev* __restr
                                                           const WorkItem* __restrict__ items) {
   const WorkItem wi = items[blockIdx.x];
   const ProbDev& p = probs[wi.prob];
+  if (p.negative && *p.negative) return;   // left to DMMA
   constexpr int kWb = 16;
   __shared__ double sd[kWb][64];
   const int tid = threadIdx.x, row = tid & 127, half = tid >> 7;
@@ -201,31 +210,26 @@ __global__ void __launch_bounds__(256) digit_slice_kernel(const ProbDev* __restr
   for (int c = 0; c < 2; ++c)
 #pragma unroll
     for (int i = 0; i < 16; ++i) v[c][i] = p.mp[size_t(t0 + (half * 2 + c) * 16 + i) * p.npad + r];
-  if (wi.c < 0) {
-    const int e = row_exponent(p.dmax[r]);
-    if (kt == 0 && half == 0) p.xexp[r] = e;
-    const double sc = pow2(8 * NS - 1 - (e == kNaNExp ? 0 : e));
-#pragma unroll
-    for (int c = 0; c < 2; ++c) write_digits<NS>(v[c], sc, dig + digit_offset(0, nrb, rb, nkt, kt, NS, row, half * 2 + c));
-    return;
-  }
   const int w0 = wi.c, w1 = min(p.nomega, w0 + p.wgroup);
   for (int wb = w0; wb < w1; wb += kWb) {
     const int nwb = min(kWb, w1 - wb);
     __syncthreads();
-    for (int i = tid; i < nwb * 64; i += 256) sd[i >> 6][i & 63] = factor(p, wb + (i >> 6), t0 + (i & 63));
+    for (int i = tid; i < nwb * 64; i += 256)
+      sd[i >> 6][i & 63] = sqrt(p.dscale[size_t(wb + (i >> 6)) * p.nia_pad + t0 + (i & 63)]);
     __syncthreads();
     for (int w = 0; w < nwb; ++w) {
-      const int e = row_exponent(p.dmax[size_t(1 + wb + w) * p.npad + r]);
-      if (kt == 0 && half == 0) p.xexp[size_t(1 + wb + w) * p.npad + r] = e;
+      const int e = row_exponent(p.dmax[size_t(wb + w) * p.npad + r]);
+      if (kt == 0 && half == 0) p.xexp[size_t(wb + w) * p.npad + r] = e;
       const double sc = pow2(8 * NS - 1 - (e == kNaNExp ? 0 : e));
+      int sq = 0;
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
         double x[16];
 #pragma unroll
         for (int i = 0; i < 16; ++i) x[i] = v[c][i] * sd[w][(half * 2 + c) * 16 + i];
-        write_digits<NS>(x, sc, dig + digit_offset(1 + wb - w0 + w, nrb, rb, nkt, kt, NS, row, half * 2 + c));
+        sq += write_digits<NS>(x, sc, dig + digit_offset(wb - w0 + w, nrb, rb, nkt, kt, NS, row, half * 2 + c));
       }
+      if (NS % 2 == 0) atomicAdd(p.squares + size_t(wb + w) * p.npad + r, (unsigned long long)(sq));
     }
   }
 }
@@ -267,18 +271,17 @@ __device__ __forceinline__ void digit_product(const Item& it, const int jw) {
   tc::cluster_sync();        // the peer's barriers are initialised
   tc::tc_fence_after();
   const uint32_t tmem = *tslot;
-  int nk, chunk, slab_a, slab_b;      // k-tiles summed, k-tiles per chunk, operand slabs
+  int nk, chunk, slab;                // k-tiles summed, k-tiles per chunk, slab of both operands
   int c0 = 0;                         // first chunk
   if constexpr (kUpdate) {
     nk = it.nk;
     chunk = it.chunk;
     c0 = it.first;
-    slab_a = slab_b = it.slab + jw * it.step;
+    slab = it.slab + jw * it.step;
   } else {
     nk = it.nkt;
     chunk = kChunkTiles;
-    slab_a = it.slab_a + jw;
-    slab_b = it.slab_b;
+    slab = jw;
   }
   const int nchunks = (nk + chunk - 1) / chunk;
   constexpr int kPasses = Cfg::kHi > 0 ? 2 : 1;
@@ -290,8 +293,8 @@ __device__ __forceinline__ void digit_product(const Item& it, const int jw) {
     // ---- TMA producer of this CTA; rank 0's full barrier counts the bytes of both
     const uint8_t* maps = static_cast<const uint8_t*>(it.maps);
     for (int m = 0; m < (kPasses > 1 ? 4 : 2); ++m) tc::tmap_acquire(maps + 128 * m);
-    const int rowA = (slab_a * it.nrb + it.rb_a + rank) * it.nkt;
-    const int rowB = (slab_b * it.nrb + it.rb_b) * it.nkt;
+    const int rowA = (slab * it.nrb + it.rb_a + rank) * it.nkt;
+    const int rowB = (slab * it.nrb + it.rb_b) * it.nkt;
     uint32_t issued = 0;
     bool ok = true;
     for (int c = c0; c < nchunks && ok; ++c)
@@ -414,7 +417,7 @@ __device__ __forceinline__ void digit_product(const Item& it, const int jw) {
         double wr = wq;
         const int* ecol = nullptr;
         if constexpr (kUpdate) {
-          const int* e = it.exps + (size_t(slab_a) * it.ngroups + c) * it.nrb * 128;
+          const int* e = it.exps + (size_t(slab) * it.ngroups + c) * it.nrb * 128;
           wr *= pow2_of(e[min(it.rb_a + rank, it.nrb - 1) * 128 + quad * 32 + lane]);
           ecol = e + it.rb_b * 128 + half * 64;
         }
@@ -459,17 +462,22 @@ __device__ __forceinline__ void digit_product(const Item& it, const int jw) {
       const int rb = it.rb_a + rank, cb = it.rb_b;
       if (rb < it.nrb && rb <= cb) {               // blocks below the diagonal are not stored
         const int row = rb * 128 + quad * 32 + lane, col0 = cb * 128 + half * 64;
-        const int er = it.exps[size_t(it.slab_e + jw) * it.ld + row];
+        const int* exps = it.exps + size_t(it.w0 + jw) * it.ld;
+        const int er = exps[row];
         double* dst = it.C + jw * it.sC + size_t(row) * it.ld + col0;
 #pragma unroll
         for (int j = 0; j < 64; j += 2) {
           double v[2];
 #pragma unroll
           for (int u = 0; u < 2; ++u) {
-            const int ec = it.exps[col0 + j + u];
+            const int ec = exps[col0 + j + u];
             v[u] = (er == kNaNExp || ec == kNaNExp) ? __longlong_as_double(0x7ff8000000000000ll)
                                                      : ldexp(acc[j + u], er + ec + kShift);
-            if (col0 + j + u == row) v[u] += 1.0;
+            if (col0 + j + u == row) {
+              if (NS % 2 == 0)   // level NS + 2, one below the lowest
+                v[u] += ldexp(double(it.squares[size_t(it.w0 + jw) * it.ld + row]), 2 * er + kShift - 8);
+              v[u] += 1.0;
+            }
           }
           *reinterpret_cast<double2*>(dst + j) = make_double2(v[0], v[1]);
         }
@@ -489,7 +497,8 @@ template <int NS>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kDigThreads, 1)
     digit_syrk_kernel(const DigitItem* __restrict__ items) {
   const DigitItem it = items[blockIdx.x >> 1];
-  if (int(blockIdx.y) >= it.nw) return;   // both CTAs of the pair, before any barrier or TMEM use
+  // both CTAs of the pair, before any barrier or TMEM use
+  if (int(blockIdx.y) >= it.nw || (it.negative && *it.negative)) return;
   digit_product<NS>(it, blockIdx.y);
 }
 

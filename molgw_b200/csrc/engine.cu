@@ -405,7 +405,7 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
     return size_t(sh.nomega) * factor_blocks(d) * kPanel * d.npad * kFp64Digits;
   };
   struct Off {
-    size_t fmap, fexp, mp, xs, tmap, dmax, xexp, tnorm, dscale, eps, winv, logdet, rhs, colsq, mnorm, vchiv, ew, tr, en, sc, sr, qp;
+    size_t fmap, fexp, mp, xs, tmap, dmap, dmax, xexp, sq, neg, tnorm, dscale, eps, winv, logdet, rhs, colsq, mnorm, vchiv, ew, tr, en, sc, sr, qp;
   };
   std::vector<Off> off(np);
   for (int i = 0; i < np; ++i) {
@@ -431,7 +431,7 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
       // the chi0 operands and, after them, the digits of the factor
       const int planes = operand_planes(sh);
       const bool fd = use_factor_digits(sh);
-      off[i].xs = L.take(std::max(planes ? size_t((planes > 2) + split_group(sh)) * split_bytes_per_frequency(sh) : 0,
+      off[i].xs = L.take(std::max(planes ? size_t(split_group(sh)) * split_bytes_per_frequency(sh) : 0,
                                   fd ? factor_bytes(sh, d) : 0));
       if (fd) {
         off[i].fmap = L.take(512);
@@ -441,12 +441,13 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
       if (planes) {
         off[i].tmap = L.take(512);
         if (planes > 2) {
-          off[i].dmax = L.take(size_t(1 + sh.nomega) * d.npad * sizeof(unsigned));
-          off[i].xexp = L.take(size_t(1 + sh.nomega) * d.npad * sizeof(int));
+          off[i].dmax = L.take(size_t(sh.nomega) * d.npad * sizeof(unsigned));
+          off[i].xexp = L.take(size_t(sh.nomega) * d.npad * sizeof(int));
+          if (planes % 2 == 0) off[i].sq = L.take(size_t(sh.nomega) * d.npad * sizeof(unsigned long long));
+          off[i].neg = L.take(sizeof(int));
         }
-      } else {
-        off[i].tmap = L.take(256);   // tensor maps of mp and dscale (TMA-staged FP64 chi0)
       }
+      if (sh.precision == RIGW_FP64) off[i].dmap = L.take(256);   // tensor maps of mp and dscale (TMA-staged DMMA)
       off[i].tnorm = L.take(size_t(d.nia_pad) * D);
       off[i].dscale = L.take(size_t(sh.nomega) * d.nia_pad * D);
       off[i].eps = L.take(size_t(sh.nomega) * d.npad * d.npad * D);
@@ -500,7 +501,7 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
         const int g = split_group(sh);
         const size_t groups = size_t(sh.nomega + g - 1) / g;
         lists += (groups + 2) * (d.nia_pad / 64) * d.npanel * sizeof(WorkItem) +
-                 (size_t(1 + sh.nomega) * d.npad / 4096 + 1) * sizeof(WorkItem) +
+                 (size_t(sh.nomega) * d.npad / 4096 + 1) * sizeof(WorkItem) +
                  groups * (d.npanel / 2 + 1) * d.npanel * sizeof(DigitItem);
       }
     }
@@ -542,7 +543,6 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
     if (factor) {
       p.mp = dp(off[i].mp);
       p.wgroup = split_group(sh);
-      p.signed_d = sh.precision == RIGW_FP64;
       p.split_t = split_item_t(d);
       p.tnorm = dp(off[i].tnorm);
       p.dscale = dp(off[i].dscale);
@@ -551,15 +551,18 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
         if (planes > 2) {
           p.dmax = reinterpret_cast<unsigned*>(base + off[i].dmax);
           p.xexp = reinterpret_cast<int*>(base + off[i].xexp);
+          if (planes % 2 == 0) p.squares = reinterpret_cast<unsigned long long*>(base + off[i].sq);
+          if (sh.precision == RIGW_FP64) p.negative = reinterpret_cast<int*>(base + off[i].neg);
         }
         alignas(64) unsigned char maps[512];
-        RIGW_TRY(make_digit_tmaps(maps, p.xs, (long long)((planes > 2) + p.wgroup) * d.npanel * (d.nia_pad / 64) * planes, planes,
+        RIGW_TRY(make_digit_tmaps(maps, p.xs, (long long)p.wgroup * d.npanel * (d.nia_pad / 64) * planes, planes,
                                   planes == 2 ? 128 : 64));
         RIGW_CUDA_TRY(cudaMemcpyAsync(base + off[i].tmap, maps, sizeof(maps), cudaMemcpyHostToDevice, ctx->stream));
-      } else {
+      }
+      if (sh.precision == RIGW_FP64) {
         alignas(64) unsigned char maps[256];
         RIGW_TRY(make_f64_tmaps(maps, p.mp, d.npad, d.nia_pad, p.dscale, sh.nomega));
-        RIGW_CUDA_TRY(cudaMemcpyAsync(base + off[i].tmap, maps, sizeof(maps), cudaMemcpyHostToDevice, ctx->stream));
+        RIGW_CUDA_TRY(cudaMemcpyAsync(base + off[i].dmap, maps, sizeof(maps), cudaMemcpyHostToDevice, ctx->stream));
       }
       if (use_factor_digits(sh)) {
         alignas(64) unsigned char maps[512];
@@ -634,11 +637,11 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
     if (factor) {
       for (int t0 = 0; t0 < p.nia_pad; t0 += 8) wl_pack_.push_back({i, t0, 0, 0});
       if (const int planes = operand_planes(sh)) {
-        // per frequency group the planes of M sqrt(D_w) (bf16) or M D_w (digits; before the first
-        // group those of M, and the row maxima of all of them), then the products
+        // (digits: the row maxima of every frequency, then) per frequency group the planes of
+        // M sqrt(D_w) and the products
         const int nkt = p.nia_pad / 64;
         if (planes > 2) {
-          for (size_t e = 0; e < size_t(1 + sh.nomega) * npad; e += 4096) wl_dzero_.push_back({i, int(e), 0, 0});
+          for (size_t e = 0; e < size_t(sh.nomega) * npad; e += 4096) wl_dzero_.push_back({i, int(e), 0, 0});
           for (int t0 = 0; t0 < p.nia_pad; t0 += p.split_t)
             for (int rb = 0; rb < p.npanel; ++rb) wl_dmax_.push_back({i, t0, rb, 0});
         }
@@ -650,10 +653,7 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
             products.resize(g + 1);
           }
           for (int rb = 0; rb < p.npanel; ++rb)
-            for (int kt = 0; kt < nkt; ++kt) {
-              slices[g].push_back({i, kt, rb, w0});
-              if (g == 0 && planes > 2) slices[g].push_back({i, kt, rb, -1});
-            }
+            for (int kt = 0; kt < nkt; ++kt) slices[g].push_back({i, kt, rb, w0});
           for (int ra = 0; ra < p.npanel; ra += 2)
             for (int cb = ra; cb < p.npanel; ++cb) {
               DigitItem t{};
@@ -661,38 +661,42 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
               t.C = p.eps + size_t(w0) * npad * npad;
               t.err = err_dev_;
               t.exps = p.xexp;
+              t.squares = p.squares;
+              t.negative = p.negative;
               t.rb_a = ra;
               t.rb_b = cb;
               t.nrb = p.npanel;
               t.nkt = nkt;
-              t.slab_a = planes > 2;
-              t.slab_b = 0;
-              t.slab_e = 1 + w0;
+              t.w0 = w0;
               t.ld = npad;
               t.nw = std::min(p.wgroup, sh.nomega - w0);
               t.sC = (long long)npad * npad;
               products[g].push_back(t);
             }
         }
-      } else {
-        // one item per tile covering every frequency (blockIdx.y); the tiles of a
+      }
+      if (sh.precision == RIGW_FP64) {
+        // DMMA: the whole of chi0, or what is left to it when some D_w is negative.
+        // One item per tile covering every frequency (blockIdx.y); the tiles of a
         // row block start at its diagonal, so only the lower half of the
         // diagonal BMC x BMC block lies below it, and end at naux
         if (npad > sh.naux)
           for (int w = 0; w < sh.nomega; ++w) wl_pad_.push_back({i, w, 0, 0});
         // 64-row items: the TMA-staged kernel (its operands by TMA from the tensor
         // maps of mp and dscale); 128-row items (a tuner candidate): the cp.async engine
-        if (BMC == 64)
-          for (int ti = 0; ti < sh.naux; ti += BMC)
+        const bool staged = BMC == 64 || p.negative;
+        if (staged)
+          for (int ti = 0; ti < sh.naux; ti += 64)
             for (int tj = ti; tj < sh.naux; tj += BMN) {
               F64SyrkItem f{};
-              f.tmap_m = base + off[i].tmap;
-              f.tmap_d = base + off[i].tmap + 128;
+              f.tmap_m = base + off[i].dmap;
+              f.tmap_d = base + off[i].dmap + 128;
               f.C = p.eps + size_t(ti) * npad + tj;
               f.err = p.err;
+              f.only_if = p.negative;
               f.ti = ti;
               f.tj = tj;
-              f.m = std::min(BMC, sh.naux - ti);
+              f.m = std::min(64, sh.naux - ti);
               f.n = std::min(BMN, sh.naux - tj);
               f.ktiles = p.nia_pad / 16;
               f.ldc = npad;
@@ -701,7 +705,7 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
               f.sC = (long long)npad * npad;
               fl_syrk_.push_back(f);
             }
-        for (int ti = 0; BMC != 64 && ti < sh.naux; ti += BMC)
+        for (int ti = 0; !staged && ti < sh.naux; ti += BMC)
           for (int tj = ti; tj < sh.naux; tj += BMN) {
             GemmItem g{};
             g.A = p.mp + ti;
@@ -977,7 +981,6 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
   add(2, wl_rhs_.data(), sizeof(WorkItem), wl_rhs_.size(), 0);
   add(3, wl_mnorm_.data(), sizeof(WorkItem), wl_mnorm_.size(), 0);
   add(1, gl_syrk_.data(), sizeof(GemmItem), gl_syrk_.size(), 0);
-  add(22, fl_syrk_.data(), sizeof(F64SyrkItem), fl_syrk_.size(), 0);
   add(23, wl_dzero_.data(), sizeof(WorkItem), wl_dzero_.size(), 0);
   add(24, wl_dmax_.data(), sizeof(WorkItem), wl_dmax_.size(), 0);
   for (int np2 = 2; np2 < 8; ++np2) {
@@ -986,6 +989,7 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
       add(26, dl_syrk_[np2][g].data(), sizeof(DigitItem), dl_syrk_[np2][g].size(), np2);
     }
   }
+  add(22, fl_syrk_.data(), sizeof(F64SyrkItem), fl_syrk_.size(), 0);   // after 24, which sets `only_if`
   add(16, wl_pad_.data(), sizeof(WorkItem), wl_pad_.size(), 0);
   add(15, wl_trace_.data(), sizeof(WorkItem), wl_trace_.size(), 0);
   // Panel loop of each chain with a one-panel lookahead.  After the diagonal block

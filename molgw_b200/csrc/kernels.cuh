@@ -90,6 +90,7 @@ struct F64SyrkItem {
   const void* tmap_d;   // CUtensorMap of dscale [nomega][nia_pad] (16 x 1 boxes)
   double* C;            // &eps[0][ti][tj]
   int* err;
+  const int* only_if;   // run only when set (negative factors, which the digits do not take); nullptr: always
   int ti, tj;           // first auxiliary row (A) and column (B) of the tile
   int m, n;             // rows and columns stored (<= 64, <= 128, even)
   int ktiles;           // nia_pad / 16
@@ -102,18 +103,19 @@ void launch_syrk_f64_tma(const F64SyrkItem* items, int n, int ny, cudaStream_t s
 cudaError_t prepare_syrk_f64_tma();
 
 // chi0 on the tcgen05 cores: one 256 x 128 upper tile of eps(iw) = 1 + M D_w M^T per pair of
-// CTAs, frequency = blockIdx.y.  The operands are planes of M and M D_w, 3 to 7 int8 digits
-// (digit_gemm.cu; FP64: 7, RIGW_OZAKI(s): s), or the two bf16 parts of M sqrt(D_w) on both
-// sides (syrk_bf16x3.cu; slab_b and exps unused).
+// CTAs, frequency = blockIdx.y (slab blockIdx.y).  The operand planes of M sqrt(D_w) are 3 to 7
+// int8 digits (digit_gemm.cu; FP64: 7, RIGW_OZAKI(s): s) or two bf16 parts (syrk_bf16x3.cu; exps
+// unused).
 struct DigitItem {
   const void* maps;     // CUtensorMaps of the problem's planes (make_digit_tmaps)
   double* C;            // &eps[w0][0][0]
   int* err;
-  const int* exps;      // digits, row exponents: [0][ld] of M, [1 + w][ld] of M D_w
+  const int* exps;      // digits, row exponents [w][ld]
+  const unsigned long long* squares;   // an even number of digits: ProbDev::squares
+  const int* negative;  // digits of FP64: not this kernel's problem when set (nullptr: always its)
   int rb_a, rb_b;       // 128-row blocks: output rows from 128 rb_a (two blocks), columns from 128 rb_b
   int nrb, nkt;         // row blocks and k-tiles (64 transitions) of a slab
-  int slab_a, slab_b;   // slab of M D_w for j = 0 (+ j), slab of M
-  int slab_e;           // exponent row of M D_w for j = 0 (+ j)
+  int w0;               // frequency of slab 0
   int ld, nw;           // npad; frequencies covered
   long long sC;         // doubles between the eps blocks of two frequencies
 };

@@ -424,6 +424,7 @@ __global__ void __launch_bounds__(256) pad_eps_kernel(const ProbDev* __restrict_
                                                       const WorkItem* __restrict__ items) {
   const WorkItem wi = items[blockIdx.x];
   const ProbDev& p = probs[wi.prob];
+  if (p.negative && !*p.negative) return;   // the digit products write whole tiles
   double* E = p.eps + size_t(wi.a) * p.npad * p.npad;
   const int npadc = p.npad - p.naux;
   for (int idx = threadIdx.x; idx < npadc * p.npad; idx += 256) {

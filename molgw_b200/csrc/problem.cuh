@@ -52,13 +52,16 @@ struct ProbDev {
   const double* zcalc;       // [nc] complex (re, im) evaluation points
   // ---- workspace (device)
   double* mp;
-  void* xs;                  // chi0 operand planes (layout in digit_gemm.cu): int8 digits, [1 + wgroup]
-                             // slabs of M, then of M D_w; bf16 hi/lo, [wgroup] slabs of M sqrt(D_w)
+  void* xs;                  // chi0 operand planes (layout in digit_gemm.cu), [wgroup] slabs of
+                             // M sqrt(D_w): int8 digits or bf16 hi/lo
   int wgroup;                // frequencies per group (one set of slabs, reused group by group)
-  int signed_d;              // D_w(t) < 0 is taken (FP64); the split precisions refuse it
+  int* negative;             // FP64 digits: set when some D_w(t) < 0, and chi0 is then left to DMMA
+                             // (nullptr: the split precisions, which refuse such factors, and DMMA)
   int split_t;               // transitions per item of the row-maximum kernel
-  unsigned* dmax;            // digits: [1 + nomega][npad] high words of max_t |M_pt|, max_t |(M D_w)_pt|
-  int* xexp;                 // digits: [1 + nomega][npad] row exponents
+  unsigned* dmax;            // digits: [nomega][npad] high words of max_t |M_pt| sqrt(D_w(t))
+  int* xexp;                 // digits: [nomega][npad] row exponents
+  unsigned long long* squares;   // an even number of digits: [nomega][npad] sums over t of the square of digit
+                             // planes / 2 + 1 (digit_gemm.cu)
   double* tnorm;
   double* dscale;
   double* eps;

@@ -166,8 +166,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kSpThreads, 1)
     const uint8_t* maps = static_cast<const uint8_t*>(it.maps);
     tc::tmap_acquire(maps);
     tc::tmap_acquire(maps + 128);
-    const int rowA = ((it.slab_a + jw) * it.nrb + it.rb_a + rank) * nk;
-    const int rowB = ((it.slab_a + jw) * it.nrb + it.rb_b) * nk;
+    const int rowA = (jw * it.nrb + it.rb_a + rank) * nk;
+    const int rowB = (jw * it.nrb + it.rb_b) * nk;
     int issued = 0;
     bool ok = true;
     for (int kt = 0; kt < nk; ++kt, ++issued) {

@@ -42,7 +42,8 @@ RIGW_DEVICE_INLINE uint32_t sw128(int r, int c) { return uint32_t(r * 128 + ((c 
 __global__ void __launch_bounds__(kF64Threads, 2) syrk_f64_tma_kernel(const F64SyrkItem* __restrict__ items) {
   const F64SyrkItem it = items[blockIdx.x];
   const int jw = blockIdx.y;
-  if (jw >= (it.nw > 0 ? it.nw : 1)) return;   // the whole CTA, before any barrier
+  // the whole CTA, before any barrier
+  if (jw >= (it.nw > 0 ? it.nw : 1) || (it.only_if && !*it.only_if)) return;
   double* C = it.C + jw * it.sC;
   extern __shared__ uint8_t f64_smem_raw[];
   uint8_t* smem =

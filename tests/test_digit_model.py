@@ -2,8 +2,9 @@
 rows scaled to their largest entry, rounded to 55 bits, cut into seven balanced base-256
 digits, digit products with i + j <= 8 summed exactly.  It pins what the kernel claims: the
 digits are int8 and rebuild the integer, the INT32 sums of a chunk cannot overflow, and the
-result is at least as close to an extended-precision sum as an FP64 sum is (normal entries; with
-entries spread over three decades few terms carry the sum, and both stay within 2e-15)."""
+result is at least as close to an extended-precision sum as an FP64 sum is, whatever the range of
+the energy differences (normal entries; with entries spread over three decades few terms carry the
+sum)."""
 import numpy as np
 import pytest
 
@@ -66,21 +67,53 @@ def test_largest_levels_stay_inside_int32():
 
 @pytest.mark.parametrize("k", [512, 1890, 4347, 25000])
 @pytest.mark.parametrize("spread", [0.0, 3.0])
-def test_error_is_no_larger_than_an_fp64_sum(k, spread):
+@pytest.mark.parametrize("gaps,rising", [(0.0, False), (3.0, False), (3.0, True)])
+def test_error_is_no_larger_than_an_fp64_sum(k, spread, gaps, rising):
     """2-norm of the error, relative to sqrt(C_pp C_qq), against an extended-precision sum;
-    ``spread``: decades over which the transitions of a row vary (0: the normal draw).  With a
-    spread the digit sum, whose unit is the row maximum, may be the larger of the two for few
-    transitions, by less than the two products per level more that it leaves out: factor 2."""
+    ``spread``: decades over which the entries of a row vary (0: the normal draw), ``gaps``: decades
+    of the energy differences, ``rising``: amplitudes that grow as their roots.  With a spread the
+    digit sum, whose unit is the row maximum, may be the larger of the two for few transitions:
+    factor 2.5."""
     rng = np.random.default_rng(k)
     m = rng.standard_normal((24, k)) * 10.0 ** (-spread * rng.random((24, k)))
-    a = m * rng.uniform(0.05, 0.5, k)[None, :]
+    de = 10.0 ** (-1.0 + gaps * rng.random(k)) if gaps else rng.uniform(0.3, 2.5, k)
+    if rising:
+        m *= np.sqrt(de)
+    d = 4.0 / de
     ref = np.zeros((24, 24), np.longdouble)
     for c in range(0, k, 500):
-        ref += (a[:, c:c + 500, None].astype(np.longdouble) *
-                m.T[None, c:c + 500, :].astype(np.longdouble)).sum(axis=1)
+        ref += ((m[:, c:c + 500].astype(np.longdouble) * d[c:c + 500])[:, None, :] *
+                m[None, :, c:c + 500].astype(np.longdouble)).sum(axis=2)
+    a = m * d
     seq = np.zeros((24, 24))
     for t in range(0, k, 4):                      # four transitions per DMMA step
         seq += a[:, t:t + 4] @ m[:, t:t + 4].T
+    s = m * np.sqrt(d)
     scale = np.sqrt(np.outer(np.diag(ref), np.diag(ref)))
-    err = [float(np.linalg.norm(((c - ref) / scale).astype(float))) for c in (digit_product(a, m), seq)]
-    assert err[0] <= (1.0 if spread == 0.0 else 2.0) * err[1], err
+    err = [float(np.linalg.norm(((c - ref) / scale).astype(float))) for c in (digit_product(s, s), seq)]
+    assert err[0] <= (1.0 if spread == 0.0 else 2.5) * err[1], err
+
+
+@pytest.mark.parametrize("ns", [4, 6])
+def test_squares_of_the_middle_digit_on_the_diagonal(ns):
+    """An even number of digits: the level left out first holds the squares of digit ns/2 + 1 on the
+    diagonal, whose mean is not zero; with their sum added the diagonal is as close as the rest."""
+    rng = np.random.default_rng(ns)
+    x = rng.standard_normal((16, 3000))
+    bits = 8 * ns - 1
+    e = exponents(x)
+    big = np.rint(np.ldexp(x, (bits - e)[:, None])).astype(np.int64)
+    bias = np.int64(sum(128 << (8 * k) for k in range(ns - 1)))
+    y = (big + bias) ^ bias
+    d = [((y >> (8 * (ns - i))) & 255).astype(np.uint8).view(np.int8).astype(np.int64) for i in range(1, ns + 1)]
+    out = sum((d[i - 1] @ d[j - 1].T).astype(np.longdouble) * np.longdouble(2.0) ** (8 * (2 * ns - i - j))
+              for i in range(1, ns + 1) for j in range(1, ns + 1) if i + j <= ns + 1)
+    ref = big.astype(np.longdouble) @ big.T.astype(np.longdouble)
+    norm = np.sqrt(np.outer(np.diag(ref), np.diag(ref)))
+    off = ~np.eye(16, dtype=bool)
+    rest = np.sqrt(np.mean(((out - ref) / norm)[off] ** 2))
+    plain = np.diag((out - ref) / norm)
+    squares = (d[ns // 2] ** 2).sum(axis=1).astype(np.longdouble) * np.longdouble(2.0) ** (8 * (ns - 2))
+    fixed = np.diag((out + np.diag(squares) - ref) / norm)
+    assert np.abs(plain).min() > 10 * rest
+    assert np.sqrt(np.mean(fixed ** 2)) < 3 * rest

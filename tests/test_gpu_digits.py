@@ -5,10 +5,12 @@ Tolerance: an FP64 sum of K products of entries with row norms |A_p|, |B_q| is o
 about K u |A_p| |B_q|, u = 2^-53; chi = eps^-1 - 1 is a contraction of that error (eps >= 1), so
 |d chi| <= 2 K u max diag(eps) with both sides' errors, and ten times that is allowed.  The row
 exponents and the layout of the digits would show as errors of 1e-2 and more."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
-from molgw_b200.rigw import Engine, RigwError
+from molgw_b200.rigw import Engine, RigwError, WPol
 from molgw_b200.synth import GWInstance, make_instance
 
 pytestmark = pytest.mark.gpu
@@ -62,6 +64,88 @@ def test_tile_and_chunk_edges(engine, nocc, nvirt, naux, nomega):
 
 def test_rows_of_very_different_size(engine):
     check(engine, molecule(10, 70, 400, 3, seed=5, decades=150.0))
+
+
+OMEGA = (1.0e-4, 1.0e-2, 1.0)       # low frequencies, where D_w has the range of the gaps
+
+
+def wide_gaps(nvirt, naux, decades, seed):
+    """Two occupied states, gaps over ``decades`` decades, amplitudes that grow as their roots: what
+    a small gap beside core states gives."""
+    rng = np.random.default_rng(seed)
+    inst = molecule(2, nvirt, naux, len(OMEGA), seed=seed)
+    inst.energy[:] = np.concatenate([[-1.0e-5, 0.0], np.sort(10.0 ** (2.0 - decades * rng.random(nvirt)))])
+    de = inst.energy[2:][None, :] - inst.energy[:2][:, None]
+    inst.m_ia[:] = rng.standard_normal(inst.m_ia.shape) * np.sqrt(de / (4.0 * de.size))[:, :, None]
+    return inst
+
+
+def exact_chi(inst, omega):
+    """eps^-1 - 1 in extended precision: the FP64 inverse and one Newton step."""
+    no, nv, n = inst.nocc, inst.nvirt, inst.naux
+    de = (inst.energy[no:][None, :] - inst.energy[:no][:, None]).ravel().astype(np.longdouble)
+    docc = (inst.occupation[:no][:, None] - inst.occupation[no:][None, :]).ravel()
+    m = inst.m_ia.reshape(no * nv, n).astype(np.longdouble)
+    eye, out = np.eye(n, dtype=np.longdouble), []
+    for w in omega:
+        w = np.longdouble(w)
+        eps = eye + m.T @ (m * (2.0 * docc * de / (w * w + de * de))[:, None])
+        x = np.linalg.inv(eps.astype(float)).astype(np.longdouble)
+        out.append(x + x @ (eye - eps @ x) - eye)
+    return np.array(out)
+
+
+def chi_and_bytes(eng, inst):
+    """chi at OMEGA, and the device memory held with that W."""
+    p, keep = eng.make_problem(inst, freq=(np.array(OMEGA), np.ones(len(OMEGA))))
+    h = C.c_void_p()
+    eng._check(eng._lib.rigw_polarizability_imag(eng._h, C.byref(p), None, None, C.byref(h)), "polarizability")
+    w = WPol(eng, h, inst.naux, len(OMEGA))
+    used = eng.last_stats()["device_bytes_in_use"]
+    chi = w.chi()
+    w.release()
+    return chi, used
+
+
+def chi_on_dmma(inst, bytes_with_digits):
+    """The same W from a context without room for its digits."""
+    eng = Engine(0, hbm_budget_bytes=bytes_with_digits - (1 << 20))
+    chi, used = chi_and_bytes(eng, inst)
+    eng.close()
+    assert used < bytes_with_digits - (1 << 20)
+    return chi
+
+
+@pytest.mark.parametrize("nvirt", [300, 1100])
+@pytest.mark.parametrize("decades", [1.0, 3.0, 5.0])
+def test_no_further_from_64_bits_than_dmma(nvirt, decades):
+    """The digits are no further from extended precision than the FP64 sums of the DMMA kernel,
+    however wide the range of the gaps: what both sides share (the rounding of eps and the
+    factorization) is in both errors, and 10% covers that it is not the same rounding.  M D_w and
+    M as operands, whose scales are not bounded by sqrt(eps_pp eps_qq), give 2 times the error
+    at three decades and 10 times at five."""
+    inst = wide_gaps(nvirt, 400, decades, seed=11)
+    eng = Engine(0)
+    chi, used = chi_and_bytes(eng, inst)
+    eng.close()
+    dmma = chi_on_dmma(inst, used)
+    ref = exact_chi(inst, OMEGA)
+    err = [float(np.sqrt(np.mean((c - ref) ** 2))) for c in (chi, dmma)]
+    assert err[0] <= 1.1 * err[1], err
+
+
+def test_negative_factors_are_left_to_dmma():
+    """Some D_w < 0: bit for bit the result of the DMMA kernel, in a plan that ran with positive
+    factors before and runs with them afterwards."""
+    good, bad = molecule(10, 70, 400, 3, seed=6), molecule(10, 70, 400, 3, seed=6)
+    bad.occupation[9], bad.occupation[10] = 0.5, 1.5
+    eng = Engine(0)
+    ref, used = chi_and_bytes(eng, good)
+    dmma = chi_on_dmma(bad, used)
+    for _ in range(2):                         # the second round replays captured graphs
+        assert np.array_equal(chi_and_bytes(eng, bad)[0], dmma)
+        assert np.array_equal(chi_and_bytes(eng, good)[0], ref)
+    eng.close()
 
 
 def test_negative_factors(engine):
