@@ -6,28 +6,35 @@
 // Row p of S is scaled by a power of two to its largest entry and rounded once
 // to an integer X of 8 NS - 1 bits; X is cut into NS balanced base-256 digits d_1 (most
 // significant) .. d_NS, each an int8:  x = 2^(e_p - (8 NS - 1)) sum_i d_i 256^(NS - i).
-//   (S S^T)_pq = 2^(e_p + e_q - 2 (8 NS - 1)) sum_{d=2}^{NS+1} 256^(2 NS - d) L_d(p,q),
-//   L_d = sum_{i+j=d} S_i S_j^T      (NS (NS + 1) / 2 digit products: 28 of 49 for NS = 7)
+//   (S S^T)_pq = 2^(e_p + e_q - 2 (8 NS - 1)) sum_{d=2}^{D} 256^(2 NS - d) L_d(p,q),
+//   L_d = sum_{i+j=d} S_i S_j^T      (D = NS + 1, NS (NS + 1) / 2 digit products; D = 9, 34 of 49, for NS = 7)
 // L_d is an exact INT32 sum (tcgen05.mma kind::i8) over chunks of kChunkTiles k-tiles: for
 // NS = 7, |L_d| <= 7 * 128^2 * 16384 < 2^31.  The levels are joined in 64-bit integers,
 // converted to FP64 once per chunk and summed in FP64.
 //
-// Error, NS = 7 (55-bit X): the products left out (i + j > 8) are digit products of zero
-// mean with weight 2^-70 of the two row scales; K of them add up to about
-// 2^-56 sqrt(K) max|S_p| max|S_q|, at most 2^-56 sqrt(K) sqrt(eps_pp eps_qq), because a row
-// maximum never exceeds the row's norm.  An FP64 sum of K products rounds its running sum K
-// times.  (M D_w and M in place of S on both sides would not be bounded so: max|M_q| can
-// exceed sqrt(eps_qq) by sqrt(max D / min D), 9 times the error of the FP64 sum for gaps over
-// three decades and amplitudes that grow as their square roots, 512 transitions.)
+// Error, NS = 7 (55-bit X): the entries are rounded to 2^-56 of their row's maximum, which
+// puts a random error of 2^-56 max|S_p| |S_q| and its mirror image into the sum, at most
+// 2^-55 sqrt(eps_pp eps_qq) whatever the spread of the entries and however long the sum,
+// because a row maximum never exceeds the row's norm.  The products left out (i + j > 9) are
+// digit products of zero mean with weight 2^-78 of the two row scales; K of them add up to
+// 2^-64 sqrt(K) max|S_p| max|S_q|, which is less.  (Without level 9 they are 256 times that and
+// the larger part: in rows that a few large entries dominate, 3 to 4 times the error of an
+// FP64 sum.)  An FP64 sum rounds its running sum K times, about 2^-54 sqrt(K).  Error against
+// extended precision over that of FP64 sums (rms, relative to sqrt(eps_pp eps_qq)): normal
+// entries 0.20 at 512 transitions, 0.05 at 4347; entries over three decades 0.23 and 0.05; three
+// large entries a row 0.27 and 0.17.  (M D_w and M in place of S on both sides would not be
+// bounded so: max|M_q| can exceed sqrt(eps_qq) by sqrt(max D / min D), 9 times the error of the
+// FP64 sum for gaps over three decades and amplitudes that grow as their square roots, 512
+// transitions.)
 //
 // 840 auxiliary functions, 4347 transitions, 32 frequencies: row maxima 0.04 ms, digits
 // 0.16 ms, products 1.23 ms (3.4 Pop/s int8), against 4.25 ms on DMMA (23 of 35 TF/s);
 // 2000 / 25000 / 32: 0.37 + 2.26 + 30.2 ms against 112 ms.
 // The operands are the same on both sides, so on the diagonal the products that are left out
-// hold squares, whose mean is not zero.  For even NS the largest of them, digit NS/2 + 1 against
-// itself, has the weight of the first level left out and would lower eps_pp by 1e-9 for NS = 4:
-// digit_slice_kernel sums it per row, and it is added to the diagonal.  For odd NS the first
-// squares are 2^-8 below that level.
+// hold squares, whose mean is not zero.  If D + 1 is even, the first level left out has one, of
+// digit (D + 1) / 2, which would lower eps_pp by 1e-9 for NS = 4 and by K 2^-66 max|S_p|^2 for
+// NS = 7: digit_slice_kernel sums it per row, and it is added to the diagonal.  Otherwise the
+// first square is 2^-8 below that level.
 // A row that holds an infinity or a NaN gives NaN, as the FP64 sums did.  A negative D_w
 // (inverted occupations) has no root: RIGW_FP64 then takes the DMMA kernel, which is launched
 // behind these and returns at once unless digit_rowmax_kernel met one; in the sliced
@@ -59,8 +66,13 @@ constexpr int kTileB = 64 * 64;                  // bytes of one digit of half a
 
 template <int NS>
 struct DigCfg {
-  static constexpr int kLo = NS < 4 ? NS : 4;    // levels of the low pass: NS + 2 - kLo .. NS + 1
-  static constexpr int kHi = NS - kLo;           // levels of the high pass: 2 .. kHi + 1 (digits 1 .. kHi)
+  // last level summed: seven digits stand for FP64 and take one more than the NS + 1 whose weight
+  // is that of the rounding of the entries
+  static constexpr int kTop = NS == 7 ? NS + 2 : NS + 1;
+  static constexpr int kLo = kTop - 1 < 4 ? kTop - 1 : 4;   // levels of the low pass: kTop + 1 - kLo .. kTop
+  static constexpr int kHi = kTop - 1 - kLo;     // levels of the high pass: 2 .. kHi + 1 (digits 1 .. kHi)
+  // the digit whose squares are added to the diagonal (0: none)
+  static constexpr int kSquare = kTop % 2 ? (kTop + 1) / 2 : 0;
   static constexpr int kSlot = NS * (kTileA + kTileB);
   static constexpr int kSlots = (216 * 1024) / kSlot;
   static constexpr int kPerHi = kHi > 0 ? NS / kHi : 1;   // k-tiles of the high pass per slot
@@ -95,7 +107,7 @@ __global__ void __launch_bounds__(256) digit_zero_kernel(const ProbDev* __restri
   for (int k = threadIdx.x; k < 4096; k += 256)
     if (wi.a + k < n) {
       p.dmax[wi.a + k] = 0u;
-      if (p.squares) p.squares[wi.a + k] = 0;
+      p.squares[wi.a + k] = 0;
     }
 }
 
@@ -150,7 +162,7 @@ RIGW_DEVICE_INLINE void bytes4(uint32_t w0, uint32_t w1, uint32_t w2, uint32_t w
 // The NS digits of 16 consecutive transitions of one row: X = rint(v scale), a carry-in of
 // 128 in every byte but the leading one makes the digits balanced, and 16 bytes per digit
 // go to core-matrix row `dst` (digit planes kTileA bytes apart).  Returns the sum of the squares
-// of digit NS/2 + 1.
+// of digit kSquare.
 template <int NS>
 RIGW_DEVICE_INLINE int write_digits(const double (&v)[16], double scale, int8_t* dst) {
   constexpr uint64_t kBias = NS >= 8 ? 0x0080808080808080ull : (0x8080808080808080ull & ((1ull << (8 * (NS - 1))) - 1));
@@ -177,8 +189,11 @@ RIGW_DEVICE_INLINE int write_digits(const double (&v)[16], double scale, int8_t*
   for (int s = 0; s < NS; ++s)
     *reinterpret_cast<uint4*>(dst + size_t(s) * kTileA) = make_uint4(out[s][0], out[s][1], out[s][2], out[s][3]);
   int sq = 0;
+  if constexpr (DigCfg<NS>::kSquare > 0) {
+    const auto& m = out[DigCfg<NS>::kSquare - 1];
 #pragma unroll
-  for (int g = 0; g < 4; ++g) sq = __dp4a(int(out[NS / 2][g]), int(out[NS / 2][g]), sq);
+    for (int g = 0; g < 4; ++g) sq = __dp4a(int(m[g]), int(m[g]), sq);
+  }
   return sq;
 }
 
@@ -229,7 +244,7 @@ __global__ void __launch_bounds__(256) digit_slice_kernel(const ProbDev* __restr
         for (int i = 0; i < 16; ++i) x[i] = v[c][i] * sd[w][(half * 2 + c) * 16 + i];
         sq += write_digits<NS>(x, sc, dig + digit_offset(wb - w0 + w, nrb, rb, nkt, kt, NS, row, half * 2 + c));
       }
-      if (NS % 2 == 0) atomicAdd(p.squares + size_t(wb + w) * p.npad + r, (unsigned long long)(sq));
+      if (DigCfg<NS>::kSquare > 0) atomicAdd(p.squares + size_t(wb + w) * p.npad + r, (unsigned long long)(sq));
     }
   }
 }
@@ -241,8 +256,8 @@ __global__ void __launch_bounds__(256) digit_slice_kernel(const ProbDev* __restr
 // in; tcgen05 reads 96 bytes of shared memory per clock and CTA and
 // TMA writes 30, below the 128 that shared memory delivers (a 128 x 128 tile of one CTA
 // would read 128 and write 45).  TMEM holds four 128-column accumulators, so the levels go
-// in two passes over a chunk: NS + 1 down to NS - 2 (22 of the 28 products for NS = 7), and
-// the rest from the leading digits alone, several k-tiles per slot.
+// in two passes over a chunk: the four lowest levels (24 of the 34 products for NS = 7), and
+// the rest from the leading digits alone, as many k-tiles per slot as fit.
 template <int NS, class Item>
 __device__ __forceinline__ void digit_product(const Item& it, const int jw) {
   using Cfg = DigCfg<NS>;
@@ -364,7 +379,7 @@ __device__ __forceinline__ void digit_product(const Item& it, const int jw) {
             const uint64_t ad = tc::desc_kmajor_cores(base, 512);
             const uint64_t bd = tc::desc_kmajor_cores(base + nd * kTileA, 512);
             const int nl = q == 0 ? Cfg::kLo : Cfg::kHi;
-            const int d0 = q == 0 ? NS + 2 - Cfg::kLo : 2;
+            const int d0 = q == 0 ? Cfg::kTop + 1 - Cfg::kLo : 2;
 #pragma unroll
             for (int a = 0; a < nl; ++a) {
               const int d = d0 + a;
@@ -397,7 +412,7 @@ __device__ __forceinline__ void digit_product(const Item& it, const int jw) {
     const int half = (warp - 2) >> 2;          // columns 64 half ..
     const uint32_t done = tc::mapa(acce, 0);
     // weight of the lowest level of unit-scaled operands
-    constexpr int kShift = 8 * (NS - 1) - 2 * (8 * NS - 1);
+    constexpr int kShift = 8 * (2 * NS - Cfg::kTop) - 2 * (8 * NS - 1);
     double acc[64];
 #pragma unroll
     for (int j = 0; j < 64; ++j) acc[j] = 0.0;
@@ -414,7 +429,7 @@ __device__ __forceinline__ void digit_product(const Item& it, const int jw) {
         constexpr int kLoL = Cfg::kLo, kHiL = Cfg::kHi;
         const double wq = q == 0 ? 1.0 : double(1ull << (8 * kLoL));
         // update: every chunk has row and column exponents of its own
-        double wr = wq;
+        double wr = wq * pow2(kShift);   // a power of two, at least 2^-1030
         const int* ecol = nullptr;
         if constexpr (kUpdate) {
           const int* e = it.exps + (size_t(slab) * it.ngroups + c) * it.nrb * 128;
@@ -436,7 +451,7 @@ __device__ __forceinline__ void digit_product(const Item& it, const int jw) {
 #pragma unroll
             for (int a = 1; a < 4; ++a)
               if (a < nl) x = x * 256 + int(r[a][j]);
-            if constexpr (kUpdate) acc[cb * 8 + j] += double(x) * (wr * pow2_of(ecol[cb * 8 + j] + kShift));
+            if constexpr (kUpdate) acc[cb * 8 + j] += double(x) * (wr * pow2_of(ecol[cb * 8 + j]));
             else acc[cb * 8 + j] += double(x) * wq;
           }
         }
@@ -474,7 +489,7 @@ __device__ __forceinline__ void digit_product(const Item& it, const int jw) {
             v[u] = (er == kNaNExp || ec == kNaNExp) ? __longlong_as_double(0x7ff8000000000000ll)
                                                      : ldexp(acc[j + u], er + ec + kShift);
             if (col0 + j + u == row) {
-              if (NS % 2 == 0)   // level NS + 2, one below the lowest
+              if (Cfg::kSquare > 0)   // of the level below the lowest
                 v[u] += ldexp(double(it.squares[size_t(it.w0 + jw) * it.ld + row]), 2 * er + kShift - 8);
               v[u] += 1.0;
             }
@@ -582,7 +597,7 @@ Status make_digit_tmaps(void* host_maps, const void* digits, long long planes, i
     g_encode_dig = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
   }
   CUtensorMap* maps = reinterpret_cast<CUtensorMap*>(host_maps);
-  const int nhi = ns > 4 ? ns - 4 : 1;
+  const int nhi = ns == 7 ? 4 : (ns > 4 ? ns - 4 : 1);   // DigCfg::kHi
   for (int m = 0; m < 4; ++m) {
     cuuint64_t dims[3] = {128, cuuint64_t(cores), cuuint64_t(planes)};
     cuuint64_t strides[2] = {128, cuuint64_t(128 * cores)};

@@ -443,7 +443,7 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
         if (planes > 2) {
           off[i].dmax = L.take(size_t(sh.nomega) * d.npad * sizeof(unsigned));
           off[i].xexp = L.take(size_t(sh.nomega) * d.npad * sizeof(int));
-          if (planes % 2 == 0) off[i].sq = L.take(size_t(sh.nomega) * d.npad * sizeof(unsigned long long));
+          off[i].sq = L.take(size_t(sh.nomega) * d.npad * sizeof(unsigned long long));
           off[i].neg = L.take(sizeof(int));
         }
       }
@@ -551,7 +551,7 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
         if (planes > 2) {
           p.dmax = reinterpret_cast<unsigned*>(base + off[i].dmax);
           p.xexp = reinterpret_cast<int*>(base + off[i].xexp);
-          if (planes % 2 == 0) p.squares = reinterpret_cast<unsigned long long*>(base + off[i].sq);
+          p.squares = reinterpret_cast<unsigned long long*>(base + off[i].sq);
           if (sh.precision == RIGW_FP64) p.negative = reinterpret_cast<int*>(base + off[i].neg);
         }
         alignas(64) unsigned char maps[512];

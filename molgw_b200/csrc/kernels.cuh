@@ -111,7 +111,7 @@ struct DigitItem {
   double* C;            // &eps[w0][0][0]
   int* err;
   const int* exps;      // digits, row exponents [w][ld]
-  const unsigned long long* squares;   // an even number of digits: ProbDev::squares
+  const unsigned long long* squares;   // digits: ProbDev::squares
   const int* negative;  // digits of FP64: not this kernel's problem when set (nullptr: always its)
   int rb_a, rb_b;       // 128-row blocks: output rows from 128 rb_a (two blocks), columns from 128 rb_b
   int nrb, nkt;         // row blocks and k-tiles (64 transitions) of a slab

@@ -60,8 +60,7 @@ struct ProbDev {
   int split_t;               // transitions per item of the row-maximum kernel
   unsigned* dmax;            // digits: [nomega][npad] high words of max_t |M_pt| sqrt(D_w(t))
   int* xexp;                 // digits: [nomega][npad] row exponents
-  unsigned long long* squares;   // an even number of digits: [nomega][npad] sums over t of the square of digit
-                             // planes / 2 + 1 (digit_gemm.cu)
+  unsigned long long* squares;   // digits: [nomega][npad] sums over t of the squares of one digit
   double* tnorm;
   double* dscale;
   double* eps;
