@@ -120,7 +120,7 @@ Status gw_density_matrix_imag(Context& c, const Wpol& w, const rigw_dm_problem& 
   if (ldm >= (1LL << 31)) return Status::fail(RIGW_ERR_ARG, "gw_density_matrix_imag: window too large");
   const size_t need = (size_t(nwp) * npad * npad + size_t(nwp) * naux_e * wq + size_t(naux) * ldm +
                        size_t(ng) * nwp + size_t(ng) * ng) * 8;
-  if (c.budget > 0 && need > (c.budget > c.in_use ? c.budget - c.in_use : 0))
+  if (c.budget > 0 && need > c.budget_left())
     return Status::fail(RIGW_ERR_NOMEM, "gw_density_matrix_imag: %zu bytes needed beyond the HBM budget", need);
   NvtxRange range("GW density matrix");
   const bool on_dev = (pr.flags & RIGW_PROBLEM_DEVICE_POINTERS) != 0;

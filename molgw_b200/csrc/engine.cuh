@@ -247,6 +247,11 @@ class Context {
   void put_idle(std::unique_ptr<Plan> plan, const Plan* parent);
   void drop_children(const Plan* parent);   // idle Sigma plans of a W that goes
   size_t idle_bytes() const;
+  // What the HBM budget still admits: idle plans and the spare block give way to an allocation.
+  size_t budget_left() const {
+    const size_t held = in_use - spare_bytes - idle_bytes();
+    return budget > held ? budget - held : 0;
+  }
   bool use_graphs = true;
   rigw_stats last_stats{};
   double host_build_ms = 0.0, host_capture_ms = 0.0;   // host time in plan builds / graph captures

@@ -259,7 +259,7 @@ Status sox_selfenergy_imag(Context& c, const rigw_sox_problem& pr, double* sigma
   // what the context's HBM budget has left
   const size_t per_p = size_t(ngp) * novp * 8;
   size_t cap = size_t(2) << 30;
-  if (c.budget > 0) cap = std::min(cap, c.budget > c.in_use ? (c.budget - c.in_use) / 2 : size_t(0));
+  if (c.budget > 0) cap = std::min(cap, c.budget_left() / 2);
   const int pc = int(std::max<size_t>(1, std::min<size_t>(size_t(nsig), cap / per_p)));
   RIGW_TRY(b_c.allocate(&c, per_p * pc, "sox (p q|j c)"));
   double* cbuf = reinterpret_cast<double*>(b_c.data());
@@ -659,7 +659,7 @@ Status sosex_selfenergy_imag(Context& c, const Wpol& w, const rigw_sosex_problem
   // of what the HBM budget has left
   const size_t per_m = (size_t(3) * wq * niap + size_t(naux_e) * wq) * 8;
   size_t cap = size_t(2) << 30;
-  if (c.budget > 0) cap = std::min(cap, c.budget > c.in_use ? (c.budget - c.in_use) / 2 : size_t(0));
+  if (c.budget > 0) cap = std::min(cap, c.budget_left() / 2);
   const int pc = int(std::max<size_t>(1, std::min<size_t>(size_t(nsig), cap / per_m)));
   DeviceBuffer b_t, b_b1, b_b2, b_r, b_wt, b_k, b_out, b_iw;
   RIGW_TRY(b_t.allocate(&c, size_t(pc) * wq * niap * 8, "sosex T"));
@@ -833,7 +833,7 @@ Status g3w2_selfenergy_imag(Context& c, const Wpol& w, const rigw_g3w2_problem& 
   // Gn and Gp of every frequency stay resident for the frequency pairs
   const size_t need = (size_t(2) * nwp * sk + size_t(nwp) * npad * npad + size_t(nwp) * naux_e * wq +
                        size_t(naux) * ldm + size_t(nwp) * nwp * nz * 2) * 8;
-  if (c.budget > 0 && need > (c.budget > c.in_use ? c.budget - c.in_use : 0))
+  if (c.budget > 0 && need > c.budget_left())
     return Status::fail(RIGW_ERR_NOMEM, "g3w2_selfenergy_imag: %zu bytes needed beyond the HBM budget", need);
   NvtxRange range("G3W2 self-energy");
   const bool on_dev = (pr.flags & RIGW_PROBLEM_DEVICE_POINTERS) != 0;

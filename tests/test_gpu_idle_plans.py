@@ -6,8 +6,8 @@ from dataclasses import replace
 import numpy as np
 import pytest
 
-from molgw_b200.rigw import Engine, RigwError
-from molgw_b200.synth import make_instance
+from molgw_b200.rigw import Engine, RigwError, efermi_of
+from molgw_b200.synth import make_instance, with_window
 
 pytestmark = pytest.mark.gpu
 
@@ -76,4 +76,41 @@ def test_kept_plans_give_way_to_an_allocation():
     sequence(eng, small)
     sequence(eng, replace(small, nomega=6))
     assert same(sequence(eng, large), ref)
+    eng.close()
+
+
+def vertex_call(eng, name, inst, mf):
+    """One of the calls that check their workspace against the HBM budget, or chunk by it."""
+    z = efermi_of(inst) + 1j * inst.step_sigma_calc * np.arange(inst.nomega_sigma_calc)
+    if name == "density matrix":
+        return eng.gw_density_matrix_imag(inst, mf, 8)[0]
+    if name == "sox":
+        return eng.sox_selfenergy_imag_grid(inst, z)
+    _, _, w = eng.polarizability_grid_scalapack(inst)
+    try:
+        return (eng.g3w2_selfenergy_imag_grid if name == "g3w2" else eng.sosex_selfenergy_imag_grid)(w, inst, mf, z)
+    finally:
+        w.release()
+
+
+@pytest.mark.parametrize("name", ["g3w2", "density matrix", "sosex", "sox"])
+def test_kept_plans_do_not_count_against_the_budget(name):
+    """In a context whose budget is full of kept plans (the W of the call among them) every call
+    gives the bits that it gives without a budget."""
+    inst, mf = with_window(make_instance(4, 25, 64, 6, seed=31), seed=32)
+    inst.nomega_sigma_calc = 9
+    other = make_instance(6, 40, 500, 8, seed=5)
+
+    def fill(eng):
+        eng.polarizability_grid_scalapack(inst)[2].release()
+        sequence(eng, other)
+        return eng.last_stats()["device_bytes_in_use"]
+
+    probe = Engine(0)
+    used = fill(probe)
+    ref = vertex_call(probe, name, inst, mf)
+    probe.close()
+    eng = Engine(0, hbm_budget_bytes=used + (256 << 10))
+    assert fill(eng) == used                   # nothing was dropped
+    assert np.array_equal(vertex_call(eng, name, inst, mf), ref)
     eng.close()
