@@ -25,9 +25,11 @@ int finish(rigw_ctx* ctx, const Status& s) {
 }
 
 Status run_batch(Context& c, rigw::PlanMode mode, int n, const rigw_problem* probs, rigw_result* res,
-                 std::unique_ptr<Plan>* owned_plan, const Plan* parent, const double* const* sigma_in) {
+                 std::unique_ptr<Plan>* owned_plan, const rigw::Wpol* w, const double* const* sigma_in) {
   std::vector<const rigw::ProbDev*> factors;   // of the W a Sigma plan reads
-  if (parent) factors.push_back(&const_cast<Plan*>(parent)->problems()[0].dev);
+  if (w) factors.push_back(&w->plan->problems()[0].dev);
+  const bool keep = !w || w->ctx == &c;        // whether this context sees the W go
+  const uint64_t parent = w ? w->plan->id() : 0;
   std::vector<Shape> shapes(n);
   for (int i = 0; i < n; ++i) RIGW_TRY(rigw::make_shape(probs[i], &shapes[i]));
   if (mode != rigw::kPlanPolar)
@@ -38,7 +40,8 @@ Status run_batch(Context& c, rigw::PlanMode mode, int n, const rigw_problem* pro
     if (probs[i].precision != RIGW_FP64 && !rigw::bf16x3_available())
       return Status::fail(RIGW_ERR_UNSUPPORTED, "precision %d not available", probs[i].precision);
   // a plan of an earlier call of this kind, or a new one
-  std::unique_ptr<Plan> fresh = c.take_idle(mode, shapes, parent);
+  std::unique_ptr<Plan> fresh;
+  if (keep) fresh = c.take_idle(mode, shapes, parent);
   Status bs;
   if (!fresh) {
     fresh.reset(new Plan());
@@ -67,7 +70,7 @@ Status run_batch(Context& c, rigw::PlanMode mode, int n, const rigw_problem* pro
     Context& c;
     std::unique_ptr<Plan>& p;
     ~Guard() {
-      if (p) c.drop_children(p.get());
+      if (p) c.drop_children(p->id());
     }
   } guard{c, fresh};
   RIGW_TRY(plan->stage_inputs(probs, c.stream));
@@ -87,7 +90,7 @@ Status run_batch(Context& c, rigw::PlanMode mode, int n, const rigw_problem* pro
   RIGW_TRY(err);
   if (res) RIGW_TRY(plan->fetch_results(probs, res, c.stream));
   if (owned_plan) *owned_plan = std::move(fresh);
-  else c.put_idle(std::move(fresh), parent);
+  else if (keep) c.put_idle(std::move(fresh), parent);
   return Status::ok();
 }
 
@@ -199,7 +202,7 @@ int rigw_gw_selfenergy_imag(rigw_ctx* ctx, const rigw_wpol* wpol, const rigw_pro
     return finish(ctx, Status::fail(RIGW_ERR_ARG, "problem does not match the resident polarizability"));
   std::lock_guard<std::mutex> lock(ctx->impl.mu);
   cudaSetDevice(ctx->impl.device);
-  return finish(ctx, run_batch(ctx->impl, rigw::kPlanSigma, 1, prob, result, nullptr, wpol->impl.plan.get(), nullptr));
+  return finish(ctx, run_batch(ctx->impl, rigw::kPlanSigma, 1, prob, result, nullptr, &wpol->impl, nullptr));
 }
 
 int rigw_wpol_release(rigw_ctx* /*ctx*/, rigw_wpol* wpol) {
@@ -207,7 +210,7 @@ int rigw_wpol_release(rigw_ctx* /*ctx*/, rigw_wpol* wpol) {
   Context* own = wpol->impl.ctx;   // the context that made it (alive: it owns the plan's memory)
   std::lock_guard<std::mutex> lock(own->mu);
   cudaSetDevice(own->device);
-  own->put_idle(std::move(wpol->impl.plan), nullptr);
+  own->put_idle(std::move(wpol->impl.plan), 0);
   delete wpol;
   return RIGW_OK;
 }

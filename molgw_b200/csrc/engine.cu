@@ -1,5 +1,6 @@
 // Host engine of the RI-GW library: plans, device memory, launch sequences.
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstring>
@@ -125,7 +126,12 @@ Status Context::reserve(size_t bytes) {
   return Status::ok();
 }
 
-std::unique_ptr<Plan> Context::take_idle(int mode, const std::vector<Shape>& shapes, const Plan* parent) {
+uint64_t Plan::next_id() {
+  static std::atomic<uint64_t> n{0};
+  return ++n;
+}
+
+std::unique_ptr<Plan> Context::take_idle(int mode, const std::vector<Shape>& shapes, uint64_t parent) {
   for (size_t k = idle.size(); k-- > 0;) {
     IdlePlan& e = idle[k];
     if (e.mode != mode || e.parent != parent || e.shapes < shapes || shapes < e.shapes) continue;
@@ -136,7 +142,7 @@ std::unique_ptr<Plan> Context::take_idle(int mode, const std::vector<Shape>& sha
   return nullptr;
 }
 
-void Context::drop_children(const Plan* parent) {
+void Context::drop_children(uint64_t parent) {
   for (size_t k = idle.size(); k-- > 0;)
     if (idle[k].parent == parent) idle.erase(idle.begin() + k);
 }
@@ -147,10 +153,10 @@ size_t Context::idle_bytes() const {
   return n;
 }
 
-void Context::put_idle(std::unique_ptr<Plan> plan, const Plan* parent) {
+void Context::put_idle(std::unique_ptr<Plan> plan, uint64_t parent) {
   const Plan* raw = plan.get();
   if (raw->bytes() > kIdleBytes) {
-    drop_children(raw);
+    drop_children(raw->id());
     return;
   }
   const int mode = raw->mode();
@@ -159,7 +165,7 @@ void Context::put_idle(std::unique_ptr<Plan> plan, const Plan* parent) {
   while (idle.size() > kIdlePlans || idle_bytes() > kIdleBytes) {
     std::unique_ptr<Plan> old = std::move(idle.front().plan);
     idle.erase(idle.begin());
-    drop_children(old.get());
+    drop_children(old->id());
   }
 }
 

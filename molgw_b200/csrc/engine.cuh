@@ -156,6 +156,7 @@ class Plan {
   std::vector<PlanProblem>& problems() { return probs_; }
   size_t bytes() const { return arena_.size() + lists_.size(); }
   PlanMode mode() const { return mode_; }
+  uint64_t id() const { return id_; }   // of this plan alone among all of the process, never 0
   const std::vector<Shape>& shapes() const { return shapes_; }
   ~Plan();
 
@@ -164,6 +165,8 @@ class Plan {
 
  private:
   void record(cudaStream_t s, int stage);
+  static uint64_t next_id();
+  const uint64_t id_ = next_id();
   Context* ctx_ = nullptr;
   PlanMode mode_ = kPlanFused;
   Tuning tune_;
@@ -180,7 +183,7 @@ class Plan {
   std::vector<F64SyrkItem> fl_syrk_;              // FP64 chi0, TMA-staged (64-row items)
   std::vector<WorkItem> wl_dzero_, wl_dmax_;               // digits: row maxima
   // chi0 on tcgen05, by the number of operand planes (2: bf16, 3 .. 7: digits)
-  std::vector<std::vector<WorkItem>> wl_slice_[8];         // per frequency group: planes of M D_w (first: and of M)
+  std::vector<std::vector<WorkItem>> wl_slice_[8];         // per frequency group: planes of M sqrt(D_w)
   std::vector<std::vector<DigitItem>> dl_syrk_[8];         // and the products
   std::vector<std::vector<GemmItem>> gl_k2_, gl_k2n_, gl_k3_, gl_k3d_;
   std::vector<std::vector<FactorSliceItem>> fl_slice_;   // digits of a finished panel group
@@ -231,21 +234,22 @@ class Context {
   std::map<std::pair<int, std::vector<Shape>>, std::unique_ptr<Plan>> plan_cache;
   // Plans of the stand-alone calls that are not in use (a released W, the Sigma and QP plans of
   // finished calls): a repeated sequence of such calls finds its lists uploaded and its graphs
-  // captured.  A Sigma plan belongs to the W (parent) whose factors its items point to and goes
-  // with it.  At most kIdlePlans and kIdleBytes; all are given back when an allocation would
+  // captured.  A Sigma plan belongs to the W of this context (parent: its plan's id) whose factors
+  // its items point to and goes with it; one on the W of another context is not kept, because
+  // this context does not learn when that W goes.  At most kIdlePlans and kIdleBytes; all are given back when an allocation would
   // fail, before an autotuning run and with the context.
   struct IdlePlan {
     int mode;
     std::vector<Shape> shapes;
-    const Plan* parent;
+    uint64_t parent;          // Plan::id() of the W, 0: none
     std::unique_ptr<Plan> plan;
   };
   static constexpr size_t kIdlePlans = 6;
   static constexpr size_t kIdleBytes = size_t(1) << 30;
   std::vector<IdlePlan> idle;   // oldest first
-  std::unique_ptr<Plan> take_idle(int mode, const std::vector<Shape>& shapes, const Plan* parent);
-  void put_idle(std::unique_ptr<Plan> plan, const Plan* parent);
-  void drop_children(const Plan* parent);   // idle Sigma plans of a W that goes
+  std::unique_ptr<Plan> take_idle(int mode, const std::vector<Shape>& shapes, uint64_t parent);
+  void put_idle(std::unique_ptr<Plan> plan, uint64_t parent);
+  void drop_children(uint64_t parent);   // idle Sigma plans of a W that goes
   size_t idle_bytes() const;
   // What the HBM budget still admits: idle plans and the spare block give way to an allocation.
   size_t budget_left() const {

@@ -54,6 +54,28 @@ def test_two_resident_w_of_one_shape():
     eng.close()
 
 
+def test_sigma_on_the_w_of_another_context():
+    """Sigma_c from a W that another context of the device made and gives up: the second context
+    keeps no plan on its factors, whatever W comes to lie at their place."""
+    a, b = make_instance(5, 40, 90, 8, seed=1), make_instance(5, 40, 90, 8, seed=2)
+    big = make_instance(8, 60, 260, 16, seed=4)
+    one, two = Engine(0), Engine(0)
+    ref = {id(x): sequence(one, x)[2] for x in (a, b)}
+    for x in (a, b, a):
+        _, _, w = one.polarizability_grid_scalapack(x)
+        held = two.last_stats()["device_bytes_in_use"]
+        for _ in range(3):
+            assert np.array_equal(two.gw_selfenergy_imag_scalapack(w, x), ref[id(x)])
+            assert np.array_equal(one.gw_selfenergy_imag_scalapack(w, x), ref[id(x)])
+        w.release()
+        one.autotune([big])                    # drops every kept plan of the first context
+    two.qp_solve(a, ref[id(a)])
+    assert two.last_stats()["device_bytes_in_use"] <= held + (1 << 20)     # no Sigma plans kept
+    one.close()
+    assert np.array_equal(sequence(two, b)[2], ref[id(b)])
+    two.close()
+
+
 def test_failed_w_is_not_kept():
     good = make_instance(5, 40, 90, 8, seed=1)
     bad = replace(good, occupation=2.0 - good.occupation, m_ia=good.m_ia * 3.0)   # chi0 > 1: not positive definite
