@@ -42,6 +42,20 @@ Status run_batch(Context& c, rigw::PlanMode mode, int n, const rigw_problem* pro
   // a plan of an earlier call of this kind, or a new one
   std::unique_ptr<Plan> fresh;
   if (keep) fresh = c.take_idle(mode, shapes, parent);
+  // the same without the digit buffers of the FP64 products, for a W that has no room for them
+  std::vector<Shape> lean = shapes;
+  bool digits = false;
+  for (Shape& sh : lean) {
+    digits = digits || (mode == rigw::kPlanPolar && (rigw::use_digits(sh) || rigw::use_factor_digits(sh)));
+    sh.no_digits = 1;
+  }
+  if (!fresh && digits && keep)
+    if (std::unique_ptr<Plan> kept = c.take_idle(mode, lean, parent)) {
+      size_t room = rigw::available_bytes(c) + c.idle_bytes() + kept->bytes();
+      for (auto& kv : c.plan_cache) room += kv.second->bytes();
+      if (Plan::measure(shapes, mode) > room) fresh = std::move(kept);
+      else c.drop_children(kept->id());   // there is room again
+    }
   Status bs;
   if (!fresh) {
     fresh.reset(new Plan());
@@ -51,16 +65,9 @@ Status run_batch(Context& c, rigw::PlanMode mode, int n, const rigw_problem* pro
       fresh.reset(new Plan());
       bs = fresh->build(&c, mode, shapes, factors);
     }
-    if (bs.code == RIGW_ERR_NOMEM) {   // without the digit buffers of the FP64 products
-      bool any = false;
-      for (Shape& sh : shapes) {
-        any = any || rigw::use_digits(sh) || rigw::use_factor_digits(sh);
-        sh.no_digits = 1;
-      }
-      if (any) {
-        fresh.reset(new Plan());
-        bs = fresh->build(&c, mode, shapes, factors);
-      }
+    if (bs.code == RIGW_ERR_NOMEM && digits) {
+      fresh.reset(new Plan());
+      bs = fresh->build(&c, mode, lean, factors);
     }
   }
   RIGW_TRY(bs);

@@ -136,3 +136,28 @@ def test_kept_plans_do_not_count_against_the_budget(name):
     assert fill(eng) == used                   # nothing was dropped
     assert np.array_equal(vertex_call(eng, name, inst, mf), ref)
     eng.close()
+
+
+def test_a_plan_without_room_for_digits_is_kept():
+    """A W whose digit buffers the budget does not hold runs on DMMA, and its repetitions replay the
+    kept plans of W and Sigma."""
+    inst = make_instance(10, 100, 400, 8, seed=3)
+    probe = Engine(0)
+    ref = sequence(probe, inst)
+    _, _, w = probe.polarizability_grid_scalapack(inst)
+    digits = probe.last_stats()["device_bytes_in_use"]
+    w.release()
+    probe.close()
+    eng = Engine(0, hbm_budget_bytes=digits - (12 << 20))
+    replayed = []
+    for _ in range(4):
+        _, _, w = eng.polarizability_grid_scalapack(inst)
+        st = eng.last_stats()
+        replayed.append(st["graph_replayed"])
+        assert st["device_bytes_in_use"] < digits - (12 << 20)
+        s = eng.gw_selfenergy_imag_scalapack(w, inst)
+        assert np.abs(s - ref[2]).max() <= 1e-12 * np.abs(ref[2]).max()
+        replayed.append(eng.last_stats()["graph_replayed"])
+        w.release()
+    assert replayed == [False] * 2 + [True] * 6
+    eng.close()
