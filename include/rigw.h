@@ -229,6 +229,8 @@ RIGW_API int rigw_wpol_chi(rigw_ctx* ctx, const rigw_wpol* wpol, double* chi);
  * of ``prob``; writes result->sigma_calc. */
 RIGW_API int rigw_gw_selfenergy_imag(rigw_ctx* ctx, const rigw_wpol* wpol, const rigw_problem* prob,
                             rigw_result* result);
+/* Gives the W back to the context that made it.  rigw_destroy frees the memory of every W of its
+ * context; such a W can still be released (ctx may be NULL), and calls with it fail. */
 RIGW_API int rigw_wpol_release(rigw_ctx* ctx, rigw_wpol* wpol);
 /* Continuation + QP equation from sigma_calc (host arrays of ``result``). */
 RIGW_API int rigw_qp_solve(rigw_ctx* ctx, const rigw_problem* prob, const double* sigma_calc,

@@ -24,6 +24,8 @@ int finish(rigw_ctx* ctx, const Status& s) {
   return s.code;
 }
 
+Status orphan() { return Status::fail(RIGW_ERR_ARG, "the context of this polarizability is gone"); }
+
 Status run_batch(Context& c, rigw::PlanMode mode, int n, const rigw_problem* probs, rigw_result* res,
                  std::unique_ptr<Plan>* owned_plan, const rigw::Wpol* w, const double* const* sigma_in) {
   std::vector<const rigw::ProbDev*> factors;   // of the W a Sigma plan reads
@@ -187,6 +189,7 @@ int rigw_polarizability_imag(rigw_ctx* ctx, const rigw_problem* prob, double* er
     return finish(ctx, s);
   }
   w->impl.ctx = &ctx->impl;
+  ctx->impl.live.push_back(&w->impl);
   rigw::make_shape(*prob, &w->impl.sh);
   if (erpa) *erpa = r.erpa;
   if (egw) *egw = r.egw;
@@ -197,6 +200,7 @@ int rigw_polarizability_imag(rigw_ctx* ctx, const rigw_problem* prob, double* er
 int rigw_wpol_chi(rigw_ctx* ctx, const rigw_wpol* wpol, double* chi) {
   if (!ctx) return RIGW_ERR_ARG;
   if (!wpol || !chi) return finish(ctx, Status::fail(RIGW_ERR_ARG, "null argument"));
+  if (!wpol->impl.plan) return finish(ctx, orphan());
   std::lock_guard<std::mutex> lock(ctx->impl.mu);
   cudaSetDevice(ctx->impl.device);
   return finish(ctx, rigw::wpol_chi(ctx->impl, wpol->impl, chi));
@@ -205,6 +209,7 @@ int rigw_wpol_chi(rigw_ctx* ctx, const rigw_wpol* wpol, double* chi) {
 int rigw_gw_selfenergy_imag(rigw_ctx* ctx, const rigw_wpol* wpol, const rigw_problem* prob, rigw_result* result) {
   if (!ctx) return RIGW_ERR_ARG;
   if (!wpol || !prob || !result) return finish(ctx, Status::fail(RIGW_ERR_ARG, "null argument"));
+  if (!wpol->impl.plan) return finish(ctx, orphan());
   if (prob->naux != wpol->impl.sh.naux || prob->nomega != wpol->impl.sh.nomega)
     return finish(ctx, Status::fail(RIGW_ERR_ARG, "problem does not match the resident polarizability"));
   std::lock_guard<std::mutex> lock(ctx->impl.mu);
@@ -214,10 +219,12 @@ int rigw_gw_selfenergy_imag(rigw_ctx* ctx, const rigw_wpol* wpol, const rigw_pro
 
 int rigw_wpol_release(rigw_ctx* /*ctx*/, rigw_wpol* wpol) {
   if (!wpol) return RIGW_ERR_ARG;
-  Context* own = wpol->impl.ctx;   // the context that made it (alive: it owns the plan's memory)
-  std::lock_guard<std::mutex> lock(own->mu);
-  cudaSetDevice(own->device);
-  own->put_idle(std::move(wpol->impl.plan), 0);
+  if (Context* own = wpol->impl.ctx) {   // the context that made it
+    std::lock_guard<std::mutex> lock(own->mu);
+    cudaSetDevice(own->device);
+    own->live.erase(std::remove(own->live.begin(), own->live.end(), &wpol->impl), own->live.end());
+    own->put_idle(std::move(wpol->impl.plan), 0);
+  }
   delete wpol;
   return RIGW_OK;
 }
@@ -243,6 +250,7 @@ int rigw_sosex_selfenergy_imag(rigw_ctx* ctx, const rigw_wpol* wpol, const rigw_
                                double* sigma_sosex) {
   if (!ctx) return RIGW_ERR_ARG;
   if (!wpol || !prob || !sigma_sosex) return finish(ctx, Status::fail(RIGW_ERR_ARG, "null argument"));
+  if (!wpol->impl.plan) return finish(ctx, orphan());
   std::lock_guard<std::mutex> lock(ctx->impl.mu);
   cudaSetDevice(ctx->impl.device);
   return finish(ctx, rigw::sosex_selfenergy_imag(ctx->impl, wpol->impl, *prob, sigma_sosex));
@@ -252,6 +260,7 @@ int rigw_g3w2_selfenergy_imag(rigw_ctx* ctx, const rigw_wpol* wpol, const rigw_g
                               double* sigma_g3w2) {
   if (!ctx) return RIGW_ERR_ARG;
   if (!wpol || !prob || !sigma_g3w2) return finish(ctx, Status::fail(RIGW_ERR_ARG, "null argument"));
+  if (!wpol->impl.plan) return finish(ctx, orphan());
   std::lock_guard<std::mutex> lock(ctx->impl.mu);
   cudaSetDevice(ctx->impl.device);
   return finish(ctx, rigw::g3w2_selfenergy_imag(ctx->impl, wpol->impl, *prob, sigma_g3w2));
@@ -285,6 +294,7 @@ int rigw_gw_density_matrix_imag(rigw_ctx* ctx, const rigw_wpol* wpol, const rigw
                                 double* p_matrix) {
   if (!ctx) return RIGW_ERR_ARG;
   if (!wpol || !prob || !p_matrix) return finish(ctx, Status::fail(RIGW_ERR_ARG, "null argument"));
+  if (!wpol->impl.plan) return finish(ctx, orphan());
   std::lock_guard<std::mutex> lock(ctx->impl.mu);
   cudaSetDevice(ctx->impl.device);
   return finish(ctx, rigw::gw_density_matrix_imag(ctx->impl, wpol->impl, *prob, p_matrix));

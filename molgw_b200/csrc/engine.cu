@@ -245,6 +245,10 @@ Status Context::sync(cudaStream_t s) {
 }
 
 Context::~Context() {
+  for (Wpol* w : live) {
+    w->plan.reset();
+    w->ctx = nullptr;
+  }
   plan_cache.clear();
   idle.clear();
   free_spare();

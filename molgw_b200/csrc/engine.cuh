@@ -251,6 +251,9 @@ class Context {
   void put_idle(std::unique_ptr<Plan> plan, uint64_t parent);
   void drop_children(uint64_t parent);   // idle Sigma plans of a W that goes
   size_t idle_bytes() const;
+  // The W that calls have handed out; a context that ends takes their memory with it and leaves
+  // them without a plan, for their holders to release.
+  std::vector<struct Wpol*> live;
   // What the HBM budget still admits: idle plans and the spare block give way to an allocation.
   size_t budget_left() const {
     const size_t held = in_use - spare_bytes - idle_bytes();
@@ -300,7 +303,7 @@ class Context {
 };
 
 struct Wpol {
-  Context* ctx = nullptr;
+  Context* ctx = nullptr;         // nullptr: the context is gone
   std::unique_ptr<Plan> plan;     // the kPlanPolar plan that owns eps/U, winv and U^-T
   Shape sh;
 };

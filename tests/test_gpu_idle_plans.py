@@ -76,6 +76,25 @@ def test_sigma_on_the_w_of_another_context():
     two.close()
 
 
+def test_a_w_outlives_its_context():
+    """A context that ends takes the memory of the W it handed out; they can still be released, and
+    calls with them are refused."""
+    a = make_instance(5, 40, 90, 8, seed=1)
+    other = Engine(0)
+    ref = sequence(other, a)
+    for _ in range(3):
+        eng = Engine(0)
+        _, _, w = eng.polarizability_grid_scalapack(a)
+        _, _, v = eng.polarizability_grid_scalapack(a)
+        v.release()
+        eng.close()
+        with pytest.raises(RigwError):
+            other.gw_selfenergy_imag_scalapack(w, a)
+        w.release()
+        assert same(sequence(other, a), ref)
+    other.close()
+
+
 def test_failed_w_is_not_kept():
     good = make_instance(5, 40, 90, 8, seed=1)
     bad = replace(good, occupation=2.0 - good.occupation, m_ia=good.m_ia * 3.0)   # chi0 > 1: not positive definite
