@@ -53,7 +53,7 @@ Status run_batch(Context& c, rigw::PlanMode mode, int n, const rigw_problem* pro
   }
   if (!fresh && digits && keep)
     if (std::unique_ptr<Plan> kept = c.take_idle(mode, lean, parent)) {
-      size_t room = rigw::available_bytes(c) + c.idle_bytes() + kept->bytes();
+      size_t room = rigw::available_bytes(c) + c.reclaimable_bytes() + kept->bytes();
       for (auto& kv : c.plan_cache) room += kv.second->bytes();
       if (Plan::measure(shapes, mode) > room) fresh = std::move(kept);
       else c.drop_children(kept->id());   // there is room again
@@ -190,6 +190,7 @@ int rigw_polarizability_imag(rigw_ctx* ctx, const rigw_problem* prob, double* er
   }
   w->impl.ctx = &ctx->impl;
   ctx->impl.live.push_back(&w->impl);
+  if (w->impl.plan->bytes() > Context::kIdleBytes) w->impl.plan->drop_scratch();   // too large to be kept for another
   rigw::make_shape(*prob, &w->impl.sh);
   if (erpa) *erpa = r.erpa;
   if (egw) *egw = r.egw;

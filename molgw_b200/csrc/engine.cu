@@ -71,7 +71,7 @@ Status DeviceBuffer::allocate(Context* ctx, size_t bytes, const char* name) {
     return Status::ok();   // already counted in in_use
   }
   if (ctx->budget && ctx->in_use + bytes > ctx->budget) {
-    ctx->idle.clear();
+    ctx->reclaim();
     ctx->free_spare();
   }
   if (ctx->budget && ctx->in_use + bytes > ctx->budget)
@@ -81,9 +81,9 @@ Status DeviceBuffer::allocate(Context* ctx, size_t bytes, const char* name) {
   // stays mapped in the pool and is handed to the next plan without remapping.
   const auto t0 = std::chrono::steady_clock::now();
   cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(&ptr_), bytes, ctx->stream);
-  if (e != cudaSuccess && (ctx->spare_ptr || !ctx->idle.empty())) {   // what is kept may be what is missing
+  if (e != cudaSuccess && (ctx->spare_ptr || ctx->reclaimable_bytes() > 0)) {   // what is kept may be what is missing
     cudaGetLastError();
-    ctx->idle.clear();
+    ctx->reclaim();
     ctx->free_spare();
     e = cudaMallocAsync(reinterpret_cast<void**>(&ptr_), bytes, ctx->stream);
   }
@@ -100,10 +100,10 @@ Status DeviceBuffer::allocate(Context* ctx, size_t bytes, const char* name) {
   return Status::ok();
 }
 
-void DeviceBuffer::release() {
+void DeviceBuffer::release(bool keep_spare) {
   if (ptr_) {
     ctx_->sync(ctx_->stream);
-    if (bytes_ >= Context::kSpareMin && bytes_ > ctx_->spare_bytes) {
+    if (keep_spare && bytes_ >= Context::kSpareMin && bytes_ > ctx_->spare_bytes) {
       // keep the larger block for the next plan of this context
       ctx_->free_spare();
       ctx_->spare_ptr = ptr_;
@@ -153,9 +153,20 @@ size_t Context::idle_bytes() const {
   return n;
 }
 
+size_t Context::reclaimable_bytes() const {
+  size_t n = idle_bytes();
+  for (const Wpol* w : live) n += w->plan->scratch_bytes();
+  return n;
+}
+
+void Context::reclaim() {
+  idle.clear();
+  for (Wpol* w : live) w->plan->drop_scratch();
+}
+
 void Context::put_idle(std::unique_ptr<Plan> plan, uint64_t parent) {
   const Plan* raw = plan.get();
-  if (raw->bytes() > kIdleBytes) {
+  if (!raw->runnable() || raw->bytes() > kIdleBytes) {
     drop_children(raw->id());
     return;
   }
@@ -408,7 +419,8 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
   };
 
   // ---- memory layout
-  Layout L;
+  Layout L, LS;               // arena, scratch of a W
+  Layout& LX = mode == kPlanPolar ? LS : L;
   // digit blocks of the factor [U | right-hand sides], and the bytes of its digits
   auto factor_blocks = [&](const Dims& d) { return d.npanel + (d.ldb + kPanel - 1) / kPanel; };
   auto factor_bytes = [&](const Shape& sh, const Dims& d) {
@@ -441,8 +453,9 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
       // the chi0 operands and, after them, the digits of the factor
       const int planes = operand_planes(sh);
       const bool fd = use_factor_digits(sh);
-      off[i].xs = L.take(std::max(planes ? size_t(split_group(sh)) * split_bytes_per_frequency(sh) : 0,
-                                  fd ? factor_bytes(sh, d) : 0));
+      const size_t xs = std::max(planes ? size_t(split_group(sh)) * split_bytes_per_frequency(sh) : 0,
+                                 fd ? factor_bytes(sh, d) : 0);
+      if (xs) off[i].xs = LX.take(xs);
       if (fd) {
         off[i].fmap = L.take(512);
         off[i].fexp = L.take(size_t(sh.nomega) * ((d.npanel + factor_group(sh) - 1) / factor_group(sh)) * factor_blocks(d) *
@@ -515,11 +528,13 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
                  groups * (d.npanel / 2 + 1) * d.npanel * sizeof(DigitItem);
       }
     }
-    *measure_only = L.cur + lists + (size_t(1) << 20);
+    *measure_only = L.cur + LS.cur + lists + (size_t(1) << 20);
     return Status::ok();
   }
   RIGW_TRY(arena_.allocate(ctx, L.cur, "plan arena"));
+  RIGW_TRY(scratch_.allocate(ctx, LS.cur, "plan scratch"));
   char* base = arena_.data();
+  char* const xbase = mode == kPlanPolar ? scratch_.data() : base;
   probs_dev_ = reinterpret_cast<ProbDev*>(base + table_off);
   err_dev_ = reinterpret_cast<int*>(base + err_off);
   auto dp = [&](size_t o) { return reinterpret_cast<double*>(base + o); };
@@ -557,7 +572,7 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
       p.tnorm = dp(off[i].tnorm);
       p.dscale = dp(off[i].dscale);
       if (const int planes = operand_planes(sh)) {
-        p.xs = base + off[i].xs;
+        p.xs = xbase + off[i].xs;
         if (planes > 2) {
           p.dmax = reinterpret_cast<unsigned*>(base + off[i].dmax);
           p.xexp = reinterpret_cast<int*>(base + off[i].xexp);
@@ -576,7 +591,7 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
       }
       if (use_factor_digits(sh)) {
         alignas(64) unsigned char maps[512];
-        RIGW_TRY(make_digit_tmaps(maps, base + off[i].xs,
+        RIGW_TRY(make_digit_tmaps(maps, xbase + off[i].xs,
                                   (long long)sh.nomega * factor_blocks(d) * (d.npad / 64) * kFp64Digits, kFp64Digits, 64));
         RIGW_CUDA_TRY(cudaMemcpyAsync(base + off[i].fmap, maps, sizeof(maps), cudaMemcpyHostToDevice, ctx->stream));
       }
@@ -814,7 +829,7 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
           auto slice = [&](const double* X, int ldx, long long stride, int c0, int n, int rb) {
             FactorSliceItem f{};
             f.src = X + size_t(kp) * kPanel * ldx + c0;
-            f.digits = base + off[i].xs;
+            f.digits = xbase + off[i].xs;
             f.exps = fexp;
             f.ld = ldx;
             f.ncol = n;

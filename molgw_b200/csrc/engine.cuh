@@ -70,7 +70,7 @@ class DeviceBuffer {
   DeviceBuffer(const DeviceBuffer&) = delete;
   DeviceBuffer& operator=(const DeviceBuffer&) = delete;
   Status allocate(Context* ctx, size_t bytes, const char* name);
-  void release();
+  void release(bool keep_spare = true);
   char* data() const { return ptr_; }
   size_t size() const { return bytes_; }
 
@@ -154,7 +154,14 @@ class Plan {
   Status check_errors(cudaStream_t s);
   float last_ms() const { return last_ms_; }
   std::vector<PlanProblem>& problems() { return probs_; }
-  size_t bytes() const { return arena_.size() + lists_.size(); }
+  size_t bytes() const { return arena_.size() + scratch_.size() + lists_.size(); }
+  // A W that has been solved needs its operand planes and digits only to be solved again.
+  size_t scratch_bytes() const { return scratch_.size(); }
+  void drop_scratch() {
+    dropped_ = dropped_ || scratch_.size() > 0;
+    scratch_.release(false);
+  }
+  bool runnable() const { return !dropped_; }
   PlanMode mode() const { return mode_; }
   uint64_t id() const { return id_; }   // of this plan alone among all of the process, never 0
   const std::vector<Shape>& shapes() const { return shapes_; }
@@ -173,6 +180,8 @@ class Plan {
   std::vector<Shape> shapes_;
   std::vector<PlanProblem> probs_;
   DeviceBuffer arena_;
+  DeviceBuffer scratch_;      // kPlanPolar: ProbDev::xs (in the arena in the other modes)
+  bool dropped_ = false;
   DeviceBuffer lists_;
   ProbDev* probs_dev_ = nullptr;
   int* err_dev_ = nullptr;
@@ -251,12 +260,16 @@ class Context {
   void put_idle(std::unique_ptr<Plan> plan, uint64_t parent);
   void drop_children(uint64_t parent);   // idle Sigma plans of a W that goes
   size_t idle_bytes() const;
-  // The W that calls have handed out; a context that ends takes their memory with it and leaves
+  // The W that calls have handed out, solved and not running: what they need only to be solved
+  // again is given back with the idle plans; a context that ends takes their memory with it and leaves
   // them without a plan, for their holders to release.
   std::vector<struct Wpol*> live;
-  // What the HBM budget still admits: idle plans and the spare block give way to an allocation.
+  // What gives way to an allocation besides the spare block.
+  size_t reclaimable_bytes() const;
+  void reclaim();
+  // What the HBM budget still admits.
   size_t budget_left() const {
-    const size_t held = in_use - spare_bytes - idle_bytes();
+    const size_t held = in_use - spare_bytes - reclaimable_bytes();
     return budget > held ? budget - held : 0;
   }
   bool use_graphs = true;

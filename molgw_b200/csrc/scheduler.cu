@@ -120,7 +120,7 @@ Status solve_batch(Context& c, int n, const rigw_problem* probs, rigw_result* re
   // plans cached for other shapes count as free memory for this decision
   size_t cached = 0;
   for (auto& kv : c.plan_cache) cached += kv.second->bytes();
-  cached += c.idle_bytes();
+  cached += c.reclaimable_bytes();
   const size_t usable = avail + cached;
 
   // ---- fits: one fused plan
@@ -136,7 +136,7 @@ Status solve_batch(Context& c, int n, const rigw_problem* probs, rigw_result* re
 
   // ---- frequency chunks and waves
   c.plan_cache.clear();
-  c.idle.clear();
+  c.reclaim();
   avail = available_bytes(c);
   struct Unit {
     int prob, w0, nw;
@@ -248,7 +248,7 @@ Status autotune(Context& c, int n, const rigw_problem* probs, rigw_tune_report* 
   RIGW_TRY(validate_batch(n, probs, &shapes));
   std::memset(rep, 0, sizeof(*rep));
   c.plan_cache.clear();
-  c.idle.clear();
+  c.reclaim();
   const size_t avail = available_bytes(c);
   const int cls = precision_class(shapes);
   bool any_fp64 = false;

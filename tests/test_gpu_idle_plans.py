@@ -180,3 +180,28 @@ def test_a_plan_without_room_for_digits_is_kept():
         w.release()
     assert replayed == [False] * 2 + [True] * 6
     eng.close()
+
+
+def test_the_digits_of_a_solved_w_give_way():
+    """Three W in a budget that holds two with their digit buffers and one without, which is more
+    than three without: all are accepted, and give what they give without a budget."""
+    insts = [make_instance(10, 100, 400, 8, seed=s) for s in (3, 4, 5)]
+    probe = Engine(0)
+    ref = [sequence(probe, x)[2] for x in insts]
+    probe.close()
+    held = []
+    for budget in (0, None):
+        eng = Engine(0, hbm_budget_bytes=0 if budget == 0 else held[0] - (1 << 20))
+        w = eng.polarizability_grid_scalapack(insts[0])[2]
+        held.append(eng.last_stats()["device_bytes_in_use"])
+        w.release()
+        eng.close()
+    assert held[0] - held[1] > (20 << 20)
+    eng = Engine(0, hbm_budget_bytes=2 * held[0] + held[1] - (1 << 20))
+    w = [eng.polarizability_grid_scalapack(x)[2] for x in insts]
+    for x, v, r in zip(insts, w, ref):
+        assert np.abs(eng.gw_selfenergy_imag_scalapack(v, x) - r).max() <= 1e-12 * np.abs(r).max()
+    for v in w:
+        v.release()
+    assert np.array_equal(sequence(eng, insts[0])[2], ref[0])
+    eng.close()
