@@ -34,6 +34,7 @@ Status run_batch(Context& c, rigw::PlanMode mode, int n, const rigw_problem* pro
   const uint64_t parent = w ? w->plan->id() : 0;
   std::vector<Shape> shapes(n);
   for (int i = 0; i < n; ++i) RIGW_TRY(rigw::make_shape(probs[i], &shapes[i]));
+  rigw::choose_factor_digits(&shapes);
   if (mode != rigw::kPlanPolar)
     for (int i = 0; i < n; ++i)
       if (shapes[i].nc < 1 || shapes[i].nsig < 1 || shapes[i].nstate_p < 1)
@@ -143,8 +144,9 @@ const char* rigw_last_error(const rigw_ctx* ctx) {
 }
 
 size_t rigw_footprint_bytes(int naux, int nocc, int nvirt, int nomega, int nstate_p, int nsig, int precision) {
-  Shape sh{naux, nocc, nvirt, nomega, nstate_p, nsig, 0, 0, 0, precision, 0};
-  return rigw::footprint(sh, rigw::kPlanFused);
+  std::vector<Shape> sh{Shape{naux, nocc, nvirt, nomega, nstate_p, nsig, 0, 0, 0, precision, 0}};
+  rigw::choose_factor_digits(&sh);
+  return rigw::footprint(sh[0], rigw::kPlanFused);
 }
 
 int rigw_imag_grid(int nomega, double* omega, double* weight) {

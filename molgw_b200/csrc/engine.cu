@@ -20,8 +20,9 @@ inline int round_up(int v, int a) { return (v + a - 1) / a * a; }
 // ---------------------------------------------------------------------------
 bool Shape::operator<(const Shape& o) const {
   return std::tie(naux, nocc, nvirt, nomega, nstate_p, nsig, nc, nsigma_half, technique, precision, qp_only, nocc2,
-                  nvirt2, no_digits) < std::tie(o.naux, o.nocc, o.nvirt, o.nomega, o.nstate_p, o.nsig, o.nc, o.nsigma_half,
-                                     o.technique, o.precision, o.qp_only, o.nocc2, o.nvirt2, o.no_digits);
+                  nvirt2, factor_digits, no_digits) < std::tie(o.naux, o.nocc, o.nvirt, o.nomega, o.nstate_p, o.nsig, o.nc, o.nsigma_half,
+                                     o.technique, o.precision, o.qp_only, o.nocc2, o.nvirt2,
+                                     o.factor_digits, o.no_digits);
 }
 
 Status make_shape(const rigw_problem& p, Shape* sh) {
@@ -50,6 +51,7 @@ Status make_shape(const rigw_problem& p, Shape* sh) {
   sh->nsigma_half = p.nomega_sigma / 2;
   sh->technique = p.technique;
   sh->precision = p.precision;
+  sh->factor_digits = 0;
   sh->no_digits = 0;
   sh->qp_only = (p.flags & RIGW_PROBLEM_QP_ONLY) ? 1 : 0;
   return Status::ok();
@@ -319,15 +321,31 @@ bool use_digits(const Shape& sh) {
          (long long)sh.nocc * sh.nvirt + (long long)sh.nocc2 * sh.nvirt2 >= 512;
 }
 
-// Factorization stage, DMMA against digits in groups of four panels (32 frequencies, ms): naux
-// 500 0.46 / 0.48, 840 1.91 / 1.88, 1152 3.51 / 3.14, 1483 7.15 / 5.36, 2000 18.4 / 12.9, 4000
-// (48 frequencies, QP only) 139 / 67.
-bool use_factor_digits(const Shape& sh) { return !sh.no_digits && sh.naux > 768; }
+// The digits take a launch and a pass over the finished rows more per group, and their products
+// run in chunks of one group: the frequencies and panels of the whole batch have to fill that.
+// Factorization stage, DMMA against digits (ms): 32 frequencies naux 640 0.83 / 0.89, 768 1.23 /
+// 1.18, 800 1.72 / 1.75, 840 1.78 / 1.75, 1024 2.43 / 2.06, 1152 3.37 / 2.98, 1483 7.06 / 5.16,
+// 2000 15.6 / 10.3; 8 frequencies 840 0.73 / 0.88, 1152 1.19 / 1.22, 1483 2.11 / 1.80; 4: 1483
+// 1.49 / 1.47, 2000 2.76 / 2.73; 2: 2000 1.96 / 2.08, 2600 3.33 / 3.15; 1: 840 0.58 / 0.75,
+// 2000 1.50 / 2.00, 3000 2.95 / 2.81, 4000 5.43 / 4.70; 8 molecules of 800 to 1220 with 4
+// frequencies each 2.30 / 2.04.  The line follows frequencies x panels^2, summed over the batch.
+void choose_factor_digits(std::vector<Shape>* shapes) {
+  long long work = 0;
+  for (const Shape& sh : *shapes) {
+    const long long panels = (sh.naux + kPanel - 1) / kPanel;
+    work += sh.nomega * panels * panels;
+  }
+  for (Shape& sh : *shapes) sh.factor_digits = sh.naux > 768 && work >= 800;
+}
 
-// Two panels leave the least to DMMA; from 24 panels on the sums are long enough that the four
-// of a group, drained once per group, win (stage, groups of 2 / 4 / 8, ms: 8 molecules up to
-// 1152 7.0 / 7.7 / 7.8, 1483 5.07 / 5.28 / 5.78, 2000 12.0 / 12.5 / 15.1, 4000 71.6 / 69.7 / 72.3).
-int factor_group(const Shape& sh) { return sh.naux > 23 * kPanel ? 4 : 2; }
+bool use_factor_digits(const Shape& sh) { return !sh.no_digits && sh.factor_digits; }
+
+// Two panels leave the least to DMMA; from 13 panels on the sums are long enough that the four of
+// a group, drained once per group, do as well or better (stage, groups of 2 / 4, ms: 8 frequencies
+// naux 1640 2.44 / 2.35, 1900 3.24 / 2.98, 2300 4.34 / 4.15; 16: 1500 2.89 / 2.95, 1640 3.98 /
+// 3.99, 2040 5.74 / 5.66, 2940 15.0 / 13.3; 32: 1640 6.99 / 7.00, 1900 9.58 / 9.44, 2040 10.4 /
+// 10.5, without the identity part 7.6 / 7.2).
+int factor_group(const Shape& sh) { return sh.naux > 12 * kPanel ? 4 : 2; }
 
 int operand_planes(const Shape& sh) {
   if (sh.precision == RIGW_BF16X3) return 2;

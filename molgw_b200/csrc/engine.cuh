@@ -90,6 +90,7 @@ struct Shape {
   int naux, nocc, nvirt, nomega, nstate_p, nsig, nc, nsigma_half, technique, precision;
   int qp_only;
   int nocc2 = 0, nvirt2 = 0;   // second spin channel of the W window
+  int factor_digits = 0;       // choose_factor_digits
   int no_digits = 0;           // FP64 products by DMMA alone: set where the digit buffers do not fit
   bool operator<(const Shape& o) const;
 };
@@ -108,8 +109,10 @@ struct Tuning {
 int precision_class(const std::vector<Shape>& shapes);
 // Whether the FP64 chi0 of a problem goes through the int8 digit products.
 bool use_digits(const Shape& sh);
-// Whether the updates between panel groups of the factorization go through digit products, and
-// the panels of such a group (even: rows are updated in pairs of panels).
+// Whether the updates between panel groups of the factorization go through digit products (set
+// for the problems of a batch together, before any plan of it or of parts of it), and the panels
+// of such a group (even: rows are updated in pairs of panels).
+void choose_factor_digits(std::vector<Shape>* shapes);
 bool use_factor_digits(const Shape& sh);
 int factor_group(const Shape& sh);
 // Planes of the chi0 operands: 2 (bf16 hi/lo), 3 .. 7 (int8 digits), 0 (FP64 on DMMA).

@@ -102,6 +102,7 @@ Status validate_batch(int n, const rigw_problem* probs, std::vector<Shape>* shap
     if (probs[i].precision != RIGW_FP64 && !bf16x3_available())
       return Status::fail(RIGW_ERR_UNSUPPORTED, "precision %d not available", probs[i].precision);
   }
+  choose_factor_digits(shapes);
   return Status::ok();
 }
 

@@ -242,6 +242,7 @@ RIGW_API int rigw_server_submit(rigw_server* srv, const rigw_problem* prob, rigw
   auto r = std::make_shared<rigw::Request>();
   r->prob = *prob;
   r->res = result;
+  sh.factor_digits = sh.naux > 768;   // at most: the batch that it is solved in decides
   r->bytes = rigw::Plan::measure({sh}, rigw::kPlanFused);
   r->large = r->bytes > srv->impl.share / rigw::Server::kLargeShare;
   {

@@ -195,10 +195,16 @@ def sigma_reference(inst, omega, weight, z):
 
 
 @pytest.mark.parametrize("nocc,nvirt,naux,nomega", [
-    (9, 60, 769, 3),       # seven panels in groups of two: the last group has one
-    (8, 70, 1030, 5),      # nine panels, one column block of the right-hand sides ends early
-    (10, 65, 1100, 2),     # M columns that end inside a 128-column block
-    (6, 86, 3200, 1),      # 25 panels in groups of four: the last group has one
+    # on DMMA: too few frequencies for their panels
+    (9, 60, 769, 3),
+    (8, 70, 1030, 5),
+    (10, 65, 1100, 2),
+    (6, 86, 3200, 1),
+    # as many frequencies as the digit products take up (frequencies x panels^2 >= 800)
+    (9, 60, 769, 17),      # seven panels in groups of two: the last group has one
+    (8, 70, 1030, 10),     # nine panels, one column block of the right-hand sides ends early
+    (10, 65, 1100, 10),    # M columns that end inside a 128-column block
+    (6, 86, 3200, 2),      # 25 panels in groups of four: the last group has one
 ])
 @pytest.mark.parametrize("qp_only", [False, True])
 def test_factorization_updates_by_digits(engine, nocc, nvirt, naux, nomega, qp_only):
@@ -214,6 +220,15 @@ def test_factorization_updates_by_digits(engine, nocc, nvirt, naux, nomega, qp_o
     ef = 0.5 * (inst.energy[nocc - 1] + inst.energy[nocc])
     ref = sigma_reference(inst, om, wt, ef + 1j * inst.step_sigma_calc * np.arange(inst.nomega_sigma_calc))
     assert np.abs(out.sigma_calc - ref).max() <= 1e-13 * np.abs(ref).max()
+
+
+def test_a_batch_takes_up_the_digits_together(engine):
+    """Two problems that factorize on DMMA alone and on digit products together, beside one that is
+    too small for them."""
+    insts = [make_instance(8, 90, n, 7, seed=n) for n in (900, 1000, 420)]
+    for one, both in zip([engine.g0w0(i) for i in insts], engine.g0w0_batch(insts)):
+        assert abs(one.erpa - both.erpa) <= 1e-10 * abs(one.erpa)
+        assert np.abs(one.sigma_calc - both.sigma_calc).max() <= 1e-12 * np.abs(one.sigma_calc).max()
 
 
 @pytest.mark.parametrize("bad", [np.nan, np.inf])
