@@ -146,12 +146,19 @@ Status solve_batch(Context& c, int n, const rigw_problem* probs, rigw_result* re
   std::vector<std::vector<double>> om(n), wt(n);
   for (int i = 0; i < n; ++i) {
     Shape& sh = shapes[i];
+    // the fewest chunks, of one size but for the last; a chunk of fewer frequencies may need more
+    // memory (all of its operand planes at once), so both sizes are looked at
+    auto fits = [&](int nw) {
+      Shape s2 = sh;
+      s2.nomega = nw;
+      return Plan::measure({s2}, kPlanPartial) <= avail;
+    };
     int wc = 0;
     for (;;) {
       for (wc = sh.nomega; wc >= 1; --wc) {
-        Shape s2 = sh;
-        s2.nomega = wc;
-        if (Plan::measure({s2}, kPlanPartial) <= avail) break;
+        const int last = sh.nomega % wc;
+        if ((sh.nomega + wc - 1) / wc == (sh.nomega + wc - 2) / std::max(wc - 1, 1)) continue;   // as many of a smaller size
+        if (fits(wc) && (last == 0 || fits(last))) break;
       }
       if (wc >= 1 || !(use_digits(sh) || use_factor_digits(sh))) break;
       sh.no_digits = 1;   // one frequency with its digit buffers does not fit: DMMA needs none

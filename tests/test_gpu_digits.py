@@ -250,3 +250,19 @@ def test_without_room_for_the_digits(engine):
     small.close()
     assert abs(out.erpa - ref.erpa) <= 1e-10
     assert np.abs(out.sigma_calc - ref.sigma_calc).max() <= 1e-11 * np.abs(ref.sigma_calc).max()
+
+
+def test_every_budget_finds_chunks_that_fit():
+    """Chunks of fewer frequencies keep all their operand planes at once and can need more memory than
+    longer ones (digits 57 MB a frequency here, up to 18 of them at once or 8 in turn): no budget
+    above that of one frequency is refused."""
+    inst = molecule(30, 547, 390, 90, seed=9)
+    eng = Engine(0)
+    ref = eng.g0w0(inst, qp_only=True)
+    peak = eng.last_stats()["device_bytes_peak"]
+    eng.close()
+    for budget in range(240 << 20, peak, 10 << 20):
+        eng = Engine(0, hbm_budget_bytes=budget)
+        out = eng.g0w0(inst, qp_only=True)
+        eng.close()
+        assert np.abs(out.sigma_calc - ref.sigma_calc).max() <= 1e-11 * np.abs(ref.sigma_calc).max()
