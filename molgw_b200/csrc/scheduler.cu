@@ -42,6 +42,8 @@ size_t available_bytes(Context& c) {
 
 namespace {
 
+constexpr double kLeanFlops = 2e11;   // chi0 of a batch that rather does without digits than in waves
+
 Status get_plan(Context& c, PlanMode mode, const std::vector<Shape>& shapes, Plan** out) {
   auto key = std::make_pair(int(mode), shapes);
   auto it = c.plan_cache.find(key);
@@ -117,23 +119,39 @@ Status solve_batch(Context& c, int n, const rigw_problem* probs, rigw_result* re
     c.last_stats.waves = 1;
     return Status::ok();
   }
-  size_t avail = available_bytes(c);
-  // plans cached for other shapes count as free memory for this decision
-  size_t cached = 0;
-  for (auto& kv : c.plan_cache) cached += kv.second->bytes();
-  cached += c.reclaimable_bytes();
-  const size_t usable = avail + cached;
-
-  // ---- fits: one fused plan
-  const Tuning tune = c.tuning_for(kPlanFused, shapes);
-  if (Plan::measure(shapes, kPlanFused, &tune) <= usable) {
+  auto run_fused = [&](const std::vector<Shape>& sh) -> Status {
     Plan* plan = nullptr;
-    RIGW_TRY(get_plan(c, kPlanFused, shapes, &plan));
+    RIGW_TRY(get_plan(c, kPlanFused, sh, &plan));
     RIGW_TRY(run_plan(c, plan, probs, res, nullptr, true));
     c.last_stats.chunks = n;
     c.last_stats.waves = 1;
     return Status::ok();
+  };
+  // plans cached for other shapes count as free memory for this decision
+  size_t cached = 0;
+  for (auto& kv : c.plan_cache) cached += kv.second->bytes();
+  const Tuning tune = c.tuning_for(kPlanFused, shapes);
+  const size_t fused = Plan::measure(shapes, kPlanFused, &tune);
+  // Without the digit buffers a small batch may fit in one plan, which is kept from call to call;
+  // the plans of waves are built anew (ms per call with 32 frequencies, in waves with digits /
+  // without: naux 400 4.2 / 1.2, 640 5.3 / 2.7, 840 7.4 / 6.2, 1152 12.2 / 15.5, 1483 23 / 40).
+  std::vector<Shape> lean = shapes;
+  double flops = 0.0;
+  for (Shape& sh : lean) {
+    sh.no_digits = 1;
+    const double nia = double(sh.nocc) * sh.nvirt + double(sh.nocc2) * sh.nvirt2;
+    flops += double(sh.nomega) * sh.naux * (sh.naux + 1.0) * nia;
   }
+  // beyond the budget whatever gives way: its plan without digits is ready if it ran before
+  if (c.budget && fused > c.budget_left() + cached &&
+      c.plan_cache.count(std::make_pair(int(kPlanFused), lean)))
+    return run_fused(lean);
+  size_t avail = available_bytes(c);
+  const size_t usable = avail + cached + c.reclaimable_bytes();
+
+  // ---- fits: one fused plan
+  if (fused <= usable) return run_fused(shapes);
+  if (flops < kLeanFlops && Plan::measure(lean, kPlanFused, &tune) <= usable) return run_fused(lean);
 
   // ---- frequency chunks and waves
   c.plan_cache.clear();

@@ -252,6 +252,22 @@ def test_without_room_for_the_digits(engine):
     assert np.abs(out.sigma_calc - ref.sigma_calc).max() <= 1e-11 * np.abs(ref.sigma_calc).max()
 
 
+def test_a_small_batch_does_without_digits_before_it_is_cut():
+    """A budget that holds the batch in one plan without the digit buffers only: one plan, kept."""
+    inst = make_instance(9, 90, 400, 16, seed=12)
+    eng = Engine(0)
+    ref = eng.g0w0(inst)
+    peak = eng.last_stats()["device_bytes_peak"]
+    eng.close()
+    eng = Engine(0, hbm_budget_bytes=peak - (4 << 20))
+    for k in range(3):
+        out = eng.g0w0(inst)
+        st = eng.last_stats()
+        assert (st["waves"], st["graph_replayed"]) == (1, k > 0)
+        assert np.abs(out.sigma_calc - ref.sigma_calc).max() <= 1e-11 * np.abs(ref.sigma_calc).max()
+    eng.close()
+
+
 def test_every_budget_finds_chunks_that_fit():
     """Chunks of fewer frequencies keep all their operand planes at once and can need more memory than
     longer ones (digits 57 MB a frequency here, up to 18 of them at once or 8 in turn): no budget
