@@ -22,6 +22,7 @@ namespace {
 
 constexpr int kSoxThreads = 256;
 constexpr int kSoxW = 8;      // evaluation points per pass (register accumulators; 8 leaves room
+constexpr size_t kSoxL2Bytes = size_t(64) << 20;   // half of L2
                               // for two blocks per SM: 8 > 16 by 30%, > 4 by 25% on B200)
 constexpr int kSoxTile = 32;  // empty-state tile of the second sum
 constexpr int kSoxBlockB = kSoxThreads;   // empty states b per unit of the first sum
@@ -74,7 +75,7 @@ struct SoxArgs {
   double* partial;     // [pc][gridDim.x][nw][2]
 };
 
-// One block per (unit stripe, Sigma state of the chunk, kSoxW points).  Every thread keeps
+// One block per (unit stripe, Sigma state of the chunk, points kSoxW z, kSoxW (z + grid z) ..).  Every thread keeps
 // sum_e w_e (x / d) and sum_e w_e / d for kSoxW points (x = Re z - delta,
 // d = |z - delta|^2), so that sum_e w_e / (z - delta) = ar - i Im(z) as.  The
 // per-block sums go to `partial` in a fixed order (deterministic results).
@@ -85,8 +86,7 @@ __global__ void __launch_bounds__(kSoxThreads, 2) sox_contract_kernel(SoxArgs a)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const double* C = a.C + (long long)blockIdx.y * a.sp;
   const double* ev = a.e + a.no;
-  {
-    const int w0 = blockIdx.z * kSoxW;
+  for (int w0 = blockIdx.z * kSoxW; w0 < a.nw; w0 += gridDim.z * kSoxW) {
     const int nwc = min(kSoxW, a.nw - w0);
     double zr[kSoxW], zi2[kSoxW], ar[kSoxW], as[kSoxW];
 #pragma unroll
@@ -278,8 +278,14 @@ Status sox_selfenergy_imag(Context& c, const rigw_sox_problem& pr, double* sigma
   a.vt = (nv + kSoxTile - 1) / kSoxTile;
   a.tpairs = a.vt * (a.vt + 1) / 2;
   a.units = a.units1 + no * a.tpairs;
-  // the points go over grid z, so two blocks per SM and point group balance the unit stripes
-  const int nblk = std::max(1, std::min(a.units, sms * 2 / pc));
+  // The points go over grid z, and two blocks per SM and point group balance the unit stripes; but
+  // each group reads all of C, so a chunk that L2 does not hold beside the partial sums is walked
+  // once per block, with its points in turn, and four blocks per SM (50 / 100 points, over the grid
+  // against in turn, us: C of 16 MB 463 / 548 against 524 / 622, 46 MB 1666 / 1963 against 1746 /
+  // 2052, 92 MB 2685 / 3423 against 2615 / 3223, 180 MB 5266 / 6694 against 5282 / 6617).
+  const int wgroups = (nw + kSoxW - 1) / kSoxW;
+  const int zgrid = per_p * pc > kSoxL2Bytes ? 1 : wgroups;
+  const int nblk = std::max(1, std::min(a.units, sms * (zgrid < wgroups ? 4 : 2) / pc));
   RIGW_TRY(b_part.allocate(&c, size_t(pc) * nblk * nw * 16, "sox partial sums"));
   a.partial = reinterpret_cast<double*>(b_part.data());
   double* out = sigma_sox;
@@ -323,7 +329,7 @@ Status sox_selfenergy_imag(Context& c, const rigw_sox_problem& pr, double* sigma
     RIGW_CUDA_TRY(cudaGetLastError());
     RIGW_CUDA_TRY(cudaEventRecord(e[3], s));
     a.C = cbuf;
-    sox_contract_kernel<<<dim3(nblk, pcn, (nw + kSoxW - 1) / kSoxW), kSoxThreads, 0, s>>>(a);
+    sox_contract_kernel<<<dim3(nblk, pcn, zgrid), kSoxThreads, 0, s>>>(a);
     RIGW_CUDA_TRY(cudaGetLastError());
     const int nred = pcn * nw;
     sox_reduce_kernel<<<(nred + 3) / 4, 128, 0, s>>>(a.partial, nblk, nw, pcn, out + size_t(p0) * nw * 2);

@@ -34,6 +34,17 @@ def test_sox_matches_oracle(engine, shape):
     assert np.abs(out - ref).max() <= 1e-11 * np.abs(ref).max()
 
 
+@pytest.mark.parametrize("nw", [8, 9, 21])
+def test_sox_products_beyond_l2(engine, nw):
+    """(p q|j c) of 71 MB: the blocks take their evaluation points in turn."""
+    inst = synth.make_instance(42, 300, 12, 4, seed=13)
+    z = _points(inst)
+    out = engine.sox_selfenergy_imag_grid(inst, z[:nw])
+    ref = _oracle_sox(inst, z[:nw])
+    assert np.abs(out - ref).max() <= 1e-11 * np.abs(ref).max()
+    assert np.array_equal(out, engine.sox_selfenergy_imag_grid(inst, z[:nw]))
+
+
 def test_sox_is_repeatable(engine):
     inst = synth.make_instance(9, 80, 200, 16, seed=3)
     z = _points(inst)
