@@ -425,7 +425,9 @@ RIGW_API int rigw_g0w0_batch(rigw_ctx* ctx, int nprob, const rigw_problem* probs
  * row height of the FP64 chi0 and trailing-update tiles (64 or 128 rows x 128
  * columns), the number of frequency chains, the panels per trailing update and,
  * for split precision, the frequencies per split buffer (automatic, a group
- * whose buffers fit in L2, or 8).  The fastest shapes are kept in the context
+ * whose buffers fit in L2, or 8).  A field that the batch does not use (row heights and panel
+ * groups of the DMMA kernels, where digit products take their place) is not tried and stays as
+ * it is.  The fastest shapes are kept in the context
  * for every later batch of the same precision class (FP64, BF16x3, Ozaki,
  * mixed); results of a solve do not depend on them beyond floating-point
  * summation order. */

@@ -277,8 +277,13 @@ Status autotune(Context& c, int n, const rigw_problem* probs, rigw_tune_report* 
   c.reclaim();
   const size_t avail = available_bytes(c);
   const int cls = precision_class(shapes);
-  bool any_fp64 = false;
-  for (const Shape& sh : shapes) any_fp64 = any_fp64 || sh.precision == RIGW_FP64;
+  // A field that no problem of the batch uses is not tried: noise would choose, for every later
+  // batch of the class.
+  bool any_dmma = false, any_groups = false;   // chi0 on DMMA, panel groups on DMMA
+  for (const Shape& sh : shapes) {
+    any_dmma = any_dmma || operand_planes(sh) == 0;
+    any_groups = any_groups || !use_factor_digits(sh);
+  }
   Tuning best = c.tuning_for(kPlanFused, shapes);
   if (Plan::measure(shapes, kPlanFused, &best) > avail)
     return Status::fail(RIGW_ERR_NOMEM, "autotune: the batch does not fit the device in one plan");
@@ -315,7 +320,8 @@ Status autotune(Context& c, int n, const rigw_problem* probs, rigw_tune_report* 
   RIGW_TRY(run(best, bst));
   record(best, bst);
   rep->default_ms = bst[0] + bst[1] + bst[2] + bst[3];
-  // try one field at a time; keep a candidate when its stage is faster
+  // try one field at a time; keep a candidate when its stage is faster by more than repeated
+  // replays of one plan differ
   auto try_field = [&](int Tuning::*field, std::initializer_list<int> values, int stage) -> Status {
     const int cur = best.*field;
     for (int v : values) {
@@ -327,16 +333,17 @@ Status autotune(Context& c, int n, const rigw_problem* probs, rigw_tune_report* 
       if (s.code == RIGW_ERR_NOMEM) continue;
       RIGW_TRY(s);
       record(t, st);
-      if (st[stage] < bst[stage]) {
+      if (st[stage] < 0.98f * bst[stage]) {
         best = t;
         std::memcpy(bst, st, sizeof(bst));
       }
     }
     return Status::ok();
   };
-  if (any_fp64) RIGW_TRY(try_field(&Tuning::chi0_rows, {64, 128}, 1));
+  if (any_dmma) RIGW_TRY(try_field(&Tuning::chi0_rows, {64, 128}, 1));
   // split precision: frequencies per hi/lo buffer, including a group whose
-  // buffers stay resident in L2 between the split and the tensor-core launch
+  // buffers stay resident in L2 between the split and the tensor-core launch (the digits
+  // of FP64 keep the default group)
   bool any_split = false;
   size_t per_w = 0;
   for (const Shape& sh : shapes)
@@ -350,7 +357,7 @@ Status autotune(Context& c, int n, const rigw_problem* probs, rigw_tune_report* 
   }
   RIGW_TRY(try_field(&Tuning::update_rows, {64, 128}, 2));
   RIGW_TRY(try_field(&Tuning::chains, {1, 2, 4, 8}, 2));
-  RIGW_TRY(try_field(&Tuning::panel_group, {2, 8, 16}, 2));
+  if (any_groups) RIGW_TRY(try_field(&Tuning::panel_group, {2, 8, 16}, 2));
   c.tuned[{int(kPlanFused), cls}] = best;
   c.plan_cache.clear();
   c.idle.clear();

@@ -57,3 +57,21 @@ def test_tuning_applies_to_other_batches_of_the_class():
     assert rep["tuned_ms"] > 0
     assert abs(a.erpa - b.erpa) <= 1e-12 * abs(a.erpa)
     assert np.abs(a.energy_qp_g - b.energy_qp_g).max() * HA_EV <= 1e-8
+
+
+@pytest.mark.parametrize("naux,nomega,fields", [
+    (900, 16, set()),                          # digits in chi0 and in the factorization
+    (500, 8, {"panel_group"}),                 # digits in chi0 only
+    (200, 8, {"chi0_rows", "panel_group"}),    # DMMA
+])
+def test_fields_without_effect_are_not_tried(naux, nomega, fields):
+    """Row heights of the DMMA chi0 and panel groups of the DMMA factorization are candidates only
+    where the batch uses them, and stay at their defaults otherwise."""
+    eng = Engine(0)
+    rep = eng.autotune([synth.make_instance(8, 90, naux, nomega, 75)], RIGW_FP64)
+    eng.close()
+    for name in ("chi0_rows", "panel_group"):
+        tried = {c[name] for c in rep["candidates"]}
+        assert (len(tried) > 1) == (name in fields), (name, tried)
+        if name not in fields:
+            assert {rep[name]} == tried == {64 if name == "chi0_rows" else 2}
