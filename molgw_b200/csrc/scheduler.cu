@@ -277,6 +277,9 @@ Status autotune(Context& c, int n, const rigw_problem* probs, rigw_tune_report* 
   c.reclaim();
   const size_t avail = available_bytes(c);
   const int cls = precision_class(shapes);
+  Tuning best = c.tuning_for(kPlanFused, shapes);
+  if (Plan::measure(shapes, kPlanFused, &best) > avail)
+    for (Shape& sh : shapes) sh.no_digits = 1;   // as a batch without room for its digits runs
   // A field that no problem of the batch uses is not tried: noise would choose, for every later
   // batch of the class.
   bool any_dmma = false, any_groups = false;   // chi0 on DMMA, panel groups on DMMA
@@ -284,7 +287,6 @@ Status autotune(Context& c, int n, const rigw_problem* probs, rigw_tune_report* 
     any_dmma = any_dmma || operand_planes(sh) == 0;
     any_groups = any_groups || !use_factor_digits(sh);
   }
-  Tuning best = c.tuning_for(kPlanFused, shapes);
   if (Plan::measure(shapes, kPlanFused, &best) > avail)
     return Status::fail(RIGW_ERR_NOMEM, "autotune: the batch does not fit the device in one plan");
 

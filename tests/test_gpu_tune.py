@@ -75,3 +75,16 @@ def test_fields_without_effect_are_not_tried(naux, nomega, fields):
         assert (len(tried) > 1) == (name in fields), (name, tried)
         if name not in fields:
             assert {rep[name]} == tried == {64 if name == "chi0_rows" else 2}
+
+
+def test_autotune_without_room_for_the_digits():
+    """A budget that holds the batch in one plan without its digit buffers only: tuned on DMMA."""
+    insts = [synth.make_instance(9, 90, 400, 16, 76)]
+    probe = Engine(0)
+    probe.g0w0_batch(insts, RIGW_FP64)
+    peak = probe.last_stats()["device_bytes_peak"]
+    probe.close()
+    eng = Engine(0, hbm_budget_bytes=peak - (4 << 20))
+    rep = eng.autotune(insts, RIGW_FP64)
+    eng.close()
+    assert {c["chi0_rows"] for c in rep["candidates"]} == {64, 128}
