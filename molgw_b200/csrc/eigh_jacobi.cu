@@ -7,14 +7,16 @@
 // rotation formula, round-robin pairs of its 64 indices) runs on the 64 x 64
 // subproblem S = [A_II A_IJ; A_JI A_JJ] in shared memory and accumulates the
 // orthogonal Q.  (Solving S to convergence instead changes neither the number
-// of outer sweeps nor the result: on the test matrices both take 11 outer
-// sweeps at n = 512, the single inner sweep with a quarter of the inner work.)
+// of outer sweeps nor the result; the single inner sweep has a quarter of the
+// inner work.)
 // The entries inside A_II and A_JJ are rotated in the first round of a sweep
 // only, where every block is in one pair (63 inner rounds); the other rounds
 // rotate the 32 x 32 entries of A_IJ alone (32 inner rounds), so a sweep visits
-// every entry once instead of the inner ones nb - 1 times.  That takes one outer
-// sweep more (12 at n = 512) and half the inner work: 22 matrices of 512,
-// subproblems 21.2 -> 11 ms, the whole batch 32.3 -> 23 ms.
+// every entry once instead of the inner ones nb - 1 times.  That takes one or two
+// outer sweeps more (12 instead of 11 at n = 512; 19 instead of 15 for a matrix of
+// rank 240) of half the inner work each, and leaves smaller errors: 22 matrices of
+// 512, subproblems 21.2 -> 11 ms, the whole batch 32.3 -> 21 ms; with 240 transitions
+// contour deformation at 480 auxiliary functions 32.6 -> 25.4 ms.
 // The whole matrix is then updated with the round's rotation J (the pairs' Q
 // embedded at their rows and columns): every row and column belongs to exactly
 // one pair, so tile (p, q) of J^T A J is Q_p^T A[P, Q] Q_q and depends only on

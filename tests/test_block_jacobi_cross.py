@@ -1,7 +1,9 @@
 """The sweep of the device eigensolver in NumPy (molgw_b200/csrc/eigh_jacobi.cu): every entry
 inside a block is rotated in the first round of a sweep only, the other rounds rotate the
-entries between the two blocks of a pair.  It converges to LAPACK's eigenpairs in at most one
-sweep more than rotating everything in every round."""
+entries between the two blocks of a pair.  It converges to LAPACK's eigenpairs, no further from
+them than rotating everything in every round, in up to two sweeps more; matrices of low rank, which
+contour deformation meets when there are fewer transitions than auxiliary functions, take up to
+four more (15 to 19 at n = 512, rank 240), each of about half the work."""
 import numpy as np
 import pytest
 
@@ -53,14 +55,22 @@ def block_jacobi_cross(A, max_sweeps=60):
 
 @pytest.mark.parametrize("n", [64, 128, 256])
 @pytest.mark.parametrize("decades", [0.0, 4.0])
-def test_cross_sweeps_converge(n, decades):
+@pytest.mark.parametrize("rank", [3.0, 0.8, 0.24])
+def test_cross_sweeps_converge(n, decades, rank):
     rng = np.random.default_rng(n)
-    X = rng.standard_normal((n, 3 * n)) * 10.0 ** (-decades * rng.random((n, 1)))
-    A = -(X @ X.T) / (3 * n)
+    k = int(rank * n)
+    X = rng.standard_normal((n, k)) * 10.0 ** (-decades * rng.random((n, 1)))
+    A = -(X @ X.T) / k
     lam, V, sweeps = block_jacobi_cross(A)
     ref = np.linalg.eigvalsh(A)
     scale = np.abs(ref).max()
-    assert np.abs(np.sort(lam) - ref).max() < 2e-13 * scale
-    assert np.abs(V.T @ V - np.eye(n)).max() < 2e-13
+    # rounding of the rotations: about sweeps x n of them act on every entry, 2^-53 sqrt(2 n sweeps)
+    tol = 20 * 2.0 ** -53 * np.sqrt(2.0 * n * sweeps)
+    assert np.abs(np.sort(lam) - ref).max() < tol * scale
+    assert np.abs(V.T @ V - np.eye(n)).max() < tol
     assert np.abs(A @ V - V * lam).max() < 2e-12 * scale
-    assert sweeps <= block_jacobi(A)[2] + 2
+    lam_all, V_all, sweeps_all = block_jacobi(A)
+    assert sweeps <= sweeps_all + (2 if rank > 1.0 else 4)
+    for err, err_all in ((np.sort(lam) - ref, np.sort(lam_all) - ref),
+                         (V.T @ V - np.eye(n), V_all.T @ V_all - np.eye(n))):
+        assert np.linalg.norm(err) <= 1.2 * np.linalg.norm(err_all) + 1e-15
