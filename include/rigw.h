@@ -67,13 +67,19 @@ enum rigw_status {
   RIGW_ERR_CANCELLED = 8   /* request loop destroyed before the request ran               */
 };
 
-/* Arithmetic of the chi0 = M D M^T contraction (the eps factorization, Sigma and
- * the QP solve are FP64 in every mode). */
+/* Arithmetic of the chi0 = M D M^T contraction.  The eps factorization, Sigma and the QP solve
+ * have FP64 accuracy in every mode; above 768 auxiliary functions, where frequencies x panels of
+ * 128 squared reach 800 in a call, the factorization takes the digit products of RIGW_FP64 for the
+ * updates between groups of panels. */
 enum rigw_precision {
-  RIGW_FP64 = 0,           /* FP64 end to end (the drop-in): chi0 on the FP64 DMMA cores, or,
-                              from 384 auxiliary functions on, from exact int8 digit products
-                              of 55-bit operands whose error is no larger than that of the
-                              FP64 sums                                                  */
+  RIGW_FP64 = 0,           /* FP64 accuracy (the drop-in): chi0 on the FP64 DMMA cores, or, from
+                              384 auxiliary functions and 512 transitions on, from int8 digit
+                              products of M sqrt(D) rounded to 55 bits of the largest entry of
+                              each row.  Beside the FP64 rounding of M sqrt(D) itself (2^-52 of
+                              each product) that puts a random error of at most
+                              2^-55 sqrt(eps_pp eps_qq) into an element of eps; FP64 sums of K
+                              terms add about 2^-54 sqrt(K) of it to the rounding of M D.
+                              Negative factors (inverted occupations) always run on DMMA  */
   RIGW_BF16X3 = 1,         /* split BF16 hi/lo products on tcgen05, FP32 accumulation    */
   RIGW_OZAKI_INT8 = 16     /* + s (3 <= s <= 7): Ozaki-sliced INT8 products on tcgen05,
                               s signed slices per row (8 bits each for chi0, 7 for AO->MO),

@@ -12,14 +12,14 @@
 // NS = 7, |L_d| <= 7 * 128^2 * 16384 < 2^31.  The levels are joined in 64-bit integers,
 // converted to FP64 once per chunk and summed in FP64.
 //
-// Error, NS = 7 (55-bit X): the entries are rounded to 2^-56 of their row's maximum, which
-// puts a random error of 2^-56 max|S_p| |S_q| and its mirror image into the sum, at most
+// Error, NS = 7 (55-bit X), beside that of S in FP64 (2^-52 of each product): the entries are
+// rounded to 2^-56 of their row's maximum, which puts a random error of 2^-56 max|S_p| |S_q| and its mirror image into the sum, at most
 // 2^-55 sqrt(eps_pp eps_qq) whatever the spread of the entries and however long the sum,
 // because a row maximum never exceeds the row's norm.  The products left out (i + j > 9) are
 // digit products of zero mean with weight 2^-78 of the two row scales; K of them add up to
 // 2^-64 sqrt(K) max|S_p| max|S_q|, which is less.  (Without level 9 they are 256 times that and
 // the larger part: in rows that a few large entries dominate, 3 to 4 times the error of an
-// FP64 sum.)  An FP64 sum rounds its running sum K times, about 2^-54 sqrt(K).  Error against
+// FP64 sum.)  An FP64 sum rounds its running sum K times, about 2^-54 sqrt(K), beside M D_w.  Error against
 // extended precision over that of FP64 sums (rms, relative to sqrt(eps_pp eps_qq)): normal
 // entries 0.20 at 512 transitions, 0.05 at 4347; entries over three decades 0.23 and 0.05; three
 // large entries a row 0.27 and 0.17.  (M D_w and M in place of S on both sides would not be

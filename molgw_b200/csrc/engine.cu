@@ -310,12 +310,14 @@ Dims dims_of(const Shape& sh, PlanMode mode) {
 
 }  // namespace
 
-// The digit products need whole 256 x 128 tiles per pair of CTAs and three passes over the
-// operands before the product.  chi0 stage, DMMA against digits (12 / 32 frequencies, ms):
-// naux 200 0.051 / 0.064 against 0.066 / 0.096, 300 0.104 / 0.137 against 0.078 / 0.162,
-// 384 0.117 / 0.299 against 0.094 / 0.188, 512 0.262 / 0.664 against 0.127 / 0.317,
-// 840 (32) 4.25 against 1.41, 2000 (32) 112 against 33.  Below 512 transitions the passes
-// and the drains, which do not shrink with the sum, take over.
+// The digit products need whole 256 x 128 tiles per pair of CTAs and two passes over the operands
+// before the product, all of them once per frequency.  chi0 stage, DMMA against digits (ms): naux
+// 384 with 1 / 12 / 16 / 24 / 32 / 48 frequencies 0.114 / 0.119 / 0.160 / 0.160 / 0.301 / 0.309
+// against 0.078 / 0.108 / 0.123 / 0.200 / 0.217 / 0.311 (waves of tiles), 400 (32) 0.352 against
+// 0.286, 512 (1 / 32) 0.188 / 0.666 against 0.100 / 0.372, 840 (1 / 32) 0.53 / 4.25 against 0.22 /
+// 1.64, 2000 (32) 112 against 39.  Below 512 transitions the passes and the drains, which do not
+// shrink with the sum, take over: at 512 naux 400 (16 / 32) 0.131 / 0.213 against 0.153 / 0.225, 840
+// 0.37 / 0.66 against 0.26 / 0.44, 2000 1.62 / 3.12 against 0.86 / 1.64.
 bool use_digits(const Shape& sh) {
   return !sh.no_digits && sh.precision == RIGW_FP64 && sh.naux >= 384 &&
          (long long)sh.nocc * sh.nvirt + (long long)sh.nocc2 * sh.nvirt2 >= 512;

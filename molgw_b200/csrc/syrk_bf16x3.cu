@@ -60,7 +60,7 @@ __global__ void __launch_bounds__(256) split_bf16_kernel(const ProbDev* __restri
         const double x0 = v[k] * d[k], x1 = v[k + 1] * d[k + 1];
         const __nv_bfloat162 h = __floats2bfloat162_rn(float(x0), float(x1));
         hi[i] = *reinterpret_cast<const uint32_t*>(&h);
-        // the low part from the FP64 remainder, rounded once
+        // the low part from the FP64 remainder (through FP32, whose rounding is 2^-16 of its own)
         const __nv_bfloat162 l = __floats2bfloat162_rn(float(x0 - widen(hi[i] << 16)),
                                                        float(x1 - widen(hi[i] & 0xffff0000u)));
         lo[i] = *reinterpret_cast<const uint32_t*>(&l);

@@ -183,7 +183,7 @@ def sigma_reference(inst, omega, weight, z):
     de = (inst.energy[no:][None, :] - inst.energy[:no][:, None]).ravel()
     docc = (inst.occupation[:no][:, None] - inst.occupation[no:][None, :]).ravel()
     m = inst.m_ia.reshape(no * nv, -1)
-    out = np.zeros((2, z.size), complex)
+    out, erpa = np.zeros((2, z.size), complex), 0.0
     for w, wt in zip(omega, weight):
         eps = np.eye(inst.naux) + m.T @ (m * (2.0 * docc * de / (w * w + de * de))[:, None])
         for s in range(2):
@@ -191,7 +191,8 @@ def sigma_reference(inst, omega, weight, z):
                 np.sum(inst.m_sigma[s] ** 2, axis=1)
             x = z[:, None] - inst.energy[None, :]
             out[s] -= wt / (2 * np.pi) * ((1.0 / (x + 1j * w) + 1.0 / (x - 1j * w)) @ v)
-    return out
+        erpa += wt / (2 * np.pi) * (np.linalg.slogdet(eps)[1] + inst.naux - np.trace(eps))
+    return out, erpa
 
 
 @pytest.mark.parametrize("nocc,nvirt,naux,nomega", [
@@ -210,7 +211,9 @@ def sigma_reference(inst, omega, weight, z):
 def test_factorization_updates_by_digits(engine, nocc, nvirt, naux, nomega, qp_only):
     """The updates between panel groups on digit products: chi from the identity part and
     Sigma_c from the M columns.  |U^-T M|^2 - |M|^2 is a difference of sums of naux terms, each
-    rounded: 1e-13 of the largest Sigma covers naux u sqrt(naux) for these sizes."""
+    rounded: 1e-13 of the largest Sigma covers naux u sqrt(naux) for these sizes.  The integrand of
+    E_RPA is a difference of two sums of naux terms of about 1, on either side; a sum in blocks
+    rounds log2(naux) times, by up to u naux: 4 log2(naux) u naux sum |weight| / (2 pi)."""
     from molgw_b200.rigw import imag_grid
     inst = molecule(nocc, nvirt, naux, nomega, seed=naux)
     if not qp_only:
@@ -218,8 +221,9 @@ def test_factorization_updates_by_digits(engine, nocc, nvirt, naux, nomega, qp_o
     om, wt = imag_grid(nomega)
     out = engine.g0w0(inst, qp_only=qp_only)
     ef = 0.5 * (inst.energy[nocc - 1] + inst.energy[nocc])
-    ref = sigma_reference(inst, om, wt, ef + 1j * inst.step_sigma_calc * np.arange(inst.nomega_sigma_calc))
+    ref, erpa = sigma_reference(inst, om, wt, ef + 1j * inst.step_sigma_calc * np.arange(inst.nomega_sigma_calc))
     assert np.abs(out.sigma_calc - ref).max() <= 1e-13 * np.abs(ref).max()
+    assert abs(out.erpa - erpa) <= 4 * np.log2(naux) * 2.0 ** -53 * naux * np.abs(wt).sum() / (2 * np.pi)
 
 
 def test_a_batch_takes_up_the_digits_together(engine):
