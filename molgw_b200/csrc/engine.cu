@@ -330,14 +330,24 @@ bool use_digits(const Shape& sh) {
 // 2000 15.6 / 10.3; 8 frequencies 840 0.73 / 0.88, 1152 1.19 / 1.22, 1483 2.11 / 1.80; 4: 1483
 // 1.49 / 1.47, 2000 2.76 / 2.73; 2: 2000 1.96 / 2.08, 2600 3.33 / 3.15; 1: 840 0.58 / 0.75,
 // 2000 1.50 / 2.00, 3000 2.95 / 2.81, 4000 5.43 / 4.70; 8 molecules of 800 to 1220 with 4
-// frequencies each 2.30 / 2.04.  The line follows frequencies x panels^2, summed over the batch.
+// frequencies each 2.30 / 2.04.  The line follows frequencies x panels^2 of the problems on digits,
+// summed over the batch.  Where smaller problems do much of the work, the two kinds of launches of
+// a mixed batch wait for each other (32 frequencies, DMMA / digits: 760 + 768 + 776 2.62 / 2.79, 200 +
+// 400 + 600 + 840 1.99 / 2.16, 600 + 700 + 840 + 860 3.30 / 3.46, but 600 + 700 + 840 + 900 3.78 /
+// 3.69, ten from 200 to 1100 7.63 / 7.34): the digits take 70% of the work (panels^3) or none.
 void choose_factor_digits(std::vector<Shape>* shapes) {
-  long long work = 0;
+  long long area = 0;
+  double on_digits = 0.0, all = 0.0;
   for (const Shape& sh : *shapes) {
     const long long panels = (sh.naux + kPanel - 1) / kPanel;
-    work += sh.nomega * panels * panels;
+    const double volume = double(sh.nomega) * panels * panels * panels;
+    all += volume;
+    if (sh.naux <= 768) continue;
+    on_digits += volume;
+    area += sh.nomega * panels * panels;
   }
-  for (Shape& sh : *shapes) sh.factor_digits = sh.naux > 768 && work >= 800;
+  const bool worth = area >= 800 && on_digits >= 0.7 * all;
+  for (Shape& sh : *shapes) sh.factor_digits = worth && sh.naux > 768;
 }
 
 bool use_factor_digits(const Shape& sh) { return !sh.no_digits && sh.factor_digits; }

@@ -226,10 +226,14 @@ def test_factorization_updates_by_digits(engine, nocc, nvirt, naux, nomega, qp_o
     assert abs(out.erpa - erpa) <= 4 * np.log2(naux) * 2.0 ** -53 * naux * np.abs(wt).sum() / (2 * np.pi)
 
 
-def test_a_batch_takes_up_the_digits_together(engine):
-    """Two problems that factorize on DMMA alone and on digit products together, beside one that is
-    too small for them."""
-    insts = [make_instance(8, 90, n, 7, seed=n) for n in (900, 1000, 420)]
+@pytest.mark.parametrize("sizes,nomega", [
+    ((900, 1000, 420), 7),     # two that factorize on DMMA alone and on digit products together
+    ((780, 700, 500), 18),     # one that takes digits alone and leaves them beside the others
+])
+def test_a_batch_takes_up_the_digits_together(engine, sizes, nomega):
+    """The factorization of a batch takes digit products, beside problems too small for them, or none,
+    and gives what each problem gives alone."""
+    insts = [make_instance(8, 90, n, nomega, seed=n) for n in sizes]
     for one, both in zip([engine.g0w0(i) for i in insts], engine.g0w0_batch(insts)):
         assert abs(one.erpa - both.erpa) <= 1e-10 * abs(one.erpa)
         assert np.abs(one.sigma_calc - both.sigma_calc).max() <= 1e-12 * np.abs(one.sigma_calc).max()
