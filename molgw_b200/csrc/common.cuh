@@ -15,7 +15,7 @@ constexpr int kMaxChains = 8;                  // frequency chains of the factor
 constexpr int kAutoChains = 2;                 // chains without a tuning
 constexpr int kChainPairs = 4;                 // (problem, frequency) pairs per chain at least
 constexpr size_t kNarrowCtas = 148;            // factorization launches of at most this many tiles are cut into
-                                               // 32-column ones
+                                               // 32-column ones (a quarter of it with many problems)
 constexpr int kSplitGroup = 8;                 // frequencies sharing one bf16 hi/lo split buffer
 constexpr size_t kSplitWholeBytes = size_t(1) << 30;   // below this, one buffer for all frequencies
 constexpr size_t kSplitProblemBytes = size_t(4) << 30; // split buffer of one problem at most (>= one frequency)

@@ -976,12 +976,16 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
     for (auto& l : planes)
       std::stable_sort(l.begin(), l.end(), [](const DigitItem& a, const DigitItem& b) { return a.nkt > b.nkt; });
 
-  // Products of the factorization that would leave SMs idle are cut into 32-column tiles.
-  // Returns whether the list was cut (the launch argument).
+  // Products of the factorization that would leave SMs idle are cut into 32-column tiles.  With
+  // more than 36 (problem, frequency) pairs the other chains' launches fill the GPU, and only the
+  // smallest lists are cut (stage, lists of up to 148 / up to 37 tiles, ms: 8 molecules of 700, 32
+  // frequencies 5.55 / 5.40, 8 of 250 0.83 / 0.80, one of 500 with 48 frequencies 0.70 / 0.66; but
+  // 4 of 700 with 8 frequencies 0.87 / 0.90).  Returns whether the list was cut (the launch argument).
+  const size_t narrow_ctas = npairs > 36 ? kNarrowCtas / 4 : kNarrowCtas;
   auto narrow = [&](std::vector<GemmItem>& l) {
     size_t ctas = 0;
     for (const GemmItem& g : l) ctas += std::max(g.nw, 1);
-    if (l.empty() || ctas > kNarrowCtas) return 0;
+    if (l.empty() || ctas > narrow_ctas) return 0;
     std::vector<GemmItem> cut;
     for (const GemmItem& g : l)
       for (int c = 0; c < g.n; c += 32) {
@@ -995,6 +999,24 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
       }
     l.swap(cut);
     return 1;
+  };
+
+  // The next diagonal blocks, 128 x 128 items: 32-column tiles, or two 64-row ones (two CTAs of
+  // which share an SM: 8 molecules of 700 5.40 -> 5.33 ms).
+  auto narrow_diag = [&](std::vector<GemmItem>& l) {
+    if (narrow(l)) return 1;
+    std::vector<GemmItem> cut;
+    for (const GemmItem& g : l)
+      for (int r = 0; r < g.m; r += 64) {
+        GemmItem t = g;
+        t.A += r;
+        t.C += size_t(r) * g.ldc;
+        t.Cin += size_t(r) * g.ldc;
+        t.m = std::min(64, g.m - r);
+        cut.push_back(t);
+      }
+    l.swap(cut);
+    return 0;
   };
 
   // ---- upload the lists and the launch sequence
@@ -1070,7 +1092,7 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
       std::vector<GemmItem>& rest3 = gl_k3_[L(k)];
       if (next && ul_update_[L(k)].empty() && !gl_k2n_[L(k)].empty() && !gl_k3d_[L(k)].empty()) {
         const int ea = nev++, eb = nev++;
-        const int nn = narrow(gl_k2n_[L(k)]), nd = narrow(gl_k3d_[L(k)]), n2 = narrow(gl_k2_[L(k)]), n3 = narrow(rest3);
+        const int nn = narrow(gl_k2n_[L(k)]), nd = narrow_diag(gl_k3d_[L(k)]), n2 = narrow(gl_k2_[L(k)]), n3 = narrow(rest3);
         add(5, gl_k2n_[L(k)].data(), sizeof(GemmItem), gl_k2n_[L(k)].size(), nn, sm, pending, ea);
         pending = -1;
         add(14, gl_k3d_[L(k)].data(), sizeof(GemmItem), gl_k3d_[L(k)].size(), nd, sl, ea);
@@ -1082,7 +1104,7 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
       }
       // no next panel, nothing to update ahead of it, or a panel group on digit products ends
       // here (its digits need the whole panel solve): everything on the main stream
-      const int nn = narrow(gl_k2n_[L(k)]), nd = narrow(gl_k3d_[L(k)]), n2 = narrow(gl_k2_[L(k)]), n3 = narrow(rest3);
+      const int nn = narrow(gl_k2n_[L(k)]), nd = narrow_diag(gl_k3d_[L(k)]), n2 = narrow(gl_k2_[L(k)]), n3 = narrow(rest3);
       if (add(5, gl_k2n_[L(k)].data(), sizeof(GemmItem), gl_k2n_[L(k)].size(), nn, sm, pending)) pending = -1;
       if (add(5, gl_k2_[L(k)].data(), sizeof(GemmItem), gl_k2_[L(k)].size(), n2, sm, pending)) pending = -1;
       if (add(14, gl_k3d_[L(k)].data(), sizeof(GemmItem), gl_k3d_[L(k)].size(), nd, sm, pending)) pending = -1;
@@ -1156,9 +1178,9 @@ void Plan::record(cudaStream_t s0, int stage) {
         if (tune_.chi0_rows == 128) launch_dgemm_128x128(gl, L.count, L.ny, s);
         else launch_dgemm_64x128(gl, L.count, L.ny, s);
         break;
-      case 14:   // the next diagonal block: one 128 x 128 item per frequency set
+      case 14:   // the next diagonal blocks
         if (L.arg) launch_dgemm_128x32(gl, L.count, L.ny, s);
-        else launch_dgemm_128x128(gl, L.count, L.ny, s);
+        else launch_dgemm_64x128(gl, L.count, L.ny, s);
         break;
       case 6:
         if (L.arg && tune_.update_rows == 128) launch_dgemm_128x32(gl, L.count, L.ny, s);
