@@ -555,7 +555,7 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
         const size_t groups = size_t(sh.nomega + g - 1) / g;
         lists += (groups + 2) * (d.nia_pad / 64) * d.npanel * sizeof(WorkItem) +
                  (size_t(sh.nomega) * d.npad / 4096 + 1) * sizeof(WorkItem) +
-                 groups * (d.npanel / 2 + 1) * d.npanel * sizeof(DigitItem);
+                 groups * (d.npanel / 2 + 2) * d.npanel * sizeof(DigitItem);
       }
     }
     *measure_only = L.cur + LS.cur + lists + (size_t(1) << 20);
@@ -709,7 +709,7 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
           }
           for (int rb = 0; rb < p.npanel; ++rb)
             for (int kt = 0; kt < nkt; ++kt) slices[g].push_back({i, kt, rb, w0});
-          for (int ra = 0; ra < p.npanel; ra += 2)
+          for (int ra = 0; ra < p.npanel; ra += planes > 2 ? 2 : 1)
             for (int cb = ra; cb < p.npanel; ++cb) {
               DigitItem t{};
               t.maps = base + off[i].tmap;

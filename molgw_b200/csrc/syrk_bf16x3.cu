@@ -6,7 +6,7 @@
 // split_bf16_kernel: scales the packed FP64 tensor by sqrt(D_w(t)) for every frequency of a
 //   group and writes the hi/lo pair in the order in which the tensor cores read it
 //   (8 x 16-byte core matrices, as digit_gemm.cu).
-// split_syrk_kernel: one 256 x 128 upper tile of eps(iw) per pair of CTAs (cta_group::2).
+// split_syrk_kernel: one 128 x 128 upper tile of eps(iw) per CTA.
 // split_kmajor_kernel, syrk_bf16x3_kernel: the general products of the AO->MO transform,
 //   one 128 x 128 tile per CTA from K-major operands (128-byte swizzle).
 // All mbarrier waits are bounded.
@@ -111,37 +111,34 @@ __global__ void __launch_bounds__(256) split_kmajor_kernel(const SplitOp op) {
 // registers while the MMA warp fills the other, so the fp32 accumulation length is bounded
 // whatever the number of transitions.
 //
-// Tile 256 x 128 per CTA pair: what bounds the products is shared memory, 128 bytes per
-// clock.  A 128 x 128 tile of one CTA reads 128 bytes per clock of MMA time and TMA writes
-// 85 more (64 KB per 768 clocks), so it could not pass 60%; the pair reads 96 (each CTA its
-// A rows and half of B; the hi part of A is held in the collector for two products, which
-// saves a sixth of that) and writes 62.  What remains is the traffic between L2 and shared
-// memory, 31 bytes per clock and SM (50% of the tensor pipe); half-size slots, twice as many of
-// them and wider TMA rows change nothing.  chi0 stage, one CTA per tile before: 840 auxiliary
-// functions, 32 frequencies 0.539 -> 0.530 ms, 4000 / 48 317 -> 290 ms, 16 ragged molecules
-// 98.4 -> 94.6 ms.
-constexpr int kSpPlaneA = 128 * 128;                       // hi or lo of 128 A rows, 64 transitions
-constexpr int kSpPlaneB = 64 * 128;                        // of half a B tile
-constexpr int kSpSlot = 2 * (kSpPlaneA + kSpPlaneB);       // 48 KB
-constexpr int kSpSlots = 4;
+// One 128 x 128 tile per CTA.  What bounds the products is the traffic into shared memory: 64 KB
+// per k-tile of 64 transitions from L2, two boxes of both parts of an operand each, in the order in
+// which the tensor cores read them.  A 256 x 128 tile per CTA pair (cta_group::2) loads a quarter
+// less, but computes rows beyond the last block and blocks below the diagonal, and its two CTAs
+// wait for each other; the row-major form with four 128-byte-swizzled boxes per k-tile needs more
+// instructions and transactions.  chi0 stage, row-major / pairs / this (ms): 64 molecules of 128
+// auxiliary functions 0.301 / 0.381 / 0.242, 32 of 300 1.11 / 1.28 / 0.97, 8 of 700 2.36 / 2.41 /
+// 2.08; one of 768 0.348 / 0.387 / 0.321, 840 0.502 / 0.490 / 0.452, 1700 5.39 / 5.73 / 4.98, 2000
+// 9.74 / 9.14 / 8.97, 4000 (48 frequencies) 249 / 246 / 239.
+constexpr int kSpPlane = 128 * 128;                        // hi or lo of 128 rows, 64 transitions
+constexpr int kSpSlot = 4 * kSpPlane;                      // 64 KB
+constexpr int kSpSlots = 3;
 constexpr int kSpChunk = 8;                                // k-tiles per fp32 accumulation
 constexpr int kSpThreads = 320;                            // warp 0 TMA, warp 1 MMA, warps 2..9 drain
 constexpr size_t kSpSmem = size_t(kSpSlots) * kSpSlot + 1024 + 256;
 
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kSpThreads, 1)
-    split_syrk_kernel(const DigitItem* __restrict__ items) {
-  const DigitItem it = items[blockIdx.x >> 1];
+__global__ void __launch_bounds__(kSpThreads, 1) split_syrk_kernel(const DigitItem* __restrict__ items) {
+  const DigitItem it = items[blockIdx.x];
   const int jw = blockIdx.y;
-  if (jw >= it.nw) return;   // both CTAs of the pair, before any barrier or TMEM use
+  if (jw >= it.nw) return;   // before any barrier or TMEM use
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + kSpSlots * kSpSlot);   // used in rank 0
-  uint64_t* empty = full + kSpSlots;        // slot read by the MMAs (both ranks)
-  uint64_t* accf = empty + kSpSlots;        // [2] chunk accumulated (both ranks)
-  uint64_t* acce = accf + 2;                // [2] chunk drained by the 16 warps of the pair (rank 0)
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + kSpSlots * kSpSlot);
+  uint64_t* empty = full + kSpSlots;        // slot read by the MMAs
+  uint64_t* accf = empty + kSpSlots;        // [2] chunk accumulated
+  uint64_t* acce = accf + 2;                // [2] chunk drained by the 8 warps
   uint32_t* tslot = reinterpret_cast<uint32_t*>(acce + 2);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int rank = int(tc::cluster_rank());
   if (tid == 0) {
     for (int s = 0; s < kSpSlots; ++s) {
       tc::mbar_init(&full[s], 1);
@@ -149,24 +146,21 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kSpThreads, 1)
     }
     for (int b = 0; b < 2; ++b) {
       tc::mbar_init(&accf[b], 1);
-      tc::mbar_init(&acce[b], 16);
+      tc::mbar_init(&acce[b], 8);
     }
     tc::fence_mbar_init();
   }
-  if (warp == 0) tc::tmem_alloc_pair(tslot, 256);
+  if (warp == 0) tc::tmem_alloc(tslot, 256);
   __syncthreads();
-  tc::cluster_sync();        // the peer's barriers are initialised
   tc::tc_fence_after();
   const uint32_t tmem = *tslot;
   const int nk = it.nkt;
   const int nchunks = (nk + kSpChunk - 1) / kSpChunk;
 
   if (tid == 0) {
-    // ---- TMA producer of this CTA; rank 0's full barrier counts the bytes of both
-    const uint8_t* maps = static_cast<const uint8_t*>(it.maps);
-    tc::tmap_acquire(maps);
-    tc::tmap_acquire(maps + 128);
-    const int rowA = (jw * it.nrb + it.rb_a + rank) * nk;
+    // ---- TMA producer
+    tc::tmap_acquire(it.maps);
+    const int rowA = (jw * it.nrb + it.rb_a) * nk;
     const int rowB = (jw * it.nrb + it.rb_b) * nk;
     int issued = 0;
     bool ok = true;
@@ -176,25 +170,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kSpThreads, 1)
         ok = false;
         break;
       }
-      if (rank == 0) tc::mbar_arrive_expect_tx(&full[s], 2 * kSpSlot);
-      const uint32_t bar = tc::mapa(&full[s], 0);
+      tc::mbar_arrive_expect_tx(&full[s], kSpSlot);
       uint8_t* d = smem + s * kSpSlot;
-      tc::tma_load_3d_pair(d, maps, bar, 0, 0, (rowA + kt) * 2);
-      tc::tma_load_3d_pair(d + 2 * kSpPlaneA, maps + 128, bar, 0, 64 * rank, (rowB + kt) * 2);
+      tc::tma_load_3d(d, it.maps, &full[s], 0, 0, (rowA + kt) * 2);
+      tc::tma_load_3d(d + 2 * kSpPlane, it.maps, &full[s], 0, 0, (rowB + kt) * 2);
     }
     if (!ok) atomicOr(it.err, kErrTimeout);
     // copies still in flight on a timeout land before the CTA leaves (bounded wait)
-    if (rank == 0) {
-      for (int s = 0; s < kSpSlots && s < issued; ++s)
-        if (!tc::mbar_wait(&full[s], (((issued - 1 - s) / kSpSlots)) & 1)) atomicOr(it.err, kErrTimeout);
-    } else if (!ok) {
-      const uint64_t t0 = tc::global_ns();
-      while (tc::global_ns() - t0 < 1000000ull) {
-      }
-    }
-  } else if (tid == 32 && rank == 0) {
-    // ---- MMA issuer of the pair
-    constexpr uint32_t idesc = tc::idesc_bf16_f32(256, 128);
+    for (int s = 0; s < kSpSlots && s < issued; ++s)
+      if (!tc::mbar_wait(&full[s], (((issued - 1 - s) / kSpSlots)) & 1)) atomicOr(it.err, kErrTimeout);
+  } else if (tid == 32) {
+    // ---- MMA issuer
+    constexpr uint32_t idesc = tc::idesc_bf16_f32(128, 128);
     bool ok = true;
     for (int kt = 0; kt < nk && ok; ++kt) {
       const int c = kt / kSpChunk, b = c & 1;
@@ -211,18 +198,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kSpThreads, 1)
       tc::tc_fence_after();
       const uint32_t d = tmem + uint32_t(b * 128);
       const uint8_t* base = smem + s * kSpSlot;
-      const uint64_t ah = tc::desc_kmajor_cores(base, 1024), al = tc::desc_kmajor_cores(base + kSpPlaneA, 1024);
-      const uint64_t bh = tc::desc_kmajor_cores(base + 2 * kSpPlaneA, 1024);
-      const uint64_t bl = tc::desc_kmajor_cores(base + 2 * kSpPlaneA + kSpPlaneB, 1024);
+      const uint64_t ah = tc::desc_kmajor_cores(base, 1024), al = tc::desc_kmajor_cores(base + kSpPlane, 1024);
+      const uint64_t bh = tc::desc_kmajor_cores(base + 2 * kSpPlane, 1024);
+      const uint64_t bl = tc::desc_kmajor_cores(base + 3 * kSpPlane, 1024);
 #pragma unroll
       for (int sub = 0; sub < 4; ++sub) {
         const uint64_t o = uint64_t(sub * 16);   // 16 bf16 along K = two core matrices = 256 bytes
-        tc::mma_bf16_pair<1>(d, ah + o, bh + o, idesc, (first && sub == 0) ? 0u : 1u);
-        tc::mma_bf16_pair<2>(d, ah + o, bl + o, idesc, 1u);
-        tc::mma_bf16_pair<0>(d, al + o, bh + o, idesc, 1u);
+        tc::mma_bf16(d, ah + o, bh + o, idesc, (first && sub == 0) ? 0u : 1u);
+        tc::mma_bf16(d, ah + o, bl + o, idesc, 1u);
+        tc::mma_bf16(d, al + o, bh + o, idesc, 1u);
       }
-      tc::mma_commit_pair(&empty[s]);
-      if ((kt % kSpChunk) == kSpChunk - 1 || kt == nk - 1) tc::mma_commit_pair(&accf[b]);
+      tc::mma_commit(&empty[s]);
+      if ((kt % kSpChunk) == kSpChunk - 1 || kt == nk - 1) tc::mma_commit(&accf[b]);
     }
     if (!ok) atomicOr(it.err, kErrTimeout);
   } else if (warp >= 2) {
@@ -249,12 +236,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kSpThreads, 1)
       }
       tc::tc_fence_before();
       __syncwarp();
-      if (lane == 0) tc::mbar_arrive_cluster(tc::mapa(&acce[b], 0));
+      if (lane == 0) tc::mbar_arrive(&acce[b]);
     }
-    const int rb = it.rb_a + rank, cb = it.rb_b;
+    const int rb = it.rb_a, cb = it.rb_b;
     if (!ok) {
       if (lane == 0) atomicOr(it.err, kErrTimeout);
-    } else if (rb < it.nrb && rb <= cb) {      // blocks below the diagonal are not stored
+    } else {
       const int row = rb * 128 + quad * 32 + lane, col0 = cb * 128 + half * 64;
       double* dst = it.C + jw * it.sC + size_t(row) * it.ld + col0;
 #pragma unroll
@@ -268,10 +255,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kSpThreads, 1)
   }
   tc::tc_fence_before();
   __syncthreads();
-  tc::cluster_sync();        // no CTA leaves while its peer may still reach its memory
   if (warp == 0) {
     __syncwarp();
-    tc::tmem_dealloc_pair(tmem, 256);
+    tc::tmem_dealloc(tmem, 256);
   }
 }
 
@@ -453,7 +439,7 @@ void launch_split_bf16(const ProbDev* probs, const WorkItem* items, int n, cudaS
 }
 
 void launch_split_syrk(const DigitItem* items, int n, int ny, cudaStream_t s) {
-  if (n > 0 && ny > 0) split_syrk_kernel<<<dim3(2 * n, ny), kSpThreads, kSpSmem, s>>>(items);
+  if (n > 0 && ny > 0) split_syrk_kernel<<<dim3(n, ny), kSpThreads, kSpSmem, s>>>(items);
 }
 
 void launch_split_kmajor(const SplitOp& op, cudaStream_t s) {
