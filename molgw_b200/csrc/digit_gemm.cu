@@ -45,7 +45,8 @@
 //   cores read them: [slab][row block of 128][k-tile of 64][digit][row group of 8][16-byte
 //   k chunk][row][16 bytes], i.e. contiguous 8 x 16-byte core matrices, so that one TMA box
 //   fetches all the digits of a tile.  One slab per frequency of the group.
-// digit_syrk_kernel:   one 256 x 128 tile of eps(iw) per pair of CTAs (cta_group::2).
+// digit_syrk_kernel:   one 256 x 128 tile of eps(iw) per pair of CTAs (cta_group::2), or, for
+//   small problems of up to six digits, one 128 x 128 tile per CTA.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
@@ -61,10 +62,10 @@ namespace {
 constexpr int kNaNExp = 1 << 20;                 // row exponent of a row with a non-finite entry
 constexpr int kDigThreads = 320;                 // warp 0 TMA, warp 1 MMA, warps 2..9 drain
 constexpr int kChunkTiles = 256;                 // k-tiles (of 64) per exact INT32 accumulation
-constexpr int kTileA = 128 * 64;                 // bytes of one digit of an A tile (128 rows)
-constexpr int kTileB = 64 * 64;                  // bytes of one digit of half a B tile (64 rows)
+constexpr int kTileA = 128 * 64;                 // bytes of one digit of 128 rows
 
-template <int NS>
+// CT: CTAs of a tile, a pair (256 x 128) or one (128 x 128; NS <= 6, whose slots leave room for two).
+template <int NS, int CT = 2>
 struct DigCfg {
   // last level summed: seven digits stand for FP64 and take one more than the NS + 1 whose weight
   // is that of the rounding of the entries
@@ -73,6 +74,8 @@ struct DigCfg {
   static constexpr int kHi = kTop - 1 - kLo;     // levels of the high pass: 2 .. kHi + 1 (digits 1 .. kHi)
   // the digit whose squares are added to the diagonal (0: none)
   static constexpr int kSquare = kTop % 2 ? (kTop + 1) / 2 : 0;
+  static constexpr int kCtas = CT;
+  static constexpr int kTileB = kTileA / kCtas;  // bytes of one digit of this CTA's rows of a B tile
   static constexpr int kSlot = NS * (kTileA + kTileB);
   static constexpr int kSlots = (216 * 1024) / kSlot;
   static constexpr int kPerHi = kHi > 0 ? NS / kHi : 1;   // k-tiles of the high pass per slot
@@ -258,9 +261,11 @@ __global__ void __launch_bounds__(256) digit_slice_kernel(const ProbDev* __restr
 // would read 128 and write 45).  TMEM holds four 128-column accumulators, so the levels go
 // in two passes over a chunk: the four lowest levels (24 of the 34 products for NS = 7), and
 // the rest from the leading digits alone, as many k-tiles per slot as fit.
-template <int NS, class Item>
+template <int NS, int CT, class Item>
 __device__ __forceinline__ void digit_product(const Item& it, const int jw) {
-  using Cfg = DigCfg<NS>;
+  using Cfg = DigCfg<NS, CT>;
+  constexpr int kTileB = Cfg::kTileB;
+  constexpr bool kPair = Cfg::kCtas == 2;
   constexpr bool kUpdate = std::is_same<Item, UpdateItem>::value;
   extern __shared__ uint8_t dig_smem_raw[];
   uint8_t* smem =
@@ -271,19 +276,22 @@ __device__ __forceinline__ void digit_product(const Item& it, const int jw) {
   uint64_t* acce = accf + 1;                // pass drained by the 16 warps of the pair (rank 0)
   uint32_t* tslot = reinterpret_cast<uint32_t*>(acce + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int rank = int(tc::cluster_rank());
+  const int rank = kPair ? int(tc::cluster_rank()) : 0;
   if (tid == 0) {
     for (int s = 0; s < Cfg::kSlots; ++s) {
       tc::mbar_init(&full[s], 1);
       tc::mbar_init(&empty[s], 1);
     }
     tc::mbar_init(accf, 1);
-    tc::mbar_init(acce, 16);
+    tc::mbar_init(acce, 8 * Cfg::kCtas);
     tc::fence_mbar_init();
   }
-  if (warp == 0) tc::tmem_alloc_pair(tslot, 512);
+  if (warp == 0) {
+    if constexpr (kPair) tc::tmem_alloc_pair(tslot, 512);
+    else tc::tmem_alloc(tslot, 512);
+  }
   __syncthreads();
-  tc::cluster_sync();        // the peer's barriers are initialised
+  if constexpr (kPair) tc::cluster_sync();        // the peer's barriers are initialised
   tc::tc_fence_after();
   const uint32_t tmem = *tslot;
   int nk, chunk, slab;                // k-tiles summed, k-tiles per chunk, slab of both operands
@@ -324,12 +332,17 @@ __device__ __forceinline__ void digit_product(const Item& it, const int jw) {
             break;
           }
           const int nt = min(ps, k1 - k0);
-          if (rank == 0) tc::mbar_arrive_expect_tx(&full[s], uint32_t(2 * nt * nd * (kTileA + kTileB)));
-          const uint32_t bar = tc::mapa(&full[s], 0);
+          if (rank == 0) tc::mbar_arrive_expect_tx(&full[s], uint32_t(Cfg::kCtas * nt * nd * (kTileA + kTileB)));
+          const uint32_t bar = kPair ? tc::mapa(&full[s], 0) : 0;
           for (int t = 0; t < nt; ++t) {
             uint8_t* d = slot(s) + t * nd * (kTileA + kTileB);
-            tc::tma_load_3d_pair(d, maps + 256 * q, bar, 0, 0, (rowA + k0 + t) * NS);
-            tc::tma_load_3d_pair(d + nd * kTileA, maps + 256 * q + 128, bar, 0, 32 * rank, (rowB + k0 + t) * NS);
+            if constexpr (kPair) {
+              tc::tma_load_3d_pair(d, maps + 256 * q, bar, 0, 0, (rowA + k0 + t) * NS);
+              tc::tma_load_3d_pair(d + nd * kTileA, maps + 256 * q + 128, bar, 0, 32 * rank, (rowB + k0 + t) * NS);
+            } else {
+              tc::tma_load_3d(d, maps + 256 * q, &full[s], 0, 0, (rowA + k0 + t) * NS);
+              tc::tma_load_3d(d + nd * kTileA, maps + 256 * q, &full[s], 0, 0, (rowB + k0 + t) * NS);
+            }
           }
         }
       }
@@ -347,7 +360,7 @@ __device__ __forceinline__ void digit_product(const Item& it, const int jw) {
     }
   } else if (tid == 32 && rank == 0) {
     // ---- MMA issuer of the pair
-    constexpr uint32_t idesc = tc::idesc_s8_s32(256, 128);
+    constexpr uint32_t idesc = tc::idesc_s8_s32(128 * Cfg::kCtas, 128);
     bool ok = true;
     uint32_t step = 0;
     int pass = 0;
@@ -392,25 +405,31 @@ __device__ __forceinline__ void digit_product(const Item& it, const int jw) {
 #pragma unroll
                 for (int sub = 0; sub < 2; ++sub) {
                   // 32 int8 along K = two core matrices = 256 bytes
-                  tc::mma_s8_pair(dt, ad + uint64_t(((i - 1) * kTileA + sub * 256) >> 4),
-                                  bd + uint64_t(((j - 1) * kTileB + sub * 256) >> 4), idesc,
-                                  (fresh && sub == 0) ? first : 1u);
+                  const uint64_t ai = ad + uint64_t(((i - 1) * kTileA + sub * 256) >> 4);
+                  const uint64_t bj = bd + uint64_t(((j - 1) * kTileB + sub * 256) >> 4);
+                  const uint32_t keep = (fresh && sub == 0) ? first : 1u;
+                  if constexpr (kPair) tc::mma_s8_pair(dt, ai, bj, idesc, keep);
+                  else tc::mma_s8(dt, ai, bj, idesc, keep);
                 }
                 fresh = false;
               }
             }
             first = 1u;
           }
-          tc::mma_commit_pair(&empty[s]);
+          if constexpr (kPair) tc::mma_commit_pair(&empty[s]);
+          else tc::mma_commit(&empty[s]);
         }
-        if (ok) tc::mma_commit_pair(accf);
+        if (ok) {
+          if constexpr (kPair) tc::mma_commit_pair(accf);
+          else tc::mma_commit(accf);
+        }
       }
     if (!ok) atomicOr(it.err, kErrTimeout);
   } else if (warp >= 2) {
     // ---- drain: join the levels of a pass in 64-bit integers, add to FP64 registers
     const int quad = warp & 3;                 // TMEM lanes 32 quad .. (rows)
     const int half = (warp - 2) >> 2;          // columns 64 half ..
-    const uint32_t done = tc::mapa(acce, 0);
+    const uint32_t done = kPair ? tc::mapa(acce, 0) : 0;
     // weight of the lowest level of unit-scaled operands
     constexpr int kShift = 8 * (2 * NS - Cfg::kTop) - 2 * (8 * NS - 1);
     double acc[64];
@@ -457,7 +476,10 @@ __device__ __forceinline__ void digit_product(const Item& it, const int jw) {
         }
         tc::tc_fence_before();
         __syncwarp();
-        if (lane == 0) tc::mbar_arrive_cluster(done);
+        if (lane == 0) {
+          if constexpr (kPair) tc::mbar_arrive_cluster(done);
+          else tc::mbar_arrive(acce);
+        }
       }
     if (!ok) {
       if (lane == 0) atomicOr(it.err, kErrTimeout);
@@ -502,20 +524,22 @@ __device__ __forceinline__ void digit_product(const Item& it, const int jw) {
   }
   tc::tc_fence_before();
   __syncthreads();
-  tc::cluster_sync();        // no CTA leaves while its peer may still reach its memory
+  if constexpr (kPair) tc::cluster_sync();        // no CTA leaves while its peer may still reach its memory
   if (warp == 0) {
     __syncwarp();
-    tc::tmem_dealloc_pair(tmem, 512);
+    if constexpr (kPair) tc::tmem_dealloc_pair(tmem, 512);
+    else tc::tmem_dealloc(tmem, 512);
   }
 }
 
-template <int NS>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kDigThreads, 1)
+// Grid x: the items times CT, in clusters of that size.
+template <int NS, int CT>
+__global__ void __cluster_dims__(CT, 1, 1) __launch_bounds__(kDigThreads, 1)
     digit_syrk_kernel(const DigitItem* __restrict__ items) {
-  const DigitItem it = items[blockIdx.x >> 1];
+  const DigitItem it = items[blockIdx.x / CT];
   // both CTAs of the pair, before any barrier or TMEM use
   if (int(blockIdx.y) >= it.nw || (it.negative && *it.negative)) return;
-  digit_product<NS>(it, blockIdx.y);
+  digit_product<NS, CT>(it, blockIdx.y);
 }
 
 // C -= A^T B for the rows of one panel group, A and B columns of the finished rows above it
@@ -529,7 +553,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kDigThreads, 1)
     digit_update_kernel(const UpdateItem* __restrict__ items) {
   const UpdateItem it = items[blockIdx.x >> 1];
   if (int(blockIdx.y) >= it.nw) return;
-  digit_product<kFp64Digits>(it, blockIdx.y);
+  digit_product<kFp64Digits, 2>(it, blockIdx.y);
 }
 
 // One block of 128 columns of a group of finished rows: column maxima, then the digits, both
@@ -572,14 +596,14 @@ __global__ void __launch_bounds__(256) factor_slice_kernel(const FactorSliceItem
 namespace {
 PFN_cuTensorMapEncodeTiled_v12000 g_encode_dig = nullptr;
 
-template <int NS>
+template <int NS, int CT>
 cudaError_t prepare_ns() {
-  return cudaFuncSetAttribute(digit_syrk_kernel<NS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              int(DigCfg<NS>::kSmem));
+  return cudaFuncSetAttribute(digit_syrk_kernel<NS, CT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              int(DigCfg<NS, CT>::kSmem));
 }
-template <int NS>
+template <int NS, int CT>
 void syrk_ns(const DigitItem* items, int n, int ny, cudaStream_t s) {
-  digit_syrk_kernel<NS><<<dim3(2 * n, ny), kDigThreads, DigCfg<NS>::kSmem, s>>>(items);
+  digit_syrk_kernel<NS, CT><<<dim3(CT * n, ny), kDigThreads, DigCfg<NS, CT>::kSmem, s>>>(items);
 }
 }  // namespace
 
@@ -635,18 +659,25 @@ void launch_digit_update(const UpdateItem* items, int n, int ny, cudaStream_t s)
   if (n > 0 && ny > 0)
     digit_update_kernel<<<dim3(2 * n, ny), kDigThreads, DigCfg<kFp64Digits>::kSmem, s>>>(items);
 }
-void launch_digit_syrk(int planes, const DigitItem* items, int n, int ny, cudaStream_t s) {
+// ctas: of a tile (see DigCfg); 1 for planes <= 6 only
+void launch_digit_syrk(int planes, int ctas, const DigitItem* items, int n, int ny, cudaStream_t s) {
   if (n <= 0 || ny <= 0) return;
-  switch (planes) {
-    case 3: syrk_ns<3>(items, n, ny, s); break;
-    case 4: syrk_ns<4>(items, n, ny, s); break;
-    case 5: syrk_ns<5>(items, n, ny, s); break;
-    case 6: syrk_ns<6>(items, n, ny, s); break;
-    default: syrk_ns<7>(items, n, ny, s); break;
+  switch (planes * 10 + ctas) {
+    case 31: syrk_ns<3, 1>(items, n, ny, s); break;
+    case 32: syrk_ns<3, 2>(items, n, ny, s); break;
+    case 41: syrk_ns<4, 1>(items, n, ny, s); break;
+    case 42: syrk_ns<4, 2>(items, n, ny, s); break;
+    case 51: syrk_ns<5, 1>(items, n, ny, s); break;
+    case 52: syrk_ns<5, 2>(items, n, ny, s); break;
+    case 61: syrk_ns<6, 1>(items, n, ny, s); break;
+    case 62: syrk_ns<6, 2>(items, n, ny, s); break;
+    default: syrk_ns<7, 2>(items, n, ny, s); break;
   }
 }
 cudaError_t prepare_digit_kernels() {
-  for (cudaError_t e : {prepare_ns<3>(), prepare_ns<4>(), prepare_ns<5>(), prepare_ns<6>(), prepare_ns<7>()})
+  for (cudaError_t e : {prepare_ns<3, 1>(), prepare_ns<3, 2>(), prepare_ns<4, 1>(), prepare_ns<4, 2>(),
+                        prepare_ns<5, 1>(), prepare_ns<5, 2>(), prepare_ns<6, 1>(), prepare_ns<6, 2>(),
+                        prepare_ns<7, 2>()})
     if (e != cudaSuccess) return e;
   return cudaFuncSetAttribute(digit_update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               int(DigCfg<kFp64Digits>::kSmem));

@@ -365,6 +365,15 @@ int operand_planes(const Shape& sh) {
   return use_digits(sh) ? kFp64Digits : 0;
 }
 
+// CTAs of a chi0 tile: one for bf16 (syrk_bf16x3.cu), a pair for the seven digits of FP64, whose
+// slot takes half of a CTA's shared memory in a pair and all of it alone.  Pairs compute rows
+// beyond the last block and blocks below the diagonal (2, 4, 8, 24, 40 blocks for 1, 3, 6, 21, 36), so up
+// to eight row blocks of three to six digits go one by one; beyond, pairs read less.  chi0 stage,
+// pairs / single (ms), four and six digits: 64 molecules of 128 auxiliary functions 0.641 / 0.348 and
+// 0.809 / 0.414, 32 of 300 1.76 / 1.32 and 2.46 / 1.88, one of 840 0.643 / 0.630 and 1.075 / 1.073, 1000
+// 1.01 / 0.94 and 2.26 / 1.71, 1483 4.11 / 4.20 and 7.84 / 8.10, 2000 11.5 / 11.8 and 22.8 / 23.9.
+int tile_ctas(int planes, int npanel) { return planes == 2 || (planes < 7 && npanel <= 8) ? 1 : 2; }
+
 // Bytes of one frequency's split operands (bf16 hi/lo, or the digits).
 size_t split_bytes_per_frequency(const Shape& sh) {
   const int planes = operand_planes(sh);
@@ -701,15 +710,14 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
             for (int rb = 0; rb < p.npanel; ++rb) wl_dmax_.push_back({i, t0, rb, 0});
         }
         auto& slices = wl_slice_[planes];
-        auto& products = dl_syrk_[planes];
+        const int ctas = tile_ctas(planes, p.npanel);
+        auto& products = dl_syrk_[ctas - 1][planes];
         for (int w0 = 0, g = 0; w0 < sh.nomega; w0 += p.wgroup, ++g) {
-          if (int(slices.size()) <= g) {
-            slices.resize(g + 1);
-            products.resize(g + 1);
-          }
+          if (int(slices.size()) <= g) slices.resize(g + 1);
+          if (int(products.size()) <= g) products.resize(g + 1);
           for (int rb = 0; rb < p.npanel; ++rb)
             for (int kt = 0; kt < nkt; ++kt) slices[g].push_back({i, kt, rb, w0});
-          for (int ra = 0; ra < p.npanel; ra += planes > 2 ? 2 : 1)
+          for (int ra = 0; ra < p.npanel; ra += ctas)
             for (int cb = ra; cb < p.npanel; ++cb) {
               DigitItem t{};
               t.maps = base + off[i].tmap;
@@ -972,9 +980,10 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
   std::stable_sort(gl_syrk_.begin(), gl_syrk_.end(), [](const GemmItem& a, const GemmItem& b) {
     return double(a.k) * a.m * a.n * std::max(a.nw, 1) > double(b.k) * b.m * b.n * std::max(b.nw, 1);
   });
-  for (auto& planes : dl_syrk_)
-    for (auto& l : planes)
-      std::stable_sort(l.begin(), l.end(), [](const DigitItem& a, const DigitItem& b) { return a.nkt > b.nkt; });
+  for (auto& ctas : dl_syrk_)
+    for (auto& planes : ctas)
+      for (auto& l : planes)
+        std::stable_sort(l.begin(), l.end(), [](const DigitItem& a, const DigitItem& b) { return a.nkt > b.nkt; });
 
   // Products of the factorization that would leave SMs idle are cut into 32-column tiles.  With
   // more than 36 (problem, frequency) pairs the other chains' launches fill the GPU, and only the
@@ -1063,7 +1072,11 @@ Status Plan::build(Context* ctx, PlanMode mode, const std::vector<Shape>& shapes
   for (int np2 = 2; np2 < 8; ++np2) {
     for (size_t g = 0; g < wl_slice_[np2].size(); ++g) {
       add(25, wl_slice_[np2][g].data(), sizeof(WorkItem), wl_slice_[np2][g].size(), np2);
-      add(26, dl_syrk_[np2][g].data(), sizeof(DigitItem), dl_syrk_[np2][g].size(), np2);
+      for (int ct = 1; ct <= 2; ++ct) {
+        auto& products = dl_syrk_[ct - 1][np2];
+        if (g < products.size())
+          add(26, products[g].data(), sizeof(DigitItem), products[g].size(), 10 * np2 + ct);
+      }
     }
   }
   add(22, fl_syrk_.data(), sizeof(F64SyrkItem), fl_syrk_.size(), 0);   // after 24, which sets `only_if`
@@ -1198,8 +1211,8 @@ void Plan::record(cudaStream_t s0, int stage) {
         break;
       case 26: {
         const DigitItem* dl = reinterpret_cast<const DigitItem*>(lb + L.off);
-        if (L.arg == 2) launch_split_syrk(dl, L.count, L.ny, s);
-        else launch_digit_syrk(L.arg, dl, L.count, L.ny, s);
+        if (L.arg / 10 == 2) launch_split_syrk(dl, L.count, L.ny, s);
+        else launch_digit_syrk(L.arg / 10, L.arg % 10, dl, L.count, L.ny, s);
         break;
       }
       case 27:

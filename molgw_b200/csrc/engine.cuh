@@ -117,6 +117,8 @@ bool use_factor_digits(const Shape& sh);
 int factor_group(const Shape& sh);
 // Planes of the chi0 operands: 2 (bf16 hi/lo), 3 .. 7 (int8 digits), 0 (FP64 on DMMA).
 int operand_planes(const Shape& sh);
+// CTAs of a chi0 tile on tcgen05: 1 (128 x 128) or 2 (256 x 128).
+int tile_ctas(int planes, int npanel);
 // Bytes of one frequency's split operands of a problem (0 for FP64 on DMMA).
 size_t split_bytes_per_frequency(const Shape& sh);
 
@@ -196,7 +198,7 @@ class Plan {
   std::vector<WorkItem> wl_dzero_, wl_dmax_;               // digits: row maxima
   // chi0 on tcgen05, by the number of operand planes (2: bf16, 3 .. 7: digits)
   std::vector<std::vector<WorkItem>> wl_slice_[8];         // per frequency group: planes of M sqrt(D_w)
-  std::vector<std::vector<DigitItem>> dl_syrk_[8];         // and the products
+  std::vector<std::vector<DigitItem>> dl_syrk_[2][8];      // and the products, by the CTAs of a tile - 1
   std::vector<std::vector<GemmItem>> gl_k2_, gl_k2n_, gl_k3_, gl_k3d_;
   std::vector<std::vector<FactorSliceItem>> fl_slice_;   // digits of a finished panel group
   std::vector<std::vector<UpdateItem>> ul_update_;       // and the update of the next group's rows

@@ -103,7 +103,7 @@ void launch_syrk_f64_tma(const F64SyrkItem* items, int n, int ny, cudaStream_t s
 cudaError_t prepare_syrk_f64_tma();
 
 // chi0 on the tcgen05 cores: one upper tile of eps(iw) = 1 + M D_w M^T, 256 x 128 per pair of CTAs
-// (digits) or 128 x 128 per CTA (bf16), frequency = blockIdx.y (slab blockIdx.y).  The operand planes of M sqrt(D_w) are 3 to 7
+// (digits) or 128 x 128 per CTA (tile_ctas), frequency = blockIdx.y (slab blockIdx.y).  The operand planes of M sqrt(D_w) are 3 to 7
 // int8 digits (digit_gemm.cu; FP64: 7, RIGW_OZAKI(s): s) or two bf16 parts (syrk_bf16x3.cu; exps
 // unused).
 struct DigitItem {
@@ -113,7 +113,7 @@ struct DigitItem {
   const int* exps;      // digits, row exponents [w][ld]
   const unsigned long long* squares;   // digits: ProbDev::squares
   const int* negative;  // digits of FP64: not this kernel's problem when set (nullptr: always its)
-  int rb_a, rb_b;       // 128-row blocks: output rows from 128 rb_a (two blocks, bf16: one), columns from 128 rb_b
+  int rb_a, rb_b;       // 128-row blocks: output rows from 128 rb_a (two blocks of a pair, or one), columns from 128 rb_b
   int nrb, nkt;         // row blocks and k-tiles (64 transitions) of a slab
   int w0;               // frequency of slab 0
   int ld, nw;           // npad; frequencies covered
@@ -152,9 +152,9 @@ void launch_factor_slice(const FactorSliceItem* items, int n, int ny, cudaStream
 void launch_digit_update(const UpdateItem* items, int n, int ny, cudaStream_t s);
 void launch_digit_zero(const ProbDev* probs, const WorkItem* items, int n, cudaStream_t s);
 void launch_digit_rowmax(const ProbDev* probs, const WorkItem* items, int n, cudaStream_t s);
-// planes: digits per operand, 3 .. 7
+// planes: digits per operand, 3 .. 7; ctas of a tile: 2, or 1 for up to six digits
 void launch_digit_slice(int planes, const ProbDev* probs, const WorkItem* items, int n, cudaStream_t s);
-void launch_digit_syrk(int planes, const DigitItem* items, int n, int ny, cudaStream_t s);
+void launch_digit_syrk(int planes, int ctas, const DigitItem* items, int n, int ny, cudaStream_t s);
 void launch_split_bf16(const ProbDev* probs, const WorkItem* items, int n, cudaStream_t s);
 void launch_split_syrk(const DigitItem* items, int n, int ny, cudaStream_t s);
 cudaError_t prepare_digit_kernels();
