@@ -210,9 +210,12 @@ dgemm_mn_kernel(const GemmItem* __restrict__ items) {
       }
     return;
   }
-  double csq[4][2];
+  // Column sums of squares: one binary tree over the tile's rows, whatever the warps' share of it,
+  // so that the same product gives the same bits in every tile shape (a batch picks the shape by its
+  // size).  Rows 0 and 1, 2 and 3 of a lane, then their sums, then the lane's quads, lanes, warps.
+  double csq[4][2], half[4][2], quad[4][2];   // finished quads; rows 0 1 of a quad; its last pair
 #pragma unroll
-  for (int j = 0; j < 4; ++j) csq[j][0] = csq[j][1] = 0.0;
+  for (int j = 0; j < 4; ++j) csq[j][0] = csq[j][1] = half[j][0] = half[j][1] = quad[j][0] = quad[j][1] = 0.0;
 #pragma unroll
   for (int i = 0; i < FM; ++i) {
     const int row = wm0 + FM * q + i;
@@ -233,8 +236,13 @@ dgemm_mn_kernel(const GemmItem* __restrict__ items) {
         if (col + 1 - row == it.diag) v1 += idv;
       }
       *reinterpret_cast<double2*>(it.C + size_t(row) * it.ldc + col) = make_double2(v0, v1);
-      csq[j][0] += v0 * v0;
-      csq[j][1] += v1 * v1;
+      const double s[2] = {__dmul_rn(v0, v0), __dmul_rn(v1, v1)};
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        if (i % 4 < 2) half[j][e] = i % 4 == 0 ? s[e] : __dadd_rn(half[j][e], s[e]);
+        else quad[j][e] = i % 4 == 2 ? s[e] : __dadd_rn(quad[j][e], s[e]);
+        if (i % 4 == 3) csq[j][e] = __dadd_rn(csq[j][e], __dadd_rn(half[j][e], quad[j][e]));
+      }
     }
   }
   if (it.colsq != nullptr) {
@@ -259,10 +267,14 @@ dgemm_mn_kernel(const GemmItem* __restrict__ items) {
     }
     __syncthreads();
     for (int c = tid; c < BN && c < it.n; c += NT) {
-      double v = 0.0;
+      double v[Cfg::kWarpsM];
 #pragma unroll
-      for (int w = 0; w < Cfg::kWarpsM; ++w) v += red[w * BN + c];
-      it.colsq[c] = v;
+      for (int w = 0; w < Cfg::kWarpsM; ++w) v[w] = red[w * BN + c];
+#pragma unroll
+      for (int d = 1; d < Cfg::kWarpsM; d *= 2)
+#pragma unroll
+        for (int w = 0; w < Cfg::kWarpsM; w += 2 * d) v[w] += v[w + d];
+      it.colsq[c] = v[0];
     }
   }
 }

@@ -116,6 +116,18 @@ def test_ragged_batch_equals_single_solves(engine):
         assert np.abs(b.energy_qp_g - s.energy_qp_g).max() < 1e-13
 
 
+@pytest.mark.parametrize("naux,count,nomega", [(70, 12, 32), (130, 3, 16), (200, 12, 32), (256, 6, 24)])
+def test_tile_shapes_give_the_same_bits(engine, naux, count, nomega):
+    """Up to two panels a solve has the same bits alone, where the products of the factorization run
+    in narrow tiles, and in batches of any size, where they do not."""
+    insts = [synth.make_instance(5, 40, naux + k % 3, nomega, 90 + k) for k in range(count)]
+    alone = [engine.g0w0(i) for i in insts]
+    for a, b in zip(alone, engine.g0w0_batch(insts)):
+        assert (a.erpa, a.egw) == (b.erpa, b.egw)
+        assert np.array_equal(a.sigma_calc, b.sigma_calc)
+        assert np.array_equal(a.energy_qp_g, b.energy_qp_g)
+
+
 def test_qp_only_mode_gives_the_same_qp_energies(engine, golden_synth):
     """RIGW_PROBLEM_QP_ONLY skips the tr eps^-1 solve (E_GW); every other output is unchanged."""
     inst = instance_from_golden(golden_synth)
