@@ -28,8 +28,8 @@
 // transitions.)
 //
 // 840 auxiliary functions, 4347 transitions, 32 frequencies: row maxima 0.04 ms, digits
-// 0.16 ms, products 1.23 ms (3.4 Pop/s int8), against 4.25 ms on DMMA (23 of 35 TF/s);
-// 2000 / 25000 / 32: 0.37 + 2.26 + 30.2 ms against 112 ms.
+// 0.16 ms, products 1.43 ms (3.5 Pop/s int8 over the executed tiles), against 4.25 ms on DMMA (23
+// of 35 TF/s); 2000 / 25000 / 32: 0.37 + 2.19 + 35.4 ms against 111 ms.
 // The operands are the same on both sides, so on the diagonal the products that are left out
 // hold squares, whose mean is not zero.  If D + 1 is even, the first level left out has one, of
 // digit (D + 1) / 2, which would lower eps_pp by 1e-9 for NS = 4 and by K 2^-66 max|S_p|^2 for
@@ -548,7 +548,7 @@ __global__ void __cluster_dims__(CT, 1, 1) __launch_bounds__(kDigThreads, 1)
 // U's entries far above the diagonal are small, and one scale for a whole column would have to
 // cover its largest entry.  DMMA did these updates at 20 TF/s (64 x 128 tiles, K = 256 at a
 // time, every trailing tile read and written once per group); here each tile is written once
-// in all, with K of all rows above, at 100 TF/s (2000 auxiliary functions, K = 512).
+// in all, with K of all rows above (2000 auxiliary functions, 32 frequencies: stage 15.6 -> 10.3 ms).
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kDigThreads, 1)
     digit_update_kernel(const UpdateItem* __restrict__ items) {
   const UpdateItem it = items[blockIdx.x >> 1];

@@ -315,7 +315,7 @@ Dims dims_of(const Shape& sh, PlanMode mode) {
 // 384 with 1 / 12 / 16 / 24 / 32 / 48 frequencies 0.114 / 0.119 / 0.160 / 0.160 / 0.301 / 0.309
 // against 0.078 / 0.108 / 0.123 / 0.200 / 0.217 / 0.311 (waves of tiles), 400 (32) 0.352 against
 // 0.286, 512 (1 / 32) 0.188 / 0.666 against 0.100 / 0.372, 840 (1 / 32) 0.53 / 4.25 against 0.22 /
-// 1.64, 2000 (32) 112 against 39.  Below 512 transitions the passes and the drains, which do not
+// 1.64, 2000 (32) 111 against 38.  Below 512 transitions the passes and the drains, which do not
 // shrink with the sum, take over: at 512 naux 400 (16 / 32) 0.131 / 0.213 against 0.153 / 0.225, 840
 // 0.37 / 0.66 against 0.26 / 0.44, 2000 1.62 / 3.12 against 0.86 / 1.64.
 bool use_digits(const Shape& sh) {
